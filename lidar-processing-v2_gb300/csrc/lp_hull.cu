@@ -380,66 +380,6 @@ __device__ bool pca_axes(double sxx, double sxy, double syy, double& v00, double
     return true;
 }
 
-// PCA box (polygonizer.cpp:280-362) in FP64 by one thread: mean, centred X^T X / (n - 1), the
-// JacobiSVD axes, rotate, min/max, corners back to the original frame.
-__device__ void pca_box(const double2* P, int n, lp_bounding_box* out)
-{
-    lp_bounding_box box;
-    for (int k = 0; k < 4; ++k)
-        box.corners[k][0] = box.corners[k][1] = 0.0;
-    box.area = 0.0f;
-    box.angle_rad = 0.0f;
-    box.is_valid = 0;
-    if (n >= 3)
-    {
-        double mx = 0.0, my = 0.0;
-        for (int i = 0; i < n; ++i)
-        {
-            mx += P[i].x;
-            my += P[i].y;
-        }
-        mx /= n;
-        my /= n;
-        double sxx = 0.0, sxy = 0.0, syy = 0.0;
-        for (int i = 0; i < n; ++i)
-        {
-            const double dx = P[i].x - mx, dy = P[i].y - my;
-            sxx += dx * dx;
-            sxy += dx * dy;
-            syy += dy * dy;
-        }
-        sxx /= (n - 1);
-        sxy /= (n - 1);
-        syy /= (n - 1);
-        double v00, v01, v10, v11;
-        if (pca_axes(sxx, sxy, syy, v00, v01, v10, v11))
-        {
-            double mnx = DBL_MAX, mxx = -DBL_MAX, mny = DBL_MAX, mxy = -DBL_MAX;
-            for (int i = 0; i < n; ++i)
-            {
-                const double dx = P[i].x - mx, dy = P[i].y - my;
-                const double rx = dx * v00 + dy * v10;
-                const double ry = dx * v01 + dy * v11;
-                mnx = fmin(mnx, rx);
-                mxx = fmax(mxx, rx);
-                mny = fmin(mny, ry);
-                mxy = fmax(mxy, ry);
-            }
-            const double xs[4] = {mnx, mxx, mxx, mnx};
-            const double ys[4] = {mny, mny, mxy, mxy};
-            for (int k = 0; k < 4; ++k)
-            {
-                box.corners[k][0] = xs[k] * v00 + ys[k] * v01 + mx;
-                box.corners[k][1] = xs[k] * v10 + ys[k] * v11 + my;
-            }
-            box.area = __double2float_rn((mxx - mnx) * (mxy - mny));
-            box.angle_rad = __double2float_rn(atan2(v10, v00));
-            box.is_valid = 1;
-        }
-    }
-    *out = box;
-}
-
 // Sums of the x and of the y coordinates of P[0..n) as the reference's loop computes them in
 // binary64 (left to right), by one warp; every lane returns both. Each term is a multiple of
 // 2^g (g from its exponent and the trailing zeros of its significand) and below 2^t in
@@ -500,8 +440,8 @@ __device__ __forceinline__ void sum_xy_fp64(const double2* P, int n, double& sx,
 // PCA box by one warp, every step in FP64 in the reference's order: the mean, the covariance sums
 // (the principal axis is ill-conditioned exactly where they nearly cancel), the JacobiSVD axes
 // (pca_axes, evaluated by every lane alike), the rotated extents (lanes stride over the vertices;
-// min and max do not depend on order) and the corners. The box equals the single-thread pca_box
-// bit for bit.
+// min and max do not depend on order) and the corners. The box equals the reference loop's bit
+// for bit.
 __device__ void pca_box_warp(const double2* P, int n, lp_bounding_box* out)
 {
     const uint32_t lane = lane_id();
@@ -2393,56 +2333,329 @@ __global__ void k_hull_compact(BatchDev b, const uint32_t* work)
 
 // ---------------------------------------------------------------------------------------------
 // Standalone single-polygon entry points (double inputs): one CTA.
+//
+// What bounds them: nearly every point of a cluster lies inside its hull, and sorting all of them
+// (24-byte records, about log2(n)^2 / 2 passes) and walking them with one thread's FP64 orientation
+// tests took most of the 62 ms that twelve polygons of 3 to 20,000 points needed for hull and both
+// boxes (now 1.9 ms, 54 us a call). The points proven inside a polygon of input points
+// are dropped first (Quickhull rounds as in hull_one, coordinates as floats), so the sort and the
+// chain see a few dozen to a few hundred; 1,024 threads because the rounds stream over all points.
+// Points whose coordinates are binary32 values (the processor's are) also take the FP32-screened
+// orientation test, whose decisions are those of the FP64 expression.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kHullThreads) k_hull_single(const double2* pts, uint32_t n, HPt<double>* scratch,
-                                                            int* stack, int32_t* out, uint32_t* n_out)
+constexpr int kSingleThreads = 1024;
+constexpr uint32_t kSingleCand = 512;     // candidates sorted in shared memory
+constexpr uint32_t kSingleFilterMin = 64; // fewer points go straight to the sort
+constexpr uint32_t kSingleEnough = 96;    // candidates few enough to end the rounds
+
+struct SingleSmem
 {
-    // the sort runs in global scratch (capacity next_pow2(n)); no prefilter (the polygon is
-    // the caller's whole input)
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-        scratch[i] = HPt<double>{pts[i].x, pts[i].y, i};
+    HPt<double> cand[kSingleCand]; // as HPt<float> for binary32 points
+    int stack[2 * kSingleCand + 2];
+    float2 poly[2][kPolyCap];
+    float4 erec[kPolyCap];
+    float2 emar[kPolyCap];
+    unsigned long long pkey[kPolyCap];
+    unsigned long long ext[kDirs][kSingleThreads / 32];
+    float2 dirs[kDirs];
+    float red[kSingleThreads / 32];
+    int npoly, grew, nact;
+};
+
+// Lists (act[0], n entries) the points not proven inside the hull and returns their number, or n
+// when nothing can be dropped (the list is then not valid). `lf` receives the points as floats:
+// themselves when `exact` (all binary32 values), else relative to the first point, where each
+// coordinate is within 2^-24 R of the exact difference (R: the largest); the tests' margins add that
+// error (a cross product of |e|, |q| errs by less than 2^-22 R (|e| + |q|)).
+__device__ uint32_t single_filter(SingleSmem& sm, const double2* pts, uint32_t n, bool exact, float2* lf, uint32_t* act0,
+                                  uint32_t* act1)
+{
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, tid = threadIdx.x, nt = blockDim.x;
+    hull_dirs(sm.dirs);
+    const double ox = exact ? 0.0 : pts[0].x, oy = exact ? 0.0 : pts[0].y;
     __syncthreads();
-    block_sort_global(scratch, n);
-    __syncthreads();
-    __shared__ int hn;
-    __shared__ isort::SortShared ss;
-    if (threadIdx.x == 0)
-        hn = monotone_chain(scratch, static_cast<int>(n), stack);
-    __syncthreads();
-    bool tie = false;
-    for (int j = threadIdx.x; j < hn; j += blockDim.x)
+    Extremes16 ex;
+    ex.init();
+    float R = 0.0f;
+    for (uint32_t i = tid; i < n; i += nt)
     {
-        const int q = stack[j];
-        const HPt<double> c = scratch[q];
-        out[j] = static_cast<int32_t>(c.key);
-        tie |= (q > 0 && scratch[q - 1].x == c.x && scratch[q - 1].y == c.y) ||
-               (q + 1 < static_cast<int>(n) && scratch[q + 1].x == c.x && scratch[q + 1].y == c.y);
+        const double2 p = pts[i];
+        const float2 q = make_float2(static_cast<float>(p.x - ox), static_cast<float>(p.y - oy));
+        lf[i] = q;
+        R = fmaxf(R, fmaxf(fabsf(q.x), fabsf(q.y)));
+        ex.add(sm.dirs, q.x, q.y, i);
     }
+    R = warp_max_f(R);
+    if (lane == 0)
+        sm.red[warp] = R;
+#pragma unroll
+    for (int d = 0; d < kDirs; ++d)
+    {
+        const unsigned long long v = warp_max64(ex.key(d));
+        if (lane == 0)
+            sm.ext[d][warp] = v;
+    }
+    __syncthreads();
+    R = warp_max_f(sm.red[lane]); // every warp alike (kSingleThreads / 32 == 32)
+    if (!(R > 1e-12f && R < 1e15f))
+        return n; // float products would leave the normal range
+    const float slack = exact ? 0.0f : 1e-6f * R;
+    if (warp < static_cast<uint32_t>(kDirs))
+    {
+        const unsigned long long v = warp_max64(sm.ext[warp][lane]);
+        if (lane == 0)
+            sm.pkey[warp] = v;
+    }
+    __syncthreads();
+    if (tid == 0)
+        sm.npoly = first_polygon(lf, n, sm.pkey, sm.poly[0]);
+    __syncthreads();
+    uint32_t* act[2] = {act0, act1};
+    int cur = -1, pb = 0; // -1: the active set is all points
+    uint32_t nact = n;
+    for (int round = 0; round < kRefineRounds && (round == 0 || nact > kSingleEnough); ++round)
+    {
+        const int np = sm.npoly;
+        if (np < 3)
+            break;
+        const float2* poly = sm.poly[pb];
+        for (int e = static_cast<int>(tid); e < np; e += static_cast<int>(nt))
+        {
+            sm.pkey[e] = 0ull;
+            const float2 a = poly[e], c = poly[(e + 1 == np) ? 0 : e + 1];
+            const float dx = c.x - a.x, dy = c.y - a.y;
+            const float l1 = fabsf(dx) + fabsf(dy);
+            sm.erec[e] = make_float4(a.x, a.y, dx, dy);
+            sm.emar[e] = make_float2(1e-5f * l1 + slack, slack * l1 + 1e-30f);
+        }
+        if (tid == 0)
+            sm.nact = 0;
+        __syncthreads();
+        const int nxt = (cur == 0) ? 1 : 0;
+        for (uint32_t t = tid; t < ((nact + 31u) & ~31u); t += nt)
+        {
+            const bool live = t < nact;
+            const uint32_t i = live ? ((cur < 0) ? t : act[cur][t]) : 0u;
+            const float2 q = lf[i];
+            bool in = true;
+            for (int e = 0; live && e < np; ++e)
+            {
+                const float4 r = sm.erec[e];
+                const float2 mg = sm.emar[e];
+                const float qx = q.x - r.x, qy = q.y - r.y;
+                const float cr = r.z * qy - r.w * qx;
+                const float aq = fabsf(qx) + fabsf(qy);
+                if (!(cr > mg.x * aq + mg.y))
+                    in = false;
+                if (cr < -(mg.x * aq + mg.y)) // any outside point may become a vertex
+                {
+                    const unsigned long long key = fkey_payload(-cr, i);
+                    if (key > sm.pkey[e])
+                        atomicMax(&sm.pkey[e], key);
+                }
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, live && !in);
+            uint32_t at = 0u;
+            if (lane == 0 && m)
+                at = static_cast<uint32_t>(atomicAdd(&sm.nact, __popc(m)));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (live && !in)
+                act[nxt][at + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)))] = i;
+        }
+        __syncthreads();
+        cur = nxt;
+        nact = static_cast<uint32_t>(sm.nact);
+        // each edge's farthest outside point becomes a vertex behind the edge's first one (warp 0)
+        if (warp == 0)
+        {
+            int add = 0;
+            for (int e = static_cast<int>(lane); e < np; e += 32)
+                add += (sm.pkey[e] != 0ull) ? 1 : 0;
+            add = static_cast<int>(warp_sum(static_cast<uint32_t>(add)));
+            const bool grow = add > 0 && np + add <= kPolyCap;
+            int w = 0;
+            for (int base = 0; grow && base < np; base += 32)
+            {
+                const int e = base + static_cast<int>(lane);
+                const bool ins = e < np && sm.pkey[e] != 0ull;
+                const uint32_t im = __ballot_sync(0xffffffffu, ins);
+                const int at = w + static_cast<int>(lane) + __popc(im & ((1u << lane) - 1u));
+                if (e < np)
+                    sm.poly[pb ^ 1][at] = sm.poly[pb][e];
+                if (ins)
+                    sm.poly[pb ^ 1][at + 1] = lf[static_cast<uint32_t>(sm.pkey[e] & 0xffffffffull)];
+                w += 32 + __popc(im);
+            }
+            if (lane == 0)
+            {
+                sm.grew = grow ? 1 : 0;
+                if (grow)
+                    sm.npoly = np + add;
+            }
+        }
+        __syncthreads();
+        if (!sm.grew)
+            break;
+        pb ^= 1;
+    }
+    if (cur < 0)
+        return n;
+    if (cur == 1)
+    {
+        for (uint32_t t = tid; t < nact; t += nt)
+            act0[t] = act1[t];
+        __syncthreads();
+    }
+    return nact;
+}
+
+// Sort and chain of m candidates (list: their input positions, null for all points): hull indices
+// to out, returns the hull size; *tie: a vertex has an identical candidate.
+template <typename T>
+__device__ int single_chain(SingleSmem& sm, const double2* pts, const uint32_t* list, uint32_t m, HPt<T>* gl, int* gstack,
+                            int32_t* out, bool* tie)
+{
+    auto run = [&](HPt<T>* C, int* H) {
+        const uint32_t np2 = next_pow2(m);
+        for (uint32_t t = threadIdx.x; t < np2; t += blockDim.x)
+        {
+            HPt<T> c{static_cast<T>(INFINITY), static_cast<T>(INFINITY), 0xffffffffu};
+            if (t < m)
+            {
+                const uint32_t i = list ? list[t] : t;
+                const double2 p = pts[i];
+                c = HPt<T>{static_cast<T>(p.x), static_cast<T>(p.y), i};
+            }
+            C[t] = c;
+        }
+        __syncthreads();
+        block_bitonic_sort(C, np2, [](const HPt<T>& x, const HPt<T>& y) { return hpt_less(x, y); });
+        if (threadIdx.x == 0)
+            sm.npoly = chain_half(C, static_cast<int>(m), H, false);
+        else if (threadIdx.x == 32)
+            sm.grew = chain_half(C, static_cast<int>(m), H + m + 1, true);
+        __syncthreads();
+        const int kl = sm.npoly, h = kl + sm.grew - 2;
+        bool t = false;
+        for (int j = static_cast<int>(threadIdx.x); j < h; j += static_cast<int>(blockDim.x))
+        {
+            const int q = (j < kl) ? H[j] : H[static_cast<int>(m) + 2 + j - kl];
+            const HPt<T> c = C[q];
+            out[j] = static_cast<int32_t>(c.key);
+            t |= (q > 0 && C[q - 1].x == c.x && C[q - 1].y == c.y) ||
+                 (q + 1 < static_cast<int>(m) && C[q + 1].x == c.x && C[q + 1].y == c.y);
+        }
+        *tie = t;
+        return h;
+    };
+    return (m <= kSingleCand) ? run(reinterpret_cast<HPt<T>*>(sm.cand), sm.stack) : run(gl, gstack);
+}
+
+// scratch: next_pow2(n) records of 24 bytes, stack: 2n + 8 ints (8-byte aligned). The floats of the
+// filter lie in the stack area (the chain needs it only for candidates beyond shared memory, after the
+// filter), its two lists at the end of the record area.
+__global__ void __launch_bounds__(kSingleThreads) k_hull_single(const double2* pts, uint32_t n, HPt<double>* scratch,
+                                                              int* stack, int32_t* out, uint32_t* n_out)
+{
+    __shared__ __align__(16) unsigned char raw[sizeof(SingleSmem) > sizeof(isort::SortShared) ? sizeof(SingleSmem)
+                                                                                             : sizeof(isort::SortShared)];
+    SingleSmem& sm = *reinterpret_cast<SingleSmem*>(raw);
+    bool exact = true, finite = true;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+    {
+        const double2 p = pts[i];
+        exact &= static_cast<double>(static_cast<float>(p.x)) == p.x && static_cast<double>(static_cast<float>(p.y)) == p.y;
+        finite &= isfinite(p.x) && isfinite(p.y);
+    }
+    exact = __syncthreads_and(exact);
+    finite = __syncthreads_and(finite);
+    const size_t bytes = static_cast<size_t>(next_pow2(n)) * sizeof(HPt<double>);
+    const size_t lists = bytes - 8ull * n; // the two lists of n entries start here
+    uint32_t* act0 = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(scratch) + lists);
+    uint32_t m = n;
+    if (finite && n > kSingleFilterMin)
+        m = single_filter(sm, pts, n, exact, reinterpret_cast<float2*>(stack), act0, act0 + n);
+    // without a gain, or when the candidates' records would meet the list, every point takes part
+    const bool all = m == n || (m > kSingleCand && static_cast<size_t>(next_pow2(m)) * sizeof(HPt<double>) > lists);
+    if (all)
+        m = n;
+    __syncthreads();
+    bool tie;
+    int h;
+    if (exact && finite)
+        h = single_chain(sm, pts, all ? nullptr : act0, m, reinterpret_cast<HPt<float>*>(scratch), stack, out, &tie);
+    else
+        h = single_chain(sm, pts, all ? nullptr : act0, m, scratch, stack, out, &tie);
     if (threadIdx.x == 0)
-        *n_out = static_cast<uint32_t>(hn);
+        *n_out = static_cast<uint32_t>(h);
     if (__syncthreads_or(tie))
     {
         // a vertex with an identical point: the reference's std::sort order decides which one. The
         // sort buffer takes the records (24 bytes each, as its entries) and the chain stack (2n + 8
         // ints, free now) the partition lists; the vertices' coordinates are read from the input.
+        isort::SortShared& ss = *reinterpret_cast<isort::SortShared*>(raw);
         auto* rec = reinterpret_cast<HRec<double>*>(scratch);
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
             rec[i] = HRec<double>{pts[i].x, pts[i].y, i};
         __syncthreads();
         uint32_t* ge = reinterpret_cast<uint32_t*>(stack);
-        hull_repair_ties(rec, n, out, hn, [=](int j) { return pts[out[j]]; }, ge, ge + n, ss);
+        hull_repair_ties(rec, n, out, h, [=](int j) { return pts[out[j]]; }, ge, ge + n, ss);
     }
 }
 
-__global__ void k_boxes_single(const double2* P, uint32_t n, int2* pairs, int cap, int kind, lp_bounding_box* out,
-                               int* npairs_out)
+// Antipodal pairs and a box of one polygon by one warp. A polygon of at most kBoxVerts binary32
+// vertices takes the FP32-screened walk and calipers of the pipeline's hulls (same pairs, same box);
+// others run in FP64 throughout (every visited edge's extents: 4 n^2 / 32 FP64 steps).
+constexpr uint32_t kBoxVerts = 1024;
+
+__global__ void __launch_bounds__(32) k_boxes_single(const double2* P, uint32_t n, int2* pairs, int cap, int kind,
+                                                    lp_bounding_box* out, int* npairs_out)
 {
-    if (threadIdx.x >= 32)
-        return;
+    __shared__ double2 sp[kBoxVerts];
+    __shared__ float2 spf[kBoxVerts];
+    __shared__ float ea[kBoxVerts];
     const uint32_t lane = lane_id();
+    const bool local = n <= kBoxVerts;
+    bool exact = true;
+    float mabs = 0.0f, r2 = 0.0f;
+    if (local)
+    {
+        for (uint32_t k = lane; k < n; k += 32)
+        {
+            const double2 p = P[k];
+            const float2 f = make_float2(static_cast<float>(p.x), static_cast<float>(p.y));
+            exact &= static_cast<double>(f.x) == p.x && static_cast<double>(f.y) == p.y;
+            mabs = fmaxf(mabs, fmaxf(fabsf(f.x), fabsf(f.y)));
+            sp[k] = p;
+            spf[k] = f;
+        }
+        __syncwarp();
+        for (uint32_t k = lane; k < n; k += 32)
+        {
+            const float lx = spf[k].x - spf[0].x, ly = spf[k].y - spf[0].y;
+            r2 = fmaxf(r2, lx * lx + ly * ly);
+        }
+        mabs = warp_max_f(mabs);
+        r2 = warp_max_f(r2) * 1.001f;
+    }
+    const bool fast = __all_sync(0xffffffffu, exact) && local && mabs < 1e15f;
+    const double2* V = local ? sp : P;
+    if (kind == 1)
+    {
+        if (lane == 0 && npairs_out)
+            *npairs_out = 0;
+        pca_box_warp(V, static_cast<int>(n), out);
+        return;
+    }
     int np = 0;
     if (lane == 0)
-        np = antipodal_pairs(AreaCmpFp64{P}, static_cast<int>(n), pairs, cap);
+    {
+        if (fast)
+            np = antipodal_pairs(AreaCmpFiltered{V, spf, spf[0].x, spf[0].y, 2.0f * (4e-6f * r2 + 1e-13f * mabs * sqrtf(r2)) + 1e-30f},
+                                 static_cast<int>(n), pairs, cap);
+        else
+            np = antipodal_pairs(AreaCmpFp64{V}, static_cast<int>(n), pairs, cap);
+    }
     np = __shfl_sync(0xffffffffu, np, 0);
     if (lane == 0 && npairs_out)
         *npairs_out = np;
@@ -2450,9 +2663,12 @@ __global__ void k_boxes_single(const double2* P, uint32_t n, int2* pairs, int ca
         np = cap;
     __syncwarp();
     if (kind == 0)
-        calipers_warp(P, static_cast<int>(n), pairs, np, out);
-    else if (kind == 1 && lane == 0)
-        pca_box(P, static_cast<int>(n), out);
+    {
+        if (fast)
+            calipers_fast(V, spf, static_cast<int>(n), pairs, np, ea, r2, out);
+        else
+            calipers_warp(V, static_cast<int>(n), pairs, np, out);
+    }
 }
 } // namespace
 
@@ -2582,7 +2798,7 @@ int sm_count()
 void launch_hull_single(Launcher& L, const double2* pts, uint32_t n, void* scratch, int* stack, int32_t* out,
                         uint32_t* n_out)
 {
-    LP_LAUNCH(L, k_hull_single, 1, kHullThreads, pts, n, reinterpret_cast<HPt<double>*>(scratch), stack, out, n_out);
+    LP_LAUNCH(L, k_hull_single, 1, kSingleThreads, pts, n, reinterpret_cast<HPt<double>*>(scratch), stack, out, n_out);
 }
 
 void launch_boxes_single(Launcher& L, const double2* P, uint32_t n, int2* pairs, int cap, int kind, lp_bounding_box* out,
@@ -2672,7 +2888,7 @@ extern "C" lp_status lp_convex_hull_noalloc(const double* d_xy, uint32_t n, int3
         int* stack = reinterpret_cast<int*>(static_cast<unsigned char*>(scratch) + kNoallocSortBytes);
         const double2* xy = reinterpret_cast<const double2*>(d_xy);
         void* args[] = {&xy, &n, &sort_buf, &stack, &d_indices_out, &d_n_out};
-        e = cudaLaunchKernel(reinterpret_cast<const void*>(&lpg::k_hull_single), dim3(1), dim3(lpg::kHullThreads), args,
+        e = cudaLaunchKernel(reinterpret_cast<const void*>(&lpg::k_hull_single), dim3(1), dim3(lpg::kSingleThreads), args,
                              0, st);
     }
     return e == cudaSuccess ? LP_OK : LP_ERR_CUDA;

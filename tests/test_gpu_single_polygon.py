@@ -1,0 +1,53 @@
+"""lp_convex_hull and the single-polygon boxes at the edges of their dispatch: below and above the
+filter's and the shared-memory sort's sizes, binary32 and genuine binary64 coordinates, clouds that keep
+every point, ties, degenerate and far-off clouds. Index sequences and boxes equal the oracle's (the
+boxes' FP64 expressions are the oracle's, so no tolerance)."""
+import numpy as np
+import pytest
+
+import lidar_gb300 as lp
+import lp_testlib as T
+
+pytestmark = pytest.mark.gpu
+
+
+def cloud(kind, n, rng):
+    if kind == "footprint":  # two sides of a rectangle, centimetre noise, 20 m away
+        t, far = rng.random(n), rng.random(n) < 0.6
+        p = np.stack([np.where(far, 8 * t, 0), np.where(far, 0, 3 * t)], 1) + rng.normal(0, 0.02, (n, 2))
+        c, s = np.cos(0.4), np.sin(0.4)
+        return (p @ np.array([[c, s], [-s, c]]) + 20).astype(np.float32).astype(np.float64)
+    if kind == "binary64":
+        return rng.normal(size=(n, 2)) * [9.0, 0.3] + [1e4, -3e3]
+    if kind == "circle":  # every point a vertex: nothing can be dropped
+        a = rng.permutation(n) * (2 * np.pi / n)
+        return np.stack([np.cos(a), np.sin(a)], 1) * 50.0
+    if kind == "grid":  # ties and collinear runs
+        return np.round(rng.normal(size=(n, 2)) * 3.0)
+    if kind == "line":
+        return np.stack([np.arange(n) * 0.25, np.arange(n) * 0.5], 1)[rng.permutation(n)]
+    if kind == "tiny":  # float products would underflow: the filter steps aside
+        return rng.normal(size=(n, 2)) * 1e-14
+    raise ValueError(kind)
+
+
+@pytest.mark.parametrize("kind", ["footprint", "binary64", "circle", "grid", "line", "tiny"])
+@pytest.mark.parametrize("n", [3, 64, 65, 511, 513, 1023, 5000, 20011])
+def test_hull_sizes(ctx, kind, n):
+    pts = np.ascontiguousarray(cloud(kind, n, np.random.default_rng([n, len(kind)])))
+    # the device orders by exact (x, y) where the reference takes x less than DBL_EPSILON apart as equal;
+    # scaled by a power of two (exact) the tiny cloud has no such x and the oracle's order is the exact one
+    want = T.o_hull(pts * 2.0**50 if kind == "tiny" else pts, T.TIES_LIBSTDCXX)
+    assert np.array_equal(lp.Polygonizer(ctx).convexHull(pts), want)
+
+
+@pytest.mark.parametrize("n", [3, 31, 33, 1024, 1025])
+@pytest.mark.parametrize("single", [True, False])
+def test_boxes_sizes(ctx, n, single):
+    a = np.arange(n) * (2 * np.pi / n)
+    hp = np.stack([30 + 12 * np.cos(a), 5 * np.sin(a) - 8], 1)
+    hp = np.ascontiguousarray(hp.astype(np.float32).astype(np.float64) if single else hp)
+    poly = lp.Polygonizer(ctx)
+    assert np.array_equal(poly.findAntipodalPairsOfConvexHull(hp), T.o_antipodal(hp))
+    assert T.boxes_identical(poly.boundingBoxRotatingCalipers(hp), T.o_calipers(hp))
+    assert T.pca_boxes_equal(poly.boundingBoxPrincipalComponentAnalysis(hp), T.o_pca(hp)[0])
