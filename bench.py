@@ -382,7 +382,7 @@ def run_dror(args):
 # jump convolution, label write-back); prefix scans count with the stage of the kernel before them.
 SEG_KERNELS = {"k_quadrant", "k_ring_count", "k_ring_apply", "k_bin", "k_scatter", "k_cell_small", "k_cell_large",
                "k_chain", "k_near", "k_ransac_draw", "k_ransac_inliers", "k_ransac_select", "k_label_depth",
-               "k_project_key", "k_pixel", "k_dilate_rows", "k_jcp_weights", "k_jcp_rowrec", "k_jcp_rows",
+               "k_project_key", "k_pixel", "k_dilate_rows", "k_jcp_weights", "k_jcp_resolve", "k_jcp_rows",
                "k_populate"}
 
 

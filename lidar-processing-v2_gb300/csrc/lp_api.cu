@@ -152,7 +152,9 @@ lp_status plan(lp_context* ctx, lp_batch& B)
                 sd.first_ring = c.image_height - 1;
             pix += static_cast<uint64_t>(sd.H) * static_cast<uint64_t>(sd.W);
             // a queued pixel of the vote holds a point: at most min(pixels, points) per scan
-            queue += std::min<uint64_t>(static_cast<uint64_t>(sd.H) * static_cast<uint64_t>(sd.W), in.n);
+            sd.jq_off = static_cast<uint32_t>(queue);
+            sd.jq_cap = static_cast<uint32_t>(std::min<uint64_t>(static_cast<uint64_t>(sd.H) * static_cast<uint64_t>(sd.W), in.n));
+            queue += (sd.jq_cap + 15u) & ~15u;
             row += static_cast<uint64_t>(sd.H);
             cell += static_cast<uint64_t>(sd.nslice) * static_cast<uint64_t>(sd.nrad);
             slice += static_cast<uint64_t>(sd.nslice);
@@ -202,7 +204,7 @@ lp_status plan(lp_context* ctx, lp_batch& B)
     b.nrows = static_cast<uint32_t>(row);
     b.nhash = static_cast<uint32_t>(hash);
     b.ncl = static_cast<uint32_t>(cl);
-    b.jq_cap = static_cast<uint32_t>(queue);
+    b.jq_total = static_cast<uint32_t>(queue);
     return LP_OK;
 }
 
@@ -305,13 +307,13 @@ size_t carve(lp_batch& B, char* base)
         put(b.pix_map, b.npix);
         put(b.pix_state, b.npix);
         put(b.row_cols, b.npix);
-        put(b.row_cnt, b.nrows + 1); // [nrows]: queued pixels of the batch
-        put(b.row_q0, b.nrows);
-        put(b.jq, b.jq_cap + 1);
+        put(b.row_cnt, b.nrows);
+        put(b.jq, b.jq_total + 1);
         put(b.jw, static_cast<size_t>(b.nrows) * 3u * kJwStride); // the last three queued pixels of each row
-        put(b.jn, (static_cast<size_t>(b.jq_cap) + 1) * kJwStride);
-        put(b.jrow, static_cast<size_t>(b.nrows) * kJrowWords);
-        put(b.jmap, b.jq_cap + 1);
+        put(b.jst, static_cast<size_t>(b.jq_total) + 16);
+        put(b.jrec, static_cast<size_t>(b.jq_total) * kJrecFields + 1);
+        put(b.jlist, 2ull * b.jq_total + 1);
+        put(b.jborder, b.jq_total + 1);
         if (R.stages & ST_IMAGE)
             put(B.d_image, static_cast<size_t>(b.npix) * 3);
     }
@@ -473,7 +475,7 @@ lp_status execute(lp_context* ctx, lp_batch& B)
         LP_CUDA(ctx, cudaMemsetAsync(b.near_cnt, 0, (static_cast<size_t>(b.nnear) + 1) * 4, st));
         LP_CUDA(ctx, cudaMemsetAsync(b.pix_depth, 0xff, static_cast<size_t>(b.npix) * 4, st));
         LP_CUDA(ctx, cudaMemsetAsync(b.pix_key, 0xff, static_cast<size_t>(b.npix) * 8, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.row_cnt, 0, (static_cast<size_t>(b.nrows) + 1) * 4, st));
+        LP_CUDA(ctx, cudaMemsetAsync(b.row_cnt, 0, static_cast<size_t>(b.nrows) * 4, st));
         launch_segmentation(L, b, B.hb, B.d_image);
     }
     if (R.stages & ST_ALL_OBS)

@@ -36,24 +36,10 @@ enum : uint8_t
     V_O = 2
 };
 
-// Jump-convolution weight record of a queued pixel: 24 fresh weights, their sum, padding to a
-// multiple of 16 bytes (vector loads).
 constexpr uint32_t kKtPoolPerPoint = 8; // leftover search entries per point the DROR pool holds
+// Raw weight record of the jump convolution: 24 weights, padded to a multiple of 16 bytes.
 constexpr uint32_t kJwStride = 28;
-// Per image row of the jump convolution: lastq[3], pad, 24 stale weights, 24 stale label infos
-// (kJrowNoUpdate: the row leaves the slot as it was; kJrowDynamic | pixel: the final colour of
-// that pixel; else the label), padded to 64 words.
-constexpr uint32_t kJrowWords = 64;
-constexpr uint32_t kFinRingW = 4096; // image width up to which the vote keeps final colours in shared memory
-// Staging of the vote's next row: queued pixels per row and image rows it covers, bytes per buffer
-// (normalised records, the queue entries with 16-byte slack on both sides, the row record).
-constexpr uint32_t kStageRec = 256;
-constexpr uint32_t kRowCache = 1024;
-constexpr uint32_t kStageRecBytes = kStageRec * kJwStride * 4u;
-constexpr uint32_t kStageColBytes = (kStageRec * 2u + 32u + 15u) & ~15u;
-constexpr uint32_t kStageBytes = kStageRecBytes + kStageColBytes + kJrowWords * 4u; // + the row record
-constexpr uint32_t kJrowNoUpdate = 0xffffffffu;
-constexpr uint32_t kJrowDynamic = 0x80000000u;
+constexpr uint32_t kJrecFields = 10; // 16-byte fields of an open pixel's record (jrec in lp_segment.cu)
 
 // A scan's buffers in the caller's page-locked host memory (device-accessible addresses).
 struct IoScan
@@ -132,14 +118,14 @@ struct BatchDev
     // ---- jump convolution -------------------------------------------------------------------
     uint32_t nrows;
     uint16_t* row_cols;        // per pixel slot: intersection columns of the row in order
-    uint4* jq;            // flat list of the batch's queued pixels: (image row, position | column << 16, point, scan)
+    uint4* jq;            // per scan (jq_off): its queued pixels: (image row, position | column << 16, point, 0)
     uint32_t* row_cnt;         // per global row
-    float* jw;                 // per row, its last three queued pixels: 24 fresh weights + sum (stride kJwStride)
-    float* jn;                 // per queued pixel (flat queue position): 24 normalized weights, sum, slot label codes
-    uint32_t* row_q0;          // per image row: its first position in the flat queue
-    uint32_t jq_cap;           // queue capacity: sum over scans of min(pixels, points)
-    uint32_t* jrow;            // per image row: kJrowWords words (lastq, stale-buffer update)
-    unsigned long long* jmap;  // per entry: 9-state transition map
+    float* jw;                 // per row, its last three queued pixels: 24 fresh weights (stride kJwStride)
+    uint32_t jq_total;         // queue capacity: sum over scans of min(pixels, points), each rounded up to 16
+    uint8_t* jst;              // per queued pixel: its outcome, or JST_OPEN
+    uint4* jrec;               // per open pixel (list position at jq_off): kJrecFields x jq_total
+    uint32_t* jlist;           // 2 x jq_total: positions of the pixels still open, round by round
+    uint32_t* jborder;         // list positions of the open pixels whose window leaves the image
 
     // ---- segmentation output -----------------------------------------------------------------
     uint32_t* seg_label; // per compacted point

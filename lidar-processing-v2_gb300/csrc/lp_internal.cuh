@@ -39,6 +39,7 @@ struct ScanDev
     uint32_t pix_off;
     int32_t H, W;
     uint32_t row_off;   // first global row (sum of H of earlier scans)
+    uint32_t jq_off, jq_cap; // vote queue slice: jq_off a multiple of 16, at most min(pixels, points) entries
     uint32_t tile_off;  // first 1024-point ring tile
     uint32_t slice_off; // first global azimuth slice
     // polar grid
@@ -86,7 +87,10 @@ struct ScanState
     uint32_t n_clusters;
     uint32_t cl_base; // clusters of earlier scans (work-queue numbering)
     uint32_t n_hull;
-    uint32_t pad[4];
+    // jump convolution: queued pixels, those the weights pass left open, and of these the ones whose
+    // window leaves the image
+    uint32_t n_queue, n_open, n_border;
+    uint32_t pad[1];
 };
 
 __device__ __forceinline__ void raise_err(ScanState* st, uint32_t bit)

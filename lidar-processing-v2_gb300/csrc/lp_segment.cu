@@ -1170,16 +1170,16 @@ __global__ void __launch_bounds__(256) k_dilate_rows(BatchDev b)
             run += wcount[k];
         }
         b.row_cnt[r] = run;
-        // the row's segment of the flat list of queued pixels (row_cnt[nrows] counts them); the
-        // capacity bound (a queued pixel holds a point) cannot be exceeded, checked all the same
-        qbase = run ? atomicAdd(&b.row_cnt[b.nrows], run) : 0u;
-        if (qbase + run > b.jq_cap)
+        // the row's segment of the scan's queue; the capacity bound (a queued pixel holds a point)
+        // cannot be exceeded, checked all the same
+        qbase = run ? atomicAdd(&b.state[s].n_queue, run) : 0u;
+        if (qbase + run > sd.jq_cap)
         {
             raise_err(&b.state[s], ERR_INTERNAL);
             b.row_cnt[r] = 0u;
-            qbase = 0u;
+            atomicSub(&b.state[s].n_queue, run);
+            qbase = 0xffffffffu;
         }
-        b.row_q0[r] = qbase;
     }
     __syncthreads();
     // pass 2: queue entries in column order (this row's states now hold the intersections)
@@ -1193,11 +1193,14 @@ __global__ void __launch_bounds__(256) k_dilate_rows(BatchDev b)
         {
             const uint32_t j = pos + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
             b.row_cols[row_base + j] = static_cast<uint16_t>(w);
-            // (row, position | column << 16, the pixel's point, scan): the weights pass starts here
-            if (qbase + j < b.jq_cap)
-                b.jq[qbase + j] = make_uint4(r, j | (static_cast<uint32_t>(w) << 16),
-                                         static_cast<uint32_t>(b.pix_map[sd.pix_off + static_cast<uint32_t>(h * W + w)]),
-                                         static_cast<uint32_t>(s));
+            // (row, position | column << 16, the pixel's point): the weights pass starts here; the
+            // depth key, no longer needed, takes the pixel's queue index for those that read its outcome
+            if (qbase != 0xffffffffu)
+            {
+                b.jq[sd.jq_off + qbase + j] = make_uint4(r, j | (static_cast<uint32_t>(w) << 16),
+                                                         static_cast<uint32_t>(b.pix_map[row_base + static_cast<uint32_t>(w)]), 0u);
+                b.pix_depth[row_base + static_cast<uint32_t>(w)] = qbase + j;
+            }
         }
         pos += static_cast<uint32_t>(__popc(m));
     }
@@ -1223,579 +1226,572 @@ __device__ __forceinline__ uint8_t pre_view(uint8_t st)
     return (st == PX_GROUND) ? V_G : ((st == PX_OBSTACLE) ? V_O : V_U);
 }
 
-// A queued pixel's vote (segmenter.cpp:585-631) as a 9-state transition map of the in-row chain.
-// The reference sums, in slot order, the normalised weights of the slots labelled ground into g
-// and of those labelled obstacle into o (a slot with another label adds nothing), and votes
-// obstacle iff o > g. Here both sums run as one pair (a slot adds (w, 0), (0, w) or (0, 0);
-// weights and sums are never negative, so adding +0 is exactly the reference's skip, and each half
-// rounds like its scalar addition in the same order). The labels at slots 10 (column c-2) and 11
-// (c-1) are symbolic where those are queued pixels of the same row (their outcomes, the chain's
-// state; sym_b / sym_a). g after slot 11 is one of four values (whether slot 10, then slot 11, is
-// ground) and so is o, so four chains over slots 12-23 give the final sums for all nine label
-// pairs of slots 10 and 11 (an outcome table of 2 bits per pair); each chain state reads the
-// pair its labels select. The map (state = 3 x + a) is built for the column gap to the previous
-// queued pixel.
-__device__ __forceinline__ unsigned long long vote_map(const float* wn, const uint8_t* lb, bool sym_a, bool sym_b,
-                                                       bool live, int32_t gap)
+// ------------------------------------------------------------------------------------------
+// The vote of the queued pixels (segmenter.cpp:523-637). The reference takes them in row-major
+// order, in place: a pixel reads the final colours of queued pixels above it and to its left in its
+// row (kernel slots 0-11), pre-vote colours everywhere else. The sums run in slot order: a neighbour
+// labelled ground adds its normalised weight to g, one labelled obstacle to o, and the pixel becomes
+// an obstacle iff o > g.
+//
+// Taking image rows one after the other (one CTA per scan, the row as a scan of transition maps)
+// made the vote the longest kernel of every call: a chain of 64-128 rows at 2 us each. But most
+// outcomes do not depend on their open neighbours: weights are never negative and rounding is
+// monotone, so with every open neighbour counted to o and none to g (and the other way round) the
+// same chain of additions bounds o and g for any outcome of theirs. A pixel whose bounds do not
+// overlap is decided at once, in any order, with the reference's result. k_jcp_weights decides about
+// half of the pixels this way, in parallel; k_jcp_resolve repeats the test for the rest as their
+// neighbours are decided (about 20-100 hops instead of one step per row; every hop decides at
+// least the first open pixel in the reference's order).
+// ------------------------------------------------------------------------------------------
+enum : uint32_t
 {
-    auto gw = [](uint8_t l, float w) { return make_float2(l == V_G ? w : 0.0F, l == V_O ? w : 0.0F); };
-    float2 head = make_float2(0.0F, 0.0F);
+    JST_OPEN = 3u // queued pixel not decided yet (V_U, V_G, V_O otherwise)
+};
+
+// Decision from the normalised weights and the slots' labels (bit 0 of slot k's label in m0, bit 1 in
+// m1; both: the slot is open). V_G / V_O, or JST_OPEN while the open slots could change it.
+__device__ __forceinline__ uint32_t vote_bounds(const float* wn, uint32_t m0, uint32_t m1)
+{
+    float2 lo = make_float2(0.0F, 0.0F), hi = lo; // (g, o) without the open slots, with them on both sides
+    const uint32_t g = m0 & ~m1, o = m1 & ~m0;
 #pragma unroll
-    for (int k = 0; k < 10; ++k)
-        head = __fadd2_rn(head, gw(lb[k], wn[k]));
-    // start i (bit 0: slot 10 adds, bit 1: slot 11 adds): g in .x, o in .y, each slot added in order
-    float2 v[4];
-    v[0] = head;
-    v[1] = __fadd2_rn(head, make_float2(wn[10], wn[10]));
-    v[2] = __fadd2_rn(head, make_float2(wn[11], wn[11]));
-    v[3] = __fadd2_rn(v[1], make_float2(wn[11], wn[11]));
-#pragma unroll
-    for (int k = 12; k < 24; ++k)
+    for (int k = 0; k < 24; ++k)
     {
-        const float2 d = gw(lb[k], wn[k]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            v[i] = __fadd2_rn(v[i], d);
+        const uint32_t bit = 1u << k;
+        lo = __fadd2_rn(lo, make_float2((g & bit) ? wn[k] : 0.0F, (o & bit) ? wn[k] : 0.0F));
+        hi = __fadd2_rn(hi, make_float2((m0 & bit) ? wn[k] : 0.0F, (m1 & bit) ? wn[k] : 0.0F));
     }
-    // outcome of label pair (l10, l11) at bits 2 (3 l10 + l11): the starts it selects are fixed
-    uint32_t otab = 0u;
-#pragma unroll
-    for (int l10 = 0; l10 < 3; ++l10)
-#pragma unroll
-        for (int l11 = 0; l11 < 3; ++l11)
-        {
-            const int ig = (l10 == V_G ? 1 : 0) | (l11 == V_G ? 2 : 0);
-            const int io = (l10 == V_O ? 1 : 0) | (l11 == V_O ? 2 : 0);
-            otab |= static_cast<uint32_t>((v[io].y > v[ig].x) ? V_O : V_G) << (2 * (3 * l10 + l11));
-        }
-    if (!live)
-        otab = 0u; // V_U whatever the labels
-    const int g1 = gap == 1, g2 = gap == 2;
-    unsigned long long t = 0ull;
-#pragma unroll
-    for (int sidx = 0; sidx < 9; ++sidx)
-    {
-        const int a = sidx / 3, bb = sidx % 3;
-        const int ap = g1 ? a : V_U;
-        const int bp = g1 ? bb : (g2 ? a : V_U);
-        const int l10 = sym_b ? bp : lb[10];
-        const int l11 = sym_a ? ap : lb[11];
-        const uint32_t x = (otab >> (2 * (3 * l10 + l11))) & 3u;
-        t |= static_cast<unsigned long long>(3u * x + static_cast<uint32_t>(ap)) << (4 * sidx);
-    }
-    return t;
+    if ((m0 & m1) == 0u)
+        return (lo.y > lo.x) ? V_O : V_G;
+    if (lo.y > hi.x)
+        return V_O; // o >= lo.y > hi.x >= g
+    return (hi.y <= lo.x) ? V_G : JST_OPEN; // o <= hi.y <= lo.x <= g (false for nan weights: they stay open)
 }
 
-// Fresh (not stale) weight of every in-bounds neighbour slot of every queued pixel: 0 for an
-// empty neighbour or one farther than the kernel threshold, else expf(-amp * dist)
-// (segmenter.cpp:545-607). These depend on geometry only, so they are computed in parallel
-// before the ordered vote. Two records per queued pixel:
-//   jw: the raw weights and their sum (read back when a later pixel's slot leaves the image;
-//       written for the last three queued pixels of each row, the only ones read),
-//   jn: the weights divided by the sum, the sum, and a 2-bit label code per slot: the label the
-//       vote will read (unknown / ground / obstacle) wherever it is already fixed, or 3 where it
-//       is not: a queued pixel in a row above (its final colour comes from its own vote) or a
-//       queued pixel to the left in the same row (the symbolic outcome of the in-row chain).
-__global__ void __launch_bounds__(256) k_jcp_weights(BatchDev b)
+// Records of the open pixels, by list position (fields of 16 bytes, jq_total entries each):
+// 0-5 the 24 normalised weights; 6-8 for slots 0-11 the queue index behind an open slot, else
+// kDepFixed | label; 9 (label bit 0 per slot, label bit 1 per slot, queue index, weight sum).
+constexpr uint32_t kDepFixed = 0x80000000u;
+
+__device__ __forceinline__ uint4& jrec(const BatchDev& b, uint32_t field, uint32_t at)
 {
-    // one warp per queued pixel of the batch's flat list (rows of any length spread over the whole
-    // grid), lane k = kernel slot k (lanes 24-31 idle); the weights are summed by lane 0 in slot
-    // order, as the reference's loop adds them
-    const uint32_t total = min(b.row_cnt[b.nrows], b.jq_cap);
+    return b.jrec[static_cast<size_t>(field) * b.jq_total + at];
+}
+
+// Weights of the queued pixels (segmenter.cpp:545-607): 0 for an empty neighbour or one farther than
+// the kernel threshold, else expf(-amp * dist). A warp takes up to 32 consecutive pixels of a scan's
+// queue: lane k = kernel slot k for the gathers (four pixels side by side), the weights and the
+// divisions by the sum, lane = pixel for the sums (slot order, as the reference's loop adds them) and
+// the decision. Fewer pixels per warp where the queues would leave warps idle (4 to 32, from their
+// total). The exponential and the division stand in loops that are not unrolled: on a single scan
+// every warp runs this code once, and fetching it is most of the time.
+// Only open pixels leave a record. A pixel whose window leaves the image is completed by
+// k_jcp_resolve: such a slot keeps what an earlier queued pixel left there; the raw weights of each
+// row's last three queued pixels, the only ones read for that, go to jw.
+struct JcpTile // a warp's pixels
+{
+    float w[32][25]; // squared distances, then weights, then normalised weights
+    float sum[32];
+    uint32_t dep[32][13];
+    uint32_t m0[32], m1[32], oob[32], valid[32];
+};
+constexpr uint32_t kWeightThreads = 128;
+
+__global__ void __launch_bounds__(kWeightThreads) k_jcp_weights(BatchDev b)
+{
+    __shared__ JcpTile tiles[kWeightThreads / 32];
     const uint32_t lane = lane_id();
     const int k = static_cast<int>(lane);
     const int32_t dh = jcp_dh(k), dw = jcp_dw(k);
-    const uint32_t nw = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < total; q += nw)
+    JcpTile& t = tiles[threadIdx.x >> 5];
+    const uint32_t nwarp = gridDim.x * (kWeightThreads / 32u);
+    uint32_t total = 0u;
+    for (int q = 0; q < b.nscan; ++q)
+        total += b.state[q].n_queue;
+    const uint32_t per = min(32u, 4u * max(1u, div_up(total, 4u * nwarp))); // pixels per warp and turn
+    int s = 0; // the cursor: scan s owns turns [tbase, tbase + div_up(nq, per))
+    uint32_t tbase = 0u, nq = b.nscan > 0 ? b.state[0].n_queue : 0u;
+    for (uint32_t it = (blockIdx.x * kWeightThreads + threadIdx.x) >> 5;; it += nwarp)
     {
-        const uint4 e = b.jq[q];
-        const uint32_t r = e.x, j = e.y & 0xffffu;
-        const int32_t w = static_cast<int32_t>(e.y >> 16);
-        const int s = static_cast<int>(e.w);
+        while (s < b.nscan && it >= tbase + div_up(nq, per))
+        {
+            tbase += div_up(nq, per);
+            ++s;
+            nq = (s < b.nscan) ? b.state[s].n_queue : 0u;
+        }
+        if (s >= b.nscan)
+            break; // uniform over the warp
         const ScanDev& sd = b.scans[s];
-        const int32_t h = static_cast<int32_t>(r - sd.row_off);
+        const uint32_t q0 = (it - tbase) * per;
+        const uint32_t cnt = min(per, nq - q0);
         const int32_t H = sd.H, W = sd.W;
-        const uint32_t row_base = sd.pix_off + static_cast<uint32_t>(h * W);
-        const uint32_t m = b.row_cnt[r];
         const int32_t* map = b.pix_map + sd.pix_off;
+        const uint32_t* qidx = b.pix_depth + sd.pix_off;
         const uint8_t* st = b.pix_state + sd.pix_off;
         const float4* pts = b.pts + sd.pt_off;
-        const float4 cp = pts[e.z];
-        float wt = 0.0F;
-        uint32_t code = V_U;
-        const int32_t hh = h + dh, ww = w + dw;
-        if (k < 24 && hh >= 0 && hh < H && ww >= 0 && ww < W)
+        const float kthr2 = sd.kthr2, namp = -sd.amp;
+        const uint4 mine_e = b.jq[sd.jq_off + q0 + min(lane, cnt - 1u)]; // lane p: pixel p's queue entry
+        const uint32_t mine_m = b.row_cnt[mine_e.x];
+        for (uint32_t p0 = 0; p0 < cnt; p0 += 4u)
         {
-            const int32_t ni = map[hh * W + ww];
-            if (ni >= 0)
+            int32_t ni[4];
+            uint8_t ns[4];
+            uint32_t qi[4];
+            float4 cp[4], np[4];
+            bool inb[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u)
             {
-                const float4 np = pts[ni];
-                const float dx = cp.x - np.x;
-                const float dy = cp.y - np.y;
-                const float dz = cp.z - np.z;
-                const float d2 = dx * dx + dy * dy + dz * dz;
-                if (!(d2 > sd.kthr2))
-                    wt = lpm::cr_expf(-sd.amp * sqrtf(d2));
+                const int src = static_cast<int>(min(p0 + u, cnt - 1u));
+                const int32_t h = static_cast<int32_t>(__shfl_sync(0xffffffffu, mine_e.x, src) - sd.row_off);
+                const int32_t w = static_cast<int32_t>(__shfl_sync(0xffffffffu, mine_e.y, src) >> 16);
+                const int32_t hh = h + dh, ww = w + dw;
+                inb[u] = k < 24 && hh >= 0 && hh < H && ww >= 0 && ww < W;
+                const int32_t at = inb[u] ? hh * W + ww : 0;
+                ni[u] = inb[u] ? map[at] : -1;
+                ns[u] = st[at];
+                qi[u] = (k < 12) ? qidx[at] : 0u;
+                cp[u] = pts[__shfl_sync(0xffffffffu, mine_e.z, src)];
             }
-            if (wt != 0.0F)
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u)
+                np[u] = (ni[u] >= 0) ? pts[ni[u]] : cp[u];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u)
             {
-                const uint8_t ns = st[hh * W + ww];
-                if (dh > 0 || (dh == 0 && dw > 0))
-                    code = pre_view(ns); // not voted before this pixel
-                else
-                    code = (ns == PX_INTERSECT) ? 3u : final_view(ns);
+                const uint32_t p = p0 + u;
+                const float dx = cp[u].x - np[u].x;
+                const float dy = cp[u].y - np[u].y;
+                const float dz = cp[u].z - np[u].z;
+                const float d2 = dx * dx + dy * dy + dz * dz;
+                // slots 12-23 are not voted before this pixel
+                const uint32_t code = (k < 12 && ns[u] == PX_INTERSECT) ? 3u : pre_view(ns[u]);
+                const uint32_t va = __ballot_sync(0xffffffffu, ni[u] >= 0 && !(d2 > kthr2));
+                const uint32_t c0 = __ballot_sync(0xffffffffu, code & 1u), c1 = __ballot_sync(0xffffffffu, code & 2u);
+                const uint32_t ob = __ballot_sync(0xffffffffu, k < 24 && !inb[u]);
+                if (p < cnt)
+                {
+                    if (k < 24)
+                        t.w[p][k] = d2;
+                    if (k < 12) // the queue index behind an open slot, else its label
+                        t.dep[p][k] = (code == 3u) ? qi[u] : kDepFixed | code;
+                    if (lane == 0)
+                    {
+                        t.m0[p] = c0;
+                        t.m1[p] = c1;
+                        t.oob[p] = ob;
+                        t.valid[p] = va;
+                    }
+                }
             }
         }
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t p = 0; p < cnt; ++p)
+        {
+            float wt = 0.0F;
+            if ((t.valid[p] >> k) & 1u)
+                wt = lpm::cr_expf(namp * sqrtf(t.w[p][k]));
+            const uint32_t nz = __ballot_sync(0xffffffffu, wt != 0.0F);
+            if (k < 24)
+                t.w[p][k] = wt;
+            if (k < 12 && wt == 0.0F)
+                t.dep[p][k] = kDepFixed | V_U;
+            if (lane == 0) // a slot without weight has no label
+            {
+                t.m0[p] &= nz;
+                t.m1[p] &= nz;
+            }
+        }
+        __syncwarp();
+        const uint32_t p = min(lane, cnt - 1u);
+        const bool mine = lane < cnt;
+        float wn[24];
         float sum = 0.0F;
 #pragma unroll
         for (int q = 0; q < 24; ++q)
-            sum += __shfl_sync(0xffffffffu, wt, q);
-        unsigned long long codes = (k < 24) ? (static_cast<unsigned long long>(code) << (2 * k)) : 0ull;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            codes |= __shfl_xor_sync(0xffffffffu, codes, o);
-        const bool live = fabsf(sum) > FLT_EPSILON;
-        // the raw record is only read for the row's last three queued pixels (the stale-slot
-        // sources of later rows and of the row's right border)
-        const bool raw = j + 3u >= m;
-        // raw records: the row's last three positions, slot j + 3 - m; normalised: by queue position
-        float* out = raw ? b.jw + (static_cast<size_t>(r) * 3u + (j + 3u - m)) * kJwStride : nullptr;
-        float* nrm = b.jn + static_cast<size_t>(q) * kJwStride;
-        if (k < 24)
         {
-            if (raw)
-                out[k] = wt;
-            nrm[k] = live ? wt / sum : 0.0F;
+            wn[q] = t.w[p][q];
+            sum += wn[q];
         }
-        else if (k < 28)
+        const uint32_t j = mine_e.y & 0xffffu;
+        if (mine && j + 3u >= mine_m)
         {
-            if (raw)
-                out[k] = (k == 24) ? sum : 0.0F;
-            nrm[k] = (k == 24) ? sum
-                               : ((k == 25) ? __uint_as_float(static_cast<uint32_t>(codes))
-                                            : ((k == 26) ? __uint_as_float(static_cast<uint32_t>(codes >> 32)) : 0.0F));
-        }
-    }
-}
-
-// Row record of the ordered vote (kJrowWords words per image row with queued pixels), one warp per
-// row (lanes 0-23: slots), after k_jcp_weights has written every pixel's raw weight record.
-__global__ void __launch_bounds__(256) k_jcp_rowrec(BatchDev b)
-{
-    const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (r >= b.nrows || lane_id() >= 24u)
-        return;
-    const uint32_t m = b.row_cnt[r];
-    if (m == 0u)
-        return;
-    const int s = scan_of_row(b, r);
-    const ScanDev& sd = b.scans[s];
-    const int32_t h = static_cast<int32_t>(r - sd.row_off);
-    const int32_t H = sd.H, W = sd.W;
-    const uint32_t row_base = sd.pix_off + static_cast<uint32_t>(h * W);
-    const uint8_t* st = b.pix_state + sd.pix_off;
-
-    // Row record (kJrowWords words): lastq[d] = the last of the row's final three queued pixels
-    // with column <= W-1-d; per slot k, what the row leaves in the reference's stale weight/label
-    // buffer: the raw weight of the last queued pixel for which slot k is inside the image, and
-    // its label, fixed already or (a queued pixel before it in vote order) read after the vote.
-    uint32_t* rec = b.jrow + static_cast<size_t>(r) * kJrowWords;
-    const uint16_t* cols = b.row_cols + row_base;
-    int32_t lq[3];
-    for (int32_t d = 0; d < 3; ++d)
-    {
-        lq[d] = -1;
-        for (int32_t j = static_cast<int32_t>(m) - 1; j >= 0 && j >= static_cast<int32_t>(m) - 3; --j)
-            if (cols[j] <= W - 1 - d)
-            {
-                lq[d] = j;
-                break;
-            }
-    }
-    const int k = static_cast<int>(lane_id());
-    if (k < 3)
-        rec[k] = static_cast<uint32_t>(lq[k]);
-    const int32_t dh = jcp_dh(k), dw = jcp_dw(k);
-    const int32_t hh = h + dh;
-    uint32_t info = kJrowNoUpdate;
-    float qw = 0.0F;
-    if (hh >= 0 && hh < H)
-    {
-        const int32_t q = lq[dw > 0 ? dw : 0];
-        if (q >= 0 && static_cast<int32_t>(cols[q]) >= (dw < 0 ? -dw : 0))
-        {
-            qw = b.jw[(static_cast<size_t>(r) * 3u + static_cast<uint32_t>(q + 3 - static_cast<int32_t>(m))) * kJwStride + k];
-            info = V_U;
-            if (qw != 0.0F)
-            {
-                const uint32_t addr = static_cast<uint32_t>(hh * W + cols[q] + dw);
-                const uint8_t ns = st[addr];
-                const bool before = (dh < 0) || (dh == 0 && dw < 0);
-                if (!before)
-                    info = pre_view(ns);
-                else if (ns == PX_INTERSECT)
-                    info = kJrowDynamic | addr; // its colour is its own vote's outcome
-                else
-                    info = final_view(ns);
-            }
-        }
-    }
-    rec[4 + k] = __float_as_uint(qw);
-    rec[28 + k] = info;
-}
-
-__device__ __forceinline__ unsigned long long map_compose(unsigned long long later, unsigned long long earlier)
-{
-    unsigned long long r = 0ull;
-#pragma unroll
-    for (int s = 0; s < 9; ++s)
-    {
-        const uint32_t mid = static_cast<uint32_t>((earlier >> (4 * s)) & 0xfull);
-        r |= ((later >> (4 * mid)) & 0xfull) << (4 * s);
-    }
-    return r;
-}
-__device__ __forceinline__ unsigned long long map_identity()
-{
-    unsigned long long r = 0ull;
-#pragma unroll
-    for (int s = 0; s < 9; ++s)
-        r |= static_cast<unsigned long long>(s) << (4 * s);
-    return r;
-}
-
-// The ordered vote (segmenter.cpp:535-637), one block per scan, image rows in order.
-//
-// Within a row, the queued pixel at column c reads the vote outcomes of the queued pixels at
-// c-1 and c-2 (already written in the reference's FIFO); everything else it reads is fixed:
-// rows above are final, rows below and columns to the right still hold their pre-vote colour.
-// Each queued pixel therefore has a vote table f(a, b) over the outcomes a (column c-1) and
-// b (column c-2), each in {unknown, ground, obstacle}; the row is a chain of 9-state
-// transitions composed by a block-wide prefix scan, which reproduces the FIFO exactly.
-//
-// Slots outside the image keep the weight and label the previous queued pixel wrote to that
-// slot (segmenter.cpp:552-556). That pixel is the last earlier queued pixel for which the slot
-// was inside the image: for a right-border pixel it can be an earlier pixel of the same row
-// (columns <= W-1-dw); otherwise it lies in an earlier row, tracked as a running value per
-// slot across rows.
-__global__ void __launch_bounds__(256) k_jcp_rows(BatchDev b)
-{
-    __shared__ float run_w[24];
-    __shared__ uint8_t run_l[24];
-    __shared__ unsigned long long wmaps[8];
-    __shared__ unsigned long long rmap[256]; // a row's maps by position (rows of at most 256 pixels)
-    // final colour (V_U/V_G/V_O) of the queued pixels of the last three rows, by column: the
-    // labels a pixel reads from queued pixels above it, without a global load (images up to
-    // kFinRingW columns; wider ones read the pixel states)
-    __shared__ uint8_t fin[3][kFinRingW];
-    // Double-buffered staging: while a row votes, one thread copies the next non-empty row's
-    // normalised records and queue entries into shared memory with a TMA bulk copy (rows of at
-    // most kStageRec queued pixels, images of at most kRowCache rows; others load directly).
-    extern __shared__ __align__(16) unsigned char stage[];
-    __shared__ uint32_t mrow[kRowCache];
-    __shared__ unsigned long long mbar[2];
-    __shared__ int32_t st_row[2], st_coff[2];
-    __shared__ int32_t st_pend[2]; // a copy into the buffer is in flight (issued, not yet waited for)
-    const int s = blockIdx.x;
-    const ScanDev& sd = b.scans[s];
-    const int32_t H = sd.H, W = sd.W;
-    const bool ring = W <= static_cast<int32_t>(kFinRingW);
-    const bool cache = H <= static_cast<int32_t>(kRowCache);
-    if (cache)
-        for (int32_t i = threadIdx.x; i < H; i += blockDim.x)
-            mrow[i] = b.row_cnt[sd.row_off + static_cast<uint32_t>(i)];
-    if (threadIdx.x == 0)
-    {
-        mbar_init(&mbar[0], 1u);
-        mbar_init(&mbar[1], 1u);
-        st_row[0] = st_row[1] = -1;
-        st_pend[0] = st_pend[1] = 0;
-    }
-    __syncthreads();
-    // thread 0: copy row hh into buffer bf (queue entries widened to 16-byte bounds)
-    auto issue = [&](int32_t hh, int bf) {
-        const uint32_t mm = mrow[hh];
-        const uint32_t rb = sd.pix_off + static_cast<uint32_t>(hh * W);
-        const uint32_t rec_bytes = mm * kJwStride * 4u;
-        const uintptr_t c0 = reinterpret_cast<uintptr_t>(b.row_cols + rb);
-        const uintptr_t ca = c0 & ~static_cast<uintptr_t>(15);
-        const uintptr_t ce = (reinterpret_cast<uintptr_t>(b.row_cols + rb + mm) + 15) & ~static_cast<uintptr_t>(15);
-        unsigned char* dst = stage + bf * kStageBytes;
-        mbar_expect_tx(&mbar[bf], rec_bytes + static_cast<uint32_t>(ce - ca) + kJrowWords * 4u);
-        bulk_g2s(dst, b.jn + static_cast<size_t>(b.row_q0[sd.row_off + static_cast<uint32_t>(hh)]) * kJwStride, rec_bytes,
-                 &mbar[bf]);
-        bulk_g2s(dst + kStageRecBytes, reinterpret_cast<const void*>(ca), static_cast<uint32_t>(ce - ca), &mbar[bf]);
-        bulk_g2s(dst + kStageRecBytes + kStageColBytes,
-                 b.jrow + static_cast<size_t>(sd.row_off + static_cast<uint32_t>(hh)) * kJrowWords, kJrowWords * 4u,
-                 &mbar[bf]);
-        st_row[bf] = hh;
-        st_coff[bf] = static_cast<int32_t>((c0 - ca) / 2);
-        st_pend[bf] = 1;
-    };
-    auto stageable = [&](int32_t hh) { return cache && mrow[hh] > 0 && mrow[hh] <= kStageRec; };
-    auto next_row = [&](int32_t hh) {
-        for (int32_t q = hh + 1; q < H; ++q)
-            if (mrow[q] > 0)
-                return q;
-        return -1;
-    };
-    uint32_t parity[2] = {0u, 0u};
-    int cur = 0;
-    if (threadIdx.x == 0 && cache)
-    {
-        const int32_t h0 = next_row(-1);
-        if (h0 >= 0 && stageable(h0))
-            issue(h0, 0);
-    }
-    __syncthreads();
-    uint8_t* st = b.pix_state + sd.pix_off;
-    if (threadIdx.x < 24)
-    {
-        run_w[threadIdx.x] = 0.0F;
-        run_l[threadIdx.x] = V_U;
-    }
-    __syncthreads();
-    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    for (int32_t h = 0; h < H; ++h)
-    {
-        const uint32_t r = sd.row_off + static_cast<uint32_t>(h);
-        const uint32_t m = cache ? mrow[h] : b.row_cnt[r];
-        if (m == 0)
-            continue;
-        const uint32_t row_base = sd.pix_off + static_cast<uint32_t>(h * W);
-        const uint16_t* cols = b.row_cols + row_base;
-        const uint32_t q0 = b.row_q0[r]; // the row's first position in the flat queue
-        const bool staged = st_row[cur] == h;
-        const float4* srec = reinterpret_cast<const float4*>(stage + cur * kStageBytes);
-        const uint16_t* scols = reinterpret_cast<const uint16_t*>(stage + cur * kStageBytes + kStageRecBytes) + st_coff[cur];
-        __syncthreads(); // every thread has read st_row / st_coff before thread 0 reissues
-        if (threadIdx.x == 0 && cache)
-        {
-            const int32_t hn = next_row(h);
-            st_row[cur ^ 1] = -1;
-            if (hn >= 0 && stageable(hn))
-                issue(hn, cur ^ 1);
-        }
-        if (staged)
-        {
-            // every thread waits (bounded); the block decides together whether the copy landed
-            const bool landed = mbar_wait(&mbar[cur], parity[cur], 1u << 22);
-            if (!__syncthreads_and(landed))
-            {
-                // report, then give every copy still in flight (this row's and the next row's,
-                // issued above) a last bounded wait before the CTA leaves its shared memory
-                if (threadIdx.x == 0)
-                    raise_err(&b.state[s], ERR_INTERNAL);
-                for (int bf = 0; bf < 2; ++bf)
-                    if (st_pend[bf])
-                        mbar_wait(&mbar[bf], parity[bf], 1u << 24);
-                return;
-            }
-            parity[cur] ^= 1u;
-            // landed for every thread, so no thread reads st_pend in this row; thread 0 alone
-            // writes it (here and in issue), so clearing needs no further barrier
-            if (threadIdx.x == 0)
-                st_pend[cur] = 0;
-        }
-        // the row's record (from the parallel pass): lastq and the stale-buffer update
-        const uint32_t* rrec = staged ? reinterpret_cast<const uint32_t*>(stage + cur * kStageBytes + kStageRecBytes + kStageColBytes)
-                                      : b.jrow + static_cast<size_t>(r) * kJrowWords;
-        const int32_t lastq[3] = {static_cast<int32_t>(rrec[0]), static_cast<int32_t>(rrec[1]),
-                                  static_cast<int32_t>(rrec[2])};
-        float upd_w = 0.0F;
-        uint32_t upd_info = kJrowNoUpdate;
-        if (threadIdx.x < 24)
-        {
-            upd_w = __uint_as_float(rrec[4 + threadIdx.x]);
-            upd_info = rrec[28 + threadIdx.x];
-        }
-
-        // ---- per queued pixel: vote table -> 9-state transition map --------------------------
-        const int32_t fr2 = (h + 1) % 3, fr1 = (h + 2) % 3; // final-colour rows of h-2 and h-1
-        // Consecutive chunks of pixels per thread (one pixel per thread in rows of at most 256
-        // pixels, whose maps stay in shared memory).
-        const bool spread = m <= blockDim.x;
-        const uint32_t chunk = (m + blockDim.x - 1) / blockDim.x;
-        const uint32_t j0 = threadIdx.x * chunk;
-        const uint32_t j1 = min(m, j0 + chunk);
-        unsigned long long agg = map_identity();
-        for (uint32_t j = j0; j < j1; ++j)
-        {
-            // the pixel's queue entry and normalised record: staged in shared memory, or loaded
-            const int32_t c = staged ? scols[j] : cols[j];
-            const float4* rec = staged ? srec + 7u * j
-                                       : reinterpret_cast<const float4*>(b.jn + static_cast<size_t>(q0 + j) * kJwStride);
-            float wn[24];
+            float4* raw = reinterpret_cast<float4*>(b.jw + (static_cast<size_t>(mine_e.x) * 3u + (j + 3u - mine_m)) * kJwStride);
 #pragma unroll
             for (int q = 0; q < 6; ++q)
-            {
-                const float4 v = rec[q];
-                wn[4 * q] = v.x;
-                wn[4 * q + 1] = v.y;
-                wn[4 * q + 2] = v.z;
-                wn[4 * q + 3] = v.w;
-            }
-            const float4 tail = rec[6];
-            const float sum = tail.x;
-            const unsigned long long codes =
-                static_cast<unsigned long long>(__float_as_uint(tail.y)) |
-                (static_cast<unsigned long long>(__float_as_uint(tail.z)) << 32);
-            unsigned long long t;
-            if (h >= 2 && h + 2 < H && c >= 2 && c + 2 < W)
-            {
-                // the window lies inside the image: labels from the codes and the final colours
-                // above (no stale slot)
-                const bool live = fabsf(sum) > FLT_EPSILON;
-                uint8_t lb[24];
-                bool sym_a = false, sym_b = false;
-#pragma unroll
-                for (int k = 0; k < 24; ++k)
-                {
-                    const uint32_t code = static_cast<uint32_t>((codes >> (2 * k)) & 3ull);
-                    if (code != 3u)
-                        lb[k] = static_cast<uint8_t>(code);
-                    else if (k < 10)
-                    {
-                        const int32_t hh = h + jcp_dh(k), ww = c + jcp_dw(k);
-                        lb[k] = ring ? fin[k < 5 ? fr2 : fr1][ww] : final_view(st[hh * W + ww]);
-                    }
-                    else
-                    {
-                        lb[k] = V_U; // same row, left of c, queued: the chain's state
-                        if (k == 11)
-                            sym_a = true;
-                        else
-                            sym_b = true;
-                    }
-                }
-                const int32_t gap = (j > 0) ? (c - static_cast<int32_t>(staged ? scols[j - 1] : cols[j - 1])) : 1000;
-                t = vote_map(wn, lb, sym_a, sym_b, live, gap);
-            }
-            else
-            {
-                uint8_t nsv[10]; // final colour of the queued pixels above (code 3: inside the image)
-#pragma unroll
-                for (int k = 0; k < 10; ++k)
-                {
-                    const int32_t hh = h + jcp_dh(k), ww = c + jcp_dw(k);
-                    nsv[k] = V_U;
-                    if (((codes >> (2 * k)) & 3ull) == 3ull)
-                        nsv[k] = ring ? fin[hh % 3][ww] : final_view(st[hh * W + ww]);
-                }
-                const bool live = fabsf(sum) > FLT_EPSILON;
-                uint8_t lb[24];
-                bool sym_a = false, sym_b = false;
-#pragma unroll
-                for (int k = 0; k < 24; ++k)
-                {
-                    const int32_t dh = jcp_dh(k), dw = jcp_dw(k);
-                    const int32_t hh = h + dh, ww = c + dw;
-                    if (hh < 0 || hh >= H || ww < 0 || ww >= W)
-                    {
-                        // stale slot: the raw weight an earlier pixel left there, over this sum
-                        float wv = 0.0F;
-                        lb[k] = V_U;
-                        if (live)
-                        {
-                            const int32_t qd = dw > 0 ? dw : 0;
-                            const int32_t q = (dw > 0 && hh >= 0 && hh < H) ? lastq[qd] : -1;
-                            if (q >= 0)
-                            {
-                                const float qw = b.jw[(static_cast<size_t>(r) * 3u + static_cast<uint32_t>(q + 3 - static_cast<int32_t>(m))) * kJwStride + k];
-                                wv = qw;
-                                if (qw != 0.0F)
-                                {
-                                    const uint8_t ns = st[hh * W + cols[q] + dw];
-                                    lb[k] = (dh < 0) ? final_view(ns) : pre_view(ns);
-                                }
-                            }
-                            else
-                            {
-                                wv = run_w[k];
-                                lb[k] = run_l[k];
-                            }
-                            wn[k] = wv / sum;
-                        }
-                        continue;
-                    }
-                    const uint32_t code = static_cast<uint32_t>((codes >> (2 * k)) & 3ull);
-                    if (code != 3u)
-                        lb[k] = static_cast<uint8_t>(code);
-                    else if (dh < 0)
-                        lb[k] = nsv[k < 10 ? k : 0];
-                    else
-                    {
-                        // same row, left of c, queued: symbolic (the chain's outcome)
-                        lb[k] = V_U;
-                        if (dw == -1)
-                            sym_a = true;
-                        else
-                            sym_b = true;
-                    }
-                }
-                const int32_t gap = (j > 0) ? (c - static_cast<int32_t>(staged ? scols[j - 1] : cols[j - 1])) : 1000;
-                t = vote_map(wn, lb, sym_a, sym_b, live, gap);
-            }
-            if (spread)
-                rmap[j] = t;
-            else
-                b.jmap[q0 + j] = t;
-            agg = (j == j0) ? t : map_compose(t, agg);
+                raw[q] = make_float4(wn[4 * q], wn[4 * q + 1], wn[4 * q + 2], wn[4 * q + 3]);
         }
-
-        // ---- block-wide exclusive scan of the thread aggregates (composition order) -----------
-        // only the warps holding pixels scan (the others' aggregates are the identity)
-        const uint32_t wused = ((m + chunk - 1) / chunk + 31u) / 32u;
-        unsigned long long incl = agg;
-        if (warp < wused)
+        if (mine)
+            t.sum[lane] = sum;
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t p1 = 0; p1 < cnt; ++p1)
         {
+            const float sp = t.sum[p1];
+            if (k < 24)
+                t.w[p1][k] = (fabsf(sp) > FLT_EPSILON) ? t.w[p1][k] / sp : 0.0F;
+        }
+        __syncwarp();
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const unsigned long long other = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= static_cast<uint32_t>(o))
-                    incl = map_compose(incl, other);
-            }
-        }
-        if (lane == 31)
-            wmaps[warp] = incl;
-        __syncthreads();
-        unsigned long long wpre = map_identity();
-        for (uint32_t w2 = 0; w2 < min(warp, wused); ++w2)
-            wpre = map_compose(wmaps[w2], wpre);
-        unsigned long long excl = __shfl_up_sync(0xffffffffu, incl, 1);
-        if (lane == 0)
-            excl = map_identity();
-        excl = map_compose(excl, wpre);
-        // state before this thread's chunk, starting from (unknown, unknown)
-        uint32_t state = static_cast<uint32_t>(excl & 0xfull);
-        for (uint32_t j = j0; j < j1; ++j)
+        for (int q = 0; q < 24; ++q)
+            wn[q] = t.w[p][q];
+        const uint32_t m0 = t.m0[p], m1 = t.m1[p];
+        const bool border = t.oob[p] != 0u;
+        uint32_t x = JST_OPEN;
+        if (!(fabsf(sum) > FLT_EPSILON))
+            x = V_U; // keeps the queue's colour
+        else if (!border)
+            x = vote_bounds(wn, m0, m1);
+        if (mine)
+            b.jst[sd.jq_off + q0 + lane] = static_cast<uint8_t>(x);
+        const bool open = mine && x == JST_OPEN;
+        const uint32_t om = __ballot_sync(0xffffffffu, open);
+        uint32_t slot = 0u;
+        if (om && lane == 0)
+            slot = atomicAdd(&b.state[s].n_open, static_cast<uint32_t>(__popc(om)));
+        slot = __shfl_sync(0xffffffffu, slot, 0) + static_cast<uint32_t>(__popc(om & ((1u << lane) - 1u)));
+        if (open)
         {
-            state = static_cast<uint32_t>(((spread ? rmap[j] : b.jmap[q0 + j]) >> (4 * state)) & 0xfull);
-            const uint32_t x = state / 3;
-            if (x != V_U)
-                st[h * W + cols[j]] = (x == V_O) ? PX_RES_O : PX_RES_G;
-            if (ring)
-                fin[h % 3][cols[j]] = static_cast<uint8_t>(x); // final_view of the new state
+            const uint32_t r = sd.jq_off + slot;
+#pragma unroll
+            for (uint32_t f = 0; f < 6; ++f)
+                jrec(b, f, r) = make_uint4(__float_as_uint(wn[4 * f]), __float_as_uint(wn[4 * f + 1]),
+                                           __float_as_uint(wn[4 * f + 2]), __float_as_uint(wn[4 * f + 3]));
+#pragma unroll
+            for (uint32_t f = 0; f < 3; ++f)
+                jrec(b, 6u + f, r) = make_uint4(t.dep[p][4 * f], t.dep[p][4 * f + 1], t.dep[p][4 * f + 2], t.dep[p][4 * f + 3]);
+            jrec(b, 9u, r) = make_uint4(m0, m1, q0 + lane, __float_as_uint(sum));
+            if (border)
+                b.jborder[sd.jq_off + atomicAdd(&b.state[s].n_border, 1u)] = slot;
         }
-        __syncthreads();
-
-        // ---- running stale values: last queued pixel of this row with the slot in bounds ------
-        if (upd_info != kJrowNoUpdate)
-        {
-            run_w[threadIdx.x] = upd_w;
-            uint8_t l = static_cast<uint8_t>(upd_info);
-            if (upd_info & kJrowDynamic)
-            {
-                const uint32_t addr = upd_info & ~kJrowDynamic; // a queued pixel of rows h-2..h
-                l = ring ? fin[(addr / static_cast<uint32_t>(W)) % 3u][addr % static_cast<uint32_t>(W)]
-                         : final_view(st[addr]);
-            }
-            run_l[threadIdx.x] = l;
-        }
-        // no barrier here: the next row's first barrier orders these writes before its readers
-        cur ^= 1;
+        __syncwarp(); // the tile is read before the next turn fills it
     }
+}
+
+// What the reference's weight and label buffer holds for slot k (dh, dw) of a pixel of row h whose
+// slot lies outside the image (segmenter.cpp:552-556): the values of the last earlier queued pixel
+// with that slot inside. Right of the image that can be a pixel of the same row (columns up to
+// W - 1 - dw); otherwise it lies in the nearest earlier row that has one. Among a row's queued pixels
+// it is one of the last three (at most two columns lie beyond W - 1 - dw).
+__device__ __forceinline__ bool stale_slot(const BatchDev& b, const ScanDev& sd, int k, int32_t h, float& w, uint32_t& code,
+                                           uint32_t& dep)
+{
+    const int32_t dh = jcp_dh(k), dw = jcp_dw(k);
+    const int32_t H = sd.H, W = sd.W;
+    const uint8_t* st = b.pix_state + sd.pix_off;
+    w = 0.0F;
+    code = V_U;
+    dep = 0u;
+    for (int32_t r = (dw > 0 && h + dh >= 0 && h + dh < H) ? h : h - 1; r >= 0; --r)
+    {
+        const int32_t m = static_cast<int32_t>(b.row_cnt[sd.row_off + static_cast<uint32_t>(r)]);
+        const int32_t hh = r + dh;
+        if (m == 0 || hh < 0 || hh >= H)
+            continue;
+        const uint16_t* cols = b.row_cols + sd.pix_off + static_cast<uint32_t>(r * W);
+        const int32_t lim = W - 1 - (dw > 0 ? dw : 0);
+        int32_t j = m - 1;
+        while (j >= 0 && j >= m - 3 && static_cast<int32_t>(cols[j]) > lim)
+            --j;
+        if (j < 0 || j < m - 3 || static_cast<int32_t>(cols[j]) + dw < 0)
+            continue; // no queued pixel of this row has the slot inside
+        w = b.jw[(static_cast<size_t>(sd.row_off + static_cast<uint32_t>(r)) * 3u + static_cast<uint32_t>(j + 3 - m)) * kJwStride + k];
+        if (w != 0.0F)
+        {
+            const uint32_t addr = static_cast<uint32_t>(hh * W + static_cast<int32_t>(cols[j]) + dw);
+            if (k < 12 && st[addr] == PX_INTERSECT)
+            {
+                code = 3u; // that pixel's outcome
+                dep = b.pix_depth[sd.pix_off + addr];
+            }
+            else
+                code = pre_view(st[addr]);
+        }
+        return true;
+    }
+    return false;
+}
+
+// The open pixels of a scan, one cluster of kCtas CTAs each: the border pixels' stale slots
+// first, then (more open pixels than threads only) rounds over the list, then every thread watches
+// its own pixel's open neighbours and repeats the test when one is decided. Each CTA keeps every
+// queued pixel's state in its shared memory and a decision is written into all of them, so
+// watching costs local reads only (scans of more than `cap` queued pixels watch global memory).
+// Bound by the chain of hops, about 700 cycles each. Chains of pixels of one row, each hanging on the
+// one to its left, would make 60 hops on a 64 x 2048 scan and 130 on a 32 x 4096 one: where the
+// bounds show that one open neighbour alone decides (it on ground: ground, it on obstacle: obstacle,
+// whatever the others become), the pixel becomes a copy of that neighbour, and copies of copies
+// skip ahead, so the hops of a chain grow with its logarithm (15 and 29 hops).
+// Several CTAs because a hop's price grows with the warps that share an SM, and because the rounds
+// read 160 bytes per open pixel. 8 for launches of up to kResolveWide scans (28 us on a 64 x 2048
+// scan, 68 us on six mixed ones; 4 CTAs: 31 and 107 us; one CTA without copies: 102 and 417 us; the
+// row-by-row kernel: 126 and 182 us), 4 for more, whose clusters take the SMs from the other parts of a
+// split batch (64-scan batch, eight parts: 1.92 ms against 1.97 ms with 8).
+constexpr uint32_t kResolveThreads = 512;
+constexpr uint32_t kResolveStates = 24u * 1024u; // queued pixels whose states fit shared memory (4 bytes each)
+constexpr int kResolveWide = 7;           // scans of a launch up to which a scan takes 8 CTAs
+constexpr uint32_t kResolveSpins = 1u << 20; // polls of a pixel's neighbours before giving up
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of this CTA's shared variable p in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t peer_smem(const void* p, uint32_t rank)
+{
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+    return a;
+}
+
+__device__ __forceinline__ uint32_t jrec_load(const BatchDev& b, uint32_t r, float* wn, uint32_t* dep, uint32_t& m0, uint32_t& m1)
+{
+#pragma unroll
+    for (uint32_t f = 0; f < 6; ++f)
+    {
+        const uint4 v = jrec(b, f, r);
+        wn[4 * f] = __uint_as_float(v.x);
+        wn[4 * f + 1] = __uint_as_float(v.y);
+        wn[4 * f + 2] = __uint_as_float(v.z);
+        wn[4 * f + 3] = __uint_as_float(v.w);
+    }
+#pragma unroll
+    for (uint32_t f = 0; f < 3; ++f)
+    {
+        const uint4 v = jrec(b, 6u + f, r);
+        dep[4 * f] = v.x;
+        dep[4 * f + 1] = v.y;
+        dep[4 * f + 2] = v.z;
+        dep[4 * f + 3] = v.w;
+    }
+    const uint4 v = jrec(b, 9u, r);
+    m0 = v.x;
+    m1 = v.y;
+    return v.z;
+}
+
+// An entry in shared memory: the state in the lower half (label bit 0 at bit 0, label bit 1 at bit
+// 12, so that twelve of them shift and add into the two label masks of slots 0-11), in the upper half
+// the queue index + 1 of the pixel it copies. The last three entries are the labels themselves, for
+// the slots that are not open.
+__device__ __forceinline__ uint32_t wide_state(uint32_t v)
+{
+    return (v & 1u) | ((v >> 1) << 12);
+}
+
+template <uint32_t kCtas>
+__global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads) k_jcp_resolve(BatchDev b, uint32_t cap)
+{
+    constexpr uint32_t kAll = kResolveThreads * kCtas;
+    extern __shared__ __align__(16) uint32_t sst[]; // cap + 4 entries
+    __shared__ uint32_t s_n[2]; // pixels left open by a round (of the cluster's first CTA), alternating
+    const int s = static_cast<int>(blockIdx.x / kCtas);
+    const uint32_t rank = blockIdx.x % kCtas;
+    const ScanDev& sd = b.scans[s];
+    const uint32_t nq = b.state[s].n_queue, nopen = b.state[s].n_open, nborder = b.state[s].n_border;
+    if (nopen == 0u)
+        return;
+    const uint32_t tid = threadIdx.x, lane = lane_id();
+    const uint32_t warp = (tid >> 5) * kCtas + rank; // warp and thread of the cluster: neighbouring
+    const uint32_t all = warp * 32u + lane;                 // warps on different SMs
+    uint8_t* gst = b.jst + sd.jq_off;
+    const bool local = nq <= cap;
+    if (local)
+    {
+        for (uint32_t i = tid; i < (nq + 3u) / 4u; i += kResolveThreads) // jq_off is a multiple of 16, the array padded
+        {
+            const uint32_t v = reinterpret_cast<const uint32_t*>(gst)[i];
+            reinterpret_cast<uint4*>(sst)[i] = make_uint4(wide_state(v & 3u), wide_state((v >> 8) & 3u),
+                                                          wide_state((v >> 16) & 3u), wide_state((v >> 24) & 3u));
+        }
+        if (tid < 3u)
+            sst[cap + tid] = wide_state(tid);
+    }
+    for (uint32_t i = warp; i < nborder; i += kAll / 32u)
+    {
+        const uint32_t r = sd.jq_off + b.jborder[sd.jq_off + i];
+        const uint4 rec = jrec(b, 9u, r);
+        const uint4 e = b.jq[sd.jq_off + rec.z];
+        const int k = static_cast<int>(lane);
+        const int32_t h = static_cast<int32_t>(e.x - sd.row_off), hh = h + jcp_dh(k);
+        const int32_t ww = static_cast<int32_t>(e.y >> 16) + jcp_dw(k);
+        const bool oob = k < 24 && !(hh >= 0 && hh < sd.H && ww >= 0 && ww < sd.W);
+        uint32_t code = ((rec.x >> k) & 1u) | (((rec.y >> k) & 1u) << 1);
+        if (oob)
+        {
+            float w;
+            uint32_t dep;
+            stale_slot(b, sd, k, h, w, code, dep);
+            reinterpret_cast<float*>(&jrec(b, static_cast<uint32_t>(k) / 4u, r))[k & 3] = w / __uint_as_float(rec.w);
+            if (k < 12)
+                reinterpret_cast<uint32_t*>(&jrec(b, 6u + static_cast<uint32_t>(k) / 4u, r))[k & 3] =
+                    (code == 3u) ? dep : kDepFixed | code;
+        }
+        const uint32_t m0 = __ballot_sync(0xffffffffu, code & 1u), m1 = __ballot_sync(0xffffffffu, code & 2u);
+        if (lane == 0)
+            jrec(b, 9u, r) = make_uint4(m0, m1, rec.z, rec.w);
+    }
+    if (tid < 2u)
+        s_n[tid] = 0u;
+    __threadfence();
+    cluster_barrier();
+    const uint32_t n_addr[2] = {peer_smem(&s_n[0], 0u), peer_smem(&s_n[1], 0u)};
+    uint32_t peer[kCtas];
+#pragma unroll
+    for (uint32_t c = 0; c < kCtas; ++c)
+        peer[c] = peer_smem(sst, c);
+    const uint32_t own = smem_addr(sst);
+    auto tell = [&](uint32_t at, uint32_t v) { // 16 bits at byte offset `at` of every CTA's entries
+#pragma unroll
+        for (uint32_t c = 0; c < kCtas; ++c)
+            asm volatile("st.volatile.shared::cluster.u16 [%0], %1;" ::"r"(peer[c] + at), "h"(static_cast<uint16_t>(v)) : "memory");
+    };
+    auto watch = [&](uint32_t addr) -> uint32_t {
+        uint16_t v;
+        asm volatile("ld.volatile.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+        return v;
+    };
+    auto decide = [&](uint32_t q, uint32_t x) {
+        if (local)
+            tell(4u * q, wide_state(x));
+        else
+            *(reinterpret_cast<volatile uint8_t*>(gst) + q) = static_cast<uint8_t>(x);
+    };
+    // dep[0..11] (record fields 6-8) as what `labels` reads: shared-memory addresses, or indices
+    auto locate = [&](uint32_t* dep) {
+#pragma unroll
+        for (int k = 0; k < 12; ++k)
+            if (local)
+                dep[k] = own + 4u * ((dep[k] & kDepFixed) ? cap + (dep[k] & 3u) : dep[k]);
+    };
+    // the labels of slots 0-11 now: bit 0 of each in bits 0-11, bit 1 in bits 12-23
+    auto labels = [&](const uint32_t* dep) {
+        uint32_t acc = 0u;
+        if (local)
+        {
+#pragma unroll
+            for (int k = 0; k < 12; ++k)
+                acc += watch(dep[k]) << k;
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < 12; ++k)
+                acc += wide_state((dep[k] & kDepFixed) ? dep[k] & 3u
+                                                       : *(reinterpret_cast<volatile uint8_t*>(gst) + dep[k])) << k;
+        }
+        return acc;
+    };
+    auto vote = [&](const float* wn, uint32_t acc, uint32_t m0, uint32_t m1) {
+        return vote_bounds(wn, (m0 & 0xfff000u) | (acc & 0xfffu), (m1 & 0xfff000u) | (acc >> 12));
+    };
+    float wn[24];
+    uint32_t dep[12], m0, m1;
+    uint32_t n = nopen;
+    uint32_t *cur = nullptr, *next = b.jlist + sd.jq_off, *other = b.jlist + b.jq_total + sd.jq_off; // null: all positions
+    for (uint32_t round = 0; n > kAll; ++round)
+    {
+        const uint32_t cnt = n_addr[round & 1u];
+        for (uint32_t t0 = warp * 32u; t0 < n; t0 += kAll)
+        {
+            const uint32_t t = t0 + lane;
+            bool open = false;
+            uint32_t at = 0u;
+            if (t < n)
+            {
+                at = cur ? __ldcg(&cur[t]) : t;
+                const uint32_t q = jrec_load(b, sd.jq_off + at, wn, dep, m0, m1);
+                locate(dep);
+                const uint32_t x = vote(wn, labels(dep), m0, m1);
+                open = x == JST_OPEN;
+                if (!open)
+                {
+                    decide(q, x);
+                    gst[q] = static_cast<uint8_t>(x);
+                }
+            }
+            const uint32_t mask = __ballot_sync(0xffffffffu, open);
+            uint32_t base = 0u;
+            if (lane == 0 && mask)
+                asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(base) : "r"(cnt), "r"(__popc(mask)) : "memory");
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (open)
+                next[base + static_cast<uint32_t>(__popc(mask & ((1u << lane) - 1u)))] = at;
+        }
+        __threadfence();
+        cluster_barrier();
+        uint32_t left;
+        asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(left) : "r"(cnt) : "memory");
+        if (all == 0u)
+            s_n[(round & 1u) ^ 1u] = 0u; // the next round's count (its last readers passed the barrier above)
+        cluster_barrier();
+        if (left >= n)
+        {
+            if (all == 0u)
+                raise_err(&b.state[s], ERR_INTERNAL); // (the first open pixel in order is always decided)
+            n = 0u; // (every thread of the cluster alike)
+            break;
+        }
+        n = left;
+        cur = next;
+        next = other;
+        other = cur;
+    }
+    if (all < n)
+    {
+        const uint32_t q = jrec_load(b, sd.jq_off + (cur ? __ldcg(&cur[all]) : all), wn, dep, m0, m1);
+        locate(dep);
+        uint32_t x = JST_OPEN, seen = 0xffffffffu, copied = 0u; // copied: the entry this pixel copies
+        for (uint32_t spin = 0; x == JST_OPEN && spin < kResolveSpins; ++spin)
+        {
+            if (copied != 0u)
+            {
+                const uint32_t v = watch(copied), further = watch(copied + 2u);
+                if (v != wide_state(JST_OPEN))
+                    x = (v & 1u) ? V_G : V_O;
+                else if (further != 0u)
+                {
+                    copied = own + 4u * (further - 1u);
+                    tell(4u * q + 2u, further);
+                }
+            }
+            else
+            {
+                const uint32_t acc = labels(dep);
+                if (acc == seen)
+                    continue;
+                seen = acc;
+                x = vote(wn, acc, m0, m1);
+                if (x == JST_OPEN && local)
+                {
+                    // the heaviest open neighbour: does it decide alone?
+                    float w = -1.0F;
+                    uint32_t at = 0u, bit = 0u;
+#pragma unroll
+                    for (int k = 0; k < 12; ++k)
+                        if (((acc >> k) & (acc >> (k + 12)) & 1u) && wn[k] > w)
+                        {
+                            w = wn[k];
+                            at = dep[k];
+                            bit = 1u << k;
+                        }
+                    if (bit != 0u && vote(wn, acc & ~(bit << 12), m0, m1) == V_G && vote(wn, acc & ~bit, m0, m1) == V_O)
+                    {
+                        copied = at;
+                        tell(4u * q + 2u, (at - own) / 4u + 1u);
+                    }
+                }
+            }
+            if (x != JST_OPEN)
+                decide(q, x);
+        }
+        gst[q] = static_cast<uint8_t>(x);
+        if (x == JST_OPEN)
+            raise_err(&b.state[s], ERR_INTERNAL);
+    }
+    __syncwarp();
+    cluster_barrier(); // no CTA leaves while another may still write its states
 }
 
 // populateLabels (segmenter.cpp:640-669) and the colour image of Segmenter::image().
@@ -1804,11 +1800,16 @@ __global__ void k_populate(BatchDev b, uint8_t* image)
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= b.npix)
         return;
-    const uint8_t stv = b.pix_state[p];
+    uint8_t stv = b.pix_state[p];
     const int32_t li = b.pix_map[p];
     if (li >= 0)
     {
         const int s = scan_of_pix(b, p);
+        if (stv == PX_INTERSECT)
+        {
+            const uint8_t v = b.jst[b.scans[s].jq_off + b.pix_depth[p]];
+            stv = (v == V_O) ? PX_RES_O : ((v == V_G) ? PX_RES_G : PX_INTERSECT);
+        }
         const uint8_t v = final_view(stv);
         if (v != V_U)
             b.seg_label[b.scans[s].pt_off + static_cast<uint32_t>(li)] = (v == V_G) ? LP_LABEL_GROUND : LP_LABEL_OBSTACLE;
@@ -1898,8 +1899,10 @@ void init_segment_tables()
     uint32_t table[kMtTable];
     for (int k = 0; k < kMtTable; ++k)
         table[k] = static_cast<uint32_t>(gen());
-    const bool attr = cudaFuncSetAttribute(k_jcp_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(2u * kStageBytes)) == cudaSuccess;
+    const bool attr = cudaFuncSetAttribute(k_jcp_resolve<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           static_cast<int>(4u * kResolveStates + 16u)) == cudaSuccess &&
+                      cudaFuncSetAttribute(k_jcp_resolve<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           static_cast<int>(4u * kResolveStates + 16u)) == cudaSuccess;
     if (cudaMemcpyToSymbol(g_mt42, table, sizeof(table)) == cudaSuccess && attr && dev >= 0 && dev < 64)
         done[dev] = true;
 }
@@ -2011,9 +2014,15 @@ void launch_segmentation(Launcher& L, const BatchDev& b, const BatchHost& hb, ui
     LP_LAUNCH(L, k_project_key, div_up(b.npts, T), T, b);
     LP_LAUNCH(L, k_pixel, div_up(b.npix, T), T, b);
     LP_LAUNCH(L, k_dilate_rows, b.nrows, 256, b);
-    LP_LAUNCH(L, k_jcp_weights, static_cast<uint32_t>(sm_count()) * hb.jcp_ctas_per_sm, 256, b);
-    LP_LAUNCH(L, k_jcp_rowrec, div_up(b.nrows * 32u, 256u), 256, b);
-    LP_LAUNCH_SMEM(L, k_jcp_rows, static_cast<uint32_t>(b.nscan), 256, 2u * kStageBytes, b);
+    LP_LAUNCH(L, k_jcp_weights, static_cast<uint32_t>(sm_count()) * hb.jcp_ctas_per_sm, kWeightThreads, b);
+    uint32_t cap = 16u; // the queue holds at most the scan's pixels and points
+    for (const ScanDev& sd : hb.scans)
+        cap = std::max(cap, std::min((sd.jq_cap + 15u) & ~15u, kResolveStates));
+    const uint32_t ns = static_cast<uint32_t>(b.nscan);
+    if (b.nscan <= kResolveWide)
+        L.launch_smem("k_jcp_resolve", k_jcp_resolve<8>, ns * 8u, kResolveThreads, 4u * cap + 16u, b, cap);
+    else
+        L.launch_smem("k_jcp_resolve", k_jcp_resolve<4>, ns * 4u, kResolveThreads, 4u * cap + 16u, b, cap);
     LP_LAUNCH(L, k_populate, div_up(b.npix, T), T, b, d_image);
 }
 } // namespace lpg
