@@ -227,11 +227,11 @@ size_t carve(lp_batch& B, char* base)
     ScanDev* scans;
     put(scans, S);
     b.scans = scans;
-    put(b.state, S);
     put(b.io, S);
-    put(b.io_ret, S);
+    put(b.state, S);
     const uint32_t maxlen = std::max({N, b.npix, b.nhash, b.ncell, b.ncl, b.ntiles, b.nnear}) + 2;
-    put(B.scan_sums, div_up(maxlen, static_cast<uint32_t>(kScanTile)) + 4);
+    B.scan_words = static_cast<size_t>(kScansPerRun) * scan_words(maxlen);
+    put(B.scan_sums, 2 * B.scan_words);
     float4* src;
     put(src, N);
     b.src = src;
@@ -243,7 +243,11 @@ size_t carve(lp_batch& B, char* base)
         b.ring_in = r;
     }
     put(b.noise, N);
-    put(b.ring, N);
+    // rings as given are read where they arrive; compacted or computed ones need their own array
+    if (ring_in && !noise && !B.hb.any_compute_ring)
+        b.ring = const_cast<uint16_t*>(b.ring_in);
+    else
+        put(b.ring, N);
     if (noise)
     {
         put(b.src_pos, N + 1);
@@ -431,74 +435,78 @@ lp_status upload(lp_context* ctx, lp_batch& B)
     return LP_OK;
 }
 
-// The whole launch sequence of a batch (memsets + kernels), no host synchronisation.
-lp_status execute(lp_context* ctx, lp_batch& B)
+// The whole launch sequence of a batch, no host synchronisation. outputs: the labels per input point
+// in out_seg / out_cl (the direct output kernels do without).
+lp_status execute(lp_context* ctx, lp_batch& B, bool outputs)
 {
     BatchDev& b = B.b;
     const Run& R = B.run;
-    const cudaStream_t st = B.stream ? B.stream : ctx->stream;
     Launcher L;
-    L.stream = st;
+    L.stream = B.stream ? B.stream : ctx->stream;
     L.launches = &ctx->launches;
     L.scan_sums = B.scan_sums;
+    L.scan_left = B.scan_words;
     L.scan_err = &b.state->err; // scan 0's error word: a failed scan fails the batch
     L.event_pool = &ctx->events;
     if (B.profiling)
         L.prof = &B.prof;
-    const uint32_t N = b.npts, S = static_cast<uint32_t>(b.nscan);
-    LP_CUDA(ctx, cudaMemsetAsync(b.state, 0, S * sizeof(ScanState), st));
-    LP_CUDA(ctx, cudaMemsetAsync(b.seg_label, 0, static_cast<size_t>(N) * 4, st));
-    LP_CUDA(ctx, cudaMemsetAsync(b.out_seg, 0, static_cast<size_t>(N) * 4, st));
-    LP_CUDA(ctx, cudaMemsetAsync(b.out_cl, 0xff, static_cast<size_t>(N) * 4, st));
-    const bool noise = R.stages & ST_NOISE;
-    if (!noise)
-        LP_CUDA(ctx, cudaMemsetAsync(b.noise, 0, N, st));
-    if (b.ring_in && !noise)
-        LP_CUDA(ctx, cudaMemcpyAsync(b.ring, b.ring_in, static_cast<size_t>(N) * 2, cudaMemcpyDeviceToDevice, st));
-    launch_state_init(L, b, noise ? 1 : 0);
+    const size_t N = b.npts;
+    const bool noise = R.stages & ST_NOISE, clu = R.stages & (ST_CLUSTER | ST_ALL_OBS);
+    FillList f;
+    f.add(B.scan_sums, B.scan_words * 8, 0u);
+    if (outputs && noise)
+    {
+        f.add(b.out_seg, N * 4, 0u);
+        f.add(b.out_cl, N * 4, 0xffffffffu);
+    }
+    if (outputs && !noise)
+        f.add(b.noise, N, 0u);
+    if (R.stages & (ST_RING | ST_SEG))
+        f.add(b.tile_cnt, (static_cast<size_t>(b.ntiles) + 1) * 4, 0u);
+    if (R.stages & ST_SEG)
+    {
+        f.add(b.seg_label, N * 4, 0u);
+        f.add(b.cell_cnt, (static_cast<size_t>(b.ncell) + 1) * 4, 0u);
+        f.add(b.n_large, 4, 0u);
+        f.add(b.near_cnt, (static_cast<size_t>(b.nnear) + 1) * 4, 0u);
+        f.add(b.pix_depth, static_cast<size_t>(b.npix) * 4, 0xffffffffu);
+        f.add(b.pix_key, static_cast<size_t>(b.npix) * 8, 0xffffffffu);
+        f.add(b.row_cnt, static_cast<size_t>(b.nrows) * 4, 0u);
+    }
+    if (clu)
+    {
+        f.add(b.hkey, static_cast<size_t>(b.nhash) * 4, 0xffffffffu);
+        f.add(b.hmin, static_cast<size_t>(b.nhash) * 4, 0xffffffffu);
+        f.add(b.hcnt, static_cast<size_t>(b.nhash) * 4, 0u);
+        f.add(b.kflag, (N + 1) * 4, 0u);
+        f.add(b.cl_cnt, (static_cast<size_t>(b.ncl) + 1) * 4, 0u);
+        f.add(b.cl_fill, (static_cast<size_t>(b.ncl) + 1) * 4, 0u);
+        f.add(b.cl_zkey, static_cast<size_t>(b.ncl) * 8, 0u);
+    }
+    if (R.stages & ST_HULL)
+    {
+        f.add(b.hull_cnt, (static_cast<size_t>(b.ncl) + 1) * 4, 0u);
+        f.add(b.queue, 8 * 4, 0u);
+    }
+    launch_prepare(L, f, b, noise ? 1 : 0);
     if (noise)
     {
         launch_noise(L, b, B.hb, R.nr);
         if (R.stages & (ST_SEG | ST_CLUSTER | ST_ALL_OBS | ST_RING))
             launch_noise_compaction(L, b, B.hb);
     }
-    if (R.stages & (ST_RING | ST_SEG))
-    {
-        LP_CUDA(ctx, cudaMemsetAsync(b.tile_cnt, 0, (static_cast<size_t>(b.ntiles) + 1) * 4, st));
-    }
     if ((R.stages & ST_RING) && !(R.stages & ST_SEG))
         launch_ring_only(L, b, B.hb);
     if (R.stages & ST_SEG)
-    {
-        LP_CUDA(ctx, cudaMemsetAsync(b.cell_cnt, 0, (static_cast<size_t>(b.ncell) + 1) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.n_large, 0, 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.near_cnt, 0, (static_cast<size_t>(b.nnear) + 1) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.pix_depth, 0xff, static_cast<size_t>(b.npix) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.pix_key, 0xff, static_cast<size_t>(b.npix) * 8, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.row_cnt, 0, static_cast<size_t>(b.nrows) * 4, st));
         launch_segmentation(L, b, B.hb, B.d_image);
-    }
     if (R.stages & ST_ALL_OBS)
         launch_mark_all_obstacles(L, b);
-    if (R.stages & (ST_CLUSTER | ST_ALL_OBS))
-    {
-        LP_CUDA(ctx, cudaMemsetAsync(b.hkey, 0xff, static_cast<size_t>(b.nhash) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.hmin, 0xff, static_cast<size_t>(b.nhash) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.hcnt, 0, static_cast<size_t>(b.nhash) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.kflag, 0, (static_cast<size_t>(N) + 1) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.cl_cnt, 0, (static_cast<size_t>(b.ncl) + 1) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.cl_fill, 0, (static_cast<size_t>(b.ncl) + 1) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.cl_zkey, 0, static_cast<size_t>(b.ncl) * 8, st));
+    if (clu)
         launch_clustering(L, b, B.hb);
-    }
     if (R.stages & ST_HULL)
-    {
-        LP_CUDA(ctx, cudaMemsetAsync(b.hull_cnt, 0, (static_cast<size_t>(b.ncl) + 1) * 4, st));
-        LP_CUDA(ctx, cudaMemsetAsync(b.queue, 0, 8 * 4, st));
         launch_polygons(L, b, B.hb, (R.stages & ST_OBB) ? 1 : 0);
-    }
-    if (R.stages & (ST_SEG | ST_CLUSTER | ST_ALL_OBS))
-        launch_outputs(L, b, (R.stages & (ST_CLUSTER | ST_ALL_OBS)) ? 1 : 0);
+    if (outputs && (R.stages & (ST_SEG | ST_CLUSTER | ST_ALL_OBS)))
+        launch_outputs(L, b, clu ? 1 : 0);
     if (L.err != cudaSuccess)
         return cuda_fail(ctx, L.err, "kernel launch");
     return LP_OK;
@@ -568,6 +576,8 @@ void destroy_batch(lp_batch* B)
         cudaGraphExecDestroy(B->graph);
     if (B->mem)
         cudaFree(B->mem);
+    if (B->h_stage)
+        cudaFreeHost(B->h_stage);
     for (lp_batch* P : B->parts)
         destroy_batch(P);
     for (cudaEvent_t e : B->fork_join)
@@ -725,24 +735,29 @@ namespace lprt
 std::mutex g_pin_mu;
 std::map<uintptr_t, size_t> g_pinned;
 
-bool pinned_range(const void* p, size_t bytes)
-{
-    if (!p)
-        return true;
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    std::lock_guard<std::mutex> lk(g_pin_mu);
-    auto it = g_pinned.upper_bound(a);
-    if (it == g_pinned.begin())
-        return false;
-    --it;
-    return a + bytes <= it->first + it->second;
-}
-
 // Direct host I/O applies when every buffer of the call lies in lp_host_alloc memory (inputs as
-// XYZI); the GPU then reads and writes them itself over the coherent host link.
-bool direct_io_ok(const lp_batch& B, const lp_scan_input* scans, const lp_scan_output* outs)
+// XYZI); the GPU then reads and writes them itself over the coherent host link. One lock per call; a
+// caller's arrays mostly share an allocation, so the last one found is looked at first.
+bool direct_io_ok(const lp_batch& B, const lp_scan_output* outs)
 {
     const bool hull = B.run.stages & ST_HULL, obb = B.run.stages & ST_OBB;
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    uintptr_t lo = 1, hi = 0; // the last allocation found
+    auto pinned_range = [&](const void* p, size_t bytes) {
+        if (!p)
+            return true;
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+        if (a < lo || a >= hi)
+        {
+            auto it = g_pinned.upper_bound(a);
+            if (it == g_pinned.begin())
+                return false;
+            --it;
+            lo = it->first;
+            hi = it->first + it->second;
+        }
+        return a + bytes <= hi;
+    };
     for (size_t s = 0; s < B.run.scans.size(); ++s)
     {
         const ScanIn& in = B.run.scans[s];
@@ -764,8 +779,22 @@ bool direct_io_ok(const lp_batch& B, const lp_scan_input* scans, const lp_scan_o
                 return false;
         }
     }
-    (void)scans;
     return true;
+}
+
+// Page-locked host memory of the batch for the direct path, at least `bytes`; the batch's stream is idle
+// (every direct call waits for its end).
+lp_status host_stage(lp_context* ctx, lp_batch& B, size_t bytes)
+{
+    if (bytes <= B.h_stage_cap)
+        return LP_OK;
+    if (B.h_stage)
+        cudaFreeHost(B.h_stage);
+    B.h_stage = nullptr;
+    B.h_stage_cap = 0;
+    LP_CUDA(ctx, cudaMallocHost(reinterpret_cast<void**>(&B.h_stage), bytes));
+    B.h_stage_cap = bytes;
+    return LP_OK;
 }
 
 // Launches of the direct host I/O path on the batch's stream: inputs gathered from the caller's
@@ -777,7 +806,15 @@ lp_status direct_launch(lp_context* ctx, lp_batch& B, lp_scan_output* outs)
     const cudaStream_t st = B.stream ? B.stream : ctx->stream;
     const size_t S = B.run.scans.size();
     const bool hull = B.run.stages & ST_HULL, obb = B.run.stages & ST_OBB;
-    std::vector<IoScan> io(S);
+    // page-locked: the scans' descriptors and buffers as they lie on the device (one copy), then the
+    // states and hull index counts that the output kernels write back
+    const size_t io_at = static_cast<size_t>(reinterpret_cast<const char*>(b.io) - reinterpret_cast<const char*>(b.scans));
+    const size_t in_bytes = (io_at + S * sizeof(IoScan) + 255) & ~static_cast<size_t>(255);
+    LP_TRY(host_stage(ctx, B, in_bytes + S * (sizeof(ScanState) + 4)));
+    std::memcpy(B.h_stage, B.hb.scans.data(), S * sizeof(ScanDev));
+    IoScan* io = reinterpret_cast<IoScan*>(B.h_stage + io_at);
+    B.h_ret = B.h_stage + in_bytes;
+    ScanState* h_state = reinterpret_cast<ScanState*>(B.h_ret);
     uint32_t nq = 0; // 4-point chunks of the batch
     auto aligned = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
     for (size_t s = 0; s < S; ++s)
@@ -792,36 +829,30 @@ lp_status direct_launch(lp_context* ctx, lp_batch& B, lp_scan_output* outs)
                        o.cluster_capacity, o.hull_capacity, nq, vec};
         nq += (in.n + 3u) / 4u;
     }
-    LP_CUDA(ctx, cudaMemcpyAsync(const_cast<ScanDev*>(b.scans), B.hb.scans.data(), S * sizeof(ScanDev),
-                                 cudaMemcpyHostToDevice, st));
-    LP_CUDA(ctx, cudaMemcpyAsync(b.io, io.data(), S * sizeof(IoScan), cudaMemcpyHostToDevice, st));
+    LP_CUDA(ctx, cudaMemcpyAsync(const_cast<ScanDev*>(b.scans), B.h_stage, io_at + S * sizeof(IoScan), cudaMemcpyHostToDevice, st));
     Launcher L;
     L.stream = st;
     L.launches = &ctx->launches;
     launch_io_in(L, b, b.io);
     if (L.err != cudaSuccess)
         return cuda_fail(ctx, L.err, "direct input launch");
-    LP_TRY(execute(ctx, B));
-    launch_io_out(L, b, b.io, b.io_ret, hull ? 1 : 0, obb ? 1 : 0, nq);
+    LP_TRY(execute(ctx, B, false));
+    launch_io_out(L, b, b.io, reinterpret_cast<uint32_t*>(h_state + S), h_state, hull ? 1 : 0, obb ? 1 : 0, nq);
     if (L.err != cudaSuccess)
         return cuda_fail(ctx, L.err, "direct output launch");
     return LP_OK;
 }
 
-// Reads the scans' states back (a copy into pageable memory waits for the batch's stream, so it is
-// issued only here, after every part of a split call has been launched) and reports every scan's
-// status and counts in outs.
+// Waits for the batch's stream (after every part of a split call has been launched) and reports every
+// scan's status and counts, which the output kernels left in page-locked memory, in outs.
 lp_status direct_finish(lp_context* ctx, lp_batch& B, lp_scan_output* outs)
 {
     const cudaStream_t st = B.stream ? B.stream : ctx->stream;
     const size_t S = B.run.scans.size();
     const bool hull = B.run.stages & ST_HULL;
-    B.h_nh.assign(S, 0u);
-    const std::vector<uint32_t>& nh = B.h_nh;
-    LP_CUDA(ctx, cudaMemcpyAsync(B.h_state.data(), B.b.state, S * sizeof(ScanState), cudaMemcpyDeviceToHost, st));
-    if (hull)
-        LP_CUDA(ctx, cudaMemcpyAsync(B.h_nh.data(), B.b.io_ret, S * 4, cudaMemcpyDeviceToHost, st));
     LP_CUDA(ctx, cudaStreamSynchronize(st));
+    std::memcpy(B.h_state.data(), B.h_ret, S * sizeof(ScanState));
+    const uint32_t* nh = reinterpret_cast<const uint32_t*>(B.h_ret + S * sizeof(ScanState));
     lp_status worst = report_state(ctx, B);
     if (worst != LP_OK && worst != LP_ERR_CAPACITY)
         return worst;
@@ -1673,7 +1704,7 @@ lp_status lp_process_batch(lp_context* ctx, const lp_pipeline_config* cfg, const
     LP_TRY(fill_pipeline(ctx, B, cfg, scans, nscans));
     const lp_tuning tune = tuning_for(ctx, scans, nscans);
     B.tune = tune;
-    if (direct_io_ok(B, scans, outs))
+    if (direct_io_ok(B, outs))
     {
         const uint32_t K = part_count(tune, nscans);
         return K > 1 ? run_direct_split(ctx, cfg, scans, outs, nscans, tune, K) : run_direct(ctx, B, outs);

@@ -77,7 +77,6 @@ struct BatchDev
     uint16_t* ring;           // per compacted point
     const uint16_t* ring_in;  // per input point, or null
     IoScan* io;               // per scan: the caller's page-locked buffers (direct host I/O)
-    uint32_t* io_ret;         // per scan: hull index count written by the direct output kernel
 
     // ---- ring partition ---------------------------------------------------------------------
     uint8_t* quad;            // per point quadrant

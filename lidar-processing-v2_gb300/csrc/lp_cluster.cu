@@ -542,11 +542,14 @@ void launch_clustering(Launcher& L, const BatchDev& b, const BatchHost& hb)
     LP_LAUNCH(L, k_obs_gather, div_up(b.npts, kObsChunk), 256, b);
     LP_LAUNCH(L, k_dims, div_up(ns, 64u), 64, b);
     LP_LAUNCH(L, k_vox_insert, div_up(b.npts, T), T, b);
-    L.begin("k_vox_ids");
-    scan_lookback(L.stream, VoxFlagsSrc{b.hkey, b.nhash}, VoxInitDst{b.hvid, b.vslot, b.parent, b.cmin, b.ccnt, b.nhash + 1},
-                  b.nhash + 1, L.scan_sums, L.scan_err);
-    L.end();
-    L.note();
+    if (uint32_t* words = L.scan_state(b.nhash + 1))
+    {
+        L.begin("k_vox_ids");
+        scan_lookback(L.stream, VoxFlagsSrc{b.hkey, b.nhash},
+                      VoxInitDst{b.hvid, b.vslot, b.parent, b.cmin, b.ccnt, b.nhash + 1}, b.nhash + 1, words, L.scan_err, true);
+        L.end();
+        L.note();
+    }
     LP_LAUNCH(L, k_vox_count, div_up(ns, 64u), 64, b);
     const uint32_t vgrid = std::min(div_up(b.nhash, T), static_cast<uint32_t>(sm_count()) * 8u); // <= voxels
     LP_LAUNCH(L, k_uf_hook, vgrid, T, b);

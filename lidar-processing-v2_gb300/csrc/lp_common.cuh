@@ -292,6 +292,7 @@ constexpr uint32_t kLbThreads = 256;
 constexpr uint32_t kLbRows = 8;
 constexpr uint32_t kLbWarpSpan = kLbRows * 32u * 4u;           // 1024 elements per warp
 constexpr uint32_t kLbTile = (kLbThreads / 32u) * kLbWarpSpan; // 8192 elements per tile
+static_assert(kLbTile == 8192u, "Launcher::scan_state counts tiles of 8192");
 constexpr unsigned long long kLbAgg = 1ull << 62, kLbPre = 2ull << 62;
 
 __device__ __forceinline__ unsigned long long ld_status(const unsigned long long* p)
@@ -405,12 +406,19 @@ __global__ void __launch_bounds__(kLbThreads) k_scan_lb(Src src, Dst dst, unsign
     }
 }
 
+// Words a scan of n elements needs (zeroed): the ticket counter and one per tile.
+inline uint32_t scan_words(uint32_t n)
+{
+    return div_up(n, kLbTile) + 1u;
+}
+
 template <class Src, class Dst>
-void scan_lookback(cudaStream_t st, Src src, Dst dst, uint32_t n, uint32_t* sums, uint32_t* err)
+void scan_lookback(cudaStream_t st, Src src, Dst dst, uint32_t n, uint32_t* sums, uint32_t* err, bool zeroed = false)
 {
     const uint32_t nt = div_up(n, kLbTile);
     unsigned long long* state = reinterpret_cast<unsigned long long*>(sums);
-    cudaMemsetAsync(state, 0, (static_cast<size_t>(nt) + 1) * sizeof(unsigned long long), st);
+    if (!zeroed)
+        cudaMemsetAsync(state, 0, scan_words(n) * sizeof(unsigned long long), st);
     k_scan_lb<<<nt, kLbThreads, 0, st>>>(src, dst, state, err, kLbPollLimit);
 }
 

@@ -1,4 +1,4 @@
-// lp_dror.cu — batch bookkeeping around the outlier filter: state initialisation, the compaction
+// lp_dror.cu — batch bookkeeping around the outlier filter: the compaction
 // of VALID points that segmentation sees (processor order: DROR first, then the VALID points in
 // order), and the per-input-point outputs. The filter itself (NoiseRemover::filter,
 // noise_remover.cpp:38-68) is lp_kdtree.cu.
@@ -13,15 +13,6 @@ namespace
 __device__ __forceinline__ int scan_of_src(const BatchDev& b, uint32_t i)
 {
     return find_scan(b.nscan, i, [&](int s) { return b.scans[s].src_off; });
-}
-
-__global__ void k_state_init(BatchDev b, int noise)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.nscan)
-        return;
-    ScanState& st = b.state[s];
-    st.n_pts = noise ? 0u : b.scans[s].n;
 }
 
 // VALID input points are packed, in order, at the start of their scan's point slice.
@@ -56,7 +47,8 @@ __global__ void k_noise_count(BatchDev b)
     b.state[s].n_pts = b.src_pos[sd.src_off + sd.n_src] - b.src_pos[sd.src_off];
 }
 
-// Per input point outputs: segmentation label and cluster label (obstacle points only).
+// Per input point outputs: segmentation label and cluster label (obstacle points only). Points the
+// outlier filter removed keep what the arrays start with (k_prepare).
 __global__ void k_outputs(BatchDev b, int with_clusters)
 {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -68,15 +60,10 @@ __global__ void k_outputs(BatchDev b, int with_clusters)
     const uint32_t src = b.pt_src ? static_cast<uint32_t>(b.pt_src[j]) : j;
     const uint32_t lbl = b.seg_label[j];
     b.out_seg[src] = lbl;
-    if (with_clusters && lbl == LP_LABEL_OBSTACLE)
-        b.out_cl[src] = b.obs_label[b.obs_flag[j]];
+    if (with_clusters)
+        b.out_cl[src] = (lbl == LP_LABEL_OBSTACLE) ? b.obs_label[b.obs_flag[j]] : LP_INVALID_CLUSTER;
 }
 } // namespace
-
-void launch_state_init(Launcher& L, const BatchDev& b, int noise)
-{
-    LP_LAUNCH(L, k_state_init, div_up(static_cast<uint32_t>(b.nscan), 64u), 64, b, noise);
-}
 
 void launch_noise_compaction(Launcher& L, const BatchDev& b, const BatchHost& hb)
 {

@@ -18,6 +18,7 @@
 //   5. rotating-calipers box (Shamos antipodal pairs, best area kept as a float exactly like
 //      BoundingBox::area; comparisons screened in FP32) and the PCA box, one warp each (in the CTA
 //      path while the other warps count the ranks).
+#include <atomic>
 #include <cfloat>
 #include <mutex>
 
@@ -2789,10 +2790,17 @@ void init_kernel_attributes()
 
 int sm_count()
 {
+    // asked for at most launches of a run: the attribute is read once per device
+    static std::atomic<int> known[64];
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0)
+        return n;
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 1;
+    n = n > 0 ? n : 1;
+    if (dev >= 0 && dev < 64)
+        known[dev].store(n, std::memory_order_relaxed);
+    return n;
 }
 
 void launch_hull_single(Launcher& L, const double2* pts, uint32_t n, void* scratch, int* stack, int32_t* out,

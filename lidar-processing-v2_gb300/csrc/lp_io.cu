@@ -56,7 +56,8 @@ __global__ void k_io_in(BatchDev b, const IoScan* io)
 // Per-point labels of every scan into the caller's buffers, four consecutive points per thread
 // (chunk q of the batch: scan s with io[s].q_off <= q, points 4 (q - q_off) ..): the host link
 // takes whole 16-byte stores (4 B of noise labels, 16 B of segmentation and of cluster labels)
-// where the caller's buffers are aligned for them, and one store per label otherwise.
+// where the caller's buffers are aligned for them, and one store per label otherwise. The labels come
+// straight from the stages' arrays (by compacted point, by obstacle), without a pass of their own.
 __device__ __forceinline__ void io_out_chunk(const BatchDev& b, const IoScan* io, uint32_t q)
 {
     const int s = find_scan(b.nscan, q, [&](int t) { return io[t].q_off; });
@@ -74,13 +75,18 @@ __device__ __forceinline__ void io_out_chunk(const BatchDev& b, const IoScan* io
     for (uint32_t u = 0; u < 4; ++u)
         if (u < cnt)
         {
-            // a device array is read only when the caller asked for it (stages may not produce it)
-            if (d.noise)
+            uint32_t pos = i0 + u; // compacted point
+            cl[u] = LP_INVALID_CLUSTER;
+            if (b.pt_src)
+            {
                 nz[u] = b.noise[i0 + u];
-            if (d.seg)
-                sg[u] = b.out_seg[i0 + u];
-            if (d.cl)
-                cl[u] = static_cast<int32_t>(b.out_cl[i0 + u]);
+                if (nz[u] != LP_NOISE_VALID)
+                    continue;
+                pos = sd.pt_off + (b.src_pos[i0 + u] - b.src_pos[sd.src_off]);
+            }
+            sg[u] = b.seg_label[pos];
+            if (d.cl && sg[u] == LP_LABEL_OBSTACLE)
+                cl[u] = b.obs_label[b.obs_flag[pos]];
         }
     if (d.vec && cnt == 4u)
     {
@@ -105,15 +111,19 @@ __device__ __forceinline__ void io_out_chunk(const BatchDev& b, const IoScan* io
     }
 }
 
-__global__ void k_io_out_points(BatchDev b, const IoScan* io, uint32_t nq)
+// host_state: the scans' states as the host reads them (page-locked).
+__global__ void k_io_out_points(BatchDev b, const IoScan* io, ScanState* host_state, uint32_t nq)
 {
+    if (blockIdx.x == 0)
+        for (uint32_t i = threadIdx.x; i < static_cast<uint32_t>(b.nscan) * (sizeof(ScanState) / 4u); i += blockDim.x)
+            reinterpret_cast<uint32_t*>(host_state)[i] = reinterpret_cast<const uint32_t*>(b.state)[i];
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x)
         io_out_chunk(b, io, q);
 }
 
 // Per-cluster results: hull offsets (relative to the scan), hull indices, z range, boxes. A scan
 // whose clusters or hull indices exceed the caller's capacities gets none of them (the host
-// reports LP_ERR_CAPACITY for it). ret[s] = the scan's hull index count.
+// reports LP_ERR_CAPACITY for it). ret[s] = the scan's hull index count (page-locked host memory).
 __global__ void k_io_out_clusters(BatchDev b, const IoScan* io, uint32_t* ret, int with_obb)
 {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -159,10 +169,11 @@ void launch_io_in(Launcher& L, const BatchDev& b, const IoScan* io)
     LP_LAUNCH(L, k_io_in, std::min(div_up(b.nsrc, 256u), static_cast<uint32_t>(sm_count()) * 2u), 256, b, io);
 }
 
-void launch_io_out(Launcher& L, const BatchDev& b, const IoScan* io, uint32_t* ret, int with_hull, int with_obb,
-                   uint32_t nq)
+void launch_io_out(Launcher& L, const BatchDev& b, const IoScan* io, uint32_t* ret, ScanState* host_state, int with_hull,
+                   int with_obb, uint32_t nq)
 {
-    LP_LAUNCH(L, k_io_out_points, std::min(div_up(nq, 256u), static_cast<uint32_t>(sm_count()) * 2u), 256, b, io, nq);
+    LP_LAUNCH(L, k_io_out_points, std::min(div_up(std::max(nq, 1u), 256u), static_cast<uint32_t>(sm_count()) * 2u), 256, b, io,
+              host_state, nq);
     if (with_hull)
         LP_LAUNCH(L, k_io_out_clusters, div_up(b.ncl, 256u), 256, b, io, ret, with_obb);
 }

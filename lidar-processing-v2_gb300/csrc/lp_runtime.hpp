@@ -79,7 +79,8 @@ struct lp_batch
     lpg::BatchDev b{};
     char* mem = nullptr;
     size_t cap = 0;
-    uint32_t* scan_sums = nullptr;
+    uint32_t* scan_sums = nullptr; // look-back words of a run's scans
+    size_t scan_words = 0;         // 8-byte words there
     uint8_t* d_image = nullptr;
     std::vector<lpg::ScanState> h_state;
     std::vector<float4> staging; // host repack for stride-3 inputs
@@ -95,7 +96,10 @@ struct lp_batch
     std::vector<std::vector<uint32_t>> part_scans; // the batch's scan indices in part k, in batch order
     std::vector<cudaEvent_t> fork_join;            // [0] fork, [1 + k] part k done
     lp_tuning tune = lprt::tuning_default();       // the batch's split and launch shapes
-    std::vector<uint32_t> h_nh;         // direct host I/O: hull index count per scan (read back)
+    // direct host I/O: page-locked staging (descriptors out, states and hull index counts back at h_ret)
+    char* h_stage = nullptr;
+    size_t h_stage_cap = 0;
+    char* h_ret = nullptr;
 };
 
 namespace lprt
@@ -108,7 +112,7 @@ size_t measure(lp_batch& B);
 // plan + (re)allocate + carve.
 lp_status build(lp_context* ctx, lp_batch& B);
 lp_status upload(lp_context* ctx, lp_batch& B);
-lp_status execute(lp_context* ctx, lp_batch& B);
+lp_status execute(lp_context* ctx, lp_batch& B, bool outputs = true);
 lp_status fetch_state(lp_context* ctx, lp_batch& B);
 lp_status download(lp_context* ctx, lp_batch& B, lp_scan_output* outs);
 lp_status fill_pipeline(lp_context* ctx, lp_batch& B, const lp_pipeline_config* cfg, const lp_scan_input* scans,

@@ -10,9 +10,29 @@
 namespace lpg
 {
 void scan_exclusive(cudaStream_t st, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* sums, uint32_t* err,
-                    uint64_t& launches);
+                    uint64_t& launches, bool zeroed = false);
 void launch_debug_wait_timeout(cudaStream_t st, int kind, uint32_t limit, unsigned long long* state, uint32_t* err,
                                uint64_t& launches);
+
+// Ranges a run starts from (k_prepare): 16-byte units of a 32-bit pattern. Every array of a batch is
+// 256-byte aligned with 16 bytes after its end, so a range may be rounded up to whole units.
+struct FillRange
+{
+    void* p;
+    uint32_t n16, value;
+};
+struct FillList
+{
+    FillRange r[24];
+    int n = 0;
+    void add(void* p, size_t bytes, uint32_t value)
+    {
+        r[n++] = FillRange{p, static_cast<uint32_t>((bytes + 15) / 16), value};
+    }
+};
+// Device-wide scans of one run at most (ring tiles, outlier filter 3 + compaction, cells, near cells,
+// obstacles, voxels, components, clusters, hulls): each takes its own zeroed look-back words.
+constexpr uint32_t kScansPerRun = 12;
 
 // One timed launch (profiling mode only).
 struct LaunchRecord
@@ -27,7 +47,8 @@ struct Launcher
 {
     cudaStream_t stream = nullptr;
     uint64_t* launches = nullptr;
-    uint32_t* scan_sums = nullptr; // scratch for device-wide scans
+    uint32_t* scan_sums = nullptr; // next zeroed look-back words (k_prepare zeroes scan_left of them)
+    size_t scan_left = 0;          // 8-byte words left
     uint32_t* scan_err = nullptr;  // error word the device-wide scans report into
     cudaError_t err = cudaSuccess;
     std::vector<LaunchRecord>* prof = nullptr;
@@ -93,10 +114,28 @@ struct Launcher
     {
         if (n == 0)
             return;
+        uint32_t* words = scan_state(n);
+        if (!words)
+            return;
         begin("k_scan");
-        scan_exclusive(stream, in, out, n, scan_sums, scan_err, *launches);
+        scan_exclusive(stream, in, out, n, words, scan_err, *launches, true);
         end();
         note_only();
+    }
+    // Look-back words of a scan over n elements (null, with the error noted, when the run has none left).
+    uint32_t* scan_state(uint32_t n)
+    {
+        const size_t words = (static_cast<size_t>(n) + 8191u) / 8192u + 1u; // scan_words(n)
+        if (words > scan_left)
+        {
+            if (err == cudaSuccess)
+                err = cudaErrorInvalidValue;
+            return nullptr;
+        }
+        uint32_t* p = scan_sums;
+        scan_sums += 2u * words;
+        scan_left -= words;
+        return p;
     }
     void note()
     {
@@ -120,8 +159,8 @@ void init_kernel_attributes();
 void init_kdtree_attributes(); // lp_kdtree.cu
 // Direct host I/O (lp_io.cu): inputs from and results into the caller's page-locked buffers.
 void launch_io_in(Launcher& L, const BatchDev& b, const IoScan* io);
-void launch_io_out(Launcher& L, const BatchDev& b, const IoScan* io, uint32_t* ret, int with_hull, int with_obb,
-                   uint32_t nq);
+void launch_io_out(Launcher& L, const BatchDev& b, const IoScan* io, uint32_t* ret, ScanState* host_state, int with_hull,
+                   int with_obb, uint32_t nq);
 void init_segment_tables(); // per-device constant tables (the seed-42 MT19937 stream)
 // PointCloud2 bytes -> XYZI (+ ring) (lp_wire.cu); offsets: x, y, z, intensity, ring.
 void launch_unpack_pointcloud2(cudaStream_t st, const uint8_t* data, uint32_t width, uint32_t height,
@@ -189,7 +228,7 @@ void launch_clustering(Launcher& L, const BatchDev& b, const BatchHost& hb);
 void launch_polygons(Launcher& L, const BatchDev& b, const BatchHost& hb, int compute_obb);
 void launch_noise(Launcher& L, const BatchDev& b, const BatchHost& hb, const lp_noise_remover_config& cfg);
 void launch_noise_compaction(Launcher& L, const BatchDev& b, const BatchHost& hb);
-void launch_state_init(Launcher& L, const BatchDev& b, int noise);
+void launch_prepare(Launcher& L, const FillList& f, const BatchDev& b, int noise);
 void launch_outputs(Launcher& L, const BatchDev& b, int with_clusters);
 void launch_mark_all_obstacles(Launcher& L, const BatchDev& b);
 void launch_hull_single(Launcher& L, const double2* pts, uint32_t n, void* scratch, int* stack, int32_t* out,
