@@ -168,7 +168,6 @@ lp_status plan(lp_context* ctx, lp_batch& B)
         sd.res_a = R.cl.voxel_grid_azimuth_resolution_deg * kDegToRad;
         sd.res_e = R.cl.voxel_grid_elevation_resolution_deg * kDegToRad;
         sd.min_cluster = R.cl.min_cluster_size;
-        sd.hash_off = static_cast<uint32_t>(hash);
         sd.hash_cap = next_pow2(std::max(64u, 2u * in.n));
         const uint32_t minc = std::max(1u, R.cl.min_cluster_size);
         sd.cluster_cap = in.n / minc + 1;
@@ -230,7 +229,7 @@ size_t carve(lp_batch& B, char* base)
     put(b.io, S);
     put(b.state, S);
     const uint32_t maxlen = std::max({N, b.npix, b.nhash, b.ncell, b.ncl, b.ntiles, b.nnear}) + 2;
-    B.scan_words = static_cast<size_t>(kScansPerRun) * scan_words(maxlen);
+    B.scan_words = static_cast<size_t>(kScansPerRun) * scan_words_max(maxlen);
     put(B.scan_sums, 2 * B.scan_words);
     float4* src;
     put(src, N);
@@ -330,25 +329,21 @@ size_t carve(lp_batch& B, char* base)
         put(b.obs_a, N);
         put(b.obs_e, N);
         put(b.obs_hslot, N);
-        put(b.hkey, b.nhash);
-        put(b.hmin, b.nhash);
-        put(b.hcnt, b.nhash);
-        put(b.hvid, b.nhash + 1);
-        put(b.vslot, b.nhash);
-        put(b.parent, b.nhash);
-        put(b.cmin, b.nhash);
-        put(b.ccnt, b.nhash);
+        put(b.hrec, b.nhash);
+        put(b.vlist, N);
         put(b.kflag, N + 1);
         put(b.obs_label, N);
         put(b.cl_cnt, b.ncl + 1);
-        put(b.cl_start, b.ncl + 1);
-        put(b.cl_fill, b.ncl + 1);
-        put(b.members, N);
-        put(b.mxy, N);
-        put(b.cl_zkey, 2ull * b.ncl);
     }
     if (hull)
     {
+        put(b.cl_start, b.ncl);
+        put(b.cl_rank, b.ncl);
+        put(b.cl_fill, b.ncl);
+        put(b.members, N);
+        put(b.mxy, N);
+        put(b.cl_zkey, 2ull * b.ncl);
+        put(b.hull_work, b.ncl);
         put(b.hull_cnt, b.ncl + 1);
         put(b.hull_tmp, N);
         put(b.hull_out, N);
@@ -362,7 +357,7 @@ size_t carve(lp_batch& B, char* base)
         put(b.hs_stack, static_cast<size_t>(2) * N + 2ull * b.ncl + 8);
         put(b.hs_pts, static_cast<size_t>(N) + 8);
         put(b.hs_pairs, static_cast<size_t>(4) * N + 16ull * b.ncl + 16);
-        put(b.queue, 8);
+        put(b.queue, 10);
         put(b.tie_list, b.ncl + 1);
         put(b.pre_items, N / 4096u + b.ncl + 1);
         put(b.pre_ext, 16ull * b.ncl + 16);
@@ -474,20 +469,9 @@ lp_status execute(lp_context* ctx, lp_batch& B, bool outputs)
         f.add(b.row_cnt, static_cast<size_t>(b.nrows) * 4, 0u);
     }
     if (clu)
-    {
-        f.add(b.hkey, static_cast<size_t>(b.nhash) * 4, 0xffffffffu);
-        f.add(b.hmin, static_cast<size_t>(b.nhash) * 4, 0xffffffffu);
-        f.add(b.hcnt, static_cast<size_t>(b.nhash) * 4, 0u);
-        f.add(b.kflag, (N + 1) * 4, 0u);
         f.add(b.cl_cnt, (static_cast<size_t>(b.ncl) + 1) * 4, 0u);
-        f.add(b.cl_fill, (static_cast<size_t>(b.ncl) + 1) * 4, 0u);
-        f.add(b.cl_zkey, static_cast<size_t>(b.ncl) * 8, 0u);
-    }
     if (R.stages & ST_HULL)
-    {
-        f.add(b.hull_cnt, (static_cast<size_t>(b.ncl) + 1) * 4, 0u);
-        f.add(b.queue, 8 * 4, 0u);
-    }
+        f.add(b.queue, 10 * 4, 0u);
     launch_prepare(L, f, b, noise ? 1 : 0);
     if (noise)
     {
@@ -1209,7 +1193,7 @@ lp_status lp_split_clouds(lp_context* ctx, const float* xyzi, const uint32_t* la
     const size_t o_lab = al(N * 16), o_out = o_lab + al(N * 4), o_cnt = o_out + al(3 * N * sizeof(lp_xyzrgb));
     const size_t o_sums = o_cnt + 256;
     char* m = nullptr;
-    LP_TRY(scratch(ctx, o_sums + al((N + 1) / 8192 * 8 + 64), &m));
+    LP_TRY(scratch(ctx, o_sums + al(8ull * scan_words(n + 1u)), &m));
     const cudaStream_t st = ctx->stream;
     LP_CUDA(ctx, cudaMemcpyAsync(m, xyzi, N * 16, cudaMemcpyHostToDevice, st));
     LP_CUDA(ctx, cudaMemcpyAsync(m + o_lab, labels, N * 4, cudaMemcpyHostToDevice, st));
@@ -1356,7 +1340,7 @@ lp_status lp_cluster_objects(lp_context* ctx, const float* xyzi, const int32_t* 
         return at;
     };
     const size_t o_pts = take(N * 16), o_lab = take(N * 4), o_cnt = take(cells * 4),
-                 o_sums = take(8 * (cells / 2048 + 4)), o_err = take(4), o_col = take(static_cast<size_t>(K) * 4),
+                 o_sums = take(8ull * std::max(scan_words(static_cast<uint32_t>(cells)), scan_words(K + 1u))), o_err = take(4), o_col = take(static_cast<size_t>(K) * 4),
                  o_cloff = take((K + 1ull) * 4), o_cloud = take(N * sizeof(lp_xyzrgb)), o_hoff = take((K + 1ull) * 4),
                  o_hidx = take(static_cast<size_t>(H) * 4), o_zmin = take(K * 4ull), o_zmax = take(K * 4ull),
                  o_cls = take(K * 4ull), o_box = take(K * sizeof(lp_bounding_box)), o_P = take(N * 16),

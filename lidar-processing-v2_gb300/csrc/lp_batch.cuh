@@ -138,27 +138,22 @@ struct BatchDev
     float* obs_e;
     uint32_t* obs_hslot;  // per obstacle: hash slot
     uint32_t nhash;
-    uint32_t* hkey;       // per slot: voxel flat key or 0xffffffff
-    uint32_t* hmin;       // per slot: min local obstacle index
-    uint32_t* hcnt;       // per slot: points in voxel
-    uint32_t* hvid;       // per slot: number of occupied slots before it (voxel id of an occupied slot)
-    uint32_t* vslot;      // per voxel id: hash slot
-    uint32_t* parent;     // per voxel id
-    uint32_t* cmin;       // per voxel id (valid at roots)
-    uint32_t* ccnt;
-    uint32_t* kflag;      // per obstacle: 1 at the min point of a kept component -> scan
+    uint4* hrec;          // voxel hash: key (0xffffffff: free), smallest local obstacle, points, union-find parent slot
+    uint32_t* vlist;      // hash slots of the batch's voxels
+    uint32_t* kflag;      // per obstacle: kept components whose smallest obstacle lies before it
     int32_t* obs_label;   // per obstacle: cluster label or -1
 
     // ---- per-cluster ---------------------------------------------------------------------------
     uint32_t ncl;
     uint32_t hull_cta_min; // clusters of more members take a CTA of the hull kernel (tuning)
     uint32_t* cl_cnt;     // members per cluster
-    uint32_t* cl_start;   // exclusive scan of cl_cnt
+    uint32_t* cl_start;   // first member slot of each cluster (disjoint ranges, in the order of cl_rank)
+    uint32_t* cl_rank;
     uint32_t* cl_fill;
     uint32_t* members;    // obstacle indices grouped by cluster (unordered within)
     float2* mxy;          // x, y of each member, by member slot
     uint32_t* cl_zkey;    // per cluster: max of ~ord(z) (the lowest z), max of ord(z) (the highest)
-    uint32_t* hull_cnt;   // hull vertices per cluster -> exclusive scan in place
+    uint32_t* hull_cnt;   // hull vertices per cluster -> per scan, offsets into hull_out (from its pt_off)
     int32_t* hull_tmp;    // per member slot: hull local indices at cl_start
     int32_t* hull_out;    // dense hull local indices (batch)
     float* cl_zmin;
@@ -166,10 +161,12 @@ struct BatchDev
     lp_bounding_box* obb_c;
     lp_bounding_box* obb_p;
     void* hs_cand;        // hull candidates (12 B each), 2 per member slot, at 2 * cl_start
-    int32_t* hs_stack;    // monotone-chain stack, at 2 * cl_start + 2 * cluster
+    int32_t* hs_stack;    // monotone-chain stack, at 2 * cl_start + 2 * cl_rank
     double2* hs_pts;      // hull vertices as FP64, at cl_start
-    int2* hs_pairs;       // antipodal pairs, at 4 * cl_start + 16 * cluster
-    uint32_t* queue;      // [0] clusters in the batch, [1] hull work-queue head, [4] tie clusters
+    int2* hs_pairs;       // antipodal pairs, at 4 * cl_start + 16 * cl_rank
+    uint32_t* hull_work;  // hull work list: large clusters from the front, the others from the back
+    uint32_t* queue;      // [8..9] member slots and clusters given a range, [1] large-cluster head, [2] large clusters, [3] others,
+                          // [4] others' head, [5] tie clusters, [6] chunks of the member passes
     uint32_t* tie_list;
     uint2* pre_items;          // (cluster, chunk) items of the large clusters' member passes
     unsigned long long* pre_ext;  // per cluster: its 16 direction extremes (packed keys)

@@ -8,6 +8,8 @@
 // the 26-neighbour graph (the azimuth index wraps modulo num_azimuth as in clusterer.cpp:
 // 161-169), and the canonical labels from a prefix scan of "component minimum" flags. Labels
 // are identical to the reference's, not only the partition.
+#include <algorithm>
+
 #include "lp_batch.cuh"
 #include "lp_common.cuh"
 #include "lp_math.cuh"
@@ -28,7 +30,7 @@ __device__ __forceinline__ int scan_of_obs(const BatchDev& b, uint32_t o)
 }
 __device__ __forceinline__ int scan_of_hash(const BatchDev& b, uint32_t h)
 {
-    return find_scan(b.nscan, h, [&](int s) { return b.scans[s].hash_off; });
+    return find_scan(b.nscan, h, [&](int s) { return b.state[s].hash_off; });
 }
 __device__ __forceinline__ uint32_t hash_mix(uint32_t k)
 {
@@ -43,42 +45,75 @@ __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p)
     return *reinterpret_cast<const volatile uint32_t*>(p);
 }
 
-__global__ void k_obs_flag(BatchDev b)
+// Obstacle slots: the exclusive scan of "is an obstacle" over the points.
+struct ObsFlagSrc
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > b.npts)
-        return;
-    b.obs_flag[i] = (i < b.npts && b.seg_label[i] == LP_LABEL_OBSTACLE) ? 1u : 0u;
-}
+    const uint32_t* label;
+    uint32_t n;
+    __device__ __forceinline__ uint32_t end() const { return 0xffffffffu; }
+    __device__ __forceinline__ uint4 get4(uint32_t i) const
+    {
+        uint4 v = ScanSrcU32{label, n, true}.get4(i); // (no label is LP_LABEL_OBSTACLE past the end)
+        return make_uint4(v.x == LP_LABEL_OBSTACLE, v.y == LP_LABEL_OBSTACLE, v.z == LP_LABEL_OBSTACLE, v.w == LP_LABEL_OBSTACLE);
+    }
+};
 
-__global__ void k_obs_state(BatchDev b)
+// The scans' obstacle ranges and voxel hash slices, by the first warp of a block (every lane returns the
+// slots of all scans together). The slice of a scan holds next_pow2(max(64, 2 n_obs)) slots, packed
+// one scan after the other: sized by the obstacles, not by the points, the hash of a 64 x 2048 scan
+// is 16 to 64 times smaller (its clearing and every pass over it with it) and stays in L2.
+__device__ __forceinline__ uint32_t hash_layout(const BatchDev& b, bool write)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.nscan)
-        return;
-    const ScanDev& sd = b.scans[s];
-    ScanState& st = b.state[s];
-    st.obs_off = b.obs_flag[sd.pt_off];
-    st.n_obs = b.obs_flag[sd.pt_off + sd.n] - st.obs_off;
-    st.max_r_bits = 0u;
-    st.max_a_bits = 0u;
-    st.max_e_bits = 0u;
+    uint32_t base = 0u;
+    for (int s0 = 0; s0 < b.nscan; s0 += 32)
+    {
+        const int s = s0 + static_cast<int>(lane_id());
+        uint32_t slots = 0u, off = 0u, n = 0u;
+        if (s < b.nscan)
+        {
+            const ScanDev& sd = b.scans[s];
+            off = b.obs_flag[sd.pt_off];
+            n = b.obs_flag[sd.pt_off + sd.n] - off;
+            slots = next_pow2(max(64u, 2u * n)); // <= hash_cap: n <= sd.n
+        }
+        const uint32_t incl = warp_incl_scan(slots);
+        if (write && s < b.nscan)
+        {
+            ScanState& st = b.state[s];
+            st.obs_off = off;
+            st.n_obs = n;
+            st.hash_off = base + incl - slots;
+            st.hash_mask = slots - 1u;
+        }
+        base += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    return base;
 }
 
 // Obstacle cloud in input order (processor.cpp:562-579) with the spherical coordinates of
 // Clusterer::cartesianToSpherical (clusterer.cpp:55-100). A block takes 1024 consecutive points
 // and first compacts its obstacle points in shared memory, so that every lane of the arithmetic
-// below (two correctly rounded arctangents) has one.
+// below (two correctly rounded arctangents) has one. The grid also clears the voxel hash, and its first
+// block records the scans' obstacle ranges and hash slices.
 constexpr uint32_t kObsChunk = 1024;
 
 __global__ void __launch_bounds__(256) k_obs_gather(BatchDev b)
 {
     __shared__ uint32_t sidx[kObsChunk];
-    __shared__ uint32_t scnt;
+    __shared__ uint32_t scnt, s_slots;
     const uint32_t base = blockIdx.x * kObsChunk;
-    if (threadIdx.x == 0)
-        scnt = 0u;
+    if (threadIdx.x < 32u)
+    {
+        const uint32_t slots = hash_layout(b, blockIdx.x == 0u);
+        if (threadIdx.x == 0)
+        {
+            scnt = 0u;
+            s_slots = slots;
+        }
+    }
     __syncthreads();
+    for (uint32_t h = blockIdx.x * 256u + threadIdx.x; h < s_slots; h += gridDim.x * 256u)
+        b.hrec[h] = make_uint4(kEmpty, kEmpty, 0u, h);
 #pragma unroll
     for (uint32_t u = 0; u < kObsChunk / 256u; ++u)
     {
@@ -145,145 +180,115 @@ __global__ void __launch_bounds__(256) k_obs_gather(BatchDev b)
     }
 }
 
-__global__ void k_dims(BatchDev b)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.nscan)
-        return;
-    const ScanDev& sd = b.scans[s];
-    ScanState& st = b.state[s];
-    if (st.n_obs == 0)
-    {
-        st.nr = st.na = st.ne = 0;
-        return;
-    }
-    st.nr = static_cast<int32_t>(ceilf(__uint_as_float(st.max_r_bits) / sd.res_r) + 1.0f);
-    st.na = static_cast<int32_t>(ceilf(__uint_as_float(st.max_a_bits) / sd.res_a) + 1.0f);
-    st.ne = static_cast<int32_t>(ceilf(__uint_as_float(st.max_e_bits) / sd.res_e) + 1.0f);
-    const long long cells = static_cast<long long>(st.nr) * st.na * st.ne;
-    if (cells > 0x7fffffffLL)
-        raise_err(&st, ERR_INTERNAL);
-}
-
 __device__ __forceinline__ int32_t flat_voxel(int32_t nr, int32_t na, int32_t r, int32_t a, int32_t e)
 {
     return nr * (na * e + a) + r; // Clusterer::flatVoxelIndex, clusterer.hpp:136-142
 }
 
+// Voxel hash slot (hrec): key, smallest obstacle of the voxel, its point count, union-find parent (a
+// slot; itself until linked). One 16-byte record, so an insertion and a lookup touch one sector each.
+// New voxels are listed (vlist; state[0].n_comp counts the batch's). The grid dimensions
+// (clusterer.cpp:92-99) come from the maxima that k_obs_gather left; the thread of a scan's first
+// obstacle records them.
 __global__ void k_vox_insert(BatchDev b)
 {
     const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= b.obs_flag[b.npts])
+    const bool in = o < b.obs_flag[b.npts];
+    bool fresh = false;
+    uint32_t at = 0u;
+    int s = 0;
+    if (in)
+    {
+        s = scan_of_obs(b, o);
+        const ScanDev& sd = b.scans[s];
+        ScanState& st = b.state[s];
+        const int32_t nr = static_cast<int32_t>(ceilf(__uint_as_float(st.max_r_bits) / sd.res_r) + 1.0f);
+        const int32_t na = static_cast<int32_t>(ceilf(__uint_as_float(st.max_a_bits) / sd.res_a) + 1.0f);
+        if (o == st.obs_off)
+        {
+            const int32_t ne = static_cast<int32_t>(ceilf(__uint_as_float(st.max_e_bits) / sd.res_e) + 1.0f);
+            st.nr = nr;
+            st.na = na;
+            st.ne = ne;
+            if (static_cast<long long>(nr) * na * ne > 0x7fffffffLL)
+                raise_err(&st, ERR_INTERNAL);
+        }
+        const int32_t vr = static_cast<int32_t>(b.obs_r[o] / sd.res_r);
+        const int32_t va = static_cast<int32_t>(b.obs_a[o] / sd.res_a);
+        const int32_t ve = static_cast<int32_t>(b.obs_e[o] / sd.res_e);
+        const uint32_t key = static_cast<uint32_t>(flat_voxel(nr, na, vr, va, ve));
+        const uint32_t mask = st.hash_mask, off = st.hash_off;
+        uint32_t h = hash_mix(key) & mask;
+        at = kEmpty;
+        for (uint32_t probe = 0; probe <= mask; ++probe)
+        {
+            uint32_t* rec = reinterpret_cast<uint32_t*>(&b.hrec[off + h]);
+            const uint32_t prev = atomicCAS(&rec[0], kEmpty, key);
+            if (prev == kEmpty || prev == key)
+            {
+                at = off + h;
+                fresh = prev == kEmpty;
+                atomicMin(&rec[1], o - st.obs_off);
+                atomicAdd(&rec[2], 1u);
+                break;
+            }
+            h = (h + 1u) & mask;
+        }
+        if (at == kEmpty)
+            raise_err(&st, ERR_HASH_FULL);
+        b.obs_hslot[o] = at;
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, fresh);
+    if (m == 0u)
         return;
-    const int s = scan_of_obs(b, o);
-    const ScanDev& sd = b.scans[s];
-    ScanState& st = b.state[s];
-    const int32_t vr = static_cast<int32_t>(b.obs_r[o] / sd.res_r);
-    const int32_t va = static_cast<int32_t>(b.obs_a[o] / sd.res_a);
-    const int32_t ve = static_cast<int32_t>(b.obs_e[o] / sd.res_e);
-    const uint32_t key = static_cast<uint32_t>(flat_voxel(st.nr, st.na, vr, va, ve));
-    const uint32_t mask = sd.hash_cap - 1u;
-    uint32_t h = hash_mix(key) & mask;
-    for (uint32_t probe = 0; probe < sd.hash_cap; ++probe)
+    uint32_t pos = 0u;
+    const int leader = __ffs(m) - 1;
+    if (lane_id() == static_cast<uint32_t>(leader))
+        pos = atomicAdd(&b.state[0].n_comp, static_cast<uint32_t>(__popc(m)));
+    pos = __shfl_sync(0xffffffffu, pos, leader);
+    if (fresh)
+        b.vlist[pos + static_cast<uint32_t>(__popc(m & ((1u << lane_id()) - 1u)))] = at;
+    // voxels per scan (a warp's obstacles mostly belong to one)
+    const int s0 = __shfl_sync(0xffffffffu, s, leader);
+    if (__all_sync(0xffffffffu, !fresh || s == s0))
     {
-        const uint32_t slot = sd.hash_off + h;
-        const uint32_t prev = atomicCAS(&b.hkey[slot], kEmpty, key);
-        if (prev == kEmpty || prev == key)
-        {
-            b.obs_hslot[o] = slot;
-            atomicMin(&b.hmin[slot], o - st.obs_off);
-            atomicAdd(&b.hcnt[slot], 1u);
-            return;
-        }
-        h = (h + 1u) & mask;
+        if (lane_id() == static_cast<uint32_t>(leader))
+            atomicAdd(&b.state[s0].n_vox, static_cast<uint32_t>(__popc(m)));
     }
-    raise_err(&st, ERR_HASH_FULL);
-    b.obs_hslot[o] = kEmpty;
-}
-
-// Voxel ids in hash-slot order: one look-back scan reads the occupancy of the hash slots, writes
-// hvid[h] = the number of occupied slots before h (nhash + 1 entries: the last is the total) and
-// initialises the union-find record of every occupied slot's voxel.
-struct VoxFlagsSrc
-{
-    const uint32_t* hkey;
-    uint32_t nhash;
-    __device__ __forceinline__ uint4 get4(uint32_t i) const
-    {
-        uint4 k;
-        if (i + 4u <= nhash)
-            k = *reinterpret_cast<const uint4*>(hkey + i);
-        else
-        {
-            k.x = (i < nhash) ? hkey[i] : kEmpty;
-            k.y = (i + 1u < nhash) ? hkey[i + 1u] : kEmpty;
-            k.z = (i + 2u < nhash) ? hkey[i + 2u] : kEmpty;
-            k.w = (i + 3u < nhash) ? hkey[i + 3u] : kEmpty;
-        }
-        return make_uint4(k.x != kEmpty, k.y != kEmpty, k.z != kEmpty, k.w != kEmpty);
-    }
-};
-struct VoxInitDst
-{
-    uint32_t *hvid, *vslot, *parent, *cmin, *ccnt;
-    uint32_t n; // nhash + 1
-    __device__ __forceinline__ void one(uint32_t h, uint32_t v, uint32_t occupied) const
-    {
-        if (occupied)
-        {
-            vslot[v] = h;
-            parent[v] = v;
-            cmin[v] = kEmpty;
-            ccnt[v] = 0u;
-        }
-    }
-    __device__ __forceinline__ void put4(uint32_t i, uint4 e, uint4 f) const
-    {
-        ScanDstU32{hvid, n, true}.put4(i, e, f);
-        one(i, e.x, f.x);
-        one(i + 1u, e.y, f.y);
-        one(i + 2u, e.z, f.z);
-        one(i + 3u, e.w, f.w);
-    }
-};
-
-__global__ void k_vox_count(BatchDev b)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.nscan)
-        return;
-    const ScanDev& sd = b.scans[s];
-    ScanState& st = b.state[s];
-    st.n_vox = b.hvid[sd.hash_off + sd.hash_cap] - b.hvid[sd.hash_off];
-    if (st.n_vox > kVoxelCapacity)
-        raise_err(&st, ERR_VOXEL_CAPACITY); // StaticUnorderedMap::insert throws (static_unordered_map.hpp:81)
+    else if (fresh)
+        atomicAdd(&b.state[s].n_vox, 1u);
 }
 
 // Every parent pointer is strictly smaller than its index except at roots (links go from the
 // larger root to the smaller; path halving only shortens), so a find ends within x steps. The
 // per-thread budget bounds the total work anyway: exhausting it raises ERR_UF_TIMEOUT.
-__device__ uint32_t uf_find(uint32_t* parent, uint32_t x, ScanState* st, int& budget)
+__device__ __forceinline__ uint32_t* parent_of(uint4* rec, uint32_t x)
+{
+    return &rec[x].w;
+}
+
+__device__ uint32_t uf_find(uint4* rec, uint32_t x, ScanState* st, int& budget)
 {
     while (budget-- > 0)
     {
-        const uint32_t p = ld_volatile(&parent[x]);
+        const uint32_t p = ld_volatile(parent_of(rec, x));
         if (p == x)
             return x;
-        const uint32_t gp = ld_volatile(&parent[p]);
+        const uint32_t gp = ld_volatile(parent_of(rec, p));
         if (gp != p)
-            atomicCAS(&parent[x], p, gp); // path halving; parents only ever decrease
+            atomicCAS(parent_of(rec, x), p, gp); // path halving; parents only ever decrease
         x = gp;
     }
     raise_err(st, ERR_UF_TIMEOUT);
     return x;
 }
 
-__device__ void uf_union(uint32_t* parent, uint32_t a, uint32_t c, ScanState* st, int& budget)
+__device__ void uf_union(uint4* rec, uint32_t a, uint32_t c, ScanState* st, int& budget)
 {
     while (budget > 0)
     {
-        a = uf_find(parent, a, st, budget);
-        c = uf_find(parent, c, st, budget);
+        a = uf_find(rec, a, st, budget);
+        c = uf_find(rec, c, st, budget);
         if (budget <= 0)
             return;
         if (a == c)
@@ -295,7 +300,7 @@ __device__ void uf_union(uint32_t* parent, uint32_t a, uint32_t c, ScanState* st
             c = t;
         }
         // link the larger root below the smaller one
-        const uint32_t old = atomicCAS(&parent[c], c, a);
+        const uint32_t old = atomicCAS(parent_of(rec, c), c, a);
         if (old == c)
             return;
         c = old;
@@ -303,15 +308,15 @@ __device__ void uf_union(uint32_t* parent, uint32_t a, uint32_t c, ScanState* st
     raise_err(st, ERR_UF_TIMEOUT);
 }
 
-__device__ __forceinline__ uint32_t hash_lookup(const BatchDev& b, const ScanDev& sd, uint32_t key)
+__device__ __forceinline__ uint32_t hash_lookup(const BatchDev& b, const ScanState& st, uint32_t key)
 {
-    const uint32_t mask = sd.hash_cap - 1u;
+    const uint32_t mask = st.hash_mask, off = st.hash_off;
     uint32_t h = hash_mix(key) & mask;
-    for (uint32_t probe = 0; probe < sd.hash_cap; ++probe)
+    for (uint32_t probe = 0; probe <= mask; ++probe)
     {
-        const uint32_t k = b.hkey[sd.hash_off + h];
+        const uint32_t k = b.hrec[off + h].x;
         if (k == key)
-            return sd.hash_off + h;
+            return off + h;
         if (k == kEmpty)
             return kEmpty;
         h = (h + 1u) & mask;
@@ -331,12 +336,10 @@ __device__ __forceinline__ void k_uf_hook_pair(const BatchDev& b, uint32_t v, ui
     const int32_t de = (o < 4u) ? 0 : 1;
     const int32_t da = (o == 0u) ? 0 : ((o < 4u) ? 1 : static_cast<int32_t>((o - 4u) / 3u) - 1);
     const int32_t dr = (o == 0u) ? 1 : ((o < 4u) ? static_cast<int32_t>(o) - 2 : static_cast<int32_t>((o - 4u) % 3u) - 1);
-    const uint32_t slot = b.vslot[v];
-    const int s = scan_of_hash(b, slot);
-    const ScanDev& sd = b.scans[s];
-    ScanState* st = &b.state[s];
+    const uint32_t slot = b.vlist[v];
+    ScanState* st = &b.state[scan_of_hash(b, slot)];
     const int32_t nr = st->nr, na = st->na, ne = st->ne;
-    const int32_t key = static_cast<int32_t>(b.hkey[slot]);
+    const int32_t key = static_cast<int32_t>(b.hrec[slot].x);
     const int32_t r = key % nr;
     const int32_t a = (key / nr) % na;
     const int32_t e = key / (nr * na);
@@ -348,79 +351,92 @@ __device__ __forceinline__ void k_uf_hook_pair(const BatchDev& b, uint32_t v, ui
         aa += na;
     else if (aa >= na)
         aa -= na;
-    const uint32_t nslot = hash_lookup(b, sd, static_cast<uint32_t>(flat_voxel(nr, na, rr, aa, ee)));
-    if (nslot == kEmpty)
-        return;
-    const uint32_t u = b.hvid[nslot];
-    if (u != v)
+    const uint32_t nslot = hash_lookup(b, *st, static_cast<uint32_t>(flat_voxel(nr, na, rr, aa, ee)));
+    if (nslot != kEmpty && nslot != slot)
     {
         int budget = kMaxIters;
-        uf_union(b.parent, v, u, st, budget);
+        uf_union(b.hrec, slot, nslot, st, budget);
     }
 }
 
+// The union-find runs on the hash slots themselves: their order is random, so neighbouring voxels'
+// roots do not contend, and no pass has to number the voxels.
 __global__ void k_uf_hook(BatchDev b)
 {
-    const uint32_t nv = b.hvid[b.nhash]; // occupied voxels; threads stride over (offset, voxel) pairs
+    if (blockIdx.x == 0)
+        for (int s = static_cast<int>(threadIdx.x); s < b.nscan; s += static_cast<int>(blockDim.x))
+            if (b.state[s].n_vox > kVoxelCapacity)
+                raise_err(&b.state[s], ERR_VOXEL_CAPACITY); // StaticUnorderedMap::insert throws (static_unordered_map.hpp:81)
+    const uint32_t nv = b.state[0].n_comp; // voxels; threads stride over (offset, voxel) pairs
     const unsigned long long total = 13ull * nv;
     for (unsigned long long t = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; t < total;
          t += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
         k_uf_hook_pair(b, static_cast<uint32_t>(t % nv), static_cast<uint32_t>(t / nv));
 }
 
-__device__ __forceinline__ void k_uf_flatten_one(const BatchDev& b, uint32_t v)
-{
-    const uint32_t slot = b.vslot[v];
-    const int s = scan_of_hash(b, slot);
-    int budget = kMaxIters;
-    const uint32_t root = uf_find(b.parent, v, &b.state[s], budget);
-    b.parent[v] = root;
-}
-
+// Every voxel straight below its root, and the components' smallest obstacle and point count in the
+// root's record (its own are the start; the other voxels' records keep theirs).
 __global__ void k_uf_flatten(BatchDev b)
 {
-    const uint32_t nv = b.hvid[b.nhash]; // occupied voxels: persistent threads stride over them
+    const uint32_t nv = b.state[0].n_comp;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
-        k_uf_flatten_one(b, v);
+    {
+        const uint32_t slot = b.vlist[v];
+        int budget = kMaxIters;
+        const uint32_t root = uf_find(b.hrec, slot, &b.state[scan_of_hash(b, slot)], budget);
+        if (root == slot)
+            continue;
+        uint4* rec = &b.hrec[slot];
+        rec->w = root;
+        uint32_t* rr = reinterpret_cast<uint32_t*>(&b.hrec[root]);
+        atomicMin(&rr[1], rec->y);
+        atomicAdd(&rr[2], rec->z);
+    }
 }
 
-__device__ __forceinline__ void k_comp_stats_one(const BatchDev& b, uint32_t v)
+// Component flags in obstacle order: 1 at the smallest obstacle of every component that is kept
+// (removeSmallClusters, clusterer.cpp:195-239). The obstacle's root is left in obs_label for the pass
+// after the scan.
+struct KeepSrc
 {
-    const uint32_t root = b.parent[v];
-    const uint32_t slot = b.vslot[v];
-    atomicMin(&b.cmin[root], b.hmin[slot]);
-    atomicAdd(&b.ccnt[root], b.hcnt[slot]);
-}
-
-__global__ void k_comp_stats(BatchDev b)
-{
-    const uint32_t nv = b.hvid[b.nhash]; // occupied voxels: persistent threads stride over them
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
-        k_comp_stats_one(b, v);
-}
-
-__device__ __forceinline__ void k_keep_one(const BatchDev& b, uint32_t v)
-{
-    if (b.parent[v] != v)
-        return;
-    const uint32_t slot = b.vslot[v];
-    const int s = scan_of_hash(b, slot);
-    if (b.ccnt[v] >= b.scans[s].min_cluster)
-        b.kflag[b.state[s].obs_off + b.cmin[v]] = 1u;
-}
-
-__global__ void k_keep(BatchDev b)
-{
-    const uint32_t nv = b.hvid[b.nhash];
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
-        k_keep_one(b, v);
-}
+    BatchDev b;
+    __device__ __forceinline__ uint32_t end() const { return b.obs_flag[b.npts] + 1u; }
+    __device__ __forceinline__ uint32_t one(uint32_t o, uint32_t n) const
+    {
+        if (o >= n)
+            return 0u;
+        const uint32_t slot = b.obs_hslot[o];
+        if (slot == kEmpty)
+        {
+            b.obs_label[o] = -1;
+            return 0u;
+        }
+        const uint32_t root = b.hrec[slot].w;
+        b.obs_label[o] = static_cast<int32_t>(root);
+        const int s = scan_of_obs(b, o);
+        const uint4 r = b.hrec[root];
+        return (r.y == o - b.state[s].obs_off && r.z >= b.scans[s].min_cluster) ? 1u : 0u;
+    }
+    __device__ __forceinline__ uint4 get4(uint32_t i) const
+    {
+        const uint32_t n = b.obs_flag[b.npts];
+        return make_uint4(one(i, n), one(i + 1u, n), one(i + 2u, n), one(i + 3u, n));
+    }
+};
 
 // kflag now holds the exclusive scan: rank of each kept component among the scan's kept
 // components ordered by smallest point index == the reference's final label.
 __global__ void k_obs_label(BatchDev b)
 {
     __shared__ BlockAgg agg;
+    if (blockIdx.x == 0)
+        for (int s = static_cast<int>(threadIdx.x); s < b.nscan; s += static_cast<int>(blockDim.x))
+        {
+            ScanState& st = b.state[s];
+            st.n_clusters = b.kflag[st.obs_off + st.n_obs] - b.kflag[st.obs_off];
+            if (st.n_clusters > b.scans[s].cluster_cap)
+                raise_err(&st, ERR_CLUSTER_CAPACITY);
+        }
     const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = o < b.obs_flag[b.npts];
     int32_t label = LP_INVALID_CLUSTER;
@@ -430,29 +446,17 @@ __global__ void k_obs_label(BatchDev b)
         const int s = scan_of_obs(b, o);
         const ScanDev& sd = b.scans[s];
         const ScanState& st = b.state[s];
-        const uint32_t slot = b.obs_hslot[o];
-        if (slot != kEmpty)
+        const int32_t root = b.obs_label[o]; // a hash slot (KeepSrc)
+        if (root >= 0)
         {
-            const uint32_t root = b.parent[b.hvid[slot]];
-            if (b.ccnt[root] >= sd.min_cluster)
-                label = static_cast<int32_t>(b.kflag[st.obs_off + b.cmin[root]] - b.kflag[st.obs_off]);
+            const uint4 r = b.hrec[root];
+            if (r.z >= sd.min_cluster)
+                label = static_cast<int32_t>(b.kflag[st.obs_off + r.y] - b.kflag[st.obs_off]);
         }
         b.obs_label[o] = label;
         g = sd.cl_off + static_cast<uint32_t>(label);
     }
     block_aggregated_inc(b.cl_cnt, g, in && label >= 0, agg);
-}
-
-__global__ void k_cl_state(BatchDev b)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.nscan)
-        return;
-    const ScanDev& sd = b.scans[s];
-    ScanState& st = b.state[s];
-    st.n_clusters = b.kflag[st.obs_off + st.n_obs] - b.kflag[st.obs_off];
-    if (st.n_clusters > sd.cluster_cap)
-        raise_err(&st, ERR_CLUSTER_CAPACITY);
 }
 
 // Members grouped by cluster (slot order within a cluster is free), with their x, y alongside for
@@ -534,33 +538,29 @@ void launch_mark_all_obstacles(Launcher& L, const BatchDev& b)
 
 void launch_clustering(Launcher& L, const BatchDev& b, const BatchHost& hb)
 {
-    const uint32_t T = 256;
-    const uint32_t ns = static_cast<uint32_t>(b.nscan);
-    LP_LAUNCH(L, k_obs_flag, div_up(b.npts + 1, T), T, b);
-    L.scan(b.obs_flag, b.obs_flag, b.npts + 1);
-    LP_LAUNCH(L, k_obs_state, div_up(ns, 64u), 64, b);
-    LP_LAUNCH(L, k_obs_gather, div_up(b.npts, kObsChunk), 256, b);
-    LP_LAUNCH(L, k_dims, div_up(ns, 64u), 64, b);
-    LP_LAUNCH(L, k_vox_insert, div_up(b.npts, T), T, b);
-    if (uint32_t* words = L.scan_state(b.nhash + 1))
-    {
-        L.begin("k_vox_ids");
-        scan_lookback(L.stream, VoxFlagsSrc{b.hkey, b.nhash},
-                      VoxInitDst{b.hvid, b.vslot, b.parent, b.cmin, b.ccnt, b.nhash + 1}, b.nhash + 1, words, L.scan_err, true);
-        L.end();
-        L.note();
-    }
-    LP_LAUNCH(L, k_vox_count, div_up(ns, 64u), 64, b);
-    const uint32_t vgrid = std::min(div_up(b.nhash, T), static_cast<uint32_t>(sm_count()) * 8u); // <= voxels
-    LP_LAUNCH(L, k_uf_hook, vgrid, T, b);
-    LP_LAUNCH(L, k_uf_flatten, vgrid, T, b);
-    LP_LAUNCH(L, k_comp_stats, vgrid, T, b);
-    LP_LAUNCH(L, k_keep, vgrid, T, b);
-    L.scan(b.kflag, b.kflag, b.npts + 1);
-    LP_LAUNCH(L, k_obs_label, div_up(b.npts, T), T, b);
-    LP_LAUNCH(L, k_cl_state, div_up(ns, 64u), 64, b);
-    L.scan(b.cl_cnt, b.cl_start, b.ncl + 1);
-    LP_LAUNCH(L, k_cl_scatter, div_up(b.npts, T), T, b);
     (void)hb;
+    const uint32_t T = 256;
+    auto scan = [&](const char* name, auto src, uint32_t* out) {
+        if (uint32_t* words = L.scan_state(b.npts + 1))
+        {
+            L.begin(name);
+            scan_lookback(L.stream, src, ScanDstU32{out, b.npts + 1, true}, b.npts + 1, words, L.scan_err, true);
+            L.end();
+            L.note();
+        }
+    };
+    scan("k_obs_scan", ObsFlagSrc{b.seg_label, b.npts}, b.obs_flag);
+    LP_LAUNCH(L, k_obs_gather, div_up(b.npts, kObsChunk), 256, b);
+    LP_LAUNCH(L, k_vox_insert, div_up(b.npts, T), T, b);
+    const uint32_t vgrid = std::min(div_up(13u * std::max(b.npts, 1u), T), static_cast<uint32_t>(sm_count()) * 8u);
+    LP_LAUNCH(L, k_uf_hook, vgrid, T, b);
+    LP_LAUNCH(L, k_uf_flatten, std::min(div_up(b.npts, T), static_cast<uint32_t>(sm_count()) * 8u), T, b);
+    scan("k_keep_scan", KeepSrc{b}, b.kflag);
+    LP_LAUNCH(L, k_obs_label, div_up(b.npts, T), T, b);
+}
+
+void launch_cluster_scatter(Launcher& L, const BatchDev& b)
+{
+    LP_LAUNCH(L, k_cl_scatter, div_up(b.npts, 256u), 256, b);
 }
 } // namespace lpg

@@ -43,7 +43,7 @@ void launch_debug_wait_timeout(cudaStream_t st, int kind, uint32_t limit, unsign
     {
         const unsigned long long start[4] = {1ull, 0ull, 0ull, 0ull};
         cudaMemcpyAsync(state, start, sizeof(start), cudaMemcpyHostToDevice, st);
-        k_scan_lb<<<1, kLbThreads, 0, st>>>(ScanSrcU32{nullptr, 0u, false}, ScanDstU32{nullptr, 0u, false}, state, err,
+        k_scan_lb<8><<<1, kLbThreads, 0, st>>>(ScanSrcU32{nullptr, 0u, false}, ScanDstU32{nullptr, 0u, false}, state, err,
                                             limit);
     }
     else

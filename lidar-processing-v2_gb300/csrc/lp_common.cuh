@@ -276,23 +276,21 @@ __host__ __device__ inline uint32_t div_up(uint32_t a, uint32_t b)
 
 // ---------------------------------------------------------------------------------------------
 // Single-pass exclusive scan with decoupled look-back (Merrill & Garland, "Single-pass Parallel
-// Prefix Scan with Decoupled Look-back", 2016). Tiles of kLbTile elements take dynamic tickets, so
+// Prefix Scan with Decoupled Look-back", 2016). Tiles of 1024 kRows elements take dynamic tickets, so
 // every tile a block waits for has already started (and waits only for earlier ones): each
 // look-back ends. A tile publishes (flag, value) in one 64-bit word: flag 1 = the tile's own sum,
 // flag 2 = the inclusive prefix through the tile. Waits are bounded anyway; running out sets
 // ERR_INTERNAL in *err (the result of that scan is then wrong and the batch reports an error).
 // state[0] holds the ticket counter, state[1 + t] tile t's word; the launcher zeroes them.
 //
-// Each warp owns 1024 consecutive elements of its tile and moves them as 8 rows of 32 x uint4
+// Each warp owns 128 kRows consecutive elements of its tile and moves them as rows of 32 x uint4
 // (every load and store instruction of a warp covers 512 contiguous bytes). `Src::get4(i)` gives
 // elements i..i+3 (zero past the end), `Dst::put4(i, excl, val)` receives their exclusive
-// prefixes and values, so producers and consumers of a scan can be fused into it.
+// prefixes and values, so producers and consumers of a scan can be fused into it. `Src::end()`: where
+// the elements end (may lie before the grid's end, read on the device).
 // ---------------------------------------------------------------------------------------------
 constexpr uint32_t kLbThreads = 256;
-constexpr uint32_t kLbRows = 8;
-constexpr uint32_t kLbWarpSpan = kLbRows * 32u * 4u;           // 1024 elements per warp
-constexpr uint32_t kLbTile = (kLbThreads / 32u) * kLbWarpSpan; // 8192 elements per tile
-static_assert(kLbTile == 8192u, "Launcher::scan_state counts tiles of 8192");
+
 constexpr unsigned long long kLbAgg = 1ull << 62, kLbPre = 2ull << 62;
 
 __device__ __forceinline__ unsigned long long ld_status(const unsigned long long* p)
@@ -354,7 +352,7 @@ __device__ __forceinline__ uint32_t lb_tile_prefix(unsigned long long* tiles, ui
 
 constexpr uint32_t kLbPollLimit = 1u << 24; // polls of a predecessor's word before giving up
 
-template <class Src, class Dst>
+template <uint32_t kRows, class Src, class Dst>
 __global__ void __launch_bounds__(kLbThreads) k_scan_lb(Src src, Dst dst, unsigned long long* state, uint32_t* err,
                                                         uint32_t poll_limit)
 {
@@ -364,16 +362,19 @@ __global__ void __launch_bounds__(kLbThreads) k_scan_lb(Src src, Dst dst, unsign
         s_tile = atomicAdd(reinterpret_cast<unsigned int*>(state), 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
+    constexpr uint32_t kSpan = kRows * 32u * 4u, kTile = (kLbThreads / 32u) * kSpan;
+    if (tile != 0u && tile * kTile >= src.end())
+        return; // nothing from here on: no later tile waits for this one
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    const uint32_t wbase = tile * kLbTile + warp * kLbWarpSpan;
-    uint4 v[kLbRows];
+    const uint32_t wbase = tile * kTile + warp * kSpan;
+    uint4 v[kRows];
 #pragma unroll
-    for (uint32_t q = 0; q < kLbRows; ++q)
+    for (uint32_t q = 0; q < kRows; ++q)
         v[q] = src.get4(wbase + (q * 32u + lane) * 4u);
-    uint32_t rowx[kLbRows]; // exclusive prefix of this lane's 4 elements within the warp's span
+    uint32_t rowx[kRows]; // exclusive prefix of this lane's 4 elements within the warp's span
     uint32_t wrun = 0;
 #pragma unroll
-    for (uint32_t q = 0; q < kLbRows; ++q)
+    for (uint32_t q = 0; q < kRows; ++q)
     {
         const uint32_t sq = v[q].x + v[q].y + v[q].z + v[q].w;
         const uint32_t inc = warp_incl_scan(sq);
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(kLbThreads) k_scan_lb(Src src, Dst dst, unsign
     __syncthreads();
     const uint32_t wpre = s_warp[warp];
 #pragma unroll
-    for (uint32_t q = 0; q < kLbRows; ++q)
+    for (uint32_t q = 0; q < kRows; ++q)
     {
         uint4 e;
         e.x = wpre + rowx[q];
@@ -406,20 +407,17 @@ __global__ void __launch_bounds__(kLbThreads) k_scan_lb(Src src, Dst dst, unsign
     }
 }
 
-// Words a scan of n elements needs (zeroed): the ticket counter and one per tile.
-inline uint32_t scan_words(uint32_t n)
-{
-    return div_up(n, kLbTile) + 1u;
-}
-
 template <class Src, class Dst>
 void scan_lookback(cudaStream_t st, Src src, Dst dst, uint32_t n, uint32_t* sums, uint32_t* err, bool zeroed = false)
 {
-    const uint32_t nt = div_up(n, kLbTile);
+    const uint32_t nt = div_up(n, scan_tile(n));
     unsigned long long* state = reinterpret_cast<unsigned long long*>(sums);
     if (!zeroed)
         cudaMemsetAsync(state, 0, scan_words(n) * sizeof(unsigned long long), st);
-    k_scan_lb<<<nt, kLbThreads, 0, st>>>(src, dst, state, err, kLbPollLimit);
+    if (scan_tile(n) == 1024u)
+        k_scan_lb<1><<<nt, kLbThreads, 0, st>>>(src, dst, state, err, kLbPollLimit);
+    else
+        k_scan_lb<8><<<nt, kLbThreads, 0, st>>>(src, dst, state, err, kLbPollLimit);
 }
 
 // Plain u32 arrays as scan source and destination (vector accesses when 16-byte aligned).
@@ -428,6 +426,7 @@ struct ScanSrcU32
     const uint32_t* p;
     uint32_t n;
     bool vec;
+    __device__ __forceinline__ uint32_t end() const { return 0xffffffffu; } // the grid ends with the elements
     __device__ __forceinline__ uint4 get4(uint32_t i) const
     {
         if (vec && i + 4u <= n)

@@ -1242,7 +1242,7 @@ __global__ void __launch_bounds__(256) k_hull_pre_ref(BatchDev b)
                 emar[e] = make_float2(1e-5f * l1, 1e-6f * l1);
             }
             __syncthreads();
-            uint32_t* act0 = reinterpret_cast<uint32_t*>(b.hs_stack + 2ull * start + 2ull * g);
+            uint32_t* act0 = reinterpret_cast<uint32_t*>(b.hs_stack + 2ull * start + 2ull * b.cl_rank[g]);
             for (uint32_t base = i0; base < i1; base += blockDim.x)
             {
                 const uint32_t i = base + threadIdx.x;
@@ -1400,7 +1400,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
     //    while it grows and fits. Every vertex is a member, so the polygon stays inside the hull.
     //    Members proven strictly inside the current polygon leave the active set: the float test
     //    keeps a 1e-5 relative margin, far above its rounding error, so no hull vertex is dropped.
-    uint32_t* act[2] = {reinterpret_cast<uint32_t*>(b.hs_stack + 2ull * start + 2ull * g), nullptr};
+    uint32_t* act[2] = {reinterpret_cast<uint32_t*>(b.hs_stack + 2ull * start + 2ull * b.cl_rank[g]), nullptr};
     act[1] = act[0] + n; // two member lists of n entries in the chain-stack scratch (2n + 2)
     int cur = -1;        // -1: the active set is all members
     uint32_t nact = n;
@@ -1575,7 +1575,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
     {
         block_sort_global(gs, static_cast<uint32_t>(m));
         C = gs;
-        H = b.hs_stack + 2ull * start + 2ull * g; // capacity 2n + 2 >= 2m + 2
+        H = b.hs_stack + 2ull * start + 2ull * b.cl_rank[g]; // capacity 2n + 2 >= 2m + 2
     }
     __syncthreads();
     // lower half on thread 0, upper half on thread 32 (another warp) into H + m + 1; then the
@@ -1642,7 +1642,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
         // the refinement's edge records are free: float scratch of the calipers screen
         if (warp == 0)
             calipers_box(st, P, fast ? sm.pf : nullptr, reinterpret_cast<float*>(sm.erec), h,
-                         b.hs_pairs + 4ull * start + 16ull * g, &b.obb_c[g]);
+                         b.hs_pairs + 4ull * start + 16ull * b.cl_rank[g], &b.obb_c[g]);
         else
             pca_box_warp(P, h, &b.obb_p[g]);
     }
@@ -1997,7 +1997,7 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
         __syncwarp();
     }
     HPt<float>* C = small ? ws.cand : gs;
-    int* H = small ? ws.stack : (b.hs_stack + 2ull * start + 2ull * g);
+    int* H = small ? ws.stack : (b.hs_stack + 2ull * start + 2ull * b.cl_rank[g]);
     if (m <= 32u)
     {
         // one candidate per lane, sorted in registers (hpt_less is a total order: any sort agrees)
@@ -2074,17 +2074,20 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
         __syncwarp();
         // the chain stack is free again: float scratch of the calipers screen
         calipers_box(st, P, fast ? ws.pf : nullptr, reinterpret_cast<float*>(ws.stack), h,
-                     b.hs_pairs + 4ull * start + 16ull * g, &b.obb_c[g]);
+                     b.hs_pairs + 4ull * start + 16ull * b.cl_rank[g], &b.obb_c[g]);
         pca_box_warp(P, h, &b.obb_p[g]);
     }
     __syncwarp();
 }
 
 // Work items: every cluster of the batch. queue[2] counts clusters of more than kBigCluster
-// members (listed from the front of `work`, taken by whole CTAs first), queue[3] the others
-// (listed from the back, taken one warp each).
-__global__ void k_hull_worklist(BatchDev b, uint32_t* work)
+// members (listed from the front of hull_work, taken by whole CTAs first), queue[3] the others
+// (listed from the back, taken one warp each). A cluster's member range is reserved here too, with its rank
+// in the order of the ranges (queue[8..9]; scratch that has a fixed part per cluster lies at a multiple
+// of the start plus one of the rank), and its counters start at zero.
+__global__ void k_hull_worklist(BatchDev b)
 {
+    uint32_t* work = b.hull_work;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= b.ncl)
         return;
@@ -2092,6 +2095,11 @@ __global__ void k_hull_worklist(BatchDev b, uint32_t* work)
     if (g - b.scans[s].cl_off >= b.state[s].n_clusters)
         return;
     const uint32_t n = b.cl_cnt[g];
+    const unsigned long long got = atomicAdd(reinterpret_cast<unsigned long long*>(&b.queue[8]), (1ull << 32) | n);
+    b.cl_start[g] = static_cast<uint32_t>(got);
+    b.cl_rank[g] = static_cast<uint32_t>(got >> 32);
+    b.cl_fill[g] = 0u;
+    b.cl_zkey[2u * g] = b.cl_zkey[2u * g + 1u] = 0u;
     if (n > b.hull_cta_min) // hull_cta_min <= kBigCluster: the warp path's limit
         work[atomicAdd(&b.queue[2], 1u)] = g;
     else
@@ -2110,12 +2118,6 @@ __global__ void k_hull_worklist(BatchDev b, uint32_t* work)
         for (uint32_t c = 0; c < nch; ++c)
             b.pre_items[at + c] = make_uint2(g, c);
     }
-}
-
-__device__ __forceinline__ uint32_t work_item(const BatchDev& b, const uint32_t* work, uint32_t w)
-{
-    const uint32_t nbig = b.queue[2];
-    return (w < nbig) ? work[w] : work[b.ncl - 1u - (w - nbig)];
 }
 
 constexpr size_t kHullDynSmem = sizeof(HullSmem) > (kHullThreads / 32) * sizeof(WarpSmem)
@@ -2166,7 +2168,6 @@ __global__ void __launch_bounds__(kHullThreads) k_hull(BatchDev b, int compute_o
     }
 }
 
-// Dense hull output: hull_cnt holds the exclusive scan (hull offsets over the batch).
 // ---------------------------------------------------------------------------------------------
 // The reference's order among identical points (Polygonizer::convexHull, polygonizer.cpp:51-59):
 // std::sort orders the point indices by x, then (|dx| < DBL_EPSILON) y, and leaves points that
@@ -2293,12 +2294,12 @@ __global__ void __launch_bounds__(kHullThreads) k_hull_ties(BatchDev b)
     {
         const uint32_t g = b.tie_list[t];
         const uint32_t start = b.cl_start[g], n = b.cl_cnt[g];
-        const int h = static_cast<int>(b.hull_cnt[g + 1] - b.hull_cnt[g]); // scanned: offsets
+        const int h = static_cast<int>(b.hull_cnt[g]);
         const bool local = n <= kTieSmemRecs;
         HRec<float>* rec = local ? reinterpret_cast<HRec<float>*>(tsm)
                                  : reinterpret_cast<HRec<float>*>(reinterpret_cast<HPt<float>*>(b.hs_cand) + 2ull * start);
         uint32_t* ge = local ? reinterpret_cast<uint32_t*>(tsm + kTieSmemRecs * sizeof(HRec<float>))
-                             : reinterpret_cast<uint32_t*>(b.hs_stack + 2ull * start + 2ull * g);
+                             : reinterpret_cast<uint32_t*>(b.hs_stack + 2ull * start + 2ull * b.cl_rank[g]);
         uint32_t* le = ge + (local ? kTieSmemRecs : n);
         for (uint32_t k = threadIdx.x; k < n; k += blockDim.x)
         {
@@ -2319,16 +2320,46 @@ __global__ void __launch_bounds__(kHullThreads) k_hull_ties(BatchDev b)
     }
 }
 
-__global__ void k_hull_compact(BatchDev b, const uint32_t* work)
+// Dense hull output, one CTA per scan: hull_cnt becomes the exclusive scan of its hulls' sizes, from
+// the scan's pt_off (K + 1 entries), and the hulls move behind one another into hull_out.
+constexpr uint32_t kFinishThreads = 1024;
+
+__global__ void __launch_bounds__(kFinishThreads) k_hull_finish(BatchDev b)
 {
-    const uint32_t total = b.queue[2] + b.queue[3];
-    for (uint32_t w = blockIdx.x; w < total; w += gridDim.x)
+    __shared__ uint32_t sm[33];
+    __shared__ uint32_t soff[kFinishThreads + 1], sst[kFinishThreads];
+    const ScanDev& sd = b.scans[blockIdx.x];
+    const uint32_t K = min(b.state[blockIdx.x].n_clusters, sd.cluster_cap - 1u);
+    uint32_t base = sd.pt_off;
+    for (uint32_t k0 = 0; k0 <= K; k0 += kFinishThreads)
     {
-        const uint32_t g = work_item(b, work, w);
-        const uint32_t off = b.hull_cnt[g];
-        const uint32_t cnt = b.hull_cnt[g + 1] - off;
-        for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x)
-            b.hull_out[off + i] = b.hull_tmp[b.cl_start[g] + i];
+        const uint32_t k = k0 + threadIdx.x, g = sd.cl_off + k;
+        const uint32_t h = (k < K) ? b.hull_cnt[g] : 0u;
+        uint32_t total;
+        const uint32_t at = base + block_excl_scan(h, sm, &total); // (its barriers: the counts are read)
+        if (k <= K)
+            b.hull_cnt[g] = at;
+        soff[threadIdx.x] = at;
+        sst[threadIdx.x] = (k < K) ? b.cl_start[g] : 0u;
+        if (threadIdx.x == 0)
+            soff[kFinishThreads] = base + total;
+        __syncthreads();
+        // vertex by vertex: its hull is the last that starts at or before it
+        for (uint32_t v = base + threadIdx.x; v < base + total; v += kFinishThreads)
+        {
+            uint32_t lo = 0u, hi = kFinishThreads - 1u;
+            while (lo < hi)
+            {
+                const uint32_t mid = (lo + hi + 1u) / 2u;
+                if (soff[mid] <= v)
+                    lo = mid;
+                else
+                    hi = mid - 1u;
+            }
+            b.hull_out[v] = b.hull_tmp[sst[lo] + (v - soff[lo])];
+        }
+        base += total;
+        __syncthreads();
     }
 }
 
@@ -2767,18 +2798,15 @@ void launch_objects_gates(cudaStream_t st, const ObjDev& o, const VehicleTableDe
 
 void launch_polygons(Launcher& L, const BatchDev& b, const BatchHost& hb, int compute_obb)
 {
-    (void)hb;
-    // the work list reuses the cluster fill counters' scratch (cl_fill, ncl + 1 entries)
-    uint32_t* work = b.cl_fill;
-    LP_LAUNCH(L, k_hull_worklist, div_up(b.ncl, 256u), 256, b, work);
+    LP_LAUNCH(L, k_hull_worklist, div_up(b.ncl, 256u), 256, b);
+    launch_cluster_scatter(L, b);
     LP_LAUNCH(L, k_hull_pre_ext, static_cast<uint32_t>(sm_count()) * 4u, 256, b);
     LP_LAUNCH(L, k_hull_pre_ref, static_cast<uint32_t>(sm_count()) * 4u, 256, b);
     const int sms = sm_count();
     LP_LAUNCH_SMEM(L, k_hull, static_cast<uint32_t>(sms) * hb.hull_ctas_per_sm, kHullThreads, kHullDynSmem, b, compute_obb,
-                   static_cast<const uint32_t*>(work));
-    L.scan(b.hull_cnt, b.hull_cnt, b.ncl + 1);
+                   static_cast<const uint32_t*>(b.hull_work));
     LP_LAUNCH_SMEM(L, k_hull_ties, static_cast<uint32_t>(sms), kHullThreads, kTieDynSmem, b);
-    LP_LAUNCH(L, k_hull_compact, static_cast<uint32_t>(sms * 8), 128, b, static_cast<const uint32_t*>(work));
+    LP_LAUNCH(L, k_hull_finish, static_cast<uint32_t>(b.nscan), kFinishThreads, b);
 }
 
 void init_kernel_attributes()

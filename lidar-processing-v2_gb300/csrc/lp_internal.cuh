@@ -57,7 +57,7 @@ struct ScanDev
     // clustering constants (clusterer.hpp:76-90)
     float res_r, res_a, res_e;
     uint32_t min_cluster;
-    uint32_t hash_off, hash_cap; // voxel hash table slice (power of two)
+    uint32_t hash_cap; // most voxel hash slots the scan can need (power of two)
     // per-cluster output capacity
     uint32_t cluster_cap, hull_cap;
     uint32_t cl_off; // offset of this scan's cluster arrays
@@ -82,8 +82,9 @@ struct ScanState
     uint32_t n_obs, obs_off;
     uint32_t max_r_bits, max_a_bits, max_e_bits;
     int32_t nr, na, ne;
+    uint32_t hash_off, hash_mask; // voxel hash slice: first slot, slots - 1
     uint32_t n_vox;
-    uint32_t n_comp;
+    uint32_t n_comp; // of the batch's first scan: voxels listed (all scans)
     uint32_t n_clusters;
     uint32_t cl_base; // clusters of earlier scans (work-queue numbering)
     uint32_t n_hull;
@@ -123,6 +124,25 @@ __device__ __forceinline__ uint32_t fkey(float v)
 __device__ __forceinline__ uint32_t lane_id()
 {
     return threadIdx.x & 31u;
+}
+
+// Elements per tile of a device-wide scan over n elements. A tile is one CTA: short scans take small
+// tiles, so that their loads spread over the chip (1,024 elements up to 1 Mi: at most 1,024 tiles to
+// look back over), long ones large tiles, so that the look-back stays short.
+__host__ __device__ constexpr uint32_t scan_tile(uint32_t n)
+{
+    return n <= (1u << 20) ? 1024u : 8192u;
+}
+// 64-bit words a scan over n elements needs (zeroed): the ticket counter and one per tile.
+__host__ __device__ constexpr uint32_t scan_words(uint32_t n)
+{
+    return (n + scan_tile(n) - 1u) / scan_tile(n) + 1u;
+}
+
+// At least scan_words(m) for every m <= n (short scans have small tiles, so they can need more).
+__host__ __device__ constexpr uint32_t scan_words_max(uint32_t n)
+{
+    return scan_words(n) > scan_words(1u << 20) ? scan_words(n) : scan_words(n < (1u << 20) ? n : 1u << 20);
 }
 
 // Kernel launch bookkeeping (counted by the host wrapper for instrumentation).

@@ -24,6 +24,7 @@ struct SplitSrc
     const uint32_t* lab;
     uint32_t n;
     int cls;
+    __device__ __forceinline__ uint32_t end() const { return 0xffffffffu; }
     __device__ __forceinline__ uint4 get4(uint32_t i) const
     {
         uint4 f;

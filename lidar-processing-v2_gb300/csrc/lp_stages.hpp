@@ -83,8 +83,8 @@ struct Launcher
     template <typename K, typename... Args>
     void launch(const char* name, K kernel, uint32_t grid, uint32_t block, Args... args)
     {
-        if (grid == 0)
-            return;
+        if (grid == 0 || err != cudaSuccess)
+            return; // nothing runs after a failed step: its inputs would be undefined
         begin(name);
         kernel<<<grid, block, 0, stream>>>(args...);
         end();
@@ -93,7 +93,7 @@ struct Launcher
     template <typename K, typename... Args>
     void launch2d(const char* name, K kernel, dim3 grid, uint32_t block, Args... args)
     {
-        if (grid.x == 0 || grid.y == 0)
+        if (grid.x == 0 || grid.y == 0 || err != cudaSuccess)
             return;
         begin(name);
         kernel<<<grid, block, 0, stream>>>(args...);
@@ -103,8 +103,8 @@ struct Launcher
     template <typename K, typename... Args>
     void launch_smem(const char* name, K kernel, uint32_t grid, uint32_t block, size_t smem, Args... args)
     {
-        if (grid == 0)
-            return;
+        if (grid == 0 || err != cudaSuccess)
+            return; // nothing runs after a failed step: its inputs would be undefined
         begin(name);
         kernel<<<grid, block, smem, stream>>>(args...);
         end();
@@ -125,8 +125,8 @@ struct Launcher
     // Look-back words of a scan over n elements (null, with the error noted, when the run has none left).
     uint32_t* scan_state(uint32_t n)
     {
-        const size_t words = (static_cast<size_t>(n) + 8191u) / 8192u + 1u; // scan_words(n)
-        if (words > scan_left)
+        const size_t words = scan_words(n);
+        if (words > scan_left || err != cudaSuccess)
         {
             if (err == cudaSuccess)
                 err = cudaErrorInvalidValue;
@@ -225,6 +225,7 @@ struct BatchHost
 void launch_segmentation(Launcher& L, const BatchDev& b, const BatchHost& hb, uint8_t* d_image);
 void launch_ring_only(Launcher& L, const BatchDev& b, const BatchHost& hb);
 void launch_clustering(Launcher& L, const BatchDev& b, const BatchHost& hb);
+void launch_cluster_scatter(Launcher& L, const BatchDev& b); // members by cluster, for the hulls
 void launch_polygons(Launcher& L, const BatchDev& b, const BatchHost& hb, int compute_obb);
 void launch_noise(Launcher& L, const BatchDev& b, const BatchHost& hb, const lp_noise_remover_config& cfg);
 void launch_noise_compaction(Launcher& L, const BatchDev& b, const BatchHost& hb);
