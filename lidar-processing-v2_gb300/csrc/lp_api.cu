@@ -297,9 +297,9 @@ size_t carve(lp_batch& B, char* base)
         put(b.zlow, b.ncell);
         put(b.elev, b.ncell);
         put(b.large_list, b.ncell);
-        put(b.n_large, 1);
-        put(b.near_cnt, b.nnear + 1);
-        put(b.near_start, b.nnear + 1);
+        put(b.near_cnt, b.nnear);
+        put(b.near_start, static_cast<size_t>(kNearCopies) * b.nnear);
+        put(b.ransac_done, 1);
         put(b.cand, N);
         put(b.planes, S * kMaxRansacIters);
         put(b.pvalid, S);
@@ -445,7 +445,7 @@ lp_status execute(lp_context* ctx, lp_batch& B, bool outputs)
     L.event_pool = &ctx->events;
     if (B.profiling)
         L.prof = &B.prof;
-    const size_t N = b.npts;
+    const size_t N = b.npts, S = static_cast<size_t>(b.nscan);
     const bool noise = R.stages & ST_NOISE, clu = R.stages & (ST_CLUSTER | ST_ALL_OBS);
     FillList f;
     f.add(B.scan_sums, B.scan_words * 8, 0u);
@@ -462,8 +462,9 @@ lp_status execute(lp_context* ctx, lp_batch& B, bool outputs)
     {
         f.add(b.seg_label, N * 4, 0u);
         f.add(b.cell_cnt, (static_cast<size_t>(b.ncell) + 1) * 4, 0u);
-        f.add(b.n_large, 4, 0u);
-        f.add(b.near_cnt, (static_cast<size_t>(b.nnear) + 1) * 4, 0u);
+        f.add(b.ransac_done, 4, 0u);
+        f.add(b.pvalid, S * 8, 0u);
+        f.add(b.inliers, S * kMaxRansacIters * 4, 0u);
         f.add(b.pix_depth, static_cast<size_t>(b.npix) * 4, 0xffffffffu);
         f.add(b.pix_key, static_cast<size_t>(b.npix) * 8, 0xffffffffu);
         f.add(b.row_cnt, static_cast<size_t>(b.nrows) * 4, 0u);

@@ -39,6 +39,7 @@ enum : uint8_t
 constexpr uint32_t kKtPoolPerPoint = 8; // leftover search entries per point the DROR pool holds
 // Raw weight record of the jump convolution: 24 weights, padded to a multiple of 16 bytes.
 constexpr uint32_t kJwStride = 28;
+constexpr uint32_t kNearCopies = 4; // one per CTA that draws a scan's hypotheses
 constexpr uint32_t kJrecFields = 10; // 16-byte fields of an open pixel's record (jrec in lp_segment.cu)
 
 // A scan's buffers in the caller's page-locked host memory (device-accessible addresses).
@@ -94,17 +95,17 @@ struct BatchDev
     float* csr_z;
     float* zlow;       // per cell
     float* elev;       // per cell
-    uint32_t* large_list;
-    uint32_t* n_large;
+    uint32_t* large_list; // per slice (at its first cell): cells whose heights have to be sorted
 
     // ---- RANSAC ------------------------------------------------------------------------------
     uint32_t nnear;
-    uint32_t* near_cnt;
-    uint32_t* near_start;
-    float4* cand;
+    uint32_t* near_cnt;   // RANSAC candidates per near cell
+    uint32_t* near_start; // kNearCopies x nnear: first candidate rank of each near cell
+    float4* cand;         // candidates of a scan from its pt_off, unordered
     float4* planes;            // nscan * 60
     unsigned long long* pvalid; // nscan: bit it = hypothesis it usable
     uint32_t* inliers;         // nscan * 60
+    uint32_t* ransac_done;     // CTAs of the inlier count that have finished
 
     // ---- projection / range image ------------------------------------------------------------
     uint8_t* pt_label; // per point after RECM + RANSAC

@@ -24,18 +24,9 @@ constexpr float kPi2F = 1.57079637050628662109f;      // M_PI_2f
 constexpr float kPi15F = 4.71238899230957031250f;     // 1.5F * M_PIf (dataloader.cpp:108)
 constexpr float kTwoPiF = 6.28318548202514648438f;    // 2.0F * M_PIf == (float)(2*M_PI)
 constexpr int kRingTile = 1024;
-constexpr int kSmallCell = 32;   // sorted in registers by one warp
 constexpr int kMediumCell = 256; // sorted in shared memory by one warp
 constexpr uint32_t kLargeCellMax = 8192;
 
-__device__ __forceinline__ int scan_of_cell(const BatchDev& b, uint32_t c)
-{
-    return find_scan(b.nscan, c, [&](int s) { return b.scans[s].cell_off; });
-}
-__device__ __forceinline__ int scan_of_near(const BatchDev& b, uint32_t g)
-{
-    return find_scan(b.nscan, g, [&](int s) { return b.scans[s].near_off; });
-}
 __device__ __forceinline__ int scan_of_pix(const BatchDev& b, uint32_t p)
 {
     return find_scan(b.nscan, p, [&](int s) { return b.scans[s].pix_off; });
@@ -180,9 +171,7 @@ __device__ __forceinline__ int32_t bin_point(const BatchDev& b, uint32_t i, cons
     return static_cast<int32_t>(sd.cell_off + static_cast<uint32_t>(slice * sd.nrad + radial));
 }
 
-// Two points per thread (i and i + blockDim.x), both loaded before either is binned. Each
-// aggregated slot increment covers 32 consecutive points of one warp: a cell's slots come in
-// index runs of one 32-point window each (the near-cell ordering relies on it, and checks it).
+// Two points per thread (i and i + blockDim.x), both loaded before either is binned.
 __global__ void k_bin(BatchDev b)
 {
     const uint32_t i0 = blockIdx.x * blockDim.x * 2u + threadIdx.x;
@@ -196,7 +185,7 @@ __global__ void k_bin(BatchDev b)
         b.pt_cell[i0] = c0;
     if (i1 < b.npts)
         b.pt_cell[i1] = c1;
-    // slot of the point in its cell (the order within a cell is free: near cells are ordered later)
+    // slot of the point in its cell (the order within a cell is free)
     const uint32_t s0 = warp_aggregated_inc(b.cell_cnt, static_cast<uint32_t>(c0), c0 >= 0);
     const uint32_t s1 = warp_aggregated_inc(b.cell_cnt, static_cast<uint32_t>(c1), c1 >= 0);
     if (c0 >= 0)
@@ -253,14 +242,17 @@ __device__ __forceinline__ bool cell_zlow_hist(const BatchDev& b, const ScanDev&
     // (ground cells hold one or two) with warp reductions instead of contended atomics
     uint32_t cnt = 0u, lo = 0xffffffffu, hi = 0u;
     bool bad = false;
+    float znext = (lane < n) ? b.csr_z[start + lane] : 0.0f;
     for (uint32_t base = 0; base < n; base += 32)
     {
         const uint32_t k = base + lane;
         int32_t q = -1;
         uint32_t zo = 0u;
+        const float z = znext;
+        if (k + 32u < n) // the next step's load while this one is folded in
+            znext = b.csr_z[start + k + 32u];
         if (k < n)
         {
-            const float z = b.csr_z[start + k];
             const float f = floorf(2.0f * z);
             if (f >= static_cast<float>(q0) && f < static_cast<float>(q0 + nb))
             {
@@ -334,391 +326,256 @@ __device__ __forceinline__ void cell_zlow_sorted(const BatchDev& b, uint32_t c, 
     __syncwarp();
 }
 
-// large_list entries: the cell, bit 31 set when its zlow still has to be found by sorting.
-constexpr uint32_t kLargeNeedsZ = 0x80000000u;
+// One azimuth slice of the polar grid per CTA: the lowest heights of its cells (segmenter.cpp:249-260),
+// the RECM elevation chain along it (:215-267) and the RANSAC candidates of its near cells (:345-357:
+// points whose height is within 2 thr of the elevation). Bound by latency (a handful of dependent loads
+// per cell, then the chain): as six launches (cells, large cells, chain, candidate counts, their
+// scan, candidates) the steps took 90 us of a 64 x 2048 scan, four fifths of it launches and tails.
+// The candidates keep no order: the inlier counts need none, and the few that the hypotheses draw by
+// rank are found by selection in k_ransac_draw. (Ordering every near cell's points for them was most
+// of the cells' time.)
+constexpr uint32_t kRecmThreads = 256;
+constexpr uint32_t kRecmTable = 2048; // buckets of a slice in shared memory (50 cells x 15 by default)
 
-// Per-warp scratch of the near-cell ordering: run starts and run destinations.
-struct RunScratch
+__global__ void __launch_bounds__(kRecmThreads) k_recm(BatchDev b)
 {
-    uint16_t rs[kMediumCell + 1];
-    uint16_t rd[kMediumCell];
-};
-
-// Puts the indices of a near cell (32 < n <= kMediumCell) in ascending order, as the reference's
-// cell vectors hold them (segmenter.cpp:99-131 appends in cloud order).
-//
-// k_bin hands each warp's points of a cell one contiguous slot range in lane order, and a warp
-// covers 32 consecutive indices, so a cell's list is a few ascending runs (one per contributing
-// warp) over disjoint index ranges. The list is split into runs at every descent and at every
-// change of 32-index window (`wofs` = the scan's first batch index mod 32 aligns the windows with
-// the warps), the runs are ordered by their first index (a sort of r keys instead of n), and every
-// run moves as a block. The result is checked: when one run's last index is not below the next
-// run's first, the ranges overlap and the whole list is sorted instead. `is` holds n rounded up
-// to a power of two entries, `key` as many. The heights cz (csr_z) are permuted alongside.
-__device__ __forceinline__ void warp_order_near(int32_t* csr, float* cz, const float4* pts, uint32_t n, uint32_t wofs,
-                                                int32_t* is, float* zb, uint32_t* key, RunScratch& rsc)
-{
-    const uint32_t lane = lane_id();
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t r = 0;
-    int32_t prev = 0, vmin = INT32_MAX, vmax = INT32_MIN;
-    for (uint32_t base = 0; base < n; base += 32)
-    {
-        const uint32_t k = base + lane;
-        const int32_t v = (k < n) ? csr[k] : INT32_MAX;
-        is[k] = v;
-        zb[k] = (k < n) ? cz[k] : 0.0F;
-        int32_t up = __shfl_up_sync(0xffffffffu, v, 1);
-        if (lane == 0)
-            up = prev;
-        const bool head = (k < n) && (k == 0 || v <= up || ((v + wofs) >> 5) != ((up + wofs) >> 5));
-        const uint32_t hm = __ballot_sync(0xffffffffu, head);
-        if (head)
-            rsc.rs[r + __popc(hm & lt)] = static_cast<uint16_t>(k);
-        r += __popc(hm);
-        prev = __shfl_sync(0xffffffffu, v, 31);
-        if (k < n)
-        {
-            vmin = min(vmin, v);
-            vmax = max(vmax, v);
-        }
-    }
-    if (r == 1)
-        return; // already ascending
-    vmin = __reduce_min_sync(0xffffffffu, vmin);
-    vmax = __reduce_max_sync(0xffffffffu, vmax);
-    if (lane == 0)
-        rsc.rs[r] = static_cast<uint16_t>(n);
-    __syncwarp();
-    const uint32_t np2 = next_pow2(n);
-    // run keys: first index relative to the cell's smallest (24 bits), run id (8 bits)
-    bool ok = static_cast<uint32_t>(vmax - vmin) < (1u << 24);
-    if (ok && r <= 32)
-    {
-        uint32_t kv = UINT32_MAX;
-        if (lane < r)
-            kv = (static_cast<uint32_t>(is[rsc.rs[lane]] - vmin) << 8) | lane;
-        kv = warp_bitonic_sort(kv, [](uint32_t a, uint32_t bb) { return a < bb; });
-        const uint32_t rid = kv & 0xffu;
-        const bool live = lane < r;
-        const uint32_t len = live ? static_cast<uint32_t>(rsc.rs[rid + 1] - rsc.rs[rid]) : 0u;
-        const int32_t last = live ? is[rsc.rs[rid + 1] - 1] : INT32_MIN;
-        const int32_t nhead = live ? is[rsc.rs[rid]] : INT32_MAX;
-        const int32_t nxt = __shfl_down_sync(0xffffffffu, nhead, 1);
-        ok = __all_sync(0xffffffffu, lane + 1 >= r || last < nxt);
-        uint32_t dst = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, dst, o);
-            if (lane >= static_cast<uint32_t>(o))
-                dst += t;
-        }
-        if (ok && live)
-            rsc.rd[rid] = static_cast<uint16_t>(dst - len);
-    }
-    else if (ok)
-    {
-        const uint32_t rp2 = next_pow2(r);
-        for (uint32_t j = lane; j < rp2; j += 32)
-            key[j] = (j < r) ? ((static_cast<uint32_t>(is[rsc.rs[j]] - vmin) << 8) | j) : UINT32_MAX;
-        __syncwarp();
-        warp_bitonic_smem(key, rp2, [](uint32_t a, uint32_t bb) { return a < bb; });
-        uint32_t carry = 0;
-        bool good = true;
-        for (uint32_t base = 0; base < r; base += 32)
-        {
-            const uint32_t p = base + lane;
-            const bool live = p < r;
-            const uint32_t rid = live ? (key[p] & 0xffu) : 0u;
-            const uint32_t len = live ? static_cast<uint32_t>(rsc.rs[rid + 1] - rsc.rs[rid]) : 0u;
-            if (live && p + 1 < r)
-                good &= is[rsc.rs[rid + 1] - 1] < is[rsc.rs[key[p + 1] & 0xffu]];
-            uint32_t dst = len;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, dst, o);
-                if (lane >= static_cast<uint32_t>(o))
-                    dst += t;
-            }
-            if (live)
-                rsc.rd[rid] = static_cast<uint16_t>(carry + dst - len);
-            carry += __shfl_sync(0xffffffffu, dst, 31);
-        }
-        ok = __all_sync(0xffffffffu, good);
-    }
-    __syncwarp();
-    if (!ok)
-    {
-        for (uint32_t k = ((n + 31u) & ~31u) + lane; k < np2; k += 32)
-            is[k] = INT32_MAX;
-        __syncwarp();
-        warp_bitonic_smem(is, np2, [](int32_t a, int32_t bb) { return a < bb; });
-        for (uint32_t k = lane; k < n; k += 32)
-        {
-            csr[k] = is[k];
-            cz[k] = pts[is[k]].z; // the height follows its index
-        }
-        __syncwarp();
-        return;
-    }
-    uint32_t seen = 0;
-    for (uint32_t base = 0; base < n; base += 32)
-    {
-        const uint32_t k = base + lane;
-        const bool head = (k < n) && (k == 0 || is[k] <= is[k - 1] || ((is[k] + wofs) >> 5) != ((is[k - 1] + wofs) >> 5));
-        const uint32_t hm = __ballot_sync(0xffffffffu, head);
-        if (k < n)
-        {
-            const uint32_t rid = seen + __popc(hm & (lt | (1u << lane))) - 1u;
-            const uint32_t dst = rsc.rd[rid] + (k - rsc.rs[rid]);
-            csr[dst] = is[k];
-            cz[dst] = zb[k];
-        }
-        seen += __popc(hm);
-    }
-    __syncwarp();
-}
-
-__device__ __forceinline__ void cell_small_one(const BatchDev& b, uint32_t c, uint32_t n, uint32_t start, float* zs,
-                                               int32_t* is, float* zb, RunScratch& rsc)
-{
-    const uint32_t lane = lane_id();
-    const int s = scan_of_cell(b, c);
-    const ScanDev& sd = b.scans[s];
-    const bool near = static_cast<int32_t>((c - sd.cell_off) % static_cast<uint32_t>(sd.nrad)) < kRansacRadialBins;
-    bool need_z = !cell_zlow_hist(b, sd, c, n, start);
-    if (need_z && n <= static_cast<uint32_t>(kMediumCell))
-    {
-        cell_zlow_sorted(b, c, n, start, zs);
-        need_z = false;
-    }
-    // the RANSAC candidates of a near cell are read in cloud order: sort its indices
-    if (need_z || (near && n > static_cast<uint32_t>(kMediumCell)))
-    {
-        if (lane == 0)
-        {
-            const uint32_t k = atomicAdd(b.n_large, 1u);
-            b.large_list[k] = c | (need_z ? kLargeNeedsZ : 0u);
-        }
-        return;
-    }
-    if (!near)
-        return;
-    if (n > kSmallCell)
-    {
-        warp_order_near(b.csr_idx + start, b.csr_z + start, b.pts + sd.pt_off, n, sd.pt_off & 31u, is, zb,
-                        reinterpret_cast<uint32_t*>(zs), rsc);
-        return;
-    }
-    // (index, height) pairs sorted by index in registers
-    int32_t idx = (lane < n) ? b.csr_idx[start + lane] : INT32_MAX;
-    float zv = (lane < n) ? b.csr_z[start + lane] : 0.0F;
-#pragma unroll
-    for (uint32_t k = 2; k <= 32; k <<= 1)
-    {
-#pragma unroll
-        for (uint32_t j = k >> 1; j > 0; j >>= 1)
-        {
-            const int32_t oi = __shfl_xor_sync(0xffffffffu, idx, j);
-            const float oz = __shfl_xor_sync(0xffffffffu, zv, j);
-            const bool up = ((lane & k) == 0), lower = ((lane & j) == 0);
-            if ((lower == up) ? (oi < idx) : (idx < oi))
-            {
-                idx = oi;
-                zv = oz;
-            }
-        }
-    }
-    if (lane < n)
-    {
-        b.csr_idx[start + lane] = idx;
-        b.csr_z[start + lane] = zv;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_cell_small(BatchDev b)
-{
-    __shared__ float wz[8][kMediumCell];
-    __shared__ int32_t wi[8][kMediumCell];
-    __shared__ RunScratch wr[8];
-    __shared__ float wzb[8][kMediumCell];
-    const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
-    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-    // 32 consecutive cells per warp step: one coalesced read of their counts, then only the
-    // occupied ones are visited (most cells of a scan are empty)
-    for (uint32_t c0 = (blockIdx.x * (blockDim.x >> 5) + warp) * 32u; c0 < b.ncell; c0 += nwarps * 32u)
-    {
-        const uint32_t c = c0 + lane;
-        const uint32_t cnt = (c < b.ncell) ? b.cell_cnt[c] : 0u;
-        const uint32_t st = (cnt != 0u) ? b.cell_start[c] : 0u;
-        uint32_t m = __ballot_sync(0xffffffffu, cnt != 0u);
-        while (m)
-        {
-            const int j = __ffs(m) - 1;
-            m &= m - 1u;
-            cell_small_one(b, c0 + static_cast<uint32_t>(j), __shfl_sync(0xffffffffu, cnt, j),
-                           __shfl_sync(0xffffffffu, st, j), wz[warp], wi[warp], wzb[warp], wr[warp]);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(512) k_cell_large(BatchDev b)
-{
-    __shared__ float sz[kLargeCellMax];
+    __shared__ float sz[kLargeCellMax]; // the slice's bucket table, then heights to be sorted
+    static_assert(4u * kRecmTable <= kLargeCellMax, "counts, minima, maxima and the cells' starts");
+    static_assert(kRecmThreads / 32 * kMediumCell <= kLargeCellMax, "the warps' parts fit");
+    __shared__ uint32_t nlarge, ccount[kRecmThreads / 32], cbase[kRecmThreads / 32];
     __shared__ int32_t sk;
-    const uint32_t nl = *b.n_large;
-    for (uint32_t li = blockIdx.x; li < nl; li += gridDim.x)
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    const int s = scan_of_slice(b, blockIdx.x);
+    const ScanDev& sd = b.scans[s];
+    const uint32_t slice = blockIdx.x - sd.slice_off;
+    const uint32_t off = sd.cell_off + slice * static_cast<uint32_t>(sd.nrad);
+    if (threadIdx.x == 0)
+        nlarge = 0u;
+    __syncthreads();
+    const int32_t q0 = static_cast<int32_t>(floorf(2.0f * sd.zmin_adj));
+    const int32_t nb = static_cast<int32_t>(floorf(2.0f * sd.zmax_adj)) - q0 + 1;
+    const uint32_t nr = static_cast<uint32_t>(sd.nrad);
+    if (nb >= 1 && nb <= 32 && nr * static_cast<uint32_t>(nb) <= kRecmTable)
     {
-        const uint32_t entry = b.large_list[li];
-        const uint32_t c = entry & ~kLargeNeedsZ;
-        const bool need_z = (entry & kLargeNeedsZ) != 0u;
-        const uint32_t n = b.cell_cnt[c];
-        const uint32_t start = b.cell_start[c];
-        const int s = scan_of_cell(b, c);
-        const ScanDev& sd = b.scans[s];
+        // all buckets of the slice's cells in one table (bucket-major): the slice's points, which lie
+        // behind one another in the lists, are folded in one per thread, then a thread per cell
+        // walks its buckets (see cell_zlow_hist for the rule)
+        uint32_t* tcnt = reinterpret_cast<uint32_t*>(sz);
+        uint32_t *tlo = tcnt + kRecmTable, *thi = tlo + kRecmTable, *first = thi + kRecmTable;
+        for (uint32_t k = threadIdx.x; k < nr * static_cast<uint32_t>(nb); k += kRecmThreads)
+        {
+            tcnt[k] = 0u;
+            tlo[k] = 0xffffffffu;
+            thi[k] = 0u;
+        }
+        for (uint32_t k = threadIdx.x; k < nr; k += kRecmThreads)
+            first[k] = b.cell_start[off + k];
+        __syncthreads();
+        const uint32_t p0 = first[0], p1 = first[nr - 1u] + b.cell_cnt[off + nr - 1u];
+        for (uint32_t k = p0 + threadIdx.x; k < p1; k += kRecmThreads)
+        {
+            const float z = b.csr_z[k];
+            uint32_t lo = 0u, hi = nr - 1u; // the last cell that starts at or before the point
+            while (lo < hi)
+            {
+                const uint32_t mid = (lo + hi + 1u) / 2u;
+                if (first[mid] <= k)
+                    lo = mid;
+                else
+                    hi = mid - 1u;
+            }
+            const float f = floorf(2.0f * z);
+            if (f >= static_cast<float>(q0) && f < static_cast<float>(q0 + nb))
+            {
+                const uint32_t at = static_cast<uint32_t>(static_cast<int32_t>(f) - q0) * nr + lo, zo = zord(z);
+                atomicAdd(&tcnt[at], 1u);
+                atomicMin(&tlo[at], zo);
+                atomicMax(&thi[at], zo);
+            }
+            // (a nan enters no bucket: its cell's counts stay below the cell's size)
+        }
+        __syncthreads();
+        for (uint32_t c = threadIdx.x; c < nr; c += kRecmThreads)
+        {
+            const uint32_t n = b.cell_cnt[off + c];
+            if (n == 0u)
+                continue;
+            uint32_t below = 0u, pick = 0u, hprev = 0u;
+            bool any = false;
+            for (int32_t q = 0; q < nb; ++q)
+            {
+                const uint32_t at = static_cast<uint32_t>(q) * nr + c, m = tcnt[at];
+                if (m == 0u)
+                    continue;
+                const uint32_t lo = tlo[at];
+                if (!any || (below <= n / 2u && (zunord(lo) - zunord(hprev)) > 0.5F))
+                    pick = lo; // the lowest bucket, or the last gap in the lower half
+                any = true;
+                hprev = thi[at];
+                below += m;
+            }
+            b.zlow[off + c] = zunord(pick);
+            if (below != n)
+                b.large_list[off + atomicAdd(&nlarge, 1u)] = off + c;
+        }
+        __syncthreads();
+        // cells with a nan: small ones sorted by a warp, the others stay listed
+        const uint32_t nbad = nlarge;
+        if (nbad != 0u)
+        {
+            if (threadIdx.x == 0)
+                nlarge = 0u;
+            __syncthreads();
+            if (warp == 0)
+                for (uint32_t li = 0; li < nbad; ++li)
+                {
+                    const uint32_t c = b.large_list[off + li], n = b.cell_cnt[c];
+                    __syncwarp();
+                    if (n <= static_cast<uint32_t>(kMediumCell))
+                        cell_zlow_sorted(b, c, n, b.cell_start[c], sz);
+                    else if (lane == 0)
+                        b.large_list[off + nlarge++] = c;
+                    __syncwarp();
+                }
+        }
+    }
+    else
+    {
+        // more buckets than the table holds: every eighth occupied cell per warp
+        uint32_t turn = 0u;
+        for (int32_t r0 = 0; r0 < sd.nrad; r0 += 32)
+        {
+            const int32_t r = r0 + static_cast<int32_t>(lane);
+            const uint32_t cnt = (r < sd.nrad) ? b.cell_cnt[off + static_cast<uint32_t>(r)] : 0u;
+            const uint32_t st = (cnt != 0u) ? b.cell_start[off + static_cast<uint32_t>(r)] : 0u;
+            for (uint32_t m = __ballot_sync(0xffffffffu, cnt != 0u); m != 0u; m &= m - 1u, ++turn)
+            {
+                if (turn % (kRecmThreads / 32u) != warp)
+                    continue;
+                const int j = __ffs(m) - 1;
+                const uint32_t c = off + static_cast<uint32_t>(r0 + j);
+                const uint32_t n = __shfl_sync(0xffffffffu, cnt, j), start = __shfl_sync(0xffffffffu, st, j);
+                if (cell_zlow_hist(b, sd, c, n, start))
+                    continue;
+                if (n <= static_cast<uint32_t>(kMediumCell))
+                    cell_zlow_sorted(b, c, n, start, sz + warp * kMediumCell);
+                else if (lane == 0)
+                    b.large_list[off + atomicAdd(&nlarge, 1u)] = c; // heights the buckets cannot take: sorted below
+            }
+        }
+    }
+    __syncthreads();
+    const uint32_t nl = nlarge;
+    for (uint32_t li = 0; li < nl; ++li)
+    {
+        const uint32_t c = b.large_list[off + li];
+        const uint32_t n = b.cell_cnt[c], start = b.cell_start[c];
         if (n > kLargeCellMax)
         {
             if (threadIdx.x == 0)
             {
                 raise_err(&b.state[s], ERR_CELL_TOO_LARGE);
-                if (need_z)
-                    b.zlow[c] = b.csr_z[start];
+                b.zlow[c] = b.csr_z[start];
             }
             continue;
         }
         const uint32_t np2 = next_pow2(n);
-        if (need_z)
-        {
-            for (uint32_t k = threadIdx.x; k < np2; k += blockDim.x)
-                sz[k] = (k < n) ? b.csr_z[start + k] : INFINITY;
-            if (threadIdx.x == 0)
-                sk = 0;
-            __syncthreads();
-            block_bitonic_sort(sz, np2, [](float a, float bb) { return a < bb; });
-            for (uint32_t k = 1 + threadIdx.x; k <= n / 2; k += blockDim.x)
-                if (sz[k] - sz[k - 1] > 0.5F)
-                    atomicMax(&sk, static_cast<int32_t>(k));
-            __syncthreads();
-            if (threadIdx.x == 0)
-                b.zlow[c] = sz[sk];
-            __syncthreads();
-        }
-        const bool near = static_cast<int32_t>((c - sd.cell_off) % static_cast<uint32_t>(sd.nrad)) < kRansacRadialBins;
-        if (near)
-        {
-            int32_t* si = reinterpret_cast<int32_t*>(sz);
-            for (uint32_t k = threadIdx.x; k < np2; k += blockDim.x)
-                si[k] = (k < n) ? b.csr_idx[start + k] : INT32_MAX;
-            __syncthreads();
-            block_bitonic_sort(si, np2, [](int32_t a, int32_t bb) { return a < bb; });
-            for (uint32_t k = threadIdx.x; k < n; k += blockDim.x)
-            {
-                b.csr_idx[start + k] = si[k];
-                b.csr_z[start + k] = b.pts[sd.pt_off + static_cast<uint32_t>(si[k])].z; // the height follows its index
-            }
-        }
+        for (uint32_t k = threadIdx.x; k < np2; k += blockDim.x)
+            sz[k] = (k < n) ? b.csr_z[start + k] : INFINITY;
+        if (threadIdx.x == 0)
+            sk = 0;
+        __syncthreads();
+        block_bitonic_sort(sz, np2, [](float x, float y) { return x < y; });
+        for (uint32_t k = 1 + threadIdx.x; k <= n / 2; k += blockDim.x)
+            if (sz[k] - sz[k - 1] > 0.5F)
+                atomicMax(&sk, static_cast<int32_t>(k));
+        __syncthreads();
+        if (threadIdx.x == 0)
+            b.zlow[c] = sz[sk];
         __syncthreads();
     }
-}
-
-// RECM elevation chain per azimuth slice (segmenter.cpp:215-267).
-__global__ void k_chain(BatchDev b, uint32_t nslices_total)
-{
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= nslices_total)
-        return;
-    const int s = scan_of_slice(b, g);
-    const ScanDev& sd = b.scans[s];
-    const uint32_t slice = g - sd.slice_off;
-    const uint32_t off = sd.cell_off + slice * static_cast<uint32_t>(sd.nrad);
-    float prev = -sd.sensor_h + sd.thr;
-    b.elev[off] = prev;
-    // the cells' counts and lowest heights do not depend on the chain: 16 cells are loaded before
-    // their links are computed (the loads cannot pass the stores to elev otherwise)
-    constexpr int32_t kAhead = 16;
-    for (int32_t r0 = 1; r0 < sd.nrad; r0 += kAhead)
+    __syncthreads();
+    auto link = [&](float prev, uint32_t cnt, float zlo) {
+        const float lim = prev + sd.delta;
+        return (cnt == 0u) ? lim : ((lim < zlo) ? lim : zlo); // std::min(curr_z_min, prev + delta)
+    };
+    // the near cells, two warps each: their elevation (at most three links), the candidates counted
+    const int32_t rad = static_cast<int32_t>(warp / 2u);
+    const uint32_t nc = off + static_cast<uint32_t>(rad);
+    float e = -sd.sensor_h + sd.thr;
+    for (int32_t r = 1; r <= rad; ++r)
+        e = link(e, b.cell_cnt[off + static_cast<uint32_t>(r)], b.zlow[off + static_cast<uint32_t>(r)]);
+    const uint32_t n = b.cell_cnt[nc], start = b.cell_start[nc];
+    if (n > kLargeCellMax && threadIdx.x % 64u == 0u)
+        raise_err(&b.state[s], ERR_CELL_TOO_LARGE); // the capacity of a near cell
+    const uint32_t half = ((n + 63u) / 64u) * 32u; // this warp's entries: [i0, i1)
+    const uint32_t i0 = (warp & 1u) ? min(half, n) : 0u, i1 = (warp & 1u) ? n : min(half, n);
+    const float lim = 2.0F * sd.thr;
+    uint32_t found = 0u;
+#pragma unroll 4
+    for (uint32_t k = i0 + lane; k < i1; k += 32u)
+        found += (fabsf(e - b.csr_z[start + k]) < lim) ? 1u : 0u;
+    found = warp_sum(found);
+    if (lane == 0)
+        ccount[warp] = found;
+    __syncthreads();
+    if (warp == 0)
     {
-        uint32_t cnt[kAhead];
-        float zlo[kAhead];
-#pragma unroll
-        for (int32_t u = 0; u < kAhead; ++u)
+        // room for the slice's candidates, and the counts per near cell
+        const uint32_t v = (lane < kRecmThreads / 32u) ? ccount[lane] : 0u;
+        const uint32_t incl = warp_incl_scan(v);
+        uint32_t base = 0u;
+        if (lane == 31u && incl)
+            base = atomicAdd(&b.state[s].n_cand, incl);
+        base = __shfl_sync(0xffffffffu, base, 31);
+        if (lane < kRecmThreads / 32u)
+            cbase[lane] = sd.pt_off + base + incl - v;
+        const uint32_t pair = v + __shfl_down_sync(0xffffffffu, v, 1);
+        if (lane < kRecmThreads / 32u && (lane & 1u) == 0u)
+            b.near_cnt[sd.near_off + slice * static_cast<uint32_t>(kRansacRadialBins) + lane / 2u] = pair;
+    }
+    __syncthreads();
+    uint32_t pos = cbase[warp];
+    for (uint32_t k0 = i0; k0 < i1; k0 += 32u)
+    {
+        const uint32_t k = k0 + lane;
+        const bool pred = k < i1 && fabsf(e - b.csr_z[start + k]) < lim;
+        const uint32_t m = __ballot_sync(0xffffffffu, pred);
+        if (pred)
         {
-            const int32_t r = r0 + u;
-            cnt[u] = 0u;
-            zlo[u] = 0.0f;
-            if (r < sd.nrad)
-            {
-                const uint32_t c = off + static_cast<uint32_t>(r);
-                cnt[u] = b.cell_cnt[c];
-                zlo[u] = b.zlow[c];
-            }
+            const float4 p = b.pts[sd.pt_off + static_cast<uint32_t>(b.csr_idx[start + k])];
+            b.cand[pos + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)))] = make_float4(p.x, p.y, p.z, 0.0f);
         }
-#pragma unroll
-        for (int32_t u = 0; u < kAhead; ++u)
+        pos += static_cast<uint32_t>(__popc(m));
+    }
+    // the chain along the whole slice (the last warp: its near cell is the sparsest), 32 cells at a time
+    if (warp != kRecmThreads / 32u - 1u)
+        return;
+    float prev = -sd.sensor_h + sd.thr;
+    for (int32_t r0 = 0; r0 < sd.nrad; r0 += 32)
+    {
+        const int32_t r = r0 + static_cast<int32_t>(lane);
+        const uint32_t cnt = (r < sd.nrad) ? b.cell_cnt[off + static_cast<uint32_t>(r)] : 0u;
+        const float zlo = (r < sd.nrad && cnt != 0u) ? b.zlow[off + static_cast<uint32_t>(r)] : 0.0f;
+        float mine = prev;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j)
         {
-            const int32_t r = r0 + u;
-            if (r < sd.nrad)
-            {
-                float e;
-                if (cnt[u] == 0)
-                {
-                    e = prev + sd.delta;
-                }
-                else
-                {
-                    const float lim = prev + sd.delta;
-                    e = (lim < zlo[u]) ? lim : zlo[u]; // std::min(curr_z_min, prev + delta)
-                }
-                b.elev[off + static_cast<uint32_t>(r)] = e;
-                prev = e;
-            }
+            const uint32_t cj = __shfl_sync(0xffffffffu, cnt, j);
+            const float zj = __shfl_sync(0xffffffffu, zlo, j);
+            if (r0 + j > 0)
+                prev = link(prev, cj, zj);
+            if (static_cast<int>(lane) == j)
+                mine = prev;
         }
+        if (r < sd.nrad)
+            b.elev[off + static_cast<uint32_t>(r)] = mine;
     }
 }
 
 // ------------------------------------------------------------------------------------------
 // RANSAC near-field correction (correctCloseRangeFalsePositivesRANSAC, segmenter.cpp:321-479).
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t near_cell(const ScanDev& sd, uint32_t k)
-{
-    const uint32_t slice = k / static_cast<uint32_t>(sd.nnear_per_slice);
-    const uint32_t radial = k % static_cast<uint32_t>(sd.nnear_per_slice);
-    return sd.cell_off + slice * static_cast<uint32_t>(sd.nrad) + radial;
-}
-
-__global__ void __launch_bounds__(256) k_near(BatchDev b, int write)
-{
-    const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (g >= b.nnear)
-        return;
-    const uint32_t lane = lane_id();
-    const int s = scan_of_near(b, g);
-    const ScanDev& sd = b.scans[s];
-    const uint32_t c = near_cell(sd, g - sd.near_off);
-    const uint32_t n = b.cell_cnt[c];
-    const uint32_t start = b.cell_start[c];
-    const float e = b.elev[c];
-    const float lim = 2.0F * sd.thr;
-    uint32_t pos = write ? b.near_start[g] : 0u;
-    for (uint32_t base = 0; base < n; base += 32)
-    {
-        const uint32_t k = base + lane;
-        // csr_z holds the near cells' heights in index order (permuted with csr_idx)
-        const bool pred = k < n && fabsf(e - b.csr_z[start + k]) < lim;
-        const uint32_t m = __ballot_sync(0xffffffffu, pred);
-        if (write && pred)
-        {
-            const float4 p = b.pts[sd.pt_off + static_cast<uint32_t>(b.csr_idx[start + k])];
-            b.cand[pos + __popc(m & ((1u << lane) - 1u))] = make_float4(p.x, p.y, p.z, 0.0f);
-        }
-        pos += __popc(m);
-    }
-    if (!write && lane == 0)
-        b.near_cnt[g] = pos;
-}
-
 // MT19937 (Matsumoto & Nishimura, 1998) and Lemire's nearly divisionless bounded draw
 // (Lemire, "Fast Random Integer Generation in an Interval", 2019), which is how
 // std::uniform_int_distribution<uint32_t> maps a 32-bit engine onto [0, n-1].
@@ -797,105 +654,212 @@ struct Mt42Stream
     }
 };
 
-// One warp per scan: lane 0 walks the seed-42 stream (the draws are sequential: a rejected draw
-// shifts every later one) and records the index pairs; the lanes then fit the planes in parallel.
-__global__ void __launch_bounds__(32) k_ransac_draw(BatchDev b)
+// The r-th smallest index among a near cell's candidates (entries [start, start + n) of the polar
+// grid's lists, those within `lim` of elevation e; indices below `end`), by one warp. While more than
+// kSelect entries are in question, a pass counts them in 32 equal index ranges and keeps the one that
+// holds the rank; the rest is gathered once and bisected in registers (a pass over memory costs far
+// more than the 17 or so steps).
+constexpr uint32_t kSelect = 256;
+
+__device__ __forceinline__ uint32_t select_candidate(const BatchDev& b, uint32_t start, uint32_t n, float e, float lim,
+                                                     uint32_t r, uint32_t end, uint32_t* buf)
 {
-    __shared__ uint32_t di2[kMaxRansacIters], di3[kMaxRansacIters];
-    __shared__ __align__(16) uint32_t mt_table[kMtTable]; // lane 0 walks the stream: shared-memory latency per draw
-    __shared__ int bad;
-    const int s = blockIdx.x;
     const uint32_t lane = lane_id();
+    uint32_t lo = 0u, active = n; // indices in [lo, end)
+    while (active > kSelect && end - lo > 1u)
+    {
+        const uint32_t width = (end - lo + 31u) / 32u;
+        buf[lane] = 0u;
+        __syncwarp();
+#pragma unroll 4
+        for (uint32_t k = lane; k < n; k += 32u)
+        {
+            const uint32_t v = static_cast<uint32_t>(b.csr_idx[start + k]);
+            if (v >= lo && v < end && fabsf(e - b.csr_z[start + k]) < lim)
+                atomicAdd(&buf[(v - lo) / width], 1u);
+        }
+        __syncwarp();
+        const uint32_t c = buf[lane];
+        const uint32_t incl = warp_incl_scan(c);
+        const uint32_t pick = static_cast<uint32_t>(__ffs(__ballot_sync(0xffffffffu, incl > r)) - 1) & 31u; // r < candidates
+        r -= __shfl_sync(0xffffffffu, incl - c, static_cast<int>(pick));
+        active = __shfl_sync(0xffffffffu, c, static_cast<int>(pick));
+        lo += pick * width;
+        end = min(end, lo + width);
+        __syncwarp();
+    }
+    uint32_t m = 0u;
+#pragma unroll 4
+    for (uint32_t k0 = 0; k0 < n; k0 += 32u)
+    {
+        const uint32_t k = k0 + lane;
+        const uint32_t v = (k < n) ? static_cast<uint32_t>(b.csr_idx[start + k]) : 0u;
+        const bool in = k < n && v >= lo && v < end && fabsf(e - b.csr_z[start + k]) < lim;
+        const uint32_t mask = __ballot_sync(0xffffffffu, in);
+        const uint32_t at = m + static_cast<uint32_t>(__popc(mask & ((1u << lane) - 1u)));
+        if (in && at < kSelect)
+            buf[at] = v;
+        m += static_cast<uint32_t>(__popc(mask));
+    }
+    __syncwarp();
+    m = min(m, kSelect);
+    uint32_t v[kSelect / 32u];
+#pragma unroll
+    for (uint32_t q = 0; q < kSelect / 32u; ++q)
+        v[q] = (q * 32u + lane < m) ? buf[q * 32u + lane] : 0xffffffffu;
+    uint32_t x = lo; // the smallest value with more than r entries up to it
+    for (uint32_t step = (end - lo > 1u) ? 1u << (31 - __clz(static_cast<int>(end - lo - 1u))) : 0u; step != 0u; step >>= 1)
+    {
+        uint32_t below = 0u; // entries below x + step
+#pragma unroll
+        for (uint32_t q = 0; q < kSelect / 32u; ++q)
+            if (q * 32u < m)
+                below += static_cast<uint32_t>(__popc(__ballot_sync(0xffffffffu, v[q] < x + step)));
+        if (below <= r)
+            x += step;
+    }
+    __syncwarp();
+    return x;
+}
+
+// The hypotheses' points and planes (segmenter.cpp:359-407), kDrawCtas CTAs per scan, each for its share
+// of the hypotheses. The draws index the candidates in (slice, radial bin, cloud) order: the near cell
+// comes from the scan of the cells' candidate counts, the point by selection within the cell.
+// Hypothesis it takes outputs 2 it and 2 it + 1 of the seed-42 stream unless an earlier draw was
+// rejected or repeated (a rejected draw shifts every later one): all draws are checked at once, and only
+// then one thread walks the stream. With lane 0 walking it always, and ordered candidates, 20 us.
+constexpr uint32_t kDrawThreads = 1024; // a warp per draw
+constexpr uint32_t kDrawCtas = kNearCopies;
+constexpr uint32_t kDrawPer = (kMaxRansacIters + kDrawCtas - 1) / kDrawCtas; // hypotheses per CTA
+
+__global__ void __launch_bounds__(kDrawThreads) k_ransac_draw(BatchDev b)
+{
+    __shared__ uint32_t di[2 * kMaxRansacIters]; // i2, i3 of every hypothesis
+    __shared__ float4 pt[2 * kDrawPer];
+    __shared__ uint32_t sel[kDrawThreads / 32][kSelect];
+    __shared__ uint32_t sm[33];
+    __shared__ int bad;
+    const int s = static_cast<int>(blockIdx.x / kDrawCtas);
+    const uint32_t part = blockIdx.x % kDrawCtas;
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     const ScanDev& sd = b.scans[s];
     ScanState& st = b.state[s];
-    const uint32_t first = b.near_start[sd.near_off];
-    const uint32_t nnear_s = static_cast<uint32_t>(sd.nslice * sd.nnear_per_slice);
-    const uint32_t last = b.near_start[sd.near_off + nnear_s]; // near_start has nnear + 1 entries
-    const uint32_t N = last - first;
-    if (lane == 0)
-    {
-        st.cand_off = first;
-        st.n_cand = N;
-        st.ransac_ok = 0;
-        b.pvalid[s] = 0ull;
-    }
+    const uint32_t N = st.n_cand;
+    if (part == 0u && tid == 0)
+        st.cand_off = sd.pt_off;
     if (N < 2)
         return; // the reference never ends its p3 draw for N == 1 (segmenter.cpp:382-386)
+    // near cells: first candidate rank of each (this CTA's copy)
+    const uint32_t cells = static_cast<uint32_t>(sd.nslice * sd.nnear_per_slice);
+    uint32_t* rank = b.near_start + static_cast<size_t>(part) * b.nnear + sd.near_off;
+    uint32_t base = 0u;
+    for (uint32_t k0 = 0; k0 < cells; k0 += kDrawThreads)
     {
-        // 16-byte words, several loads in flight per lane
-        const uint4* src = reinterpret_cast<const uint4*>(g_mt42);
-        uint4* dst = reinterpret_cast<uint4*>(mt_table);
-#pragma unroll 5
-        for (int k = static_cast<int>(lane); k < kMtTable / 4; k += 32)
-            dst[k] = src[k];
+        const uint32_t k = k0 + tid;
+        const uint32_t v = (k < cells) ? b.near_cnt[sd.near_off + k] : 0u;
+        uint32_t total;
+        const uint32_t at = base + block_excl_scan(v, sm, &total);
+        if (k < cells)
+            rank[k] = at;
+        base += total;
     }
-    __syncwarp();
-    if (lane == 0)
+    // the draws as if none were rejected or repeated
+    bool odd = false;
+    if (tid < 2u * kMaxRansacIters)
     {
-        Mt42Stream gen;
-        gen.table = mt_table;
+        const uint64_t m = static_cast<uint64_t>(g_mt42[tid]) * N;
+        const uint32_t l = static_cast<uint32_t>(m);
+        odd = l < N && l < (0u - N) % N;
+        di[tid] = static_cast<uint32_t>(m >> 32);
+    }
+    if (tid == 0)
         bad = 0;
-        for (int it = 0; it < kMaxRansacIters; ++it)
-        {
-            const uint32_t i2 = gen.bounded(N);
-            uint32_t i3 = gen.bounded(N);
-            int guard = 0;
-            while (i3 == i2 && guard < (1 << 20))
-            {
-                i3 = gen.bounded(N);
-                ++guard;
-            }
-            if (guard >= (1 << 20))
-            {
-                bad = 1;
-                break;
-            }
-            di2[it] = i2;
-            di3[it] = i3;
-        }
-    }
-    __syncwarp();
-    if (bad)
+    __syncthreads();
+    odd |= tid < static_cast<uint32_t>(kMaxRansacIters) && di[2u * tid] == di[2u * tid + 1u];
+    if (__syncthreads_or(odd))
     {
-        if (lane == 0)
-            raise_err(&st, ERR_INTERNAL);
-        return;
-    }
-    const float p1x = 0.0F, p1y = 0.0F, p1z = -sd.sensor_h;
-    unsigned long long valid = 0ull;
-    for (int base = 0; base < kMaxRansacIters; base += 32)
-    {
-        const int it = base + static_cast<int>(lane);
-        bool ok = false;
-        if (it < kMaxRansacIters)
+        if (tid == 0)
         {
-            const float4 p2 = b.cand[first + di2[it]];
-            const float4 p3 = b.cand[first + di3[it]];
-            float nx = ((p2.y - p1y) * (p3.z - p1z)) - ((p2.z - p1z) * (p3.y - p1y));
-            float ny = ((p2.z - p1z) * (p3.x - p1x)) - ((p2.x - p1x) * (p3.z - p1z));
-            float nz = ((p2.x - p1x) * (p3.y - p1y)) - ((p2.y - p1y) * (p3.x - p1x));
-            const float den = (nx * nx) + (ny * ny) + (nz * nz);
-            float4 pl = make_float4(0, 0, 0, 0);
-            if (!(den < 1.0e-5F))
+            Mt42Stream gen;
+            gen.table = g_mt42;
+            for (int it = 0; it < kMaxRansacIters; ++it)
             {
-                const float norm = 1.0F / sqrtf(den);
-                nz *= norm;
-                if (!(fabsf(nz) < sd.max_cos))
+                const uint32_t i2 = gen.bounded(N);
+                uint32_t i3 = gen.bounded(N);
+                int guard = 0;
+                while (i3 == i2 && guard < (1 << 20))
                 {
-                    nx *= norm;
-                    ny *= norm;
-                    const float pd = (nx * p1x) + (ny * p1y) + (nz * p1z);
-                    pl = make_float4(nx, ny, nz, pd);
-                    ok = true;
+                    i3 = gen.bounded(N);
+                    ++guard;
                 }
+                if (guard >= (1 << 20))
+                {
+                    bad = 1;
+                    break;
+                }
+                di[2 * it] = i2;
+                di[2 * it + 1] = i3;
             }
-            b.planes[s * kMaxRansacIters + it] = pl;
-            b.inliers[s * kMaxRansacIters + it] = 0u;
         }
-        valid |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, ok)) << base;
+        __syncthreads();
+        if (bad)
+        {
+            if (part == 0u && tid == 0)
+                raise_err(&st, ERR_INTERNAL);
+            return;
+        }
     }
-    if (lane == 0)
-        b.pvalid[s] = valid;
+    const uint32_t it0 = part * kDrawPer, it1 = min(it0 + kDrawPer, static_cast<uint32_t>(kMaxRansacIters));
+    const float lim = 2.0F * sd.thr;
+    for (uint32_t d = warp; d < 2u * (it1 - it0); d += kDrawThreads / 32u)
+    {
+        const uint32_t i = di[2u * it0 + d];
+        uint32_t lo = 0u; // the last cell whose first rank is not above i, 32 probes a step
+        for (uint32_t len = cells; len > 1u;)
+        {
+            const uint32_t w = (len + 31u) / 32u;
+            const bool at = lane * w < len && rank[lo + lane * w] <= i; // (true for lane 0)
+            const uint32_t k = static_cast<uint32_t>(__popc(__ballot_sync(0xffffffffu, at))) - 1u;
+            lo += k * w;
+            len = min(w, len - k * w);
+        }
+        const uint32_t c = sd.cell_off + (lo / static_cast<uint32_t>(sd.nnear_per_slice)) * static_cast<uint32_t>(sd.nrad) +
+                           lo % static_cast<uint32_t>(sd.nnear_per_slice);
+        const uint32_t idx = select_candidate(b, b.cell_start[c], b.cell_cnt[c], b.elev[c], lim, i - rank[lo], st.n_pts, sel[warp]);
+        if (lane == 0)
+            pt[d] = b.pts[sd.pt_off + min(idx, sd.n - 1u)];
+    }
+    __syncthreads();
+    const uint32_t it = it0 + tid;
+    bool ok = false;
+    if (it < it1)
+    {
+        const float p1x = 0.0F, p1y = 0.0F, p1z = -sd.sensor_h;
+        const float4 p2 = pt[2u * tid], p3 = pt[2u * tid + 1u];
+        float nx = ((p2.y - p1y) * (p3.z - p1z)) - ((p2.z - p1z) * (p3.y - p1y));
+        float ny = ((p2.z - p1z) * (p3.x - p1x)) - ((p2.x - p1x) * (p3.z - p1z));
+        float nz = ((p2.x - p1x) * (p3.y - p1y)) - ((p2.y - p1y) * (p3.x - p1x));
+        const float den = (nx * nx) + (ny * ny) + (nz * nz);
+        float4 pl = make_float4(0, 0, 0, 0);
+        if (!(den < 1.0e-5F))
+        {
+            const float norm = 1.0F / sqrtf(den);
+            nz *= norm;
+            if (!(fabsf(nz) < sd.max_cos))
+            {
+                nx *= norm;
+                ny *= norm;
+                const float pd = (nx * p1x) + (ny * p1y) + (nz * p1z);
+                pl = make_float4(nx, ny, nz, pd);
+                ok = true;
+            }
+        }
+        b.planes[s * kMaxRansacIters + static_cast<int>(it)] = pl;
+    }
+    static_assert(kDrawPer <= 32u, "one warp fits the CTA's planes");
+    const unsigned long long valid = static_cast<unsigned long long>(__ballot_sync(0xffffffffu, ok)) << it0;
+    if (tid == 0 && valid)
+        atomicOr(&b.pvalid[s], valid);
 }
 
 // Inlier counts of every hypothesis plane of a scan (segmenter.cpp:409-430): lane l of every
@@ -906,8 +870,42 @@ __global__ void __launch_bounds__(32) k_ransac_draw(BatchDev b)
 // belongs to one scan), taken grid-strided: a large scan spreads over the whole grid instead of
 // its own share of it. A CTA's tiles come in increasing order, so it follows the scans with a
 // cursor, loads a scan's planes when it reaches it and adds its counts when it leaves it (integer
-// partial counts add up exactly).
+// partial counts add up exactly). The last CTA to finish picks every scan's plane (segmenter.cpp:432-443).
 constexpr uint32_t kInlierTile = 1024;
+
+__device__ __forceinline__ void ransac_select(const BatchDev& b, int s)
+{
+    ScanState& st = b.state[s];
+    const unsigned long long valid = b.pvalid[s];
+    uint32_t best = 0;
+    int bi = -1;
+#pragma unroll 10
+    for (int it = 0; it < kMaxRansacIters; ++it)
+    {
+        const uint32_t c = ((valid >> it) & 1ull) ? __ldcg(&b.inliers[s * kMaxRansacIters + it]) : 0u;
+        if (c > best)
+        {
+            best = c;
+            bi = it;
+        }
+    }
+    if (best > 0)
+    {
+        float4 q = b.planes[s * kMaxRansacIters + bi];
+        if (q.z < 0)
+        {
+            q.x = -q.x;
+            q.y = -q.y;
+            q.z = -q.z;
+            q.w = -q.w;
+        }
+        st.plane[0] = q.x;
+        st.plane[1] = q.y;
+        st.plane[2] = q.z;
+        st.plane[3] = q.w;
+        st.ransac_ok = 1;
+    }
+}
 
 __global__ void __launch_bounds__(256) k_ransac_inliers(BatchDev b)
 {
@@ -981,44 +979,17 @@ __global__ void __launch_bounds__(256) k_ransac_inliers(BatchDev b)
         }
     }
     flush();
-}
-
-__global__ void k_ransac_select(BatchDev b)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.nscan)
+    __shared__ bool last;
+    __threadfence(); // this CTA's counts before its ticket
+    __syncthreads();
+    if (threadIdx.x == 0)
+        last = atomicAdd(b.ransac_done, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!last)
         return;
-    ScanState& st = b.state[s];
-    const unsigned long long valid = b.pvalid[s];
-    uint32_t best = 0;
-    int bi = -1;
-    for (int it = 0; it < kMaxRansacIters; ++it)
-    {
-        if (!((valid >> it) & 1ull))
-            continue;
-        const uint32_t c = b.inliers[s * kMaxRansacIters + it];
-        if (c > best)
-        {
-            best = c;
-            bi = it;
-        }
-    }
-    if (best > 0)
-    {
-        float4 q = b.planes[s * kMaxRansacIters + bi];
-        if (q.z < 0)
-        {
-            q.x = -q.x;
-            q.y = -q.y;
-            q.z = -q.z;
-            q.w = -q.w;
-        }
-        st.plane[0] = q.x;
-        st.plane[1] = q.y;
-        st.plane[2] = q.z;
-        st.plane[3] = q.w;
-        st.ransac_ok = 1;
-    }
+    __threadfence();
+    for (int q = static_cast<int>(threadIdx.x); q < b.nscan; q += static_cast<int>(blockDim.x))
+        ransac_select(b, q);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2000,16 +1971,10 @@ void launch_segmentation(Launcher& L, const BatchDev& b, const BatchHost& hb, ui
     LP_LAUNCH(L, k_bin, div_up(b.npts, 2u * T), T, b);
     L.scan(b.cell_cnt, b.cell_start, b.ncell + 1);
     LP_LAUNCH(L, k_scatter, div_up(b.npts, T), T, b);
-    LP_LAUNCH(L, k_cell_small, std::min(div_up(b.ncell, 256u), static_cast<uint32_t>(sm_count()) * hb.cell_ctas_per_sm), 256, b);
-    LP_LAUNCH(L, k_cell_large, static_cast<uint32_t>(sm_count()) * 2u, 512, b);
-    LP_LAUNCH(L, k_chain, div_up(hb.nslices, 128u), 128, b, hb.nslices);
-    LP_LAUNCH(L, k_near, div_up(b.nnear * 32u, 256u), 256, b, 0);
-    L.scan(b.near_cnt, b.near_start, b.nnear + 1); // near_cnt[nnear] == 0: last entry is the total
-    LP_LAUNCH(L, k_near, div_up(b.nnear * 32u, 256u), 256, b, 1);
-    LP_LAUNCH(L, k_ransac_draw, static_cast<uint32_t>(b.nscan), 32, b);
+    LP_LAUNCH(L, k_recm, hb.nslices, kRecmThreads, b);
+    LP_LAUNCH(L, k_ransac_draw, static_cast<uint32_t>(b.nscan) * kDrawCtas, kDrawThreads, b);
     // about four CTAs per SM over the batch's tiles
     LP_LAUNCH(L, k_ransac_inliers, static_cast<uint32_t>(sm_count()) * 4u, 256, b);
-    LP_LAUNCH(L, k_ransac_select, div_up(static_cast<uint32_t>(b.nscan), 64u), 64, b);
     LP_LAUNCH(L, k_label_depth, div_up(b.npts, T), T, b);
     LP_LAUNCH(L, k_project_key, div_up(b.npts, T), T, b);
     LP_LAUNCH(L, k_pixel, div_up(b.npix, T), T, b);
