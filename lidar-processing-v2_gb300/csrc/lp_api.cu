@@ -204,6 +204,16 @@ lp_status plan(lp_context* ctx, lp_batch& B)
     b.nhash = static_cast<uint32_t>(hash);
     b.ncl = static_cast<uint32_t>(cl);
     b.jq_total = static_cast<uint32_t>(queue);
+    for (int k = 0; k < kFewScans - 1; ++k)
+    {
+        const bool have = k + 1 < hb.nscan;
+        const ScanDev* sd = have ? &hb.scans[static_cast<size_t>(k) + 1] : nullptr;
+        b.pt_few.at[k] = have ? sd->pt_off : 0xffffffffu;
+        b.pix_few.at[k] = have ? sd->pix_off : 0xffffffffu;
+        b.row_few.at[k] = have ? sd->row_off : 0xffffffffu;
+        b.slice_few.at[k] = have ? sd->slice_off : 0xffffffffu;
+        b.cl_few.at[k] = have ? sd->cl_off : 0xffffffffu;
+    }
     return LP_OK;
 }
 

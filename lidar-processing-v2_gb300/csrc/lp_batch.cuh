@@ -61,9 +61,27 @@ struct IoScan
     uint32_t vec;   // 1: the label buffers allow 4-point vector stores (4 B noise, 16 B seg and cluster)
 };
 
+// Offsets of scans 1..7 in the batch arrays (0xffffffff past the last), in the kernels' arguments: up to
+// eight scans (a part of a split batch) are told apart by seven comparisons against constant operands;
+// the search of the descriptors costs a chain of three to six loads per thread of every kernel.
+constexpr int kFewScans = 8;
+struct FewOffsets
+{
+    uint32_t at[kFewScans - 1];
+    __device__ __forceinline__ int find(uint32_t i) const
+    {
+        int s = 0;
+#pragma unroll
+        for (int k = 0; k < kFewScans - 1; ++k)
+            s += (i >= at[k]) ? 1 : 0;
+        return s;
+    }
+};
+
 struct BatchDev
 {
     int nscan;
+    FewOffsets pt_few, pix_few, row_few, slice_few, cl_few;
     const ScanDev* scans;
     ScanState* state;
 
@@ -207,6 +225,10 @@ struct BatchDev
 
 __device__ __forceinline__ int scan_of_point(const BatchDev& b, uint32_t i)
 {
-    return find_scan(b.nscan, i, [&](int s) { return b.scans[s].pt_off; });
+    return b.nscan <= kFewScans ? b.pt_few.find(i) : find_scan(b.nscan, i, [&](int s) { return b.scans[s].pt_off; });
+}
+__device__ __forceinline__ int scan_of_cluster(const BatchDev& b, uint32_t g)
+{
+    return b.nscan <= kFewScans ? b.cl_few.find(g) : find_scan(b.nscan, g, [&](int s) { return b.scans[s].cl_off; });
 }
 } // namespace lpg

@@ -26,11 +26,11 @@ constexpr int kMaxIters = 1 << 22;
 
 __device__ __forceinline__ int scan_of_obs(const BatchDev& b, uint32_t o)
 {
-    return find_scan(b.nscan, o, [&](int s) { return b.state[s].obs_off; });
+    return b.nscan == 1 ? 0 : find_scan(b.nscan, o, [&](int s) { return b.state[s].obs_off; });
 }
 __device__ __forceinline__ int scan_of_hash(const BatchDev& b, uint32_t h)
 {
-    return find_scan(b.nscan, h, [&](int s) { return b.state[s].hash_off; });
+    return b.nscan == 1 ? 0 : find_scan(b.nscan, h, [&](int s) { return b.state[s].hash_off; });
 }
 __device__ __forceinline__ uint32_t hash_mix(uint32_t k)
 {

@@ -12,7 +12,7 @@ namespace
 {
 __device__ __forceinline__ int scan_of_src(const BatchDev& b, uint32_t i)
 {
-    return find_scan(b.nscan, i, [&](int s) { return b.scans[s].src_off; });
+    return scan_of_point(b, i); // (src_off == pt_off)
 }
 
 // VALID input points are packed, in order, at the start of their scan's point slice.

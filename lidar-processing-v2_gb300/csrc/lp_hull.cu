@@ -2091,7 +2091,7 @@ __global__ void k_hull_worklist(BatchDev b)
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= b.ncl)
         return;
-    const int s = find_scan(b.nscan, g, [&](int q) { return b.scans[q].cl_off; });
+    const int s = scan_of_cluster(b, g);
     if (g - b.scans[s].cl_off >= b.state[s].n_clusters)
         return;
     const uint32_t n = b.cl_cnt[g];
@@ -2149,7 +2149,7 @@ __global__ void __launch_bounds__(kHullThreads) k_hull(BatchDev b, int compute_o
         if (w >= nbig)
             break;
         const uint32_t g = work[w];
-        const int s = find_scan(b.nscan, g, [&](int q) { return b.scans[q].cl_off; });
+        const int s = scan_of_cluster(b, g);
         hull_one(b, sm, g, s, compute_obb);
     }
     __syncthreads(); // the CTA's shared memory now becomes eight per-warp regions
@@ -2163,7 +2163,7 @@ __global__ void __launch_bounds__(kHullThreads) k_hull(BatchDev b, int compute_o
         if (w >= nsmall)
             break;
         const uint32_t g = work[b.ncl - 1u - w];
-        const int s = find_scan(b.nscan, g, [&](int q) { return b.scans[q].cl_off; });
+        const int s = scan_of_cluster(b, g);
         hull_one_warp(b, ws, dirs, g, s, compute_obb);
     }
 }

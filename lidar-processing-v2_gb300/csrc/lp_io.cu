@@ -31,7 +31,7 @@ __global__ void k_io_in(BatchDev b, const IoScan* io)
             at[u] = 0xffffffffu;
             if (i >= b.nsrc)
                 continue;
-            const int s = find_scan(b.nscan, i, [&](int q) { return b.scans[q].src_off; });
+            const int s = scan_of_point(b, i); // (src_off == pt_off)
             const ScanDev& sd = b.scans[s];
             const uint32_t k = i - sd.src_off;
             if (k >= sd.n_src)
@@ -129,7 +129,7 @@ __global__ void k_io_out_clusters(BatchDev b, const IoScan* io, uint32_t* ret, i
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= b.ncl)
         return;
-    const int s = find_scan(b.nscan, g, [&](int q) { return b.scans[q].cl_off; });
+    const int s = scan_of_cluster(b, g);
     const ScanDev& sd = b.scans[s];
     const uint32_t kcl = b.state[s].n_clusters;
     const uint32_t k = g - sd.cl_off;

@@ -925,7 +925,7 @@ __device__ __forceinline__ bool kt_may_hit(const float4* __restrict__ box, uint3
 
 __device__ __forceinline__ int kt_scan_of(const BatchDev& b, uint32_t i)
 {
-    return find_scan(b.nscan, i, [&](int s) { return b.scans[s].src_off; });
+    return scan_of_point(b, i); // (src_off == pt_off)
 }
 
 // Pool allocation of `count` entries, one atomic per group of converged lanes (the lanes loop

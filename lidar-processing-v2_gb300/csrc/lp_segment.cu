@@ -29,11 +29,11 @@ constexpr uint32_t kLargeCellMax = 8192;
 
 __device__ __forceinline__ int scan_of_pix(const BatchDev& b, uint32_t p)
 {
-    return find_scan(b.nscan, p, [&](int s) { return b.scans[s].pix_off; });
+    return b.nscan <= kFewScans ? b.pix_few.find(p) : find_scan(b.nscan, p, [&](int s) { return b.scans[s].pix_off; });
 }
 __device__ __forceinline__ int scan_of_row(const BatchDev& b, uint32_t r)
 {
-    return find_scan(b.nscan, r, [&](int s) { return b.scans[s].row_off; });
+    return b.nscan <= kFewScans ? b.row_few.find(r) : find_scan(b.nscan, r, [&](int s) { return b.scans[s].row_off; });
 }
 __device__ __forceinline__ int scan_of_tile(const BatchDev& b, uint32_t t)
 {
@@ -41,7 +41,7 @@ __device__ __forceinline__ int scan_of_tile(const BatchDev& b, uint32_t t)
 }
 __device__ __forceinline__ int scan_of_slice(const BatchDev& b, uint32_t t)
 {
-    return find_scan(b.nscan, t, [&](int s) { return b.scans[s].slice_off; });
+    return b.nscan <= kFewScans ? b.slice_few.find(t) : find_scan(b.nscan, t, [&](int s) { return b.scans[s].slice_off; });
 }
 
 // ------------------------------------------------------------------------------------------
