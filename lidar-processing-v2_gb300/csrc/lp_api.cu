@@ -452,6 +452,7 @@ lp_status execute(lp_context* ctx, lp_batch& B, bool outputs)
     L.scan_sums = B.scan_sums;
     L.scan_left = B.scan_words;
     L.scan_err = &b.state->err; // scan 0's error word: a failed scan fails the batch
+    L.overlap = B.stream == nullptr; // not a part of a split batch
     L.event_pool = &ctx->events;
     if (B.profiling)
         L.prof = &B.prof;
@@ -828,6 +829,7 @@ lp_status direct_launch(lp_context* ctx, lp_batch& B, lp_scan_output* outs)
     Launcher L;
     L.stream = st;
     L.launches = &ctx->launches;
+    L.overlap = B.stream == nullptr;
     launch_io_in(L, b, b.io);
     if (L.err != cudaSuccess)
         return cuda_fail(ctx, L.err, "direct input launch");

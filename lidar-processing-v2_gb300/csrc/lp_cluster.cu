@@ -99,6 +99,7 @@ constexpr uint32_t kObsChunk = 1024;
 
 __global__ void __launch_bounds__(256) k_obs_gather(BatchDev b)
 {
+    pdl_enter();
     __shared__ uint32_t sidx[kObsChunk];
     __shared__ uint32_t scnt, s_slots;
     const uint32_t base = blockIdx.x * kObsChunk;
@@ -192,6 +193,7 @@ __device__ __forceinline__ int32_t flat_voxel(int32_t nr, int32_t na, int32_t r,
 // obstacle records them.
 __global__ void k_vox_insert(BatchDev b)
 {
+    pdl_enter();
     const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = o < b.obs_flag[b.npts];
     bool fresh = false;
@@ -363,6 +365,7 @@ __device__ __forceinline__ void k_uf_hook_pair(const BatchDev& b, uint32_t v, ui
 // roots do not contend, and no pass has to number the voxels.
 __global__ void k_uf_hook(BatchDev b)
 {
+    pdl_enter();
     if (blockIdx.x == 0)
         for (int s = static_cast<int>(threadIdx.x); s < b.nscan; s += static_cast<int>(blockDim.x))
             if (b.state[s].n_vox > kVoxelCapacity)
@@ -378,6 +381,7 @@ __global__ void k_uf_hook(BatchDev b)
 // root's record (its own are the start; the other voxels' records keep theirs).
 __global__ void k_uf_flatten(BatchDev b)
 {
+    pdl_enter();
     const uint32_t nv = b.state[0].n_comp;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
     {
@@ -428,6 +432,7 @@ struct KeepSrc
 // components ordered by smallest point index == the reference's final label.
 __global__ void k_obs_label(BatchDev b)
 {
+    pdl_enter();
     __shared__ BlockAgg agg;
     if (blockIdx.x == 0)
         for (int s = static_cast<int>(threadIdx.x); s < b.nscan; s += static_cast<int>(blockDim.x))
@@ -471,6 +476,7 @@ __device__ __forceinline__ uint32_t z_ord(float f)
 
 __global__ void k_cl_scatter(BatchDev b)
 {
+    pdl_enter();
     __shared__ BlockAgg agg;
     const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lane = lane_id();
@@ -524,6 +530,7 @@ __global__ void k_cl_scatter(BatchDev b)
 // Clusterer::cluster on a caller-supplied cloud: every point is a member of the cloud to cluster.
 __global__ void k_mark_all(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.npts)
         return;
@@ -544,7 +551,7 @@ void launch_clustering(Launcher& L, const BatchDev& b, const BatchHost& hb)
         if (uint32_t* words = L.scan_state(b.npts + 1))
         {
             L.begin(name);
-            scan_lookback(L.stream, src, ScanDstU32{out, b.npts + 1, true}, b.npts + 1, words, L.scan_err, true);
+            scan_lookback(L.stream, src, ScanDstU32{out, b.npts + 1, true}, b.npts + 1, words, L.scan_err, true, L.overlap);
             L.end();
             L.note();
         }

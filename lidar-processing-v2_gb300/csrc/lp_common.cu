@@ -10,10 +10,10 @@ namespace lpg
 // Exclusive scan of n u32 (in place allowed). `sums` is the scan scratch (at least
 // 8 * scan_words(n) bytes, 8-byte aligned; `zeroed`: already zero), `err` the error word (or null).
 void scan_exclusive(cudaStream_t st, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* sums, uint32_t* err,
-                    uint64_t& launches, bool zeroed)
+                    uint64_t& launches, bool zeroed, bool overlap)
 {
     const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0u;
-    scan_lookback(st, ScanSrcU32{in, n, vec}, ScanDstU32{out, n, vec}, n, sums, err, zeroed);
+    scan_lookback(st, ScanSrcU32{in, n, vec}, ScanDstU32{out, n, vec}, n, sums, err, zeroed, overlap);
     launches += 1;
 }
 
@@ -23,6 +23,7 @@ namespace
 // expecting one arrival that never comes, polled `limit` times.
 __global__ void k_debug_mbar_timeout(uint32_t limit, uint32_t* err)
 {
+    pdl_enter();
     __shared__ unsigned long long bar;
     if (threadIdx.x == 0)
         mbar_init(&bar, 1u);
@@ -63,6 +64,7 @@ namespace
 {
 __global__ void __launch_bounds__(256) k_prepare(FillList f, BatchDev b, int noise)
 {
+    pdl_enter();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
     for (int q = 0; q < f.n; ++q)
     {

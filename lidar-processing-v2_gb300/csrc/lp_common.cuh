@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "lp_internal.cuh"
+#include "lp_stages.hpp"
 
 namespace lpg
 {
@@ -356,6 +357,7 @@ template <uint32_t kRows, class Src, class Dst>
 __global__ void __launch_bounds__(kLbThreads) k_scan_lb(Src src, Dst dst, unsigned long long* state, uint32_t* err,
                                                         uint32_t poll_limit)
 {
+    pdl_enter();
     __shared__ uint32_t s_warp[kLbThreads / 32];
     __shared__ uint32_t s_tile;
     if (threadIdx.x == 0)
@@ -408,16 +410,16 @@ __global__ void __launch_bounds__(kLbThreads) k_scan_lb(Src src, Dst dst, unsign
 }
 
 template <class Src, class Dst>
-void scan_lookback(cudaStream_t st, Src src, Dst dst, uint32_t n, uint32_t* sums, uint32_t* err, bool zeroed = false)
+void scan_lookback(cudaStream_t st, Src src, Dst dst, uint32_t n, uint32_t* sums, uint32_t* err, bool zeroed = false, bool overlap = false)
 {
     const uint32_t nt = div_up(n, scan_tile(n));
     unsigned long long* state = reinterpret_cast<unsigned long long*>(sums);
     if (!zeroed)
         cudaMemsetAsync(state, 0, scan_words(n) * sizeof(unsigned long long), st);
     if (scan_tile(n) == 1024u)
-        k_scan_lb<1><<<nt, kLbThreads, 0, st>>>(src, dst, state, err, kLbPollLimit);
+        launch_kernel(overlap, st, k_scan_lb<1, Src, Dst>, dim3(nt), kLbThreads, 0, src, dst, state, err, kLbPollLimit);
     else
-        k_scan_lb<8><<<nt, kLbThreads, 0, st>>>(src, dst, state, err, kLbPollLimit);
+        launch_kernel(overlap, st, k_scan_lb<8, Src, Dst>, dim3(nt), kLbThreads, 0, src, dst, state, err, kLbPollLimit);
 }
 
 // Plain u32 arrays as scan source and destination (vector accesses when 16-byte aligned).

@@ -18,6 +18,7 @@ __device__ __forceinline__ int scan_of_src(const BatchDev& b, uint32_t i)
 // VALID input points are packed, in order, at the start of their scan's point slice.
 __global__ void k_noise_flag(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > b.nsrc)
         return;
@@ -26,6 +27,7 @@ __global__ void k_noise_flag(BatchDev b)
 
 __global__ void k_noise_compact(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.nsrc || b.noise[i] != LP_NOISE_VALID)
         return;
@@ -40,6 +42,7 @@ __global__ void k_noise_compact(BatchDev b)
 
 __global__ void k_noise_count(BatchDev b)
 {
+    pdl_enter();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= b.nscan)
         return;
@@ -51,6 +54,7 @@ __global__ void k_noise_count(BatchDev b)
 // outlier filter removed keep what the arrays start with (k_prepare).
 __global__ void k_outputs(BatchDev b, int with_clusters)
 {
+    pdl_enter();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= b.npts)
         return;

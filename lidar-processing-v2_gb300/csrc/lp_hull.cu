@@ -1173,6 +1173,7 @@ __device__ int first_polygon(const float2* xy, uint32_t n, const unsigned long l
 
 __global__ void __launch_bounds__(256) k_hull_pre_ext(BatchDev b)
 {
+    pdl_enter();
     __shared__ float2 dirs[kDirs];
     __shared__ unsigned long long ext[kDirs][8];
     hull_dirs(dirs);
@@ -1213,6 +1214,7 @@ __global__ void __launch_bounds__(256) k_hull_pre_ext(BatchDev b)
 
 __global__ void __launch_bounds__(256) k_hull_pre_ref(BatchDev b)
 {
+    pdl_enter();
     __shared__ float2 poly[kDirs];
     __shared__ float4 erec[kDirs];
     __shared__ float2 emar[kDirs];
@@ -2087,6 +2089,7 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
 // of the start plus one of the rank), and its counters start at zero.
 __global__ void k_hull_worklist(BatchDev b)
 {
+    pdl_enter();
     uint32_t* work = b.hull_work;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= b.ncl)
@@ -2128,6 +2131,7 @@ constexpr size_t kHullDynSmem = sizeof(HullSmem) > (kHullThreads / 32) * sizeof(
 // small cluster (one warp each, queue[4] is the head).
 __global__ void __launch_bounds__(kHullThreads) k_hull(BatchDev b, int compute_obb, const uint32_t* work)
 {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ float2 dirs[kDirs];
     HullSmem& sm = *reinterpret_cast<HullSmem*>(smraw);
@@ -2287,6 +2291,7 @@ constexpr size_t kTieDynSmem = static_cast<size_t>(kTieSmemRecs) * (sizeof(HRec<
 
 __global__ void __launch_bounds__(kHullThreads) k_hull_ties(BatchDev b)
 {
+    pdl_enter();
     __shared__ isort::SortShared ss;
     extern __shared__ __align__(16) unsigned char tsm[];
     const uint32_t ntie = b.queue[5]; // the tie count (queue[4] is the small-cluster head)
@@ -2326,6 +2331,7 @@ constexpr uint32_t kFinishThreads = 1024;
 
 __global__ void __launch_bounds__(kFinishThreads) k_hull_finish(BatchDev b)
 {
+    pdl_enter();
     __shared__ uint32_t sm[33];
     __shared__ uint32_t soff[kFinishThreads + 1], sst[kFinishThreads];
     const ScanDev& sd = b.scans[blockIdx.x];
@@ -2589,6 +2595,7 @@ __device__ int single_chain(SingleSmem& sm, const double2* pts, const uint32_t* 
 __global__ void __launch_bounds__(kSingleThreads) k_hull_single(const double2* pts, uint32_t n, HPt<double>* scratch,
                                                               int* stack, int32_t* out, uint32_t* n_out)
 {
+    pdl_enter();
     __shared__ __align__(16) unsigned char raw[sizeof(SingleSmem) > sizeof(isort::SortShared) ? sizeof(SingleSmem)
                                                                                              : sizeof(isort::SortShared)];
     SingleSmem& sm = *reinterpret_cast<SingleSmem*>(raw);
@@ -2643,6 +2650,7 @@ constexpr uint32_t kBoxVerts = 1024;
 __global__ void __launch_bounds__(32) k_boxes_single(const double2* P, uint32_t n, int2* pairs, int cap, int kind,
                                                     lp_bounding_box* out, int* npairs_out)
 {
+    pdl_enter();
     __shared__ double2 sp[kBoxVerts];
     __shared__ float2 spf[kBoxVerts];
     __shared__ float ea[kBoxVerts];
@@ -2715,6 +2723,7 @@ namespace
 __global__ void k_obj_gate(ObjDev o, VehicleTableDev vt, int enabled, double2* P, float2* Pf, float* ea, int2* pairs,
                            ScanState* st)
 {
+    pdl_enter();
     const uint32_t l = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
     if (l >= o.K)
         return;

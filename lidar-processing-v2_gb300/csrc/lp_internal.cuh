@@ -94,6 +94,15 @@ struct ScanState
     uint32_t pad[1];
 };
 
+// First statement of every kernel. Launches of a run carry the programmatic-serialisation attribute
+// (Launcher), so a kernel's CTAs may be set up while the one before it drains: it waits here until that
+// one is complete and its writes are visible, then lets its own successor be set up. A no-op in other
+// launches.
+__device__ __forceinline__ void pdl_enter()
+{
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ void raise_err(ScanState* st, uint32_t bit)
 {
     atomicOr(&st->err, bit);

@@ -18,6 +18,7 @@ namespace
 // their compute while this part's inputs stream in.
 __global__ void k_io_in(BatchDev b, const IoScan* io)
 {
+    pdl_enter();
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < b.nsrc; i0 += 4u * stride)
     {
@@ -114,6 +115,7 @@ __device__ __forceinline__ void io_out_chunk(const BatchDev& b, const IoScan* io
 // host_state: the scans' states as the host reads them (page-locked).
 __global__ void k_io_out_points(BatchDev b, const IoScan* io, ScanState* host_state, uint32_t nq)
 {
+    pdl_enter();
     if (blockIdx.x == 0)
         for (uint32_t i = threadIdx.x; i < static_cast<uint32_t>(b.nscan) * (sizeof(ScanState) / 4u); i += blockDim.x)
             reinterpret_cast<uint32_t*>(host_state)[i] = reinterpret_cast<const uint32_t*>(b.state)[i];
@@ -126,6 +128,7 @@ __global__ void k_io_out_points(BatchDev b, const IoScan* io, ScanState* host_st
 // reports LP_ERR_CAPACITY for it). ret[s] = the scan's hull index count (page-locked host memory).
 __global__ void k_io_out_clusters(BatchDev b, const IoScan* io, uint32_t* ret, int with_obb)
 {
+    pdl_enter();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= b.ncl)
         return;

@@ -722,6 +722,7 @@ __device__ uint32_t kt_round_cluster(float4* a, uint32_t first, uint32_t last, i
 __global__ void __cluster_dims__(kKtCluster, 1, 1) __launch_bounds__(kKtThreads)
     k_kt_level_huge(BatchDev b, int level, uint32_t slots)
 {
+    pdl_enter();
     extern __shared__ float4 kt_smem[];
     __shared__ KtClusterShared csh;
     __shared__ KtShared sh;
@@ -767,6 +768,7 @@ __global__ void __cluster_dims__(kKtCluster, 1, 1) __launch_bounds__(kKtThreads)
 
 __global__ void k_kt_load(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0)
     {
@@ -787,6 +789,7 @@ __global__ void k_kt_load(BatchDev b)
 // subtree in shared memory.
 __global__ void __launch_bounds__(kKtThreads) k_kt_level(BatchDev b, int level, uint32_t slots)
 {
+    pdl_enter();
     extern __shared__ float4 kt_smem[];
     __shared__ KtShared sh;
     const uint32_t s = blockIdx.x / slots, j = blockIdx.x % slots;
@@ -825,6 +828,7 @@ __global__ void __launch_bounds__(kKtThreads) k_kt_level(BatchDev b, int level, 
 // Boxes of the nodes above the shared-memory subtrees, one level at a time from the bottom.
 __global__ void k_kt_box_level(BatchDev b, int level, uint32_t slots)
 {
+    pdl_enter();
     const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint32_t s = static_cast<uint32_t>(t / slots), j = static_cast<uint32_t>(t % slots);
     if (s >= static_cast<uint32_t>(b.nscan))
@@ -959,6 +963,7 @@ __device__ __forceinline__ uint32_t kt_pool_alloc(uint32_t* head, uint32_t cap, 
 // where input order may be shuffled); the results go to the point's input index.
 __global__ void k_kt_own(BatchDev b)
 {
+    pdl_enter();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= b.nsrc)
         return;
@@ -1002,6 +1007,7 @@ __global__ void k_kt_own(BatchDev b)
 // Leftovers into one array in point order (klo_off: exclusive scan of the counts).
 __global__ void k_kt_flat(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.nsrc)
         return;
@@ -1014,6 +1020,7 @@ __global__ void k_kt_flat(BatchDev b)
 // The short points in order (kshort: exclusive scan of the flags).
 __global__ void k_kt_short(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.nsrc)
         return;
@@ -1040,6 +1047,7 @@ __device__ __forceinline__ uint32_t kt_segment_lo(const BatchDev& b, const ScanD
 // Step 3: each short point through its own piece.
 __global__ void k_kt_segment(BatchDev b)
 {
+    pdl_enter();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nshort = b.kshort[b.nsrc];
     if (t >= nshort)
@@ -1091,6 +1099,7 @@ __global__ void k_kt_segment(BatchDev b)
 // Candidates: short points not decided in their own piece (flag -> exclusive scan -> list).
 __global__ void k_kt_cand_flag(BatchDev b)
 {
+    pdl_enter();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nshort = b.kshort[b.nsrc];
     if (t == 0)
@@ -1101,6 +1110,7 @@ __global__ void k_kt_cand_flag(BatchDev b)
 
 __global__ void k_kt_cand_list(BatchDev b)
 {
+    pdl_enter();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < b.kshort[b.nsrc] && b.kcflag[t + 1] != b.kcflag[t])
         b.kcand[b.kcflag[t]] = t;
@@ -1161,6 +1171,7 @@ __device__ bool kt_walk_pushed(const BatchDev& b, const ScanDev& sd, const float
 // lay below them (true when the previous candidate exhausted the stack).
 __global__ void k_kt_spec(BatchDev b)
 {
+    pdl_enter();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t ncand = b.kcflag[b.kshort[b.nsrc]];
     if (c >= ncand)
@@ -1204,6 +1215,7 @@ constexpr uint32_t kNextPieceMax = 1u << 23;
 // pieces is exact whatever lies below them; running out of them continues into R below.
 __global__ void k_kt_spec_next(BatchDev b)
 {
+    pdl_enter();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t ncand = b.kcflag[b.kshort[b.nsrc]];
     if (c >= ncand)
@@ -1307,6 +1319,7 @@ constexpr uint32_t kChainPieces = 32;
 
 __global__ void __launch_bounds__(kChainThreads) k_kt_chain(BatchDev b)
 {
+    pdl_enter();
     __shared__ uint32_t red[kChainThreads / 32];
     __shared__ uint32_t bc[4];
     // the window of candidates [w0, w1): walk record, left-entry count, point, its first pushing

@@ -27,6 +27,7 @@ constexpr uint32_t kObjTile = 8192;
 
 __global__ void k_obj_hist(const int32_t* labels, uint32_t n, uint32_t K, uint32_t ntiles, uint32_t* cnt, uint32_t* err)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int32_t l = (i < n) ? labels[i] : -1;
     const bool bad = l >= 0 && static_cast<uint32_t>(l) >= K;
@@ -42,6 +43,7 @@ __global__ void k_obj_hist(const int32_t* labels, uint32_t n, uint32_t K, uint32
 // First cloud slot of each label (the scanned matrix's label-major row starts), and the total.
 __global__ void k_obj_offsets(const uint32_t* start, uint32_t K, uint32_t ntiles, uint32_t* cl_off)
 {
+    pdl_enter();
     const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l <= K)
         cl_off[l] = start[static_cast<size_t>(l) * ntiles];
@@ -51,6 +53,7 @@ __global__ void k_obj_offsets(const uint32_t* start, uint32_t K, uint32_t ntiles
 // r[i] = r[i-31] + r[i-3] mod 2^32, output r[i] >> 1; colours r, g, b = three outputs % 256.
 __global__ void k_obj_colors(RandWindow w, uint32_t K, uchar4* colour)
 {
+    pdl_enter();
     if (blockIdx.x != 0 || threadIdx.x != 0)
         return;
     uint32_t pos = w.pos;
@@ -73,6 +76,7 @@ __global__ void k_obj_colors(RandWindow w, uint32_t K, uchar4* colour)
 __global__ void k_obj_place(const float4* pts, const int32_t* labels, uint32_t n, uint32_t K, uint32_t ntiles,
                             uint32_t* run, const uchar4* colour, lp_xyzrgb* cloud)
 {
+    pdl_enter();
     const uint32_t t = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
     if (t >= ntiles)
         return;
@@ -120,6 +124,7 @@ __device__ __forceinline__ double2 obj_polygon_point(const ObjDev& o, uint32_t l
 
 __global__ void k_obj_marker_count(ObjDev o)
 {
+    pdl_enter();
     const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l > o.K)
         return;
@@ -129,6 +134,7 @@ __global__ void k_obj_marker_count(ObjDev o)
 
 __global__ void k_obj_marker_write(ObjDev o)
 {
+    pdl_enter();
     const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= o.K)
         return;

@@ -50,6 +50,7 @@ __device__ __forceinline__ int scan_of_slice(const BatchDev& b, uint32_t t)
 // ------------------------------------------------------------------------------------------
 __global__ void k_quadrant(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.npts)
         return;
@@ -76,6 +77,7 @@ __device__ __forceinline__ uint32_t ring_flag(const BatchDev& b, const ScanDev& 
 
 __global__ void __launch_bounds__(256) k_ring_count(BatchDev b)
 {
+    pdl_enter();
     const uint32_t t = blockIdx.x;
     const int s = scan_of_tile(b, t);
     const ScanDev& sd = b.scans[s];
@@ -105,6 +107,7 @@ __global__ void __launch_bounds__(256) k_ring_count(BatchDev b)
 // tile_cnt holds the exclusive scan of the per-tile counts over the whole batch.
 __global__ void __launch_bounds__(256) k_ring_apply(BatchDev b)
 {
+    pdl_enter();
     __shared__ uint32_t sm[33];
     const uint32_t t = blockIdx.x;
     const int s = scan_of_tile(b, t);
@@ -174,6 +177,7 @@ __device__ __forceinline__ int32_t bin_point(const BatchDev& b, uint32_t i, cons
 // Two points per thread (i and i + blockDim.x), both loaded before either is binned.
 __global__ void k_bin(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i0 = blockIdx.x * blockDim.x * 2u + threadIdx.x;
     const uint32_t i1 = i0 + blockDim.x;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -197,6 +201,7 @@ __global__ void k_bin(BatchDev b)
 // (the per-point loads are issued before the scan lookup and the branch, which they do not need)
 __global__ void k_scatter(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.npts)
         return;
@@ -339,6 +344,7 @@ constexpr uint32_t kRecmTable = 2048; // buckets of a slice in shared memory (50
 
 __global__ void __launch_bounds__(kRecmThreads) k_recm(BatchDev b)
 {
+    pdl_enter();
     __shared__ float sz[kLargeCellMax]; // the slice's bucket table, then heights to be sorted
     static_assert(4u * kRecmTable <= kLargeCellMax, "counts, minima, maxima and the cells' starts");
     static_assert(kRecmThreads / 32 * kMediumCell <= kLargeCellMax, "the warps' parts fit");
@@ -734,6 +740,7 @@ constexpr uint32_t kDrawPer = (kMaxRansacIters + kDrawCtas - 1) / kDrawCtas; // 
 
 __global__ void __launch_bounds__(kDrawThreads) k_ransac_draw(BatchDev b)
 {
+    pdl_enter();
     __shared__ uint32_t di[2 * kMaxRansacIters]; // i2, i3 of every hypothesis
     __shared__ float4 pt[2 * kDrawPer];
     __shared__ uint32_t sel[kDrawThreads / 32][kSelect];
@@ -909,6 +916,7 @@ __device__ __forceinline__ void ransac_select(const BatchDev& b, int s)
 
 __global__ void __launch_bounds__(256) k_ransac_inliers(BatchDev b)
 {
+    pdl_enter();
     static_assert(kMaxRansacIters <= 64, "two planes per lane");
     __shared__ float4 tile[kInlierTile];
     const uint32_t lane = lane_id();
@@ -999,6 +1007,7 @@ __global__ void __launch_bounds__(256) k_ransac_inliers(BatchDev b)
 // ------------------------------------------------------------------------------------------
 __global__ void k_label_depth(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.npts)
         return;
@@ -1025,6 +1034,7 @@ __global__ void k_label_depth(BatchDev b)
 
 __global__ void k_project_key(BatchDev b)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.npts)
         return;
@@ -1046,6 +1056,7 @@ __global__ void k_project_key(BatchDev b)
 
 __global__ void k_pixel(BatchDev b)
 {
+    pdl_enter();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= b.npix)
         return;
@@ -1089,6 +1100,7 @@ __device__ __forceinline__ uint32_t obstacle_bits(const uint8_t* st, int32_t H, 
 
 __global__ void __launch_bounds__(256) k_dilate_rows(BatchDev b)
 {
+    pdl_enter();
     __shared__ uint32_t wcount[8];
     __shared__ uint32_t woff[8];
     const uint32_t r = blockIdx.x;
@@ -1270,6 +1282,7 @@ constexpr uint32_t kWeightThreads = 128;
 
 __global__ void __launch_bounds__(kWeightThreads) k_jcp_weights(BatchDev b)
 {
+    pdl_enter();
     __shared__ JcpTile tiles[kWeightThreads / 32];
     const uint32_t lane = lane_id();
     const int k = static_cast<int>(lane);
@@ -1554,6 +1567,7 @@ __device__ __forceinline__ uint32_t wide_state(uint32_t v)
 template <uint32_t kCtas>
 __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads) k_jcp_resolve(BatchDev b, uint32_t cap)
 {
+    pdl_enter();
     constexpr uint32_t kAll = kResolveThreads * kCtas;
     extern __shared__ __align__(16) uint32_t sst[]; // cap + 4 entries
     __shared__ uint32_t s_n[2]; // pixels left open by a round (of the cluster's first CTA), alternating
@@ -1768,6 +1782,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads)
 // populateLabels (segmenter.cpp:640-669) and the colour image of Segmenter::image().
 __global__ void k_populate(BatchDev b, uint8_t* image)
 {
+    pdl_enter();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= b.npix)
         return;
@@ -1826,6 +1841,7 @@ void launch_ring_only(Launcher& L, const BatchDev& b, const BatchHost& hb)
 
 __global__ void k_debug_math(int kind, const float* a, const float* bb, uint32_t n, float* out)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
@@ -1899,6 +1915,7 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long z)
 __global__ void k_debug_math_sweep(int kind, unsigned long long first, unsigned long long count,
                                    unsigned long long* stats, unsigned long long* first_bad)
 {
+    pdl_enter();
     unsigned long long dec = 0, und = 0, bad = 0;
     const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
     for (unsigned long long i = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; i < count;

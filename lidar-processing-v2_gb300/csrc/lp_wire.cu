@@ -21,6 +21,7 @@ __device__ __forceinline__ float rd_f32(const uint8_t* p)
 __global__ void k_unpack_pc2(const uint8_t* data, uint32_t width, uint32_t n, uint32_t point_step, uint32_t row_step,
                              uint4 off, uint32_t off_ring, float4* xyzi, uint16_t* ring)
 {
+    pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
