@@ -283,6 +283,7 @@ size_t carve(lp_batch& B, char* base)
         put(b.kspec_n, N);
         put(b.kpiece, 2ull * N + 2ull * S);
         put(b.kctr, 4);
+        b.kstop = b.klo_off;
     }
     else
     {

@@ -213,10 +213,12 @@ struct BatchDev
     uint4* kc;                 // per short point: count, stop entry, left entries (pool at, count)
     uint32_t* kcflag;          // per short point (+1): 1 if step 3 left it undecided -> exclusive scan
     uint32_t* kcand;           // those candidates (short indices) in order
-    uint4* kspec;              // per candidate: count, stop short index, stop entry | kind << 31, left at
+    uint4* kspec;              // per candidate: count, stop short index, stop entry | kind << 31, left at; later,
+                               // at a run's first candidate: its result (k_kt_run)
     uint32_t* kspec_n;         // per candidate: entries the stopping search left
-    uint2* kpiece;             // per scan: stack of pieces (2 n + 2 per scan)
-    uint32_t* kctr;            // [0] pool head
+    uint2* kpiece;             // per scan: stacks of pieces (2 n + 2 per scan)
+    uint32_t* kctr;            // [0] pool head, [1] stopped candidates
+    uint32_t* kstop;           // stopped candidates in order (klo_off, no longer read by then)
 
     // ---- outputs per input point ---------------------------------------------------------------
     uint32_t* out_seg;

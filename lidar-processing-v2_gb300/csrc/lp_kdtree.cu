@@ -32,17 +32,17 @@
 //      piece from the top; an entry whose subtree box is farther than the radius is consumed
 //      without a match (skipped); the others are searched exactly. Reaching the count there
 //      decides the point (VALID) and records where it stopped and the entries it left.
-//   4. Candidates (short points step 3 did not decide) in three steps. k_kt_spec, one thread per
+//   4. Candidates (short points step 3 did not decide). k_kt_spec, one thread per
 //      candidate: the walk through the pieces pushed since the previous candidate, as if nothing
 //      lay below them, which is exact whenever the previous candidate emptied the stack (running
 //      out of entries is NOISE). k_kt_spec_next, one thread per candidate whose walk ran out right
 //      after one whose walk stopped: the walk on through the pieces that stop leaves, which lie
-//      on top of whatever was below. k_kt_chain, one CTA per scan: the candidates in order with R,
-//      what earlier walks left below those pieces; a stopped walk adds its remainder to R, one
-//      that ran out continues into R: straight after a stop with the walk k_kt_spec_next made,
-//      otherwise (and below those pieces) with the threads searching 256 entries at a time, an
-//      ordered prefix of their counts finding the stop. While R is empty, runs of candidates whose
-//      walks ran out are NOISE at once.
+//      on top of whatever was below. k_kt_run, one CTA per stopped candidate: it and the candidates
+//      after it up to the next that stopped, as if nothing lay below its pieces: each continues into
+//      them, the threads searching 256 entries at a time, an ordered prefix of their counts finding
+//      the stop, until one empties them. k_kt_chain, one CTA per scan: the runs in order, with what
+//      earlier runs left; only where that is not empty and a run emptied its own pieces do candidates
+//      search on (about one run in twenty).
 // The result equals the reference's sequential search bit for bit (same binary32 expressions,
 // same visiting order, same stop points); the tree's node positions equal the reference's.
 #include <cooperative_groups.h>
@@ -1197,6 +1197,8 @@ __global__ void k_kt_spec(BatchDev b)
         raise_err(&b.state[s], ERR_HASH_FULL);
     b.kspec[c] = make_uint4(found, stop.u, stop.x | (stop.kind << 31), stop.at);
     b.kspec_n[c] = stop.n;
+    // the result unless the candidate reaches the count in what lies below (k_kt_run, k_kt_chain)
+    b.noise[i] = (stop.u != kNone) ? LP_NOISE_VALID : LP_NOISE_NOISE;
 }
 
 // Record of a candidate's walk through what its predecessor's stop left (k_kt_spec_next), in
@@ -1303,317 +1305,395 @@ __global__ void k_kt_spec_next(BatchDev b)
     b.klo_at[c] = (stopped ? kNextStop : kNextOut) | (sn << 2) | (piece << 9);
 }
 
-// Step 4b: one CTA per scan applies the candidates' walks in order. R, the stack below the pieces
-// pushed since the previous candidate, is a list of pieces (lo, hi): entries [lo, hi) of the flat
-// array (bit 31 of lo clear) or of the pool (set), consumed from hi - 1 down. A candidate whose
-// walk stopped adds what its walk left on top of R. One whose walk ran out continues into R,
-// up to kChainThreads entries at a time across the top kChainPieces pieces: every thread searches
-// one entry's subtree in full (these searches, chains of dependent node loads, are the chain's
-// cost, so a round is as wide as the CTA), and an ordered prefix of the counts finds the stop;
-// running out of R too means NOISE and an empty R. While R is empty, a run of candidates whose
-// walks ran out is NOISE as a whole. The candidates' records are staged kChainThreads at a time in
-// shared memory. Control flow is uniform: every thread holds the same R top, count and candidate;
-// thread 0 writes R and the pool, and a barrier precedes every read of them.
+// Step 4b: the stopped candidates of the batch in order (kstop).
+struct StopSrc
+{
+    BatchDev b;
+    __device__ __forceinline__ uint32_t count() const { return b.kcflag[b.kshort[b.nsrc]]; }
+    __device__ __forceinline__ uint32_t end() const { return count() + 1u; }
+    __device__ __forceinline__ uint4 get4(uint32_t i) const
+    {
+        const uint32_t n = count();
+        auto one = [&](uint32_t c) { return (c < n && b.kspec[c].y != kNone) ? 1u : 0u; };
+        return make_uint4(one(i), one(i + 1u), one(i + 2u), one(i + 3u));
+    }
+};
+struct StopDst
+{
+    BatchDev b;
+    __device__ __forceinline__ void put4(uint32_t i, uint4 e, uint4 f) const
+    {
+        if (f.x)
+            b.kstop[e.x] = i;
+        if (f.y)
+            b.kstop[e.y] = i + 1u;
+        if (f.z)
+            b.kstop[e.z] = i + 2u;
+        if (f.w)
+            b.kstop[e.w] = i + 3u;
+        const uint32_t n = b.kcflag[b.kshort[b.nsrc]];
+        if (i <= n && n < i + 4u) // the count, from the entry past the last candidate
+            b.kctr[1] = (n == i) ? e.x : ((n == i + 1u) ? e.y : ((n == i + 2u) ? e.z : e.w));
+    }
+};
+
+// A stack of pieces (lo, hi): entries [lo, hi) of the flat array (bit 31 of lo clear) or of the pool
+// (set), consumed from hi - 1 down. Control flow is uniform over the CTA: every thread holds the same
+// top, count and candidate; thread 0 writes the stack and the pool, and a barrier precedes every read.
 constexpr uint32_t kChainThreads = 256;
 constexpr uint32_t kChainPieces = 32;
 
-__global__ void __launch_bounds__(kChainThreads) k_kt_chain(BatchDev b)
+struct ChainShared
 {
-    pdl_enter();
-    __shared__ uint32_t red[kChainThreads / 32];
-    __shared__ uint32_t bc[4];
-    // the window of candidates [w0, w1): walk record, left-entry count, point, its first pushing
-    // short point, query
-    __shared__ uint4 w_spec[kChainThreads];
-    __shared__ uint32_t w_specn[kChainThreads], w_i[kChainThreads], w_tp1[kChainThreads];
-    __shared__ float4 w_q[kChainThreads];
-    __shared__ uint4 w_nx[kChainThreads]; // walk through the predecessor's stop pieces (k_kt_spec_next)
-    // the top pieces of R for one round (index 0 = the top) and their entry-count prefix
-    __shared__ uint2 r_pc[kChainPieces];
-    __shared__ uint32_t r_pre[kChainPieces + 1];
-    const int s = blockIdx.x;
-    if (s >= b.nscan)
-        return;
-    const ScanDev& sd = b.scans[s];
-    ScanState* st = &b.state[s];
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const float4* g = b.kt + sd.src_off;
-    const float4* box = b.kbb + 2ull * sd.src_off;
-    const uint32_t k = sd.dror_k;
-    uint2* R = b.kpiece + 2ull * sd.src_off + 2ull * static_cast<uint32_t>(s);
-    const uint32_t cap = 2u * sd.n_src + 2u;
-    const uint32_t t_first = b.kshort[sd.src_off], t_end = b.kshort[sd.src_off + sd.n_src];
-    const uint32_t c0 = b.kcflag[t_first], c1 = b.kcflag[t_end];
-    uint32_t top = 0; // pieces in R (the same in every thread)
-    // R's top before the last candidate's stop pushed its pieces, while that stop is the last
-    // change to R (kNone otherwise)
-    uint32_t mark = kNone;
-    bool overflow = false, pool_full = false, full = false;
-    uint32_t stk[kKtStack];
-    auto push = [&](uint32_t lo, uint32_t hi) {
+    uint32_t red[kChainThreads / 32];
+    uint32_t bc[4];
+    uint2 pc[kChainPieces]; // the top pieces of the stack for one round (index 0 = the top)
+    uint32_t pre[kChainPieces + 1]; // and their entry-count prefix
+};
+
+struct ChainStack
+{
+    uint2* R;
+    uint32_t cap, top;
+    bool overflow, pool_full, full;
+    __device__ __forceinline__ void push(uint32_t lo, uint32_t hi)
+    {
         if (hi > (lo & 0x7fffffffu))
         {
             if (top < cap)
             {
-                if (tid == 0)
+                if (threadIdx.x == 0)
                     R[top] = make_uint2(lo, hi);
                 ++top;
             }
             else
                 full = true;
         }
-    };
-    // block-wide minimum and inclusive sum (every thread gets the result)
-    auto block_min = [&](uint32_t v) {
+    }
+};
+
+// block-wide minimum and inclusive sum (every thread gets the result)
+__device__ __forceinline__ uint32_t chain_min(uint32_t* red, uint32_t v)
+{
+    v = __reduce_min_sync(0xffffffffu, v);
+    if (lane_id() == 0)
+        red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    uint32_t m = red[0];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (lane == 0)
-            red[warp] = v;
-        __syncthreads();
-        uint32_t m = red[0];
-        for (uint32_t w = 1; w < nwarps; ++w)
-            m = min(m, red[w]);
-        __syncthreads();
-        return m;
-    };
-    auto block_incl = [&](uint32_t v, uint32_t& total) {
+    for (uint32_t w = 1; w < kChainThreads / 32u; ++w)
+        m = min(m, red[w]);
+    __syncthreads();
+    return m;
+}
+__device__ __forceinline__ uint32_t chain_incl(uint32_t* red, uint32_t v, uint32_t& total)
+{
+    v = warp_incl_scan(v);
+    if (lane_id() == 31)
+        red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    uint32_t pre = 0;
+    total = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= static_cast<uint32_t>(o))
-                v += u;
-        }
-        if (lane == 31)
-            red[warp] = v;
-        __syncthreads();
-        uint32_t pre = 0;
-        total = 0;
-        for (uint32_t w = 0; w < nwarps; ++w)
-        {
-            const uint32_t x = red[w];
-            if (w < warp)
-                pre += x;
-            total += x;
-        }
-        __syncthreads();
-        return v + pre;
-    };
-    uint32_t c = c0, w0 = c0, w1 = c0;
-    while (c < c1)
+    for (uint32_t w = 0; w < kChainThreads / 32u; ++w)
     {
-        if (c >= w1)
+        const uint32_t x = red[w];
+        if (w < (threadIdx.x >> 5))
+            pre += x;
+        total += x;
+    }
+    __syncthreads();
+    return v + pre;
+}
+
+// A candidate continues into the stack from count `found`: up to kChainThreads entries at a time across
+// the top kChainPieces pieces; every thread searches one entry's subtree in full (these searches,
+// chains of dependent node loads, are the cost, so a round is as wide as the CTA), and an ordered
+// prefix of the counts finds the stop. True: the count was reached, and the stack holds what that
+// leaves; false: the stack is empty.
+__device__ bool chain_search(const BatchDev& b, const ScanDev& sd, ChainStack& S, ChainShared& sh, float4 q, uint32_t& found,
+                             uint32_t* stk)
+{
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const float4* g = b.kt + sd.src_off;
+    const float4* box = b.kbb + 2ull * sd.src_off;
+    const uint32_t k = sd.dror_k;
+    const float r2 = kt_radius2(sd, q);
+    while (S.top > 0)
+    {
+        // the top pieces (warp 0) and how many entries of them this round covers
+        const uint32_t np = min(S.top, kChainPieces);
+        if (warp == 0)
         {
-            // stage the next window of candidates (one per thread)
-            w0 = c;
-            w1 = min(c + blockDim.x, c1);
-            const uint32_t cc = c + tid;
-            if (cc < w1)
-            {
-                const uint32_t t = b.kcand[cc];
-                const uint32_t i = b.kq[t];
-                w_spec[tid] = b.kspec[cc];
-                w_specn[tid] = b.kspec_n[cc];
-                w_i[tid] = i;
-                w_tp1[tid] = (cc > c0) ? b.kcand[cc - 1] + 1 : t_first;
-                w_q[tid] = b.src[i];
-                w_nx[tid] = make_uint4(b.kown[cc], b.kscr[2ull * cc], b.kscr[2ull * cc + 1], b.klo_at[cc]);
-            }
-            __syncthreads();
+            const uint2 pc = (lane < np) ? S.R[S.top - 1 - lane] : make_uint2(0u, 0u);
+            const uint32_t sz = (lane < np) ? pc.y - (pc.x & 0x7fffffffu) : 0u;
+            const uint32_t incl = warp_incl_scan(sz);
+            if (lane < np)
+                sh.pc[lane] = pc;
+            sh.pre[lane + 1] = incl;
+            if (lane == 0)
+                sh.pre[0] = 0;
         }
-        if (top == 0)
+        __syncthreads();
+        const uint32_t covered = min(sh.pre[np], kChainThreads);
+        uint32_t cnt = 0, my_p = 0;
+        if (tid < covered)
         {
-            // candidates whose walks ran out with R empty are NOISE, up to the first that stopped
-            mark = kNone;
-            const uint32_t cc = c + tid;
-            const bool live = cc < w1;
-            const bool hit = live && w_spec[cc - w0].y != kNone;
-            const uint32_t h = min(block_min(hit ? tid : kNone), w1 - c);
-            if (live && tid < h)
-                b.noise[w_i[cc - w0]] = LP_NOISE_NOISE;
-            c += h;
-            if (c >= w1)
-                continue;
-        }
-        const uint32_t wc = c - w0;
-        const uint4 sp4 = w_spec[wc];
-        const uint32_t i = w_i[wc];
-        if (sp4.y != kNone)
-        {
-            // the walk stopped at short point u: R gains the pieces of the pushing points below u,
-            // then the rest of u's pieces below the stop, then the entries the stopping search left
-            mark = top;
-            const uint32_t tp1 = w_tp1[wc];
-            const uint32_t hu = sp4.y, hx = sp4.z & 0x7fffffffu, hkind = sp4.z >> 31;
-            for (uint32_t u = tp1; u <= hu; ++u)
+            // the piece holding this thread's entry: the last p with pre[p] <= tid
+            uint32_t lo_p = 0, hi_p = np - 1;
+            while (lo_p < hi_p)
             {
-                const uint4 cu = b.kc[u];
-                const uint32_t lo = kt_piece_lo(b, u);
-                if (u < hu)
-                {
-                    push(lo, cu.y);
-                    push(cu.z | 0x80000000u, cu.z + cu.w);
-                }
-                else if (hkind == 1)
-                {
-                    push(lo, cu.y);
-                    push(cu.z | 0x80000000u, hx);
-                }
+                const uint32_t mid = (lo_p + hi_p + 1) / 2;
+                if (sh.pre[mid] <= tid)
+                    lo_p = mid;
                 else
-                {
-                    push(lo, hx);
-                }
+                    hi_p = mid - 1;
             }
-            push(sp4.w | 0x80000000u, sp4.w + w_specn[wc]);
-            if (tid == 0)
-                b.noise[i] = LP_NOISE_VALID;
-            ++c;
-            __syncthreads(); // thread 0's pieces are read by every thread next
-            continue;
+            my_p = lo_p;
+            const uint2 pc = sh.pc[my_p];
+            const uint32_t* arr = (pc.x & 0x80000000u) ? b.kpool : b.kflat;
+            const uint32_t e = arr[pc.y - 1 - (tid - sh.pre[my_p])];
+            if (kt_may_hit(box, e >> 2, q.x, q.y, q.z, r2))
+            {
+                int sp = 0;
+                stk[sp++] = e;
+                cnt = kt_search(g, sd.n_src, q.x, q.y, q.z, r2, k, 0, stk, sp, S.overflow);
+            }
         }
-        // the walk ran out with R non-empty: continue into R
-        const float4 q = w_q[wc];
-        const float r2 = kt_radius2(sd, q);
-        uint32_t found = sp4.x;
-        bool hit = false;
-        if (mark != kNone)
+        uint32_t total = 0;
+        const uint32_t incl = chain_incl(sh.red, cnt, total);
+        if (total > 0 && found + total >= k)
         {
-            // the previous candidate stopped and nothing changed R since: its stop's pieces lie on
-            // top of R, and this candidate's walk through them is done
-            const uint4 nx = w_nx[wc];
-            const uint32_t status = nx.w & 3u, nsp = (nx.w >> 2) & 127u, p = nx.w >> 9;
-            if (status == kNextStop && mark + p < top)
+            const uint32_t hl = chain_min(sh.red, (tid < covered && cnt > 0 && found + incl >= k) ? tid : kNone);
+            if (tid == hl)
             {
-                const uint2 pc = R[top - 1 - p];
-                top -= p + 1;
-                push(pc.x, nx.y);
-                push(nx.z | 0x80000000u, nx.z + nsp);
-                found = nx.x;
-                hit = true;
-            }
-            else if (status == kNextOut)
-            {
-                found = nx.x;
-                top = mark; // those pieces are used up; R below them follows
-            }
-            mark = kNone;
-        }
-        while (top > 0 && !hit)
-        {
-            // the top pieces (warp 0) and how many entries of them this round covers
-            const uint32_t np = min(top, kChainPieces);
-            if (warp == 0)
-            {
-                const uint2 pc = (lane < np) ? R[top - 1 - lane] : make_uint2(0u, 0u);
-                const uint32_t sz = (lane < np) ? pc.y - (pc.x & 0x7fffffffu) : 0u;
-                uint32_t incl = sz;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1)
-                {
-                    const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= static_cast<uint32_t>(o))
-                        incl += u;
-                }
-                if (lane < np)
-                    r_pc[lane] = pc;
-                r_pre[lane + 1] = incl;
-                if (lane == 0)
-                    r_pre[0] = 0;
+                sh.bc[0] = found + incl - cnt; // the count before the stopping entry
+                sh.bc[3] = my_p;
             }
             __syncthreads();
-            const uint32_t covered = min(r_pre[np], blockDim.x);
-            uint32_t cnt = 0, my_p = 0;
-            if (tid < covered)
+            const uint32_t before = sh.bc[0], p = sh.bc[3];
+            const uint2 pc = sh.pc[p];
+            const uint32_t x = pc.y - 1 - (hl - sh.pre[p]);
+            const uint32_t* arr = (pc.x & 0x80000000u) ? b.kpool : b.kflat;
+            // the stopping search again on thread 0, from the count before it, for what it leaves
+            if (tid == 0)
             {
-                // the piece holding this thread's entry: the last p with r_pre[p] <= tid
-                uint32_t lo_p = 0, hi_p = np - 1;
-                while (lo_p < hi_p)
+                int sp = 0;
+                stk[sp++] = arr[x];
+                kt_search(g, sd.n_src, q.x, q.y, q.z, r2, k, before, stk, sp, S.overflow);
+                uint32_t at = kt_pool_alloc(b.kctr, b.kpool_cap, static_cast<uint32_t>(sp));
+                if (at == kNone)
                 {
-                    const uint32_t mid = (lo_p + hi_p + 1) / 2;
-                    if (r_pre[mid] <= tid)
-                        lo_p = mid;
-                    else
-                        hi_p = mid - 1;
+                    S.pool_full = true;
+                    at = 0;
+                    sp = 0;
                 }
-                my_p = lo_p;
-                const uint2 pc = r_pc[my_p];
-                const uint32_t* arr = (pc.x & 0x80000000u) ? b.kpool : b.kflat;
-                const uint32_t e = arr[pc.y - 1 - (tid - r_pre[my_p])];
-                if (kt_may_hit(box, e >> 2, q.x, q.y, q.z, r2))
-                {
-                    int sp = 0;
-                    stk[sp++] = e;
-                    cnt = kt_search(g, sd.n_src, q.x, q.y, q.z, r2, k, 0, stk, sp, overflow);
-                }
+                for (int v = 0; v < sp; ++v)
+                    b.kpool[at + v] = stk[v];
+                sh.bc[1] = static_cast<uint32_t>(sp);
+                sh.bc[2] = at;
             }
-            uint32_t total = 0;
-            const uint32_t incl = block_incl(cnt, total);
-            const bool reach_here = tid < covered && cnt > 0 && found + incl >= k;
-            const uint32_t hl = block_min(reach_here ? tid : kNone);
-            if (hl != kNone)
+            __syncthreads();
+            const uint32_t nsp = sh.bc[1], at = sh.bc[2];
+            // the pieces above p are consumed, p keeps its entries below the stop, then the left
+            // entries go on top
+            S.top -= p + 1;
+            S.push(pc.x, x);
+            S.push(at | 0x80000000u, at + nsp);
+            __syncthreads();
+            return true;
+        }
+        found += total;
+        // pieces fully covered are consumed; the last covered one keeps what lies below
+        uint32_t p = 0;
+        while (p < np && sh.pre[p + 1] <= covered)
+            ++p;
+        S.top -= p;
+        if (p < np && covered > sh.pre[p] && tid == 0)
+            S.R[S.top - 1].y = sh.pc[p].y - (covered - sh.pre[p]);
+        __syncthreads();
+    }
+    return false;
+}
+
+__device__ __forceinline__ void chain_report(ScanState* st, const ChainStack& S)
+{
+    if (__syncthreads_or(S.overflow) && threadIdx.x == 0)
+        raise_err(st, ERR_INTERNAL);
+    if (__syncthreads_or(S.pool_full) && threadIdx.x == 0)
+        raise_err(st, ERR_HASH_FULL);
+    if (S.full && threadIdx.x == 0)
+        raise_err(st, ERR_INTERNAL);
+}
+
+// Step 4c: runs. A run is a candidate whose walk stopped and the candidates after it, whose walks ran
+// out, up to the next that stopped: the stop's remainder goes onto the stack, and each of the others
+// continues into the stack until one empties it; from there to the end of the run the candidates are
+// NOISE. As if nothing lay below the run's own pieces, the runs are independent, one CTA each; only
+// one run in twenty meets a stack that is not empty (k_kt_chain puts those right), where one
+// CTA per scan taking all candidates in order spent 5.6 ms on a cloud of 1M points.
+//
+// Run j's pieces lie in kpiece from twice the scan-local index of its first pushing short point: every
+// short point of a run adds at most two pieces. Its result replaces the stop's record: (the candidate
+// that emptied the run's pieces or kNone, its count then, pieces left, their place in kpiece).
+__global__ void __launch_bounds__(kChainThreads) k_kt_run(BatchDev b)
+{
+    pdl_enter();
+    __shared__ ChainShared sh;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t nstop = b.kctr[1];
+    uint32_t stk[kKtStack];
+    for (uint32_t j = blockIdx.x; j < nstop; j += gridDim.x)
+    {
+        const uint32_t c = b.kstop[j];
+        const uint32_t i = b.kq[b.kcand[c]];
+        const int s = kt_scan_of(b, i);
+        const ScanDev& sd = b.scans[s];
+        const uint32_t t_first = b.kshort[sd.src_off];
+        const uint32_t c0 = b.kcflag[t_first], c1 = b.kcflag[b.kshort[sd.src_off + sd.n_src]];
+        const uint32_t end = (j + 1u < nstop) ? min(b.kstop[j + 1u], c1) : c1;
+        const uint32_t tp1 = (c > c0) ? b.kcand[c - 1u] + 1u : t_first;
+        const uint32_t base = 2u * (tp1 - t_first);
+        ChainStack S{b.kpiece + 2ull * sd.src_off + 2ull * static_cast<uint32_t>(s) + base, 2u * (b.kcand[end - 1u] + 1u - tp1), 0u,
+                     false, false, false};
+        // the stop: the pieces of the pushing points below the stop point, then the rest of that
+        // point's pieces below the stop, then the entries the stopping search left
+        const uint4 rec = b.kspec[c];
+        const uint32_t hu = rec.y, hx = rec.z & 0x7fffffffu, hkind = rec.z >> 31;
+        for (uint32_t u = tp1; u <= hu; ++u)
+        {
+            const uint4 cu = b.kc[u];
+            const uint32_t lo = kt_piece_lo(b, u);
+            if (u < hu)
             {
-                if (tid == hl)
-                {
-                    bc[0] = found + incl - cnt; // the count before the stopping entry
-                    bc[3] = my_p;
-                }
-                __syncthreads();
-                const uint32_t before = bc[0], p = bc[3];
-                const uint2 pc = r_pc[p];
-                const uint32_t x = pc.y - 1 - (hl - r_pre[p]);
-                const uint32_t* arr = (pc.x & 0x80000000u) ? b.kpool : b.kflat;
-                // the stopping search again on thread 0, from the count before it, for what it leaves
-                if (tid == 0)
-                {
-                    int sp = 0;
-                    stk[sp++] = arr[x];
-                    kt_search(g, sd.n_src, q.x, q.y, q.z, r2, k, before, stk, sp, overflow);
-                    uint32_t at = kt_pool_alloc(b.kctr, b.kpool_cap, static_cast<uint32_t>(sp));
-                    if (at == kNone)
-                    {
-                        pool_full = true;
-                        at = 0;
-                        sp = 0;
-                    }
-                    for (int v = 0; v < sp; ++v)
-                        b.kpool[at + v] = stk[v];
-                    bc[1] = static_cast<uint32_t>(sp);
-                    bc[2] = at;
-                }
-                __syncthreads();
-                const uint32_t nsp = bc[1], at = bc[2];
-                // R: the pieces above p are consumed, p keeps its entries below the stop, then the
-                // left entries go on top
-                top -= p + 1;
-                push(pc.x, x);
-                push(at | 0x80000000u, at + nsp);
-                hit = true;
+                S.push(lo, cu.y);
+                S.push(cu.z | 0x80000000u, cu.z + cu.w);
+            }
+            else if (hkind == 1)
+            {
+                S.push(lo, cu.y);
+                S.push(cu.z | 0x80000000u, hx);
             }
             else
             {
-                found += total;
-                // pieces fully covered are consumed; the last covered one keeps what lies below
-                uint32_t p = 0;
-                while (p < np && r_pre[p + 1] <= covered)
-                    ++p;
-                top -= p;
-                if (p < np && covered > r_pre[p] && tid == 0)
-                    R[top - 1].y = r_pc[p].y - (covered - r_pre[p]);
+                S.push(lo, hx);
             }
-            __syncthreads();
+        }
+        S.push(rec.w | 0x80000000u, rec.w + b.kspec_n[c]);
+        __syncthreads(); // thread 0's pieces are read by every thread next
+        uint32_t out = kNone, count = 0u;
+        for (uint32_t x = c + 1u; x < end; ++x)
+        {
+            const uint32_t xi = b.kq[b.kcand[x]];
+            uint32_t found = b.kspec[x].x;
+            bool hit = false;
+            if (x == c + 1u)
+            {
+                // its walk through the stop's pieces is done (k_kt_spec_next)
+                const uint32_t w = b.klo_at[x];
+                const uint32_t status = w & 3u, nsp = (w >> 2) & 127u, p = w >> 9;
+                if (status == kNextStop && p < S.top)
+                {
+                    const uint32_t sx = b.kscr[2ull * x], sat = b.kscr[2ull * x + 1u];
+                    const uint2 pc = S.R[S.top - 1u - p];
+                    __syncthreads();
+                    S.top -= p + 1u;
+                    S.push(pc.x, sx);
+                    S.push(sat | 0x80000000u, sat + nsp);
+                    __syncthreads();
+                    hit = true;
+                }
+                else if (status == kNextOut)
+                {
+                    found = b.kown[x];
+                    S.top = 0u;
+                }
+            }
+            if (!hit)
+                hit = chain_search(b, sd, S, sh, b.src[xi], found, stk);
+            if (!hit)
+            {
+                out = x;
+                count = found;
+                break;
+            }
+            if (tid == 0)
+                b.noise[xi] = LP_NOISE_VALID;
         }
         if (tid == 0)
-            b.noise[i] = hit ? LP_NOISE_VALID : LP_NOISE_NOISE;
-        ++c;
-        __syncthreads();
+            b.kspec[c] = make_uint4(out, count, S.top, base);
+        chain_report(&b.state[s], S);
     }
-    if (__syncthreads_or(overflow) && tid == 0)
-        raise_err(st, ERR_INTERNAL);
-    if (__syncthreads_or(pool_full) && tid == 0)
-        raise_err(st, ERR_HASH_FULL);
-    if (full && tid == 0)
-        raise_err(st, ERR_INTERNAL);
+}
+
+// Step 4d: one CTA per scan takes the runs in order with what earlier runs left (the stack at the front
+// of the scan's kpiece: it never reaches the pieces of the run at hand). While the stack is empty,
+// runs that left nothing stand as they are; a run that emptied its own pieces above a stack that is not
+// empty continues into it from the candidate that did.
+__global__ void __launch_bounds__(kChainThreads) k_kt_chain(BatchDev b)
+{
+    pdl_enter();
+    __shared__ ChainShared sh;
+    const int s = blockIdx.x;
+    const ScanDev& sd = b.scans[s];
+    const uint32_t tid = threadIdx.x;
+    const uint32_t c0 = b.kcflag[b.kshort[sd.src_off]], c1 = b.kcflag[b.kshort[sd.src_off + sd.n_src]];
+    const uint32_t nstop = b.kctr[1];
+    // the scan's runs [j, j1): the first stops at or after c0 and c1
+    uint32_t j1 = 0u, j = 0u;
+    for (uint32_t step = 1u << 31; step != 0u; step >>= 1)
+    {
+        if (j + step <= nstop && b.kstop[j + step - 1u] < c0)
+            j += step;
+        if (j1 + step <= nstop && b.kstop[j1 + step - 1u] < c1)
+            j1 += step;
+    }
+    uint2* R = b.kpiece + 2ull * sd.src_off + 2ull * static_cast<uint32_t>(s);
+    ChainStack S{R, 2u * sd.n_src + 2u, 0u, false, false, false};
+    uint32_t stk[kKtStack];
+    while (j < j1)
+    {
+        if (S.top == 0u)
+        {
+            // on to the next run that left pieces
+            const uint32_t jj = j + tid;
+            const bool left = jj < j1 && b.kspec[b.kstop[jj]].z != 0u;
+            const uint32_t h = chain_min(sh.red, left ? tid : kNone);
+            j += (h == kNone) ? kChainThreads : h;
+            if (h == kNone)
+                continue;
+        }
+        const uint32_t c = b.kstop[j];
+        const uint4 run = b.kspec[c];
+        ++j;
+        if (run.z != 0u)
+        {
+            // its pieces on top of the stack (they move down: every chunk is read before it is written)
+            for (uint32_t k0 = 0; k0 < run.z; k0 += kChainThreads)
+            {
+                uint2 v = make_uint2(0u, 0u);
+                if (k0 + tid < run.z)
+                    v = R[run.w + k0 + tid];
+                __syncthreads();
+                if (k0 + tid < run.z)
+                    R[S.top + k0 + tid] = v;
+                __syncthreads();
+            }
+            S.top += run.z;
+            continue;
+        }
+        if (run.x == kNone)
+            continue;
+        const uint32_t end = (j < j1) ? b.kstop[j] : c1;
+        for (uint32_t x = run.x; x < end && S.top > 0u; ++x)
+        {
+            const uint32_t xi = b.kq[b.kcand[x]];
+            uint32_t found = (x == run.x) ? run.y : b.kspec[x].x;
+            if (chain_search(b, sd, S, sh, b.src[xi], found, stk) && tid == 0)
+                b.noise[xi] = LP_NOISE_VALID;
+        }
+    }
+    chain_report(&b.state[s], S);
 }
 } // namespace
 
@@ -1668,6 +1748,14 @@ void launch_noise(Launcher& L, const BatchDev& b, const BatchHost& hb, const lp_
     LP_LAUNCH(L, k_kt_cand_list, div_up(b.nsrc, T), T, b);
     LP_LAUNCH(L, k_kt_spec, div_up(b.nsrc, 128u), 128, b);
     LP_LAUNCH(L, k_kt_spec_next, div_up(b.nsrc, 128u), 128, b);
+    if (uint32_t* words = L.scan_state(b.nsrc + 1))
+    {
+        L.begin("k_kt_stops");
+        scan_lookback(L.stream, StopSrc{b}, StopDst{b}, b.nsrc + 1, words, L.scan_err, true, L.overlap);
+        L.end();
+        L.note();
+    }
+    LP_LAUNCH(L, k_kt_run, std::min(b.nsrc, static_cast<uint32_t>(sm_count()) * 8u), kChainThreads, b);
     LP_LAUNCH(L, k_kt_chain, S, kChainThreads, b);
 }
 } // namespace lpg

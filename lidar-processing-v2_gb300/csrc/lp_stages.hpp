@@ -30,9 +30,9 @@ struct FillList
         r[n++] = FillRange{p, static_cast<uint32_t>((bytes + 15) / 16), value};
     }
 };
-// Device-wide scans of one run at most (ring tiles, outlier filter 3 + compaction, cells, near cells,
+// Device-wide scans of one run at most (ring tiles, outlier filter 4 + compaction, cells, near cells,
 // obstacles, voxels, components, clusters, hulls): each takes its own zeroed look-back words.
-constexpr uint32_t kScansPerRun = 12;
+constexpr uint32_t kScansPerRun = 13;
 
 // One timed launch (profiling mode only).
 struct LaunchRecord
