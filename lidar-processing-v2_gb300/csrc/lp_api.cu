@@ -812,19 +812,17 @@ lp_status direct_launch(lp_context* ctx, lp_batch& B, lp_scan_output* outs)
     IoScan* io = reinterpret_cast<IoScan*>(B.h_stage + io_at);
     B.h_ret = B.h_stage + in_bytes;
     ScanState* h_state = reinterpret_cast<ScanState*>(B.h_ret);
-    uint32_t nq = 0; // 4-point chunks of the batch
-    auto aligned = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
+    uint32_t nq = 0; // label tiles of the batch
     for (size_t s = 0; s < S; ++s)
     {
         const ScanIn& in = B.run.scans[s];
         const lp_scan_output& o = outs[s];
-        const uint32_t vec = aligned(o.noise_labels, 4) && aligned(o.seg_labels, 16) && aligned(o.cluster_labels, 16);
         io[s] = IoScan{in.xyzi, in.ring, o.noise_labels, o.seg_labels, o.cluster_labels,
                        hull ? o.hull_offsets : nullptr, hull ? o.hull_indices : nullptr,
                        hull ? o.z_min : nullptr, hull ? o.z_max : nullptr,
                        obb ? o.obb_calipers : nullptr, obb ? o.obb_pca : nullptr,
-                       o.cluster_capacity, o.hull_capacity, nq, vec};
-        nq += (in.n + 3u) / 4u;
+                       o.cluster_capacity, o.hull_capacity, nq};
+        nq += (in.n + kIoTile - 1u) / kIoTile;
     }
     LP_CUDA(ctx, cudaMemcpyAsync(const_cast<ScanDev*>(b.scans), B.h_stage, io_at + S * sizeof(IoScan), cudaMemcpyHostToDevice, st));
     Launcher L;

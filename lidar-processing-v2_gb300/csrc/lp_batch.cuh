@@ -57,9 +57,9 @@ struct IoScan
     lp_bounding_box* obbc;
     lp_bounding_box* obbp;
     uint32_t cluster_cap, hull_cap;
-    uint32_t q_off; // first 4-point chunk of the scan in the batch's chunk list
-    uint32_t vec;   // 1: the label buffers allow 4-point vector stores (4 B noise, 16 B seg and cluster)
+    uint32_t q_off; // first label tile of the scan in the batch's tile list
 };
+constexpr uint32_t kIoTile = 1024; // points per label tile
 
 // Offsets of scans 1..7 in the batch arrays (0xffffffff past the last), in the kernels' arguments: up to
 // eight scans (a part of a split batch) are told apart by seven comparisons against constant operands;

@@ -54,116 +54,162 @@ __global__ void k_io_in(BatchDev b, const IoScan* io)
     }
 }
 
-// Per-point labels of every scan into the caller's buffers, four consecutive points per thread
-// (chunk q of the batch: scan s with io[s].q_off <= q, points 4 (q - q_off) ..): the host link
-// takes whole 16-byte stores (4 B of noise labels, 16 B of segmentation and of cluster labels)
-// where the caller's buffers are aligned for them, and one store per label otherwise. The labels come
+// Results into the caller's page-locked buffers, one launch. What bounds it is the host link, which
+// takes 190 GB/s of whole 128-byte lines from as few as 38 CTAs and 80 GB/s or less of lines that a
+// warp's store fills in part (measured with 16-byte stores 32 bytes apart). The buffers of a batch
+// are usually slices of one array, at any offset, so no store may count on the alignment of its
+// point number: a tile's labels are gathered in shared memory and written with lanes on consecutive words
+// of the destination, each warp on one of its lines, whatever the offset. (One thread per four points
+// with 16-byte stores, or four 4-byte stores where the offset was odd, ran at 64 GB/s: 32 scans of a
+// batch 600 us; the 64-scan call 3.23 -> 2.41 ms, six scans 620 -> 578 us, with this kernel.)
+constexpr int kIoThreads = 256;
+constexpr uint32_t kIoClusterCtas = 8; // CTAs per scan for its clusters' results
+
+struct IoSmem
+{
+    uint32_t seg[kIoTile];
+    int32_t cl[kIoTile];
+    uint8_t nz[kIoTile];
+};
+
+// n words to dst, lane by lane along dst's 128-byte lines.
+template <class T>
+__device__ __forceinline__ void put_lines(T* dst, const T* from, uint32_t n)
+{
+    static_assert(sizeof(T) == 4);
+    const uint32_t lead = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(dst) >> 2) & 31u;
+    for (uint32_t i = threadIdx.x; i < n + lead; i += kIoThreads)
+        if (i >= lead)
+            dst[i - lead] = from[i - lead];
+}
+
+// n bytes to dst: whole words along its lines, bytes at the ends.
+__device__ __forceinline__ void put_lines(uint8_t* dst, const uint8_t* from, uint32_t n)
+{
+    const uint32_t lead = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(dst)) & 127u;
+    for (uint32_t w = 4u * threadIdx.x; w < n + lead; w += 4u * kIoThreads)
+    {
+        if (w >= lead && w + 4u <= n + lead)
+        {
+            const uint8_t* f = from + (w - lead);
+            *reinterpret_cast<uint32_t*>(dst + (w - lead)) = static_cast<uint32_t>(f[0]) | (static_cast<uint32_t>(f[1]) << 8) |
+                                                             (static_cast<uint32_t>(f[2]) << 16) |
+                                                             (static_cast<uint32_t>(f[3]) << 24);
+            continue;
+        }
+        for (uint32_t u = max(w, lead); u < min(w + 4u, n + lead); ++u)
+            dst[u - lead] = from[u - lead];
+    }
+}
+
+// Per-point labels, tile q of the batch (scan s with io[s].q_off <= q, its points kIoTile (q - q_off) ..),
 // straight from the stages' arrays (by compacted point, by obstacle), without a pass of their own.
-__device__ __forceinline__ void io_out_chunk(const BatchDev& b, const IoScan* io, uint32_t q)
+__device__ __forceinline__ void io_out_tile(const BatchDev& b, const IoScan* io, IoSmem& sm, uint32_t q)
 {
     const int s = find_scan(b.nscan, q, [&](int t) { return io[t].q_off; });
     const ScanDev& sd = b.scans[s];
     const IoScan& d = io[s];
-    const uint32_t k0 = 4u * (q - d.q_off);
-    if (k0 >= sd.n_src)
+    const uint32_t k0 = kIoTile * (q - d.q_off);
+    if (k0 >= sd.n_src) // (a scan without points has no tile)
         return;
     const uint32_t i0 = sd.src_off + k0;
-    const uint32_t cnt = min(4u, sd.n_src - k0);
-    uint8_t nz[4] = {0, 0, 0, 0};
-    uint32_t sg[4] = {0, 0, 0, 0};
-    int32_t cl[4] = {0, 0, 0, 0};
+    const uint32_t cnt = min(kIoTile, sd.n_src - k0);
+    const bool filtered = b.pt_src != nullptr;
+    const uint32_t src0 = filtered ? b.src_pos[sd.src_off] : 0u;
 #pragma unroll
-    for (uint32_t u = 0; u < 4; ++u)
-        if (u < cnt)
+    for (uint32_t u = 0; u < kIoTile / kIoThreads; ++u)
+    {
+        const uint32_t t = u * kIoThreads + threadIdx.x;
+        if (t < cnt)
         {
-            uint32_t pos = i0 + u; // compacted point
-            cl[u] = LP_INVALID_CLUSTER;
-            if (b.pt_src)
+            uint32_t pos = i0 + t; // compacted point
+            uint8_t nz = 0;
+            uint32_t sg = 0;
+            int32_t cl = LP_INVALID_CLUSTER;
+            if (filtered)
             {
-                nz[u] = b.noise[i0 + u];
-                if (nz[u] != LP_NOISE_VALID)
-                    continue;
-                pos = sd.pt_off + (b.src_pos[i0 + u] - b.src_pos[sd.src_off]);
+                nz = b.noise[i0 + t];
+                pos = sd.pt_off + (b.src_pos[i0 + t] - src0);
             }
-            sg[u] = b.seg_label[pos];
-            if (d.cl && sg[u] == LP_LABEL_OBSTACLE)
-                cl[u] = b.obs_label[b.obs_flag[pos]];
+            if (!filtered || nz == LP_NOISE_VALID)
+            {
+                sg = b.seg_label[pos];
+                if (d.cl && sg == LP_LABEL_OBSTACLE)
+                    cl = b.obs_label[b.obs_flag[pos]];
+            }
+            sm.nz[t] = nz;
+            sm.seg[t] = sg;
+            sm.cl[t] = cl;
         }
-    if (d.vec && cnt == 4u)
-    {
-        if (d.noise)
-            *reinterpret_cast<uint32_t*>(d.noise + k0) =
-                static_cast<uint32_t>(nz[0]) | (static_cast<uint32_t>(nz[1]) << 8) |
-                (static_cast<uint32_t>(nz[2]) << 16) | (static_cast<uint32_t>(nz[3]) << 24);
-        if (d.seg)
-            *reinterpret_cast<uint4*>(d.seg + k0) = make_uint4(sg[0], sg[1], sg[2], sg[3]);
-        if (d.cl)
-            *reinterpret_cast<int4*>(d.cl + k0) = make_int4(cl[0], cl[1], cl[2], cl[3]);
-        return;
     }
-    for (uint32_t u = 0; u < cnt; ++u)
-    {
-        if (d.noise)
-            d.noise[k0 + u] = nz[u];
-        if (d.seg)
-            d.seg[k0 + u] = sg[u];
-        if (d.cl)
-            d.cl[k0 + u] = cl[u];
-    }
+    __syncthreads();
+    if (d.noise)
+        put_lines(d.noise + k0, sm.nz, cnt);
+    if (d.seg)
+        put_lines(d.seg + k0, sm.seg, cnt);
+    if (d.cl)
+        put_lines(d.cl + k0, sm.cl, cnt);
+    __syncthreads(); // (the tile is read before the next one is gathered)
 }
 
-// host_state: the scans' states as the host reads them (page-locked).
-__global__ void k_io_out_points(BatchDev b, const IoScan* io, ScanState* host_state, uint32_t nq)
+// n words to dst, CTA `part` of kIoClusterCtas.
+__device__ __forceinline__ void put_part(void* dst, const void* from, uint32_t n, uint32_t part)
 {
-    pdl_enter();
-    if (blockIdx.x == 0)
-        for (uint32_t i = threadIdx.x; i < static_cast<uint32_t>(b.nscan) * (sizeof(ScanState) / 4u); i += blockDim.x)
-            reinterpret_cast<uint32_t*>(host_state)[i] = reinterpret_cast<const uint32_t*>(b.state)[i];
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x)
-        io_out_chunk(b, io, q);
+    for (uint32_t i = part * kIoThreads + threadIdx.x; i < n; i += kIoClusterCtas * kIoThreads)
+        static_cast<uint32_t*>(dst)[i] = static_cast<const uint32_t*>(from)[i];
 }
 
-// Per-cluster results: hull offsets (relative to the scan), hull indices, z range, boxes. A scan
-// whose clusters or hull indices exceed the caller's capacities gets none of them (the host
-// reports LP_ERR_CAPACITY for it). ret[s] = the scan's hull index count (page-locked host memory).
-__global__ void k_io_out_clusters(BatchDev b, const IoScan* io, uint32_t* ret, int with_obb)
+// Per-cluster results of scan s: hull offsets (relative to the scan), hull indices, z range, boxes, each a
+// contiguous range on both sides. A scan whose clusters or hull indices exceed the caller's capacities
+// gets none of them (the host reports LP_ERR_CAPACITY for it). ret[s] = the scan's hull index count
+// (page-locked host memory).
+__device__ __forceinline__ void io_out_clusters(const BatchDev& b, const IoScan* io, uint32_t* ret, int with_obb, int s,
+                                                uint32_t part)
 {
-    pdl_enter();
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= b.ncl)
-        return;
-    const int s = scan_of_cluster(b, g);
     const ScanDev& sd = b.scans[s];
-    const uint32_t kcl = b.state[s].n_clusters;
-    const uint32_t k = g - sd.cl_off;
-    if (k > kcl)
-        return;
-    const uint32_t base = b.hull_cnt[sd.cl_off];
-    const uint32_t nh = b.hull_cnt[sd.cl_off + kcl] - base;
-    if (k == 0)
-        ret[s] = nh;
     const IoScan& d = io[s];
-    if (kcl > d.cluster_cap || nh > d.hull_cap)
+    const uint32_t kcl = b.state[s].n_clusters;
+    const uint32_t* off = b.hull_cnt + sd.cl_off;
+    const uint32_t base = off[0];
+    const uint32_t nh = kcl <= sd.cluster_cap ? off[kcl] - base : 0u;
+    if (part == 0 && threadIdx.x == 0)
+        ret[s] = nh;
+    if (kcl > min(sd.cluster_cap, d.cluster_cap) || nh > d.hull_cap)
         return;
     if (d.hoff)
-        d.hoff[k] = b.hull_cnt[g] - base;
-    if (k == kcl)
-        return;
-    const uint32_t h0 = b.hull_cnt[g], h1 = b.hull_cnt[g + 1];
+        for (uint32_t k = part * kIoThreads + threadIdx.x; k <= kcl; k += kIoClusterCtas * kIoThreads)
+            d.hoff[k] = off[k] - base;
     if (d.hidx)
-        for (uint32_t j = h0; j < h1; ++j)
-            d.hidx[j - base] = b.hull_out[j];
+        put_part(d.hidx, b.hull_out + base, nh, part);
     if (d.zmin)
-        d.zmin[k] = b.cl_zmin[g];
+        put_part(d.zmin, b.cl_zmin + sd.cl_off, kcl, part);
     if (d.zmax)
-        d.zmax[k] = b.cl_zmax[g];
-    if (with_obb)
+        put_part(d.zmax, b.cl_zmax + sd.cl_off, kcl, part);
+    static_assert(sizeof(lp_bounding_box) % 4 == 0);
+    if (with_obb && d.obbc)
+        put_part(d.obbc, b.obb_c + sd.cl_off, kcl * static_cast<uint32_t>(sizeof(lp_bounding_box) / 4), part);
+    if (with_obb && d.obbp)
+        put_part(d.obbp, b.obb_p + sd.cl_off, kcl * static_cast<uint32_t>(sizeof(lp_bounding_box) / 4), part);
+}
+
+// CTAs [0, ncluster): kIoClusterCtas per scan, its clusters; the others the nq label tiles. host_state: the
+// scans' states as the host reads them (page-locked).
+__global__ void __launch_bounds__(kIoThreads) k_io_out(BatchDev b, const IoScan* io, uint32_t* ret, ScanState* host_state,
+                                                       int with_obb, uint32_t ncluster, uint32_t nq)
+{
+    __shared__ IoSmem sm;
+    pdl_enter();
+    if (blockIdx.x < ncluster)
     {
-        if (d.obbc)
-            d.obbc[k] = b.obb_c[g];
-        if (d.obbp)
-            d.obbp[k] = b.obb_p[g];
+        io_out_clusters(b, io, ret, with_obb, static_cast<int>(blockIdx.x / kIoClusterCtas), blockIdx.x % kIoClusterCtas);
+        return;
     }
+    const uint32_t first = blockIdx.x - ncluster;
+    if (first == 0)
+        for (uint32_t i = threadIdx.x; i < static_cast<uint32_t>(b.nscan) * (sizeof(ScanState) / 4u); i += kIoThreads)
+            reinterpret_cast<uint32_t*>(host_state)[i] = reinterpret_cast<const uint32_t*>(b.state)[i];
+    for (uint32_t q = first; q < nq; q += gridDim.x - ncluster)
+        io_out_tile(b, io, sm, q);
 }
 } // namespace
 
@@ -175,9 +221,8 @@ void launch_io_in(Launcher& L, const BatchDev& b, const IoScan* io)
 void launch_io_out(Launcher& L, const BatchDev& b, const IoScan* io, uint32_t* ret, ScanState* host_state, int with_hull,
                    int with_obb, uint32_t nq)
 {
-    LP_LAUNCH(L, k_io_out_points, std::min(div_up(std::max(nq, 1u), 256u), static_cast<uint32_t>(sm_count()) * 2u), 256, b, io,
-              host_state, nq);
-    if (with_hull)
-        LP_LAUNCH(L, k_io_out_clusters, div_up(b.ncl, 256u), 256, b, io, ret, with_obb);
+    const uint32_t ncluster = with_hull ? static_cast<uint32_t>(b.nscan) * kIoClusterCtas : 0u;
+    const uint32_t tiles = std::min(std::max(nq, 1u), static_cast<uint32_t>(sm_count()) * 2u);
+    LP_LAUNCH(L, k_io_out, ncluster + tiles, kIoThreads, b, io, ret, host_state, with_obb, ncluster, nq);
 }
 } // namespace lpg
