@@ -20,6 +20,7 @@
 //      path while the other warps count the ranks).
 #include <atomic>
 #include <cfloat>
+#include <climits>
 #include <mutex>
 
 #include "lp_introsort.cuh"
@@ -45,19 +46,12 @@ struct HPt
 template <typename T>
 __device__ __forceinline__ bool hpt_less(const HPt<T>& a, const HPt<T>& b)
 {
-    if (a.x < b.x)
-        return true;
-    if (b.x < a.x)
-        return false;
-    if (a.y < b.y)
-        return true;
-    if (b.y < a.y)
-        return false;
-    return a.key < b.key;
+    // (without branches: the sorts compare every pair or exchange every step)
+    return (a.x < b.x) | ((a.x == b.x) & ((a.y < b.y) | ((a.y == b.y) & (a.key < b.key))));
 }
 
 // polygonizer.cpp:45-50: counter-clockwise or collinear, evaluated in FP64 exactly as written
-__device__ __forceinline__ bool ccw_or_colinear(double ax, double ay, double bx, double by, double cx, double cy)
+__device__ __noinline__ bool ccw_or_colinear(double ax, double ay, double bx, double by, double cx, double cy)
 {
     return (bx - ax) * (cy - ay) - (by - ay) * (cx - ax) <= 0;
 }
@@ -78,19 +72,30 @@ __device__ __forceinline__ unsigned long long warp_max64(unsigned long long v)
     }
     return v;
 }
-__device__ __forceinline__ double warp_min_d(double v)
+// The smaller / larger of an accumulator that is not a NaN and a value (a NaN leaves the accumulator).
+__device__ __forceinline__ double min_d(double acc, double v)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    return v < acc ? v : acc;
+}
+__device__ __forceinline__ double max_d(double acc, double v)
+{
+    return v > acc ? v : acc;
+}
+// The warp's smallest / largest of values that are not NaNs: integer reductions of the two halves of the order-preserving
+// bit pattern (an FP64 tree takes five dependent comparisons of the FP64 unit and ten shuffles).
+__device__ __noinline__ double warp_min_d(double v)
+{
+    const long long u = __double_as_longlong(v);
+    const unsigned long long k = static_cast<unsigned long long>(u ^ ((u >> 63) | LLONG_MIN));
+    const uint32_t h = static_cast<uint32_t>(k >> 32);
+    const uint32_t hi = __reduce_min_sync(0xffffffffu, h);
+    const uint32_t lo = __reduce_min_sync(0xffffffffu, h == hi ? static_cast<uint32_t>(k) : 0xffffffffu);
+    const long long m = static_cast<long long>((static_cast<unsigned long long>(hi) << 32) | lo);
+    return __longlong_as_double(m ^ (~(m >> 63) | LLONG_MIN));
 }
 __device__ __forceinline__ double warp_max_d(double v)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    return -warp_min_d(-v);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -102,21 +107,75 @@ __device__ __forceinline__ double tri_area(double ax, double ay, double bx, doub
     return fabs((ax * (by - cy) + bx * (cy - ay) + cx * (ay - by)) * 0.5);
 }
 
+// What bounds these kernels on a scan is the code itself: a cluster's warp runs most of it once, and waits
+// for each instruction line to arrive. So every FP64 division and square root is one shared function (a
+// call costs a few tens of cycles, the inlined sequence about 2 KB), what runs rarely stands out of line, and
+// loops over a hull's few vertices are not unrolled further than their latency needs.
+__device__ __noinline__ double div_d(double a, double b)
+{
+    return a / b;
+}
+__device__ __noinline__ double sqrt_d(double a)
+{
+    return sqrt(a);
+}
+
+// The FP64 areas of two triangles of P compared, as the reference evaluates them (side by side: the two
+// chains overlap): 1 larger, 0 equal, -1 neither.
+__device__ __noinline__ int area_order(const double2* P, int a1, int b1, int c1, int a2, int b2, int c2)
+{
+    const double u = tri_area(P[a1].x, P[a1].y, P[b1].x, P[b1].y, P[c1].x, P[c1].y);
+    const double v = tri_area(P[a2].x, P[a2].y, P[b2].x, P[b2].y, P[c2].x, P[c2].y);
+    return u > v ? 1 : (u == v ? 0 : -1);
+}
+
+// The error of s = fl(b - a) (Knuth's TwoSum of b and -a): s + diff_err = b - a exactly.
+__device__ __forceinline__ float diff_err(float b, float a, float s)
+{
+    const float a1 = s - b;
+    const float b1 = s - a1;
+    return ((-a) - a1) + (b - b1);
+}
+
+// Twice the signed area of (a, b, c), hi + lo, from exact two-term differences and products (the last cross terms dropped).
+__device__ __forceinline__ float2 cross2(float2 a, float2 b, float2 c)
+{
+    const float u = b.x - a.x, v = c.y - a.y, w = b.y - a.y, z = c.x - a.x;
+    const float ul = diff_err(b.x, a.x, u), vl = diff_err(c.y, a.y, v), wl = diff_err(b.y, a.y, w), zl = diff_err(c.x, a.x, z);
+    const float t1 = u * v, t2 = w * z;
+    const float e1 = __fmaf_rn(u, v, -t1), e2 = __fmaf_rn(w, z, -t2);
+    const float s = t1 - t2;
+    const float lo = diff_err(t1, t2, s) + ((e1 + (u * vl + ul * v)) - (e2 + (w * zl + wl * z)));
+    const float hi = s + lo;
+    const float rest = (s - hi) + lo;
+    return hi < 0.0f ? make_float2(-hi, -rest) : make_float2(hi, rest);
+}
+
+// area_order of float vertices. Twice the areas from cross2 are within 2^-41 R^2 each (its products lie below 4 R^2
+// and err by 2^-45 of that, its sums of small terms by less), the FP64 ones within 2e-14 M R (R, M as
+// below): a difference beyond tol2 = 4e-12 R^2 + 4e-13 M R has the FP64 comparison's sign. Opposite edges of a box are
+// near parallel, so many of a walk's comparisons come here; an FP64 chain costs 64 cycles an operation.
+__device__ __noinline__ int area_order_near(const double2* P, const float2* Pf, float tol2, int a1, int b1, int c1, int a2,
+                                            int b2, int c2)
+{
+    const float2 u = cross2(Pf[a1], Pf[b1], Pf[c1]), v = cross2(Pf[a2], Pf[b2], Pf[c2]);
+    const float d = (u.x - v.x) + (u.y - v.y);
+    if (fabsf(d) > tol2)
+        return d > 0.0f ? 1 : -1;
+    return area_order(P, a1, b1, c1, a2, b2, c2);
+}
+
 // Triangle-area comparisons of the pair walk, evaluated in FP64 exactly as the reference does.
 struct AreaCmpFp64
 {
     const double2* P;
-    __device__ __forceinline__ double ad(int a, int b, int c) const
-    {
-        return tri_area(P[a].x, P[a].y, P[b].x, P[b].y, P[c].x, P[c].y);
-    }
     __device__ __forceinline__ bool gt(int a1, int b1, int c1, int a2, int b2, int c2) const
     {
-        return ad(a1, b1, c1) > ad(a2, b2, c2);
+        return area_order(P, a1, b1, c1, a2, b2, c2) > 0;
     }
     __device__ __forceinline__ bool eq(int a1, int b1, int c1, int a2, int b2, int c2) const
     {
-        return ad(a1, b1, c1) == ad(a2, b2, c2);
+        return area_order(P, a1, b1, c1, a2, b2, c2) == 0;
     }
 };
 
@@ -130,16 +189,13 @@ struct AreaCmpFiltered
     const double2* P;
     const float2* Pf; // the same vertices as floats (exact: they are float points)
     float ox, oy, tol;
+    float tol2; // of twice the areas, evaluated with two-term differences and products (area_order_near)
     __device__ __forceinline__ float af(int a, int b, int c) const
     {
         const float ax = Pf[a].x - ox, ay = Pf[a].y - oy;
         const float bx = Pf[b].x - ox, by = Pf[b].y - oy;
         const float cx = Pf[c].x - ox, cy = Pf[c].y - oy;
         return fabsf((ax * (by - cy) + bx * (cy - ay) + cx * (ay - by)) * 0.5f);
-    }
-    __device__ __forceinline__ double ad(int a, int b, int c) const
-    {
-        return tri_area(P[a].x, P[a].y, P[b].x, P[b].y, P[c].x, P[c].y);
     }
     __device__ __forceinline__ bool gt(int a1, int b1, int c1, int a2, int b2, int c2) const
     {
@@ -148,18 +204,18 @@ struct AreaCmpFiltered
             return true;
         if (d < -tol)
             return false;
-        return ad(a1, b1, c1) > ad(a2, b2, c2);
+        return area_order_near(P, Pf, tol2, a1, b1, c1, a2, b2, c2) > 0;
     }
     __device__ __forceinline__ bool eq(int a1, int b1, int c1, int a2, int b2, int c2) const
     {
         if (fabsf(af(a1, b1, c1) - af(a2, b2, c2)) > tol)
             return false;
-        return ad(a1, b1, c1) == ad(a2, b2, c2);
+        return area_order_near(P, Pf, tol2, a1, b1, c1, a2, b2, c2) == 0;
     }
 };
 
 template <typename Cmp>
-__device__ int antipodal_pairs(const Cmp& cmp, int n, int2* pairs, int cap)
+__device__ __noinline__ int antipodal_pairs(const Cmp& cmp, int n, int2* pairs, int cap)
 {
     int np = 0;
     if (n < 2)
@@ -218,7 +274,7 @@ __device__ __forceinline__ float warp_max_f(float v)
 }
 
 // Rotating calipers (polygonizer.cpp:165-278) by one warp: all lanes return the same box.
-__device__ void calipers_warp(const double2* P, int n, const int2* pairs, int npairs, lp_bounding_box* out)
+__device__ __noinline__ void calipers_warp(const double2* P, int n, const int2* pairs, int npairs, lp_bounding_box* out)
 {
     const uint32_t lane = lane_id();
     lp_bounding_box box;
@@ -239,8 +295,8 @@ __device__ void calipers_warp(const double2* P, int n, const int2* pairs, int np
         cx += P[k].x;
         cy += P[k].y;
     }
-    cx /= n;
-    cy /= n;
+    cx = div_d(cx, n);
+    cy = div_d(cy, n);
     float best = __double2float_rn(DBL_MAX); // BoundingBox::area is a float: DBL_MAX -> +inf
     for (int pi = 0; pi < npairs; ++pi)
     {
@@ -257,20 +313,20 @@ __device__ void calipers_warp(const double2* P, int n, const int2* pairs, int np
                     nb -= n;
                 const double ex = P[nb].x - P[index].x;
                 const double ey = P[nb].y - P[index].y;
-                const double len = sqrt(ex * ex + ey * ey);
+                const double len = sqrt_d(ex * ex + ey * ey);
                 if (len < 1.0e-6)
                     continue;
-                const double ux = ex / len, uy = ey / len;
+                const double ux = div_d(ex, len), uy = div_d(ey, len);
                 double mnx = DBL_MAX, mxx = -DBL_MAX, mny = DBL_MAX, mxy = -DBL_MAX;
                 for (int k = static_cast<int>(lane); k < n; k += 32)
                 {
                     const double tx = P[k].x - cx, ty = P[k].y - cy;
                     const double rx = tx * ux + ty * uy;
                     const double ry = -tx * uy + ty * ux;
-                    mnx = fmin(mnx, rx);
-                    mxx = fmax(mxx, rx);
-                    mny = fmin(mny, ry);
-                    mxy = fmax(mxy, ry);
+                    mnx = min_d(mnx, rx);
+                    mxx = max_d(mxx, rx);
+                    mny = min_d(mny, ry);
+                    mxy = max_d(mxy, ry);
                 }
                 mnx = warp_min_d(mnx);
                 mxx = warp_max_d(mxx);
@@ -329,16 +385,21 @@ __device__ bool pca_axes(double sxx, double sxy, double syy, double& v00, double
 {
     if (!(isfinite(sxx) && isfinite(sxy) && isfinite(syy)))
         return false;
-    double scale = fmax(fmax(fabs(sxx), fabs(sxy)), fmax(fabs(sxy), fabs(syy)));
+    double scale = max_d(max_d(fabs(sxx), fabs(sxy)), fabs(syy));
     if (scale == 0.0)
         scale = 1.0;
-    double w00 = sxx / scale, w01 = sxy / scale, w10 = sxy / scale, w11 = syy / scale;
+    // the divisions by the scale on lanes 0, 1 and 2 (one division sequence)
+    const uint32_t lane = lane_id();
+    const double wq = div_d(((lane == 0u) ? sxx : ((lane == 1u) ? sxy : syy)), scale);
+    double w00 = __shfl_sync(0xffffffffu, wq, 0), w01 = __shfl_sync(0xffffffffu, wq, 1), w10 = w01,
+           w11 = __shfl_sync(0xffffffffu, wq, 2);
     v00 = 1.0, v01 = 0.0, v10 = 0.0, v11 = 1.0;
     const double precision = 2.0 * DBL_EPSILON;
-    double max_diag = fmax(fabs(w00), fabs(w11));
+    double max_diag = max_d(fabs(w00), fabs(w11));
+#pragma unroll 1
     for (int sweep = 0; sweep < 64; ++sweep)
     {
-        const double threshold = fmax(DBL_MIN, precision * max_diag);
+        const double threshold = max_d(DBL_MIN, precision * max_diag);
         if (!(fabs(w10) > threshold || fabs(w01) > threshold))
             break;
         // block of the index pair (1, 0): m = [[W11, W10], [W01, W00]]
@@ -347,28 +408,28 @@ __device__ bool pca_axes(double sxx, double sxy, double syy, double& v00, double
         const double t = m00 + m11, d = m10 - m01;
         if (!(fabs(d) < DBL_MIN))
         {
-            const double u = t / d;
-            const double tmp = sqrt(1.0 + u * u);
-            r1 = Rot2{u / tmp, 1.0 / tmp};
+            const double u = div_d(t, d);
+            const double tmp = sqrt_d(1.0 + u * u);
+            r1 = Rot2{div_d(u, tmp), div_d(1.0, tmp)};
         }
         rot2_apply(m00, m01, m10, m11, r1);
         Rot2 rr{1.0, 0.0}; // the Jacobi rotation of [[m00, m01], [m01, m11]]
         const double deno = 2.0 * fabs(m01);
         if (!(deno < DBL_MIN))
         {
-            const double tau = (m00 - m11) / deno;
-            const double w = sqrt(tau * tau + 1.0);
-            const double tt = tau > 0.0 ? 1.0 / (tau + w) : 1.0 / (tau - w);
+            const double tau = div_d(m00 - m11, deno);
+            const double w = sqrt_d(tau * tau + 1.0);
+            const double tt = div_d(1.0, tau > 0.0 ? tau + w : tau - w);
             const double sign_t = tt > 0.0 ? 1.0 : -1.0;
-            const double n = 1.0 / sqrt(tt * tt + 1.0);
-            rr = Rot2{n, -sign_t * (m01 / fabs(m01)) * fabs(tt) * n};
+            const double n = div_d(1.0, sqrt_d(tt * tt + 1.0));
+            rr = Rot2{n, -sign_t * copysign(1.0, m01) * fabs(tt) * n}; // (m01 / |m01|, m01 finite and not zero)
         }
         const Rot2 rl{r1.c * rr.c - r1.s * -rr.s, r1.c * -rr.s + r1.s * rr.c}; // r1 composed with rr^T
         const Rot2 rt{rr.c, -rr.s};
         rot2_apply(w10, w11, w00, w01, rl); // rows 1 and 0 of W
         rot2_apply(w01, w11, w00, w10, rt); // columns 1 and 0 of W
         rot2_apply(v01, v11, v00, v10, rt); // columns 1 and 0 of V
-        max_diag = fmax(max_diag, fmax(fabs(w11), fabs(w00)));
+        max_diag = max_d(max_d(max_diag, fabs(w11)), fabs(w00));
     }
     if (fabs(w11) * scale > fabs(w00) * scale)
     {
@@ -381,12 +442,26 @@ __device__ bool pca_axes(double sxx, double sxy, double syy, double& v00, double
     return true;
 }
 
+// No box: every field zero, by one warp.
+__device__ __forceinline__ void no_box(lp_bounding_box* out)
+{
+    const uint32_t lane = lane_id();
+    if (lane < 8u)
+        out->corners[lane >> 1][lane & 1u] = 0.0;
+    if (lane == 0)
+    {
+        out->area = 0.0f;
+        out->angle_rad = 0.0f;
+        out->is_valid = 0;
+    }
+}
+
 // Sums of the x and of the y coordinates of P[0..n) as the reference's loop computes them in
 // binary64 (left to right), by one warp; every lane returns both. Each term is a multiple of
 // 2^g (g from its exponent and the trailing zeros of its significand) and below 2^t in
 // magnitude; when log2(n) + max t - min g <= 53 every partial sum of any order is exact, so a warp
 // tree gives the loop's result. Otherwise (tiny next to large coordinates) the loop runs as written.
-__device__ __forceinline__ void sum_xy_fp64(const double2* P, int n, double& sx, double& sy)
+__device__ __noinline__ void sum_xy_fp64(const double2* P, int n, double& sx, double& sy)
 {
     const uint32_t lane = lane_id();
     int tmax = -4096, gmin = 4096;
@@ -406,6 +481,7 @@ __device__ __forceinline__ void sum_xy_fp64(const double2* P, int n, double& sx,
         tmax = max(tmax, e - 1022);
         gmin = min(gmin, e - 1075 + (__ffsll(static_cast<long long>(m)) - 1));
     };
+#pragma unroll 1
     for (int k = static_cast<int>(lane); k < n; k += 32)
     {
         scan(P[k].x);
@@ -431,6 +507,7 @@ __device__ __forceinline__ void sum_xy_fp64(const double2* P, int n, double& sx,
     }
     sx = 0.0;
     sy = 0.0;
+#pragma unroll 1
     for (int k = 0; k < n; ++k)
     {
         sx += P[k].x;
@@ -443,25 +520,20 @@ __device__ __forceinline__ void sum_xy_fp64(const double2* P, int n, double& sx,
 // (pca_axes, evaluated by every lane alike), the rotated extents (lanes stride over the vertices;
 // min and max do not depend on order) and the corners. The box equals the reference loop's bit
 // for bit.
-__device__ void pca_box_warp(const double2* P, int n, lp_bounding_box* out)
+__device__ __noinline__ void pca_box_warp(const double2* P, int n, lp_bounding_box* out)
 {
     const uint32_t lane = lane_id();
-    lp_bounding_box box;
-    for (int k = 0; k < 4; ++k)
-        box.corners[k][0] = box.corners[k][1] = 0.0;
-    box.area = 0.0f;
-    box.angle_rad = 0.0f;
-    box.is_valid = 0;
     if (n >= 3)
     {
         double sx, sy;
         sum_xy_fp64(P, n, sx, sy);
         // mx = sx / n and my = sy / n on lanes 0 and 1 (one division sequence)
-        const double mq = ((lane & 1u) ? sy : sx) / static_cast<double>(n);
+        const double mq = div_d((lane & 1u) ? sy : sx, static_cast<double>(n));
         const double mx = __shfl_sync(0xffffffffu, mq, 0), my = __shfl_sync(0xffffffffu, mq, 1);
         // the three covariance sums keep the reference's order: the products of vertex k come from
         // lane k mod 32, lanes 0, 1 and 2 accumulate sxx, sxy and syy in one instruction per step
         double acc = 0.0;
+#pragma unroll 1
         for (int base = 0; base < n; base += 32)
         {
             const int k = base + static_cast<int>(lane);
@@ -474,6 +546,7 @@ __device__ void pca_box_warp(const double2* P, int n, lp_bounding_box* out)
                 tyy = dy * dy;
             }
             const int cnt = min(32, n - base);
+#pragma unroll 2
             for (int j = 0; j < cnt; ++j)
             {
                 const double a0 = __shfl_sync(0xffffffffu, txx, j);
@@ -482,110 +555,67 @@ __device__ void pca_box_warp(const double2* P, int n, lp_bounding_box* out)
                 acc += (lane == 0u) ? a0 : ((lane == 1u) ? a1 : a2);
             }
         }
-        const double cq = acc / static_cast<double>(n - 1);
+        const double cq = div_d(acc, static_cast<double>(n - 1));
         const double sxx = __shfl_sync(0xffffffffu, cq, 0), sxy = __shfl_sync(0xffffffffu, cq, 1),
                      syy = __shfl_sync(0xffffffffu, cq, 2);
         double v00, v01, v10, v11;
         if (pca_axes(sxx, sxy, syy, v00, v01, v10, v11))
         {
             double mnx = DBL_MAX, mxx = -DBL_MAX, mny = DBL_MAX, mxy = -DBL_MAX;
+#pragma unroll 1
             for (int i = static_cast<int>(lane); i < n; i += 32)
             {
                 const double dx = P[i].x - mx, dy = P[i].y - my;
                 const double rx = dx * v00 + dy * v10;
                 const double ry = dx * v01 + dy * v11;
-                mnx = fmin(mnx, rx);
-                mxx = fmax(mxx, rx);
-                mny = fmin(mny, ry);
-                mxy = fmax(mxy, ry);
+                mnx = min_d(mnx, rx);
+                mxx = max_d(mxx, rx);
+                mny = min_d(mny, ry);
+                mxy = max_d(mxy, ry);
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
+            mnx = warp_min_d(mnx);
+            mxx = warp_max_d(mxx);
+            mny = warp_min_d(mny);
+            mxy = warp_max_d(mxy);
+            // coordinate c of corner k from lane 2 k + c (one sequence for all eight)
+            const int k = static_cast<int>(lane >> 1) & 3;
+            const bool cy = (lane & 1u) != 0u;
+            const double xk = (k == 1 || k == 2) ? mxx : mnx, yk = (k >= 2) ? mxy : mny;
+            const double at = xk * (cy ? v10 : v00) + yk * (cy ? v11 : v01) + (cy ? my : mx);
+            if (lane < 8u)
+                out->corners[k][cy] = at;
+            if (lane == 0)
             {
-                mnx = fmin(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-                mxx = fmax(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-                mny = fmin(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-                mxy = fmax(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+                out->area = __double2float_rn((mxx - mnx) * (mxy - mny));
+                out->angle_rad = __double2float_rn(atan2(v10, v00));
+                out->is_valid = 1;
             }
-            const double xs[4] = {mnx, mxx, mxx, mnx};
-            const double ys[4] = {mny, mny, mxy, mxy};
-            for (int k = 0; k < 4; ++k)
-            {
-                box.corners[k][0] = xs[k] * v00 + ys[k] * v01 + mx;
-                box.corners[k][1] = xs[k] * v10 + ys[k] * v11 + my;
-            }
-            box.area = __double2float_rn((mxx - mnx) * (mxy - mny));
-            box.angle_rad = __double2float_rn(atan2(v10, v00));
-            box.is_valid = 1;
+            return;
         }
     }
-    if (lane == 0)
-        *out = box;
+    no_box(out);
 }
 
 // FP64 rotated extents of P about (cx, cy) for the unit direction (ux, uy), by one warp.
-__device__ __forceinline__ void extents_fp64(const double2* P, int n, double cx, double cy, double ux, double uy,
+__device__ __noinline__ void extents_fp64(const double2* P, int n, double cx, double cy, double ux, double uy,
                                              double& mnx, double& mxx, double& mny, double& mxy)
 {
     mnx = DBL_MAX, mxx = -DBL_MAX, mny = DBL_MAX, mxy = -DBL_MAX;
+#pragma unroll 1
     for (int k = static_cast<int>(lane_id()); k < n; k += 32)
     {
         const double tx = P[k].x - cx, ty = P[k].y - cy;
         const double rx = tx * ux + ty * uy;
         const double ry = -tx * uy + ty * ux;
-        mnx = fmin(mnx, rx);
-        mxx = fmax(mxx, rx);
-        mny = fmin(mny, ry);
-        mxy = fmax(mxy, ry);
+        mnx = min_d(mnx, rx);
+        mxx = max_d(mxx, rx);
+        mny = min_d(mny, ry);
+        mxy = max_d(mxy, ry);
     }
     mnx = warp_min_d(mnx);
     mxx = warp_max_d(mxx);
     mny = warp_min_d(mny);
     mxy = warp_max_d(mxy);
-}
-
-// extents_fp64 for n <= 32 (vertex k on lane k). The FP32 projections of the float vertices about
-// the float centroid along the float direction lie within tol / 2 of the FP64 ones, so a lane more
-// than tol above the FP32 minimum cannot hold the FP64 minimum: only the lanes within tol of each
-// FP32 extreme compare their FP64 values (usually one or two lanes instead of a five-level tree).
-__device__ __forceinline__ double pick_min_fp64(double v, float f, float tol)
-{
-    const float m = warp_min_f(f);
-    double r = DBL_MAX;
-    for (uint32_t c = __ballot_sync(0xffffffffu, f <= m + tol); c != 0u; c &= c - 1u)
-        r = fmin(r, __shfl_sync(0xffffffffu, v, __ffs(c) - 1));
-    return r;
-}
-__device__ __forceinline__ double pick_max_fp64(double v, float f, float tol)
-{
-    const float m = warp_max_f(f);
-    double r = -DBL_MAX;
-    for (uint32_t c = __ballot_sync(0xffffffffu, f >= m - tol); c != 0u; c &= c - 1u)
-        r = fmax(r, __shfl_sync(0xffffffffu, v, __ffs(c) - 1));
-    return r;
-}
-__device__ __forceinline__ void extents_screened(const double2* P, const float2* Pf, int n, double cx, double cy,
-                                                 double ux, double uy, float cxf, float cyf, float tol, double& mnx,
-                                                 double& mxx, double& mny, double& mxy)
-{
-    const int lane = static_cast<int>(lane_id());
-    const bool live = lane < n;
-    const float uxf = __double2float_rn(ux), uyf = __double2float_rn(uy);
-    double rx = 0.0, ry = 0.0;
-    float fx = 0.0f, fy = 0.0f;
-    if (live)
-    {
-        const double tx = P[lane].x - cx, ty = P[lane].y - cy;
-        rx = tx * ux + ty * uy;
-        ry = -tx * uy + ty * ux;
-        const float sx = Pf[lane].x - cxf, sy = Pf[lane].y - cyf;
-        fx = sx * uxf + sy * uyf;
-        fy = -sx * uyf + sy * uxf;
-    }
-    mnx = pick_min_fp64(rx, live ? fx : INFINITY, tol);
-    mxx = pick_max_fp64(rx, live ? fx : -INFINITY, tol);
-    mny = pick_min_fp64(ry, live ? fy : INFINITY, tol);
-    mxy = pick_max_fp64(ry, live ? fy : -INFINITY, tol);
 }
 
 // Rotating calipers with the candidate boxes screened in FP32 (same result as calipers_warp).
@@ -607,20 +637,13 @@ __device__ __forceinline__ void extents_screened(const double2* P, const float2*
 // misses a vertex never looks at its edges, and a contender set made only of unvisited edges
 // would leave no box where the reference keeps one.
 // Up to 32 contenders (one per lane) are handled; more fall back to calipers_warp.
-__device__ void calipers_fast(const double2* P, const float2* Pf, int n, const int2* pairs, int npairs, float* ea,
+__device__ __noinline__ void calipers_fast(const double2* P, const float2* Pf, int n, const int2* pairs, int npairs, float* ea,
                               float r2, lp_bounding_box* out)
 {
     const uint32_t lane = lane_id();
-    lp_bounding_box box;
-    for (int k = 0; k < 4; ++k)
-        box.corners[k][0] = box.corners[k][1] = 0.0;
-    box.area = 0.0f;
-    box.angle_rad = 0.0f;
-    box.is_valid = 0;
     if (n < 3)
     {
-        if (lane == 0)
-            *out = box;
+        no_box(out);
         return;
     }
     const float ox = Pf[0].x, oy = Pf[0].y;
@@ -628,9 +651,11 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
     // Only edges the walk visits can hold the reference's box: on a near-degenerate hull the pair
     // walk can miss a vertex, and with it an edge that may have the smallest area. Mark the
     // visited edges (ea[j] = 0, the edge mapping of `visit` below) before choosing contenders.
+#pragma unroll 1
     for (int j = static_cast<int>(lane); j < n; j += 32)
         ea[j] = -1.0f;
     __syncwarp();
+#pragma unroll 1
     for (int v = static_cast<int>(lane); v < 4 * npairs; v += 32)
     {
         const int2 pr = pairs[v >> 2];
@@ -639,6 +664,7 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
     }
     __syncwarp();
     float amin = INFINITY;
+#pragma unroll 1
     for (int j = static_cast<int>(lane); j < n; j += 32)
     {
         const int j1 = (j + 1 == n) ? 0 : j + 1;
@@ -648,7 +674,7 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
         if (!skip && !(fl2 > 1.0001e-12f))
         {
             const double dx = P[j1].x - P[j].x, dy = P[j1].y - P[j].y;
-            skip = sqrt(dx * dx + dy * dy) < 1.0e-6;
+            skip = sqrt_d(dx * dx + dy * dy) < 1.0e-6;
         }
         float a = INFINITY; // edges the reference skips never compete
         if (!skip)
@@ -656,6 +682,7 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
             const float fl = sqrtf(fl2);
             const float ux = fx / fl, uy = fy / fl;
             float mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
+#pragma unroll 2
             for (int k = 0; k < n; ++k)
             {
                 const float tx = Pf[k].x - ox, ty = Pf[k].y - oy;
@@ -675,16 +702,17 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
     __syncwarp();
     if (amin == INFINITY)
     {
-        if (lane == 0)
-            *out = box; // every edge is skipped: no box, as in the reference
+        no_box(out); // every edge is skipped, as in the reference
         return;
     }
     float T = amin;
+#pragma unroll 1
     for (int it = 0; it <= n; ++it)
     {
         const float G = 2.0f * e + 1e-6f * (T + 2.0f * e);
         float nt = T;
-        for (int j = static_cast<int>(lane); j < n; j += 32)
+    #pragma unroll 1
+    for (int j = static_cast<int>(lane); j < n; j += 32)
             if (ea[j] > T && ea[j] <= T + G)
                 nt = fmaxf(nt, ea[j]);
         nt = warp_max_f(nt);
@@ -695,15 +723,17 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
     // FP64 centroid of the hull vertices, as the reference's loop sums them
     double sx, sy;
     sum_xy_fp64(P, n, sx, sy);
-    const double cq = ((lane & 1u) ? sy : sx) / static_cast<double>(n);
+    const double cq = div_d((lane & 1u) ? sy : sx, static_cast<double>(n));
     const double cx = __shfl_sync(0xffffffffu, cq, 0), cy = __shfl_sync(0xffffffffu, cq, 1);
     // contender c (in edge order) is held by lane c: its edge, direction, FP64 extents and area
     int my_j = -1;
     int ncont = 0;
+#pragma unroll 1
     for (int base = 0; base < n; base += 32)
     {
         const int j = base + static_cast<int>(lane);
         const uint32_t mask = __ballot_sync(0xffffffffu, j < n && ea[j] <= T);
+#pragma unroll 1
         for (uint32_t mm = mask; mm != 0u; mm &= mm - 1u, ++ncont)
             if (static_cast<int>(lane) == ncont) // contender ncont goes to lane ncont
                 my_j = base + __ffs(mm) - 1;
@@ -721,24 +751,16 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
     {
         const int j1 = (my_j + 1 == n) ? 0 : my_j + 1;
         const double ex = P[j1].x - P[my_j].x, ey = P[j1].y - P[my_j].y;
-        const double len = sqrt(ex * ex + ey * ey);
-        my_ux = ex / len;
-        my_uy = ey / len;
+        const double len = sqrt_d(ex * ex + ey * ey);
+        my_ux = div_d(ex, len);
+        my_uy = div_d(ey, len);
     }
-    // FP32 projection error bound of extents_screened: the float centroid is within 2^-24 (|cx| +
-    // |cy|) of the FP64 one, the float direction within 2^-24 per component, and every difference,
-    // product and sum rounds by 2^-24 relative to |P - c|_1 <= 3 sqrt(r2); the window takes 4x
-    // (centroid) and 8x (rounding) those sums as tol / 2.
-    const float cxf = __double2float_rn(cx), cyf = __double2float_rn(cy);
-    const float tol = 2.0f * ((fabsf(cxf) + fabsf(cyf)) * 2.384185791015625e-7f + 3.0f * sqrtf(r2) * 1.9073486328125e-6f) + 1e-30f;
+#pragma unroll 1
     for (int c = 0; c < ncont; ++c)
     {
         const double ux = __shfl_sync(0xffffffffu, my_ux, c), uy = __shfl_sync(0xffffffffu, my_uy, c);
         double mnx, mxx, mny, mxy;
-        if (n <= 32)
-            extents_screened(P, Pf, n, cx, cy, ux, uy, cxf, cyf, tol, mnx, mxx, mny, mxy);
-        else
-            extents_fp64(P, n, cx, cy, ux, uy, mnx, mxx, mny, mxy);
+        extents_fp64(P, n, cx, cy, ux, uy, mnx, mxx, mny, mxy);
         if (static_cast<int>(lane) == c)
         {
             my_mnx = mnx;
@@ -776,6 +798,7 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
         const bool cont = ea[j] <= T;
         f = INFINITY;
         below = 0;
+#pragma unroll 1
         for (int c = 0; c < ncont; ++c)
         {
             const int jc = __shfl_sync(0xffffffffu, my_j, c);
@@ -791,6 +814,7 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
     };
     float fmin = INFINITY;
     bool any = false;
+#pragma unroll 1
     for (int v0 = 0; v0 < nvis; v0 += 32)
     {
         const int v = v0 + static_cast<int>(lane);
@@ -805,6 +829,7 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
     fmin = warp_min_f(fmin);
     any = __any_sync(0xffffffffu, any);
     int first = INT32_MAX, lastb = -1;
+#pragma unroll 1
     for (int v0 = 0; any && v0 < nvis; v0 += 32)
     {
         const int v = v0 + static_cast<int>(lane);
@@ -849,26 +874,29 @@ __device__ void calipers_fast(const double2* P, const float2* Pf, int n, const i
             mny = -mxy;
             mxy = -a1;
         }
-        box.area = best;
-        box.corners[0][0] = mnx * ux - mny * uy + cx;
-        box.corners[0][1] = mnx * uy + mny * ux + cy;
-        box.corners[1][0] = mxx * ux - mny * uy + cx;
-        box.corners[1][1] = mxx * uy + mny * ux + cy;
-        box.corners[2][0] = mxx * ux - mxy * uy + cx;
-        box.corners[2][1] = mxx * uy + mxy * ux + cy;
-        box.corners[3][0] = mnx * ux - mxy * uy + cx;
-        box.corners[3][1] = mnx * uy + mxy * ux + cy;
-        box.angle_rad = lpm::atan2_approx(__double2float_rn(uy), __double2float_rn(ux));
-        box.is_valid = 1;
+        // coordinate c of corner k from lane 2 k + c (one sequence for all eight): x ux - y uy + cx and
+        // x uy + y ux + cy
+        const int k = static_cast<int>(lane >> 1) & 3;
+        const bool yy = (lane & 1u) != 0u;
+        const double xk = (k == 1 || k == 2) ? mxx : mnx, yk = (k >= 2) ? mxy : mny;
+        const double at = xk * (yy ? uy : ux) + (yy ? yk * ux : -(yk * uy)) + (yy ? cy : cx);
+        if (lane < 8u)
+            out->corners[k][yy] = at;
+        if (lane == 0)
+        {
+            out->area = best;
+            out->angle_rad = lpm::atan2_approx(__double2float_rn(uy), __double2float_rn(ux));
+            out->is_valid = 1;
+        }
+        return;
     }
-    if (lane == 0)
-        *out = box;
+    no_box(out);
 }
 
 // Antipodal pairs and the rotating-calipers box of hull P (h vertices) by one warp. With float
 // copies Pf and h floats of scratch ea the comparisons are screened in FP32; without them
 // (Pf == nullptr) everything runs in FP64.
-__device__ void calipers_box(ScanState* st, const double2* P, const float2* Pf, float* ea, int h, int2* pairs,
+__device__ __noinline__ void calipers_box(ScanState* st, const double2* P, const float2* Pf, float* ea, int h, int2* pairs,
                              lp_bounding_box* out)
 {
     const uint32_t lane = lane_id();
@@ -886,7 +914,8 @@ __device__ void calipers_box(ScanState* st, const double2* P, const float2* Pf, 
         }
         r2 = warp_max_f(r2) * 1.001f;
         mabs = warp_max_f(mabs);
-        const AreaCmpFiltered cmp{P, Pf, ox, oy, 2.0f * (4e-6f * r2 + 1e-13f * mabs * sqrtf(r2)) + 1e-30f};
+        const float mr = mabs * sqrtf(r2);
+        const AreaCmpFiltered cmp{P, Pf, ox, oy, 2.0f * (4e-6f * r2 + 1e-13f * mr) + 1e-30f, 4e-12f * r2 + 4e-13f * mr + 1e-30f};
         if (lane == 0)
             npairs = antipodal_pairs(cmp, h, pairs, cap);
         npairs = __shfl_sync(0xffffffffu, npairs, 0);
@@ -918,92 +947,152 @@ __device__ void calipers_box(ScanState* st, const double2* P, const float2* Pf, 
 // Orientation test of the monotone chain for float points: decided in FP32 when the float
 // determinant exceeds 2^-21 (|t1| + |t2|) in magnitude (its rounding error stays below
 // 6 * 2^-24 of that sum, the FP64 form's below 3 * 2^-53), else evaluated in FP64 as written.
-// b - a is exact in binary32 (Knuth's TwoSum of b and -a leaves no error).
-__device__ __forceinline__ bool diff_exact(float b, float a, float s)
-{
-    const float a1 = s - b;
-    const float b1 = s - a1;
-    return ((-a) - a1) + (b - b1) == 0.0f;
-}
-
 // u * v has an exact binary32 error term (no underflow in the product).
 __device__ __forceinline__ bool prod_err_exact(float u, float v, float t)
 {
     return fabsf(t) >= 1e-30f || u == 0.0f || v == 0.0f;
 }
 
-__device__ __forceinline__ bool ccw_or_colinear_f(float ax, float ay, float bx, float by, float cx, float cy)
+// The near-ties of ccw_or_colinear_f, out of line: points along a wall are mostly such.
+__device__ __noinline__ bool ccw_or_colinear_near(float ax, float ay, float bx, float by, float cx, float cy)
+{
+    const float u = bx - ax, v = cy - ay, w = by - ay, z = cx - ax;
+    const float t1 = u * v;
+    const float t2 = w * z;
+    if (prod_err_exact(u, v, t1) && prod_err_exact(w, z, t2))
+    {
+        const float ul = diff_err(bx, ax, u), vl = diff_err(cy, ay, v), wl = diff_err(by, ay, w), zl = diff_err(cx, ax, z);
+        const float e1 = __fmaf_rn(u, v, -t1), e2 = __fmaf_rn(w, z, -t2);
+        // When the four differences are exact binary32 values, each product of two of them
+        // is exact in binary64 (48 significant bits), so the binary64 expression has the sign
+        // of u v - w z exactly. Rounding to binary32 is monotone, so t1 < t2 implies u v < w z (and
+        // t1 > t2 the converse); at t1 == t2 the difference is e1 - e2, the exact product errors.
+        if (ul == 0.0f && vl == 0.0f && wl == 0.0f && zl == 0.0f)
+            return t1 != t2 ? t1 < t2 : e1 <= e2;
+        // Otherwise the products of the exact two-term differences up to their last cross term: t + e + (u vl +
+        // ul v) errs by less than 2^-46 |t| (the dropped ul vl is below 2^-48, each rounding of the small
+        // terms too), t1 - t2 is exact (both lie within 2^-20 of each other), the sums of the small terms
+        // round by less than 2^-46 (|t1| + |t2|): beyond 2^-42 of that sum, the sign is the exact one, and
+        // the binary64 expression, within 3 * 2^-53 of it, has it too.
+        const float d = (t1 - t2) + ((e1 + (u * vl + ul * v)) - (e2 + (w * zl + wl * z)));
+        if (fabsf(d) > 2.2737367544323206e-13f * (fabsf(t1) + fabsf(t2)))
+            return d < 0.0f;
+    }
+    return ccw_or_colinear(ax, ay, bx, by, cx, cy);
+}
+
+// Does the candidate c pop b (a below it)? The FP32 decision; `near`: it is not one, ask chain_pops_near.
+__device__ __forceinline__ bool chain_pops(float ax, float ay, float bx, float by, float cx, float cy, bool& near)
 {
     const float u = bx - ax, v = cy - ay, w = by - ay, z = cx - ax;
     const float t1 = u * v;
     const float t2 = w * z;
     const float d = t1 - t2;
-    const float bound = (fabsf(t1) + fabsf(t2)) * 4.76837158203125e-7f + 1e-30f;
-    if (d > bound)
-        return false;
-    if (d < -bound)
-        return true;
-    // Near-tie. When the four differences are exact binary32 values, each product of two of them
-    // is exact in binary64 (48 significant bits), so the binary64 expression above has the sign
-    // of u v - w z exactly. Rounding to binary32 is monotone, so t1 < t2 implies u v < w z (and
-    // t1 > t2 the converse); at t1 == t2 the difference is e1 - e2, the exact product errors.
-    if (diff_exact(bx, ax, u) && diff_exact(cy, ay, v) && diff_exact(by, ay, w) && diff_exact(cx, ax, z) &&
-        prod_err_exact(u, v, t1) && prod_err_exact(w, z, t2))
-    {
-        if (t1 != t2)
-            return t1 < t2;
-        return __fmaf_rn(u, v, -t1) <= __fmaf_rn(w, z, -t2);
-    }
+    near = !(fabsf(d) > (fabsf(t1) + fabsf(t2)) * 4.76837158203125e-7f + 1e-30f);
+    return d < 0.0f;
+}
+__device__ __forceinline__ bool chain_pops_near(float ax, float ay, float bx, float by, float cx, float cy)
+{
+    return ccw_or_colinear_near(ax, ay, bx, by, cx, cy);
+}
+__device__ __forceinline__ bool chain_pops(double ax, double ay, double bx, double by, double cx, double cy, bool& near)
+{
+    near = false;
+    return ccw_or_colinear(ax, ay, bx, by, cx, cy);
+}
+__device__ __forceinline__ bool chain_pops_near(double ax, double ay, double bx, double by, double cx, double cy)
+{
     return ccw_or_colinear(ax, ay, bx, by, cx, cy);
 }
 
-__device__ __forceinline__ bool chain_pops(const HPt<float>& a, const HPt<float>& b, const HPt<float>& c)
-{
-    return ccw_or_colinear_f(a.x, a.y, b.x, b.y, c.x, c.y);
-}
-__device__ __forceinline__ bool chain_pops(const HPt<double>& a, const HPt<double>& b, const HPt<double>& c)
-{
-    return ccw_or_colinear(a.x, a.y, b.x, b.y, c.x, c.y);
-}
-
-// One half of the monotone chain over sorted candidates C[0..m) (polygonizer.cpp:62-88) by one
-// thread: the lower half walks C forwards, the upper half backwards from C[m - 1]. The reference's
+// One half of the monotone chain over sorted candidates C[0..m) (polygonizer.cpp:62-88) by W lanes
+// (32: a warp; 16: half of one, the other half walks the other half of the chain): the lower
+// half walks C forwards, the upper half backwards from C[m - 1]. The reference's
 // second loop continues on the stack of the first but never pops below C[m - 1] (its k >= t
-// test), so the upper half is the same walk on its own stack starting from that point. The two
-// points below the top stay in registers. Writes the stack to S, returns its size.
-template <typename T>
-__device__ int chain_half(const HPt<T>* C, int m, int* S, bool upper)
+// test), so the upper half is the same walk on its own stack starting from that point. Writes the stack
+// to S, returns its size.
+// The walk is a chain of orientation tests, each a chain of its own: one thread took 400 cycles a candidate. Here lane l
+// holds the l-th point from the top of the stack and the one below it, and tests whether the candidate pops it once
+// those above are gone; the pops are the lanes up to the first that says no, so a candidate costs one test, a ballot and
+// the shuffles, without a divergent branch (each costs some 40 cycles). Points deeper than W come back from memory when
+// they are uncovered, and only the first lane that does not pop for certain has its near-tie decided.
+template <int W, typename T>
+__device__ __noinline__ int chain_half(const HPt<T>* C, int m, int* S, bool upper)
 {
+    const int l = static_cast<int>(lane_id()) & (W - 1);
+    const int first = static_cast<int>(lane_id()) - l;
     int k = 0;
-    HPt<T> a{}, b{};
-    for (int j = 0; j < m; ++j)
-    {
-        const int i = upper ? m - 1 - j : j;
-        const HPt<T> c = C[i];
-        while (k > 1 && chain_pops(a, b, c))
+    T ax = T(0), ay = T(0), bx = T(0), by = T(0); // below, and the l-th from the top
+    auto at = [&](int depth, T& x, T& y) { // the stack's entry `depth` from the bottom, if there is one
+        if (depth >= 0)
         {
-            --k;
-            b = a;
-            if (k > 1)
-                a = C[S[k - 2]];
+            const HPt<T> p = C[S[depth]];
+            x = p.x;
+            y = p.y;
         }
-        a = b;
-        b = c;
-        S[k++] = i;
+    };
+    auto group = [&](uint32_t mask) { return (W == 32) ? mask : ((mask >> first) & ((1u << (W & 31)) - 1u)); };
+    int i = upper ? m - 1 : 0;
+    const int step = upper ? -1 : 1;
+    HPt<T> next = (m > 0) ? C[i] : HPt<T>{};
+    for (int j = 0; j < m; ++j, i += step)
+    {
+        const HPt<T> c = next;
+        next = C[min(max(i + step, 0), m - 1)];
+        const bool deep = (W == 32) ? k > W : __any_sync(0xffffffffu, k > W); // (only then can every lane pop)
+        bool near, live = l + 1 < k;
+        bool pop = chain_pops(ax, ay, bx, by, c.x, c.y, near);
+        near = near & live;
+        pop = pop & live & !near;
+        const uint32_t keep = __ballot_sync(0xffffffffu, !pop), ties = __ballot_sync(0xffffffffu, near);
+        int pops = __ffs(group(keep)) - 1;
+        const uint32_t lowest = (W == 32) ? (keep & (0u - keep))
+                                          : ((keep & (0u - keep)) | ((keep >> 16) & (0u - (keep >> 16))) << 16);
+        if ((lowest & ties) != 0u || deep) // (the same for all lanes)
+        {
+            __syncwarp(); // the entries written so far, before they are read here and below
+            for (;;)
+            {
+                if (near)
+                    pop = chain_pops_near(ax, ay, bx, by, c.x, c.y);
+                const uint32_t mine = group(__ballot_sync(0xffffffffu, !pop));
+                pops = mine ? __ffs(mine) - 1 : W;
+                if (!__any_sync(0xffffffffu, pops == W))
+                    break;
+                if (pops == W)
+                {
+                    k -= W;
+                    at(k - 1 - l, bx, by);
+                    at(k - 2 - l, ax, ay);
+                    live = l + 1 < k;
+                    pop = chain_pops(ax, ay, bx, by, c.x, c.y, near);
+                    near = near & live;
+                    pop = pop & live & !near;
+                }
+            }
+        }
+        k -= pops;
+        const int own = l - 1 + pops, below = l + pops;
+        T nx = __shfl_sync(0xffffffffu, bx, first + (own & (W - 1))), ny = __shfl_sync(0xffffffffu, by, first + (own & (W - 1)));
+        T mx = __shfl_sync(0xffffffffu, bx, first + (below & (W - 1))),
+          my = __shfl_sync(0xffffffffu, by, first + (below & (W - 1)));
+        if (deep)
+        {
+            if (own >= W)
+                at(k - l, nx, ny);
+            if (below >= W)
+                at(k - 1 - l, mx, my);
+        }
+        ax = mx;
+        ay = my;
+        bx = (l == 0) ? c.x : nx;
+        by = (l == 0) ? c.y : ny;
+        if (l == 0)
+            S[k] = i;
+        ++k;
     }
+    __syncwarp();
     return k;
-}
-
-// The whole chain by one thread: hull positions into H (capacity 2m), returns the hull size
-// (the reference's k - 1: the last point repeats the first).
-template <typename T>
-__device__ int monotone_chain(const HPt<T>* C, int m, int* H)
-{
-    if (m == 0)
-        return -1;
-    const int kl = chain_half(C, m, H, false);
-    const int ku = chain_half(C, m, H + kl - 1, true); // its first entry is H[kl - 1] = m - 1 again
-    return kl + ku - 2;
 }
 
 // Strictly left of a -> b by a relative margin of 1e-5: the float cross product errs by less
@@ -1048,14 +1137,13 @@ __device__ void block_sort_global(HPt<T>* a, uint32_t n)
 constexpr int kDirs = 16;         // extreme-point directions of the initial polygon
 constexpr int kPolyCap = 256;     // refined polygon capacity
 constexpr int kRefineRounds = 12; // farthest-point insertion rounds
+constexpr uint32_t kHullEnough = 48; // active members few enough to end them
 constexpr uint32_t kBigCluster = 512; // larger clusters take a whole CTA; smaller ones one warp
 
 struct HullSmem
 {
     HPt<float> cand[kHullSmem];
     int stack[2 * kHullSmem + 2];
-    double2 hp[kHullSmem];
-    float2 pf[kHullSmem];     // hull vertices as floats
     uint32_t hkey[kHullSmem]; // hull vertex member keys, sorted
     int32_t diff[kHullSmem + 1];
     float2 poly[kPolyCap];
@@ -1065,6 +1153,7 @@ struct HullSmem
     unsigned long long pkey[kPolyCap];
     unsigned long long ext[kDirs][kHullThreads / 32];
     float2 dirs[kDirs];
+    uint32_t scan[33];
     int npoly;
     int grew;
     int ncand;
@@ -1132,7 +1221,42 @@ struct Extremes16
     {
         return d < 8 ? fkey_payload(hi[d], ih[d]) : fkey_payload(-lo[d - 8], il[d - 8]);
     }
+    // The warp's largest key of direction d, on lane d (the other lanes: unspecified). Two integer
+    // reductions a direction, of the value and of the positions that hold it.
+    __device__ __forceinline__ unsigned long long warp_key() const
+    {
+        unsigned long long mine = 0ull;
+#pragma unroll
+        for (int d = 0; d < kDirs; ++d)
+        {
+            const unsigned long long k = key(d);
+            const uint32_t v = static_cast<uint32_t>(k >> 32);
+            const uint32_t top = __reduce_max_sync(0xffffffffu, v);
+            const uint32_t at = __reduce_max_sync(0xffffffffu, v == top ? static_cast<uint32_t>(k) : 0u);
+            if (static_cast<int>(lane_id()) == d)
+                mine = (static_cast<unsigned long long>(top) << 32) | at;
+        }
+        return mine;
+    }
 };
+
+// The polygon of the extreme members in direction order (counter-clockwise), repeats dropped, by one
+// warp: lane d < kDirs holds direction d's key, so the members load side by side. Returns its size.
+__device__ __forceinline__ int extreme_polygon(const float2* xy, uint32_t n, unsigned long long key, float2* poly)
+{
+    const uint32_t lane = lane_id();
+    const uint32_t i = static_cast<uint32_t>(key);
+    const uint32_t prev = __shfl_up_sync(0xffffffffu, i, 1);
+    const bool take = n > 0u && lane < static_cast<uint32_t>(kDirs) && (lane == 0u || i != prev);
+    const uint32_t mask = __ballot_sync(0xffffffffu, take);
+    if (take)
+        poly[__popc(mask & ((1u << lane) - 1u))] = xy[i];
+    __syncwarp();
+    int np = __popc(mask);
+    if (np > 1 && poly[np - 1].x == poly[0].x && poly[np - 1].y == poly[0].y)
+        --np;
+    return np;
+}
 
 // Large clusters: the two passes over every member (the 16 direction extremes, the first
 // refinement round against the polygon they span) run grid-wide before the hull kernel, in
@@ -1290,9 +1414,8 @@ __global__ void __launch_bounds__(256) k_hull_pre_ref(BatchDev b)
 }
 
 // Cluster g of scan s: z range, hull (local indices into hull_tmp at cl_start), boxes.
-__device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int compute_obb)
+__device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int compute_obb)
 {
-    ScanState* st = &b.state[s];
     const uint32_t n = b.cl_cnt[g];
     const uint32_t start = b.cl_start[g];
     const uint32_t* mem = b.members + start;
@@ -1335,16 +1458,9 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
     }
     if (!pre)
     {
-        unsigned long long ext[kDirs];
-#pragma unroll
-        for (int d = 0; d < kDirs; ++d)
-            ext[d] = warp_max64(ex.key(d));
-        if (lane == 0)
-        {
-#pragma unroll
-            for (int d = 0; d < kDirs; ++d)
-                sm.ext[d][warp] = ext[d];
-        }
+        const unsigned long long key = ex.warp_key();
+        if (lane < static_cast<uint32_t>(kDirs))
+            sm.ext[lane][warp] = key;
     }
     else if (threadIdx.x < kDirs * (kHullThreads / 32))
     {
@@ -1352,28 +1468,19 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
         sm.ext[d][w] = (w == 0) ? b.pre_ext[16ull * g + d] : 0ull;
     }
     __syncthreads();
-    if (threadIdx.x == 0)
+    if (warp == 0)
     {
-        b.cl_zmin[g] = zkey_min(b.cl_zkey[2u * g]);
-        b.cl_zmax[g] = zkey_max(b.cl_zkey[2u * g + 1u]);
-        // initial polygon: extreme members in direction order (counter-clockwise), repeats dropped
-        int np = 0;
-        uint32_t prev = 0xffffffffu;
-        for (int d = 0; d < kDirs; ++d)
+        unsigned long long best = 0ull;
+        if (lane < static_cast<uint32_t>(kDirs))
+            for (int w = 0; w < kHullThreads / 32; ++w)
+                best = sm.ext[lane][w] > best ? sm.ext[lane][w] : best;
+        const int np = extreme_polygon(xy, n, best, sm.poly);
+        if (lane == 0)
         {
-            unsigned long long best = sm.ext[d][0];
-            for (int w = 1; w < kHullThreads / 32; ++w)
-                best = sm.ext[d][w] > best ? sm.ext[d][w] : best;
-            const uint32_t i = static_cast<uint32_t>(best & 0xffffffffull);
-            if (n > 0 && i != prev)
-            {
-                sm.poly[np++] = xy[i];
-                prev = i;
-            }
+            b.cl_zmin[g] = zkey_min(b.cl_zkey[2u * g]);
+            b.cl_zmax[g] = zkey_max(b.cl_zkey[2u * g + 1u]);
+            sm.npoly = np;
         }
-        if (np > 1 && sm.poly[np - 1].x == sm.poly[0].x && sm.poly[np - 1].y == sm.poly[0].y)
-            --np;
-        sm.npoly = np;
     }
     __syncthreads();
 
@@ -1406,15 +1513,14 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
     act[1] = act[0] + n; // two member lists of n entries in the chain-stack scratch (2n + 2)
     int cur = -1;        // -1: the active set is all members
     uint32_t nact = n;
-    for (int round = 0; round < kRefineRounds; ++round)
+    int np = sm.npoly;
+    float2 *poly = sm.poly, *grown = sm.poly2;
+    for (int round = 0; round < kRefineRounds && np >= 3; ++round)
     {
-        const int np = sm.npoly;
-        if (np < 3)
-            break;
         for (int e = threadIdx.x; e < np; e += blockDim.x)
         {
             sm.pkey[e] = 0ull;
-            const float2 a = sm.poly[e], c = sm.poly[(e + 1 == np) ? 0 : e + 1];
+            const float2 a = poly[e], c = poly[(e + 1 == np) ? 0 : e + 1];
             const float ex = c.x - a.x, ey = c.y - a.y;
             const float l1 = fabsf(ex) + fabsf(ey);
             sm.erec[e] = make_float4(a.x, a.y, ex, ey);
@@ -1496,45 +1602,41 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
         }
         __syncthreads();
         cur = nxt;
+        const uint32_t had = nact;
         nact = static_cast<uint32_t>(sm.ncand);
-        if (threadIdx.x == 0)
-        {
-            int add = 0;
-            for (int e = 0; e < np; ++e)
-                add += (sm.pkey[e] != 0ull);
-            sm.grew = 0;
-            if (add > 0 && np + add <= kPolyCap)
-            {
-                int w = 0;
-                for (int e = 0; e < np; ++e)
-                {
-                    sm.poly2[w++] = sm.poly[e];
-                    if (sm.pkey[e] != 0ull)
-                    {
-                        const uint32_t i = static_cast<uint32_t>(sm.pkey[e] & 0xffffffffull);
-                        sm.poly2[w++] = xy[i];
-                    }
-                }
-                for (int e = 0; e < w; ++e)
-                    sm.poly[e] = sm.poly2[e];
-                sm.npoly = w;
-                sm.grew = 1;
-            }
-        }
-        __syncthreads();
-        if (!sm.grew)
+        // each edge's farthest member goes in behind the edge's start, a thread per edge
+        static_assert(kPolyCap <= kHullThreads);
+        const int me = static_cast<int>(threadIdx.x);
+        const unsigned long long far = (me < np) ? sm.pkey[me] : 0ull;
+        uint32_t add;
+        const int at = me + static_cast<int>(block_excl_scan(far != 0ull ? 1u : 0u, sm.scan, &add));
+        const int w = np + static_cast<int>(add);
+        if (add == 0u || w > kPolyCap)
             break;
+        if (me < np)
+        {
+            grown[at] = poly[me];
+            if (far != 0ull)
+                grown[at + 1] = xy[static_cast<uint32_t>(far & 0xffffffffull)];
+        }
+        float2* const was = poly;
+        poly = grown;
+        grown = was;
+        np = w;
+        __syncthreads();
+        if (nact <= kHullEnough || 4u * nact > 3u * had)
+            break; // sorting the rest costs less than another round
     }
 
     // 3. candidates: active members not strictly inside the polygon by a relative margin far
     //    above float rounding (a hull vertex is never strictly inside a polygon of members)
-    const int npf = sm.npoly;
+    const int npf = np;
     auto inside = [&](float px, float py) {
         if (npf < 3)
             return false;
         for (int d = 0; d < npf; ++d)
         {
-            const float2 a = sm.poly[d], c = sm.poly[(d + 1 == npf) ? 0 : d + 1];
+            const float2 a = poly[d], c = poly[(d + 1 == npf) ? 0 : d + 1];
             if (!left_strict_f(a.x, a.y, c.x, c.y, px, py))
                 return false;
         }
@@ -1563,7 +1665,23 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
     // 4. sort by (x, y, input order) and the monotone chain
     const HPt<float>* C;
     int* H;
-    if (small)
+    if (m <= kHullThreads)
+    {
+        // a candidate per thread, its place the number of smaller ones (a total order)
+        const bool mine = static_cast<int>(threadIdx.x) < m;
+        const HPt<float> v = mine ? sm.cand[threadIdx.x] : HPt<float>{INFINITY, INFINITY, 0xffffffffu};
+        uint32_t rank = 0;
+        if (static_cast<int>(warp * 32u) < m)
+#pragma unroll 4
+            for (int k = 0; k < m; ++k)
+                rank += hpt_less(sm.cand[k], v) ? 1u : 0u;
+        __syncthreads();
+        if (mine)
+            sm.cand[rank] = v;
+        C = sm.cand;
+        H = sm.stack;
+    }
+    else if (small)
     {
         const uint32_t np2 = next_pow2(static_cast<uint32_t>(m));
         for (uint32_t i = m + threadIdx.x; i < np2; i += blockDim.x)
@@ -1580,12 +1698,14 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
         H = b.hs_stack + 2ull * start + 2ull * b.cl_rank[g]; // capacity 2n + 2 >= 2m + 2
     }
     __syncthreads();
-    // lower half on thread 0, upper half on thread 32 (another warp) into H + m + 1; then the
+    // lower half on warp 0, upper half on warp 1 into H + m + 1; then the
     // upper half moves down behind the lower one (forwards: the source lies above the target)
-    if (threadIdx.x == 0)
-        sm.nhull = chain_half(C, m, H, false);
-    else if (threadIdx.x == 32)
-        sm.grew = chain_half(C, m, H + m + 1, true);
+    if (warp < 2u)
+    {
+        const int k = chain_half<32>(C, m, H + (warp ? m + 1 : 0), warp == 1u);
+        if (lane == 0)
+            (warp ? sm.grew : sm.nhull) = k;
+    }
     __syncthreads();
     if (threadIdx.x == 0)
     {
@@ -1598,7 +1718,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
     const int h = sm.nhull;
     {
         // a hull vertex with an identical candidate next to it: the reference's pick among them
-        // follows std::sort's order (k_hull_ties replays it)
+        // follows std::sort's order (k_hull_boxes replays it)
         bool tie = false;
         for (int j = threadIdx.x; j < h; j += blockDim.x)
         {
@@ -1611,19 +1731,14 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
             b.tie_list[atomicAdd(&b.queue[5], 1u)] = g;
     }
 
-    // 5 + 6. Local index of each hull vertex (the number of members before it in input order) and
-    //        the boxes. They only read the hull: warps 0 and 1 compute the calipers and PCA boxes
-    //        while the other warps count (all warps count when no boxes are asked for).
+    // 5. The vertices' coordinates for k_hull_boxes and their local indices: the number of
+    //    members before each in input order.
     const bool fast = h <= kHullSmem;
-    double2* P = fast ? sm.hp : (b.hs_pts + start);
-    if (compute_obb)
-        for (int j = threadIdx.x; j < h; j += blockDim.x)
-        {
-            const HPt<float> c = C[H[j]];
-            P[j] = make_double2(static_cast<double>(c.x), static_cast<double>(c.y));
-            if (fast)
-                sm.pf[j] = make_float2(c.x, c.y);
-        }
+    for (int j = threadIdx.x; j < h; j += blockDim.x)
+    {
+        const HPt<float> c = C[H[j]];
+        b.hs_pts[start + j] = make_double2(static_cast<double>(c.x), static_cast<double>(c.y));
+    }
     const uint32_t np2 = next_pow2(static_cast<uint32_t>(h));
     if (fast)
     {
@@ -1637,73 +1752,55 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
     __syncthreads();
     if (fast)
         block_bitonic_sort(sm.hkey, np2, [](uint32_t a, uint32_t c) { return a < c; });
-    const uint32_t ix0 = compute_obb ? 64u : 0u; // first counting thread
-    const uint32_t ncount = blockDim.x - ix0;
-    if (compute_obb && warp < 2)
-    {
-        // the refinement's edge records are free: float scratch of the calipers screen
-        if (warp == 0)
-            calipers_box(st, P, fast ? sm.pf : nullptr, reinterpret_cast<float*>(sm.erec), h,
-                         b.hs_pairs + 4ull * start + 16ull * b.cl_rank[g], &b.obb_c[g]);
-        else
-            pca_box_warp(P, h, &b.obb_p[g]);
-    }
-    else if (fast)
+    if (fast)
     {
         // member o adds 1 to every hull vertex with a larger key: diff[upper_bound(o)] += 1. Each
         // thread walks a contiguous chunk of the member list as aligned quadruples (slot v:
         // members 4v - a .. 4v - a + 3, a = start mod 4; entries outside [0, n) skipped, the loads
-        // stay inside the allocation). Members come in ascending index runs, so consecutive
-        // members mostly fall into the same bin: a member inside the current bin's key interval
-        // skips the search, and a bin's count is added once when the bin changes.
+        // stay inside the allocation), four at a time: a search is a chain of shared-memory loads, sixteen of
+        // them overlap (one after the other, 37,990 members took 45,000 cycles). Members come in ascending index
+        // runs, so consecutive ones mostly fall into the same bin: a bin's count is added when the bin changes.
         const uint32_t a4 = start & 3u;
         const uint4* mv = reinterpret_cast<const uint4*>(b.members + (start - a4));
         const uint32_t nq = (n + a4 + 3u) / 4u;
-        const uint32_t per = (nq + ncount - 1u) / ncount;
-        const uint32_t q0 = (threadIdx.x - ix0) * per, q1 = min(nq, q0 + per);
-        int cb = h, cc = 0;               // current bin and its pending count
-        uint32_t blo = 1u, bhi = 0u;      // its key interval [blo, bhi) (empty: no bin yet)
-        auto member = [&](uint32_t o) {
-            if (o >= blo && o < bhi)
-            {
-                ++cc;
-                return;
-            }
-            int l = 0, hi = h;
-            while (l < hi)
-            {
-                const int mid = (l + hi) >> 1;
-                if (sm.hkey[mid] > o)
-                    hi = mid;
-                else
-                    l = mid + 1;
-            }
-            if (l != cb)
-            {
-                if (cc > 0 && cb < h)
-                    atomicAdd(&sm.diff[cb], cc);
-                cb = l;
-                cc = 0;
-            }
-            ++cc;
-            blo = (l > 0) ? sm.hkey[l - 1] : 0u;
-            bhi = (l < h) ? sm.hkey[l] : 0xffffffffu;
-        };
-        for (uint32_t v0 = q0; v0 < q1; v0 += 4u)
+        const uint32_t per = (nq + kHullThreads - 1u) / kHullThreads;
+        const uint32_t q0 = threadIdx.x * per, q1 = min(nq, q0 + per);
+        int cb = h, cc = 0; // current bin and its pending count
+        for (uint32_t v = q0; v < q1; v += 4u)
         {
-            uint4 q[4];
+            uint32_t o[16], l[16];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                q[u] = (v0 + u < q1) ? mv[v0 + u] : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (uint32_t u = 0; u < 4; ++u)
             {
-                const int32_t i = 4 * static_cast<int32_t>(v0 + u) - static_cast<int32_t>(a4);
-                const uint32_t oo[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
+                const uint4 q = (v + u < q1) ? mv[v + u] : make_uint4(0u, 0u, 0u, 0u);
+                o[4 * u] = q.x;
+                o[4 * u + 1] = q.y;
+                o[4 * u + 2] = q.z;
+                o[4 * u + 3] = q.w;
+            }
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (v0 + u < q1 && i + c >= 0 && i + c < static_cast<int32_t>(n))
-                        member(oo[c]);
+            for (int c = 0; c < 16; ++c)
+                l[c] = 0u;
+#pragma unroll 1
+            for (uint32_t step = np2 >> 1; step > 0u; step >>= 1)
+#pragma unroll
+                for (int c = 0; c < 16; ++c)
+                    l[c] += (sm.hkey[l[c] + step - 1u] <= o[c]) ? step : 0u;
+            const uint32_t i = 4u * v - a4; // (wraps below the first member: not less than n)
+            const uint32_t end = min(n, 4u * q1 - a4);
+#pragma unroll
+            for (int c = 0; c < 16; ++c)
+            {
+                const int bin = static_cast<int>(l[c] + ((sm.hkey[l[c]] <= o[c]) ? 1u : 0u));
+                const bool in = i + c < end;
+                if (in && bin != cb)
+                {
+                    if (cc > 0 && cb < h)
+                        atomicAdd(&sm.diff[cb], cc);
+                    cb = bin;
+                    cc = 0;
+                }
+                cc += in ? 1 : 0;
             }
         }
         if (cc > 0 && cb < h)
@@ -1711,7 +1808,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int s, int
     }
     else
     {
-        for (int j = static_cast<int>(warp - ix0 / 32u); j < h; j += static_cast<int>(ncount / 32u))
+        for (int j = static_cast<int>(warp); j < h; j += kHullThreads / 32)
         {
             const uint32_t key = C[H[j]].key;
             uint32_t cnt = 0;
@@ -1767,17 +1864,7 @@ constexpr int kWarpCand = 256;
 constexpr uint32_t kWarpRefineMin = 48; // more candidates than this: refine the polygon first
 constexpr int kWarpPoly = 64;           // refined polygon capacity of the warp path
 
-struct WarpSmem
-{
-    HPt<float> cand[kWarpCand];
-    int stack[2 * kWarpCand + 2];
-    double2 hp[kWarpCand];
-    float2 pf[kWarpCand];
-    float2 poly[kDirs];
-    int npoly;
-};
-
-// Scratch of the warp path's polygon refinement (inside WarpSmem::hp, unused until the boxes).
+// Scratch of the warp path's polygon refinement.
 struct WarpRefine
 {
     float2 rp[kWarpPoly], rp2[kWarpPoly];
@@ -1785,7 +1872,14 @@ struct WarpRefine
     float2 emar[kWarpPoly];
     unsigned long long pkey[kWarpPoly];
 };
-static_assert(sizeof(WarpRefine) <= sizeof(double2) * kWarpCand, "refinement scratch exceeds the box scratch");
+
+struct WarpSmem
+{
+    WarpRefine refine;
+    HPt<float> cand[kWarpCand];
+    int stack[2 * kWarpCand + 2];
+    float2 poly[kDirs];
+};
 
 // Quickhull rounds over the candidates C[0..m) (at most 16 per lane), starting from the warp's
 // 16-direction polygon: each round tests every candidate against the polygon's edges (keeping
@@ -1793,7 +1887,7 @@ static_assert(sizeof(WarpRefine) <= sizeof(double2) * kWarpCand, "refinement scr
 // inserts the farthest ones. Returns the number of candidates left in C.
 __device__ uint32_t warp_refine(WarpSmem& ws, HPt<float>* C, uint32_t m, int np)
 {
-    WarpRefine& wr = *reinterpret_cast<WarpRefine*>(ws.hp);
+    WarpRefine& wr = ws.refine;
     const uint32_t lane = lane_id();
     for (int e = static_cast<int>(lane); e < np; e += 32)
         wr.rp[e] = ws.poly[e];
@@ -1839,34 +1933,33 @@ __device__ uint32_t warp_refine(WarpSmem& ws, HPt<float>* C, uint32_t m, int np)
             inbits |= (in ? 1u : 0u) << q;
         }
         __syncwarp();
-        // lane 0 inserts each edge's farthest outside candidate (positions before compaction)
-        int grew = 0, nnew = np;
-        if (lane == 0)
+        // each edge's farthest outside candidate goes in behind the edge's start (positions before compaction)
+        static_assert(kWarpPoly == 64);
+        const int e0 = static_cast<int>(lane), e1 = e0 + 32;
+        const unsigned long long f0 = (e0 < np) ? wr.pkey[e0] : 0ull, f1 = (e1 < np) ? wr.pkey[e1] : 0ull;
+        const uint32_t m0 = __ballot_sync(0xffffffffu, f0 != 0ull), m1 = __ballot_sync(0xffffffffu, f1 != 0ull);
+        const int add = __popc(m0) + __popc(m1);
+        const bool grew = add > 0 && np + add <= kWarpPoly;
+        if (grew)
         {
-            int add = 0;
-            for (int e = 0; e < np; ++e)
-                add += (wr.pkey[e] != 0ull);
-            if (add > 0 && np + add <= kWarpPoly)
-            {
-                int w = 0;
-                for (int e = 0; e < np; ++e)
+            auto put = [&](int e, unsigned long long f, int before) {
+                if (e >= np)
+                    return;
+                wr.rp2[e + before] = wr.rp[e];
+                if (f != 0ull)
                 {
-                    wr.rp2[w++] = wr.rp[e];
-                    if (wr.pkey[e] != 0ull)
-                    {
-                        const HPt<float> c = C[static_cast<uint32_t>(wr.pkey[e] & 0xffffffffull)];
-                        wr.rp2[w++] = make_float2(c.x, c.y);
-                    }
+                    const HPt<float> c = C[static_cast<uint32_t>(f & 0xffffffffull)];
+                    wr.rp2[e + before + 1] = make_float2(c.x, c.y);
                 }
-                for (int e = 0; e < w; ++e)
-                    wr.rp[e] = wr.rp2[e];
-                nnew = w;
-                grew = 1;
-            }
+            };
+            put(e0, f0, __popc(m0 & ((1u << lane) - 1u)));
+            put(e1, f1, __popc(m0) + __popc(m1 & ((1u << lane) - 1u)));
+            __syncwarp();
+            np += add;
+            for (int e = e0; e < np; e += 32)
+                wr.rp[e] = wr.rp2[e];
         }
         __syncwarp();
-        grew = __shfl_sync(0xffffffffu, grew, 0);
-        np = __shfl_sync(0xffffffffu, nnew, 0);
         // compact in place (every chunk is read before any of its positions is written)
         uint32_t wpos = 0;
         for (uint32_t base = 0, q = 0; base < m; base += 32, ++q)
@@ -1890,9 +1983,8 @@ __device__ uint32_t warp_refine(WarpSmem& ws, HPt<float>* C, uint32_t m, int np)
     return m;
 }
 
-__device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dirs, uint32_t g, int s, int compute_obb)
+__device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dirs, uint32_t g, int compute_obb)
 {
-    ScanState* st = &b.state[s];
     const uint32_t n = b.cl_cnt[g];
     const uint32_t start = b.cl_start[g];
     const uint32_t* mem = b.members + start;
@@ -1900,35 +1992,23 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
     const float2* xy = b.mxy + start;
     Extremes16 ex;
     ex.init();
-    for (uint32_t i = lane; i < n; i += 32)
+    for (uint32_t i0 = lane; i0 < n; i0 += 128u)
     {
-        const float2 p = xy[i];
-        ex.add(dirs, p.x, p.y, i);
-    }
-    unsigned long long ext[kDirs];
+        float2 p[4];
 #pragma unroll
-    for (int d = 0; d < kDirs; ++d)
-        ext[d] = warp_max64(ex.key(d));
+        for (uint32_t u = 0; u < 4; ++u)
+            p[u] = (i0 + 32u * u < n) ? xy[i0 + 32u * u] : make_float2(NAN, NAN); // (never an extreme)
+#pragma unroll 1
+        for (uint32_t u = 0; u < 4 && i0 + 32u * u < n; ++u)
+            ex.add(dirs, u < 2 ? (u == 0 ? p[0].x : p[1].x) : (u == 2 ? p[2].x : p[3].x),
+                   u < 2 ? (u == 0 ? p[0].y : p[1].y) : (u == 2 ? p[2].y : p[3].y), i0 + 32u * u);
+    }
+    const int npf = extreme_polygon(xy, n, ex.warp_key(), ws.poly);
     if (lane == 0)
     {
         b.cl_zmin[g] = zkey_min(b.cl_zkey[2u * g]);
         b.cl_zmax[g] = zkey_max(b.cl_zkey[2u * g + 1u]);
-        int np = 0;
-        uint32_t prev = 0xffffffffu;
-        for (int d = 0; d < kDirs; ++d)
-        {
-            const uint32_t i = static_cast<uint32_t>(ext[d] & 0xffffffffull);
-            if (n > 0 && i != prev)
-            {
-                ws.poly[np++] = xy[i];
-                prev = i;
-            }
-        }
-        if (np > 1 && ws.poly[np - 1].x == ws.poly[0].x && ws.poly[np - 1].y == ws.poly[0].y)
-            --np;
-        ws.npoly = np;
     }
-    __syncwarp();
     int32_t* hull_dst = b.hull_tmp + start;
     if (n < 3)
     {
@@ -1948,20 +2028,30 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
         __syncwarp();
         return;
     }
-    const int npf = ws.npoly;
-    auto inside = [&](float px, float py) {
-        if (npf < 3)
-            return false;
+    // the polygon's edges (start, direction; |direction|_1), in the refinement's scratch
+    if (lane < static_cast<uint32_t>(npf))
+    {
+        const float2 a = ws.poly[lane], c = ws.poly[(static_cast<int>(lane) + 1 == npf) ? 0 : lane + 1];
+        ws.refine.erec[lane] = make_float4(a.x, a.y, c.x - a.x, c.y - a.y);
+        ws.refine.emar[lane].x = fabsf(c.x - a.x) + fabsf(c.y - a.y);
+    }
+    __syncwarp();
+    auto inside = [&](float px, float py) { // left_strict_f of every edge
+        bool in = npf >= 3;
+#pragma unroll 4
         for (int d = 0; d < npf; ++d)
         {
-            const float2 a = ws.poly[d], c = ws.poly[(d + 1 == npf) ? 0 : d + 1];
-            if (!left_strict_f(a.x, a.y, c.x, c.y, px, py))
-                return false;
+            const float4 r = ws.refine.erec[d];
+            const float qx = px - r.x, qy = py - r.y;
+            const float cr = r.z * qy - r.w * qx;
+            const float scale = ws.refine.emar[d].x * (fabsf(qx) + fabsf(qy));
+            in = in && cr > 1e-5f * scale + 1e-30f;
         }
-        return true;
+        return in;
     };
     HPt<float>* gs = reinterpret_cast<HPt<float>*>(b.hs_cand) + 2ull * start; // capacity 2n >= next_pow2(n)
     uint32_t m = 0;
+#pragma unroll 1
     for (uint32_t base = 0; base < n; base += 32)
     {
         const uint32_t i = base + lane;
@@ -1987,7 +2077,7 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
     __syncwarp();
     // Many candidates (members spread along the boundary, e.g. an arc): refine the polygon as the
     // CTA path does (insert the candidate farthest outside each edge, drop the candidates proven
-    // strictly inside by the 1e-5 relative margin), a few rounds, in the box scratch (ws.hp).
+    // strictly inside by the 1e-5 relative margin), a few rounds.
     HPt<float>* C0 = (m <= static_cast<uint32_t>(kWarpCand)) ? ws.cand : gs;
     if (m > kWarpRefineMin && npf >= 3)
         m = warp_refine(ws, C0, m, npf);
@@ -2000,28 +2090,31 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
     }
     HPt<float>* C = small ? ws.cand : gs;
     int* H = small ? ws.stack : (b.hs_stack + 2ull * start + 2ull * b.cl_rank[g]);
-    if (m <= 32u)
+    if (small)
     {
-        // one candidate per lane, sorted in registers (hpt_less is a total order: any sort agrees)
-        HPt<float> v = (lane < m) ? C[lane] : HPt<float>{INFINITY, INFINITY, 0xffffffffu};
-#pragma unroll
-        for (uint32_t k = 2; k <= 32; k <<= 1)
+        // two candidates per lane, the place of each the number of smaller ones (hpt_less is a total order), into
+        // the refinement's scratch: 120 candidates take a tenth of the exchange sort's 50,000 cycles
+        static_assert(sizeof(WarpRefine) >= sizeof(HPt<float>) * kWarpCand);
+        HPt<float>* D = reinterpret_cast<HPt<float>*>(&ws.refine);
+        const HPt<float> last{INFINITY, INFINITY, 0xffffffffu};
+        for (uint32_t base = lane; base < m + lane; base += 64u)
         {
-#pragma unroll
-            for (uint32_t j = k >> 1; j > 0; j >>= 1)
+            const HPt<float> v0 = (base < m) ? ws.cand[base] : last, v1 = (base + 32u < m) ? ws.cand[base + 32u] : last;
+            uint32_t r0 = 0, r1 = 0;
+#pragma unroll 2
+            for (uint32_t k = 0; k < m; ++k)
             {
-                HPt<float> o;
-                o.x = __shfl_xor_sync(0xffffffffu, v.x, j);
-                o.y = __shfl_xor_sync(0xffffffffu, v.y, j);
-                o.key = __shfl_xor_sync(0xffffffffu, v.key, j);
-                const bool up = ((lane & k) == 0), lower = ((lane & j) == 0);
-                if ((lower == up) ? hpt_less(o, v) : hpt_less(v, o))
-                    v = o;
+                const HPt<float> c = ws.cand[k];
+                r0 += hpt_less(c, v0) ? 1u : 0u;
+                r1 += hpt_less(c, v1) ? 1u : 0u;
             }
+            if (base < m)
+                D[r0] = v0;
+            if (base + 32u < m)
+                D[r1] = v1;
         }
         __syncwarp();
-        if (lane < m)
-            C[lane] = v;
+        C = D;
     }
     else
     {
@@ -2031,11 +2124,21 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
         __syncwarp();
         warp_bitonic_smem(C, np2, [](const HPt<float>& x, const HPt<float>& y) { return hpt_less(x, y); });
     }
-    int h = 0;
-    if (lane == 0)
-        h = monotone_chain(C, static_cast<int>(m), H);
-    h = __shfl_sync(0xffffffffu, h, 0);
+    // lanes 0 to 15 walk the lower half, the others the upper one into H + m + 1, which then moves down behind
+    // the lower half (chunk by chunk, forwards: the source lies above the target)
+    const int kh = chain_half<16>(C, static_cast<int>(m), H + (lane >= 16u ? m + 1u : 0u), lane >= 16u);
+    const int kl = __shfl_sync(0xffffffffu, kh, 0), ku = __shfl_sync(0xffffffffu, kh, 16);
     __syncwarp();
+    for (int j0 = 1; j0 < ku - 1; j0 += 32)
+    {
+        const int j = j0 + static_cast<int>(lane);
+        const int v = (j < ku - 1) ? H[static_cast<int>(m) + 1 + j] : 0;
+        __syncwarp();
+        if (j < ku - 1)
+            H[kl - 1 + j] = v;
+        __syncwarp();
+    }
+    const int h = kl + ku - 2; // (m >= 1: the extreme members stay)
     {
         bool tie = false;
         for (int j = static_cast<int>(lane); j < h; j += 32)
@@ -2048,37 +2151,35 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
         if (__any_sync(0xffffffffu, tie) && lane == 0)
             b.tie_list[atomicAdd(&b.queue[5], 1u)] = g;
     }
-    for (int j = 0; j < h; ++j)
+    // the members once in registers (n <= kBigCluster), then counted for every vertex
+    uint32_t mk[kBigCluster / 32u];
+#pragma unroll
+    for (uint32_t q = 0; q < kBigCluster / 32u; ++q)
+        mk[q] = (32u * q + lane < n) ? mem[32u * q + lane] : 0xffffffffu; // (never below a key)
+    for (int j0 = 0; j0 < h; j0 += 32)
     {
-        const uint32_t key = C[H[j]].key;
-        uint32_t cnt = 0;
-        for (uint32_t base = 0; base < n; base += 32)
+        const int j = j0 + static_cast<int>(lane);
+        const HPt<float> c = (j < h) ? C[H[j]] : HPt<float>{0.0f, 0.0f, 0u};
+        uint32_t before = 0;
+        for (int u = 0; u < min(32, h - j0); ++u)
         {
-            const uint32_t i = base + lane;
-            cnt += __popc(__ballot_sync(0xffffffffu, (i < n) && (mem[i] < key)));
+            const uint32_t key = __shfl_sync(0xffffffffu, c.key, u);
+            uint32_t cnt = 0;
+#pragma unroll
+            for (uint32_t q = 0; q < kBigCluster / 32u; ++q)
+                cnt += (mk[q] < key) ? 1u : 0u;
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
+            if (static_cast<int>(lane) == u)
+                before = cnt;
         }
-        if (lane == 0)
-            hull_dst[j] = static_cast<int32_t>(cnt);
+        if (j < h)
+        {
+            hull_dst[j] = static_cast<int32_t>(before);
+            b.hs_pts[start + j] = make_double2(static_cast<double>(c.x), static_cast<double>(c.y));
+        }
     }
     if (lane == 0)
         b.hull_cnt[g] = static_cast<uint32_t>(h);
-    if (compute_obb)
-    {
-        const bool fast = h <= kWarpCand;
-        double2* P = fast ? ws.hp : (b.hs_pts + start);
-        for (int j = static_cast<int>(lane); j < h; j += 32)
-        {
-            const HPt<float> c = C[H[j]];
-            P[j] = make_double2(static_cast<double>(c.x), static_cast<double>(c.y));
-            if (fast)
-                ws.pf[j] = make_float2(c.x, c.y);
-        }
-        __syncwarp();
-        // the chain stack is free again: float scratch of the calipers screen
-        calipers_box(st, P, fast ? ws.pf : nullptr, reinterpret_cast<float*>(ws.stack), h,
-                     b.hs_pairs + 4ull * start + 16ull * b.cl_rank[g], &b.obb_c[g]);
-        pca_box_warp(P, h, &b.obb_p[g]);
-    }
     __syncwarp();
 }
 
@@ -2153,8 +2254,7 @@ __global__ void __launch_bounds__(kHullThreads) k_hull(BatchDev b, int compute_o
         if (w >= nbig)
             break;
         const uint32_t g = work[w];
-        const int s = scan_of_cluster(b, g);
-        hull_one(b, sm, g, s, compute_obb);
+        hull_one(b, sm, g, compute_obb);
     }
     __syncthreads(); // the CTA's shared memory now becomes eight per-warp regions
     WarpSmem& ws = reinterpret_cast<WarpSmem*>(smraw)[threadIdx.x >> 5];
@@ -2167,8 +2267,7 @@ __global__ void __launch_bounds__(kHullThreads) k_hull(BatchDev b, int compute_o
         if (w >= nsmall)
             break;
         const uint32_t g = work[b.ncl - 1u - w];
-        const int s = scan_of_cluster(b, g);
-        hull_one_warp(b, ws, dirs, g, s, compute_obb);
+        hull_one_warp(b, ws, dirs, g, compute_obb);
     }
 }
 
@@ -2289,39 +2388,110 @@ __device__ void hull_repair_ties(HRec<T>* rec, uint32_t n, int32_t* hull, int h,
 constexpr uint32_t kTieSmemRecs = 4096;
 constexpr size_t kTieDynSmem = static_cast<size_t>(kTieSmemRecs) * (sizeof(HRec<float>) + 8);
 
-__global__ void __launch_bounds__(kHullThreads) k_hull_ties(BatchDev b)
+// Cluster g's tie repair, by one CTA with kTieDynSmem bytes of shared memory.
+__device__ __noinline__ void repair_cluster(const BatchDev& b, uint32_t g, unsigned char* tsm, isort::SortShared& ss)
+{
+    const uint32_t start = b.cl_start[g], n = b.cl_cnt[g];
+    const int h = static_cast<int>(b.hull_cnt[g]);
+    const bool local = n <= kTieSmemRecs;
+    HRec<float>* rec = local ? reinterpret_cast<HRec<float>*>(tsm)
+                             : reinterpret_cast<HRec<float>*>(reinterpret_cast<HPt<float>*>(b.hs_cand) + 2ull * start);
+    uint32_t* ge = local ? reinterpret_cast<uint32_t*>(tsm + kTieSmemRecs * sizeof(HRec<float>))
+                         : reinterpret_cast<uint32_t*>(b.hs_stack + 2ull * start + 2ull * b.cl_rank[g]);
+    uint32_t* le = ge + (local ? kTieSmemRecs : n);
+    for (uint32_t k = threadIdx.x; k < n; k += blockDim.x)
+    {
+        const float2 p = b.mxy[start + k];
+        rec[k] = HRec<float>{p.x, p.y, b.members[start + k]};
+    }
+    __syncthreads();
+    isort::cta_sort(rec, n, IdxLess<float>{}, ge, le, ss);
+    for (uint32_t k = threadIdx.x; k < n; k += blockDim.x)
+        rec[k].idx = k; // local index: position in input order
+    __syncthreads();
+    const double2* hv = b.hs_pts + start; // the vertices' coordinates, from k_hull
+    hull_repair_ties(rec, n, b.hull_tmp + start, h, [=](int j) { return hv[j]; }, ge, le, ss);
+    __syncthreads();
+}
+
+// A cluster's hull vertices while its boxes are computed, N at most.
+template <int N>
+struct BoxSmem
+{
+    double2 hp[N];
+    float2 pf[N];
+    float ea[N];
+};
+constexpr int kBoxWarpVerts = 256; // more: the warps of a CTA share one region, up to kHullSmem
+static_assert(sizeof(BoxSmem<kBoxWarpVerts>) * (kHullThreads / 32) <= kTieDynSmem && sizeof(BoxSmem<kHullSmem>) <= kTieDynSmem);
+
+// The tie repairs (rare), then both boxes of every cluster, a warp for each box. The boxes' FP64 chains
+// (the SM retires an FP64 instruction of a warp every 16 cycles) take longer than finding the hull: one after the other
+// behind the hull, they were more than half of the 62 us that a small scan's longest cluster took; here the two boxes run
+// on different SMs where the scan is small, and the hull kernel's code fits the instruction cache better without them.
+// Item i of 2 K (K clusters, the large ones first; calipers, then PCA) goes to CTA i mod grid, so that a small
+// scan's boxes share no SM's FP64 unit. A tie repair moves no coordinate: the boxes need not wait for it.
+__global__ void __launch_bounds__(kHullThreads) k_hull_boxes(BatchDev b, int compute_obb, const uint32_t* work)
 {
     pdl_enter();
     __shared__ isort::SortShared ss;
     extern __shared__ __align__(16) unsigned char tsm[];
     const uint32_t ntie = b.queue[5]; // the tie count (queue[4] is the small-cluster head)
     for (uint32_t t = blockIdx.x; t < ntie; t += gridDim.x)
+        repair_cluster(b, b.tie_list[t], tsm, ss);
+    if (!compute_obb)
+        return;
+    const uint32_t nbig = b.queue[2], nsmall = b.queue[3];
+    const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
+    // hulls of more vertices than a warp's region holds (their clusters are large): one per CTA, one box a warp
+    for (uint32_t w = blockIdx.x; w < nbig; w += gridDim.x)
     {
-        const uint32_t g = b.tie_list[t];
-        const uint32_t start = b.cl_start[g], n = b.cl_cnt[g];
+        const uint32_t g = work[w];
         const int h = static_cast<int>(b.hull_cnt[g]);
-        const bool local = n <= kTieSmemRecs;
-        HRec<float>* rec = local ? reinterpret_cast<HRec<float>*>(tsm)
-                                 : reinterpret_cast<HRec<float>*>(reinterpret_cast<HPt<float>*>(b.hs_cand) + 2ull * start);
-        uint32_t* ge = local ? reinterpret_cast<uint32_t*>(tsm + kTieSmemRecs * sizeof(HRec<float>))
-                             : reinterpret_cast<uint32_t*>(b.hs_stack + 2ull * start + 2ull * b.cl_rank[g]);
-        uint32_t* le = ge + (local ? kTieSmemRecs : n);
-        for (uint32_t k = threadIdx.x; k < n; k += blockDim.x)
+        if (h <= kBoxWarpVerts)
+            continue;
+        const uint32_t start = b.cl_start[g];
+        BoxSmem<kHullSmem>& bs = *reinterpret_cast<BoxSmem<kHullSmem>*>(tsm);
+        const bool fast = h <= kHullSmem;
+        if (fast)
+            for (int j = threadIdx.x; j < h; j += kHullThreads)
+            {
+                const double2 p = b.hs_pts[start + j];
+                bs.hp[j] = p;
+                bs.pf[j] = make_float2(static_cast<float>(p.x), static_cast<float>(p.y)); // (float vertices: exact)
+            }
+        __syncthreads();
+        const double2* P = fast ? bs.hp : (b.hs_pts + start);
+        if (warp == 0)
+            calipers_box(&b.state[scan_of_cluster(b, g)], P, fast ? bs.pf : nullptr, bs.ea, h,
+                         b.hs_pairs + 4ull * start + 16ull * b.cl_rank[g], &b.obb_c[g]);
+        else if (warp == 1)
+            pca_box_warp(P, h, &b.obb_p[g]);
+        __syncthreads();
+    }
+    BoxSmem<kBoxWarpVerts>& bs = reinterpret_cast<BoxSmem<kBoxWarpVerts>*>(tsm)[warp];
+    const uint32_t K = nbig + nsmall;
+    for (uint32_t i = blockIdx.x + gridDim.x * warp; i < 2u * K; i += gridDim.x * (kHullThreads / 32))
+    {
+        const uint32_t w = i < K ? i : i - K;
+        const uint32_t g = w < nbig ? work[w] : work[b.ncl - 1u - (w - nbig)];
+        const int h = static_cast<int>(b.hull_cnt[g]);
+        if (h > kBoxWarpVerts || b.cl_cnt[g] < 3u) // (fewer than three members: zero, written with the hull)
+            continue;
+        const uint32_t start = b.cl_start[g];
+        for (int j = static_cast<int>(lane); j < h; j += 32)
         {
-            const float2 p = b.mxy[start + k];
-            rec[k] = HRec<float>{p.x, p.y, b.members[start + k]};
+            const double2 p = b.hs_pts[start + j];
+            bs.hp[j] = p;
+            bs.pf[j] = make_float2(static_cast<float>(p.x), static_cast<float>(p.y));
         }
-        __syncthreads();
-        isort::cta_sort(rec, n, IdxLess<float>{}, ge, le, ss);
-        for (uint32_t k = threadIdx.x; k < n; k += blockDim.x)
-            rec[k].idx = k; // local index: position in input order
-        __syncthreads();
-        int32_t* hull = b.hull_tmp + start;
-        double2* hv = b.hs_pts + start; // the vertices' coordinates, kept before the records re-sort
-        for (int j = threadIdx.x; j < h; j += blockDim.x)
-            hv[j] = make_double2(static_cast<double>(rec[hull[j]].x), static_cast<double>(rec[hull[j]].y));
-        __syncthreads();
-        hull_repair_ties(rec, n, hull, h, [=](int j) { return hv[j]; }, ge, le, ss);
+        __syncwarp();
+        if (i < K)
+            calipers_box(&b.state[scan_of_cluster(b, g)], bs.hp, bs.pf, bs.ea, h,
+                         b.hs_pairs + 4ull * start + 16ull * b.cl_rank[g], &b.obb_c[g]);
+        else
+            pca_box_warp(bs.hp, h, &b.obb_p[g]);
+        __syncwarp();
     }
 }
 
@@ -2568,10 +2738,13 @@ __device__ int single_chain(SingleSmem& sm, const double2* pts, const uint32_t* 
         }
         __syncthreads();
         block_bitonic_sort(C, np2, [](const HPt<T>& x, const HPt<T>& y) { return hpt_less(x, y); });
-        if (threadIdx.x == 0)
-            sm.npoly = chain_half(C, static_cast<int>(m), H, false);
-        else if (threadIdx.x == 32)
-            sm.grew = chain_half(C, static_cast<int>(m), H + m + 1, true);
+        if (threadIdx.x < 64u)
+        {
+            const bool upper = threadIdx.x >= 32u;
+            const int k = chain_half<32>(C, static_cast<int>(m), H + (upper ? m + 1 : 0), upper);
+            if (lane_id() == 0)
+                (upper ? sm.grew : sm.npoly) = k;
+        }
         __syncthreads();
         const int kl = sm.npoly, h = kl + sm.grew - 2;
         bool t = false;
@@ -2814,7 +2987,8 @@ void launch_polygons(Launcher& L, const BatchDev& b, const BatchHost& hb, int co
     const int sms = sm_count();
     LP_LAUNCH_SMEM(L, k_hull, static_cast<uint32_t>(sms) * hb.hull_ctas_per_sm, kHullThreads, kHullDynSmem, b, compute_obb,
                    static_cast<const uint32_t*>(b.hull_work));
-    LP_LAUNCH_SMEM(L, k_hull_ties, static_cast<uint32_t>(sms), kHullThreads, kTieDynSmem, b);
+    LP_LAUNCH_SMEM(L, k_hull_boxes, static_cast<uint32_t>(sms) * (compute_obb ? 2u : 1u), kHullThreads, kTieDynSmem, b, compute_obb,
+                   static_cast<const uint32_t*>(b.hull_work));
     LP_LAUNCH(L, k_hull_finish, static_cast<uint32_t>(b.nscan), kFinishThreads, b);
 }
 
@@ -2822,7 +2996,7 @@ void init_kernel_attributes()
 {
     init_kdtree_attributes();
     cudaFuncSetAttribute(k_hull, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kHullDynSmem));
-    cudaFuncSetAttribute(k_hull_ties, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTieDynSmem));
+    cudaFuncSetAttribute(k_hull_boxes, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTieDynSmem));
 }
 
 int sm_count()

@@ -171,10 +171,10 @@ __device__ __forceinline__ void io_out_clusters(const BatchDev& b, const IoScan*
     const uint32_t kcl = b.state[s].n_clusters;
     const uint32_t* off = b.hull_cnt + sd.cl_off;
     const uint32_t base = off[0];
-    const uint32_t nh = kcl <= sd.cluster_cap ? off[kcl] - base : 0u;
+    const uint32_t nh = kcl < sd.cluster_cap ? off[kcl] - base : 0u;
     if (part == 0 && threadIdx.x == 0)
         ret[s] = nh;
-    if (kcl > min(sd.cluster_cap, d.cluster_cap) || nh > d.hull_cap)
+    if (kcl >= sd.cluster_cap || kcl > d.cluster_cap || nh > d.hull_cap)
         return;
     if (d.hoff)
         for (uint32_t k = part * kIoThreads + threadIdx.x; k <= kcl; k += kIoClusterCtas * kIoThreads)
