@@ -1137,7 +1137,8 @@ __device__ void block_sort_global(HPt<T>* a, uint32_t n)
 constexpr int kDirs = 16;         // extreme-point directions of the initial polygon
 constexpr int kPolyCap = 256;     // refined polygon capacity
 constexpr int kRefineRounds = 12; // farthest-point insertion rounds
-constexpr uint32_t kHullEnough = 48; // active members few enough to end them
+constexpr int kCountLater = 128;   // hulls of at most this many vertices have a large cluster's members counted later
+constexpr uint32_t kHullEnough = 96; // active members few enough to end them (a round costs about 30 candidates' sort and chain)
 constexpr uint32_t kBigCluster = 512; // larger clusters take a whole CTA; smaller ones one warp
 
 struct HullSmem
@@ -1716,6 +1717,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int comput
     }
     __syncthreads();
     const int h = sm.nhull;
+    bool tied;
     {
         // a hull vertex with an identical candidate next to it: the reference's pick among them
         // follows std::sort's order (k_hull_boxes replays it)
@@ -1727,7 +1729,8 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int comput
             tie |= (q > 0 && C[q - 1].x == c.x && C[q - 1].y == c.y) ||
                    (q + 1 < static_cast<int>(m) && C[q + 1].x == c.x && C[q + 1].y == c.y);
         }
-        if (__syncthreads_or(tie) && threadIdx.x == 0)
+        tied = __syncthreads_or(tie);
+        if (tied && threadIdx.x == 0)
             b.tie_list[atomicAdd(&b.queue[5], 1u)] = g;
     }
 
@@ -1739,21 +1742,62 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int comput
         const HPt<float> c = C[H[j]];
         b.hs_pts[start + j] = make_double2(static_cast<double>(c.x), static_cast<double>(c.y));
     }
+    if (pre && small && h <= kCountLater)
+    {
+        // a cluster of the grid-wide passes: its members are counted grid-wide too (k_hull_boxes, one item per
+        // kPreChunk members); not where a tie repair needs the indices first
+        if (threadIdx.x == 0)
+            b.pre_nact[g] = tied ? 0u : static_cast<uint32_t>(h);
+        if (!tied)
+        {
+            int* keys = b.hs_stack + 2ull * start + 2ull * b.cl_rank[g];
+            for (int j = threadIdx.x; j < h; j += blockDim.x)
+            {
+                keys[j] = static_cast<int>(C[H[j]].key);
+                hull_dst[j] = 0;
+            }
+            if (threadIdx.x == 0)
+                b.hull_cnt[g] = static_cast<uint32_t>(h);
+            __syncthreads();
+            return;
+        }
+    }
+    else if (pre && threadIdx.x == 0)
+        b.pre_nact[g] = 0u;
     const uint32_t np2 = next_pow2(static_cast<uint32_t>(h));
-    if (fast)
+    int place = -1; // of the thread's vertex in key order (up to a vertex per thread)
+    if (h <= kHullThreads)
+    {
+        if (static_cast<int>(threadIdx.x) < h)
+            sm.diff[threadIdx.x] = static_cast<int32_t>(C[H[threadIdx.x]].key);
+        __syncthreads();
+        if (static_cast<int>(threadIdx.x) < h)
+        {
+            const uint32_t key = static_cast<uint32_t>(sm.diff[threadIdx.x]);
+            place = 0;
+#pragma unroll 4
+            for (int k = 0; k < h; ++k)
+                place += (static_cast<uint32_t>(sm.diff[k]) < key) ? 1 : 0;
+            sm.hkey[place] = key;
+        }
+        for (uint32_t j = h + threadIdx.x; j < np2; j += blockDim.x)
+            sm.hkey[j] = 0xffffffffu;
+        __syncthreads();
+    }
+    else if (fast)
     {
         for (int j = threadIdx.x; j < h; j += blockDim.x)
             sm.hkey[j] = C[H[j]].key;
         for (uint32_t j = h + threadIdx.x; j < np2; j += blockDim.x)
             sm.hkey[j] = 0xffffffffu;
-        for (int j = threadIdx.x; j <= h; j += blockDim.x)
-            sm.diff[j] = 0;
-    }
-    __syncthreads();
-    if (fast)
+        __syncthreads();
         block_bitonic_sort(sm.hkey, np2, [](uint32_t a, uint32_t c) { return a < c; });
+    }
     if (fast)
     {
+        for (int j = threadIdx.x; j <= h; j += blockDim.x)
+            sm.diff[j] = 0;
+        __syncthreads();
         // member o adds 1 to every hull vertex with a larger key: diff[upper_bound(o)] += 1. Each
         // thread walks a contiguous chunk of the member list as aligned quadruples (slot v:
         // members 4v - a .. 4v - a + 3, a = start mod 4; entries outside [0, n) skipped, the loads
@@ -1835,7 +1879,9 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int comput
             }
         }
         __syncthreads();
-        for (int j = threadIdx.x; j < h; j += blockDim.x)
+        if (place >= 0)
+            hull_dst[threadIdx.x] = sm.diff[place];
+        for (int j = threadIdx.x; h > kHullThreads && j < h; j += blockDim.x)
         {
             const uint32_t key = C[H[j]].key;
             int lo = 0, hi = h - 1;
@@ -1861,7 +1907,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int comput
 // and then the sort and the chain stack move to global scratch).
 // ---------------------------------------------------------------------------------------------
 constexpr int kWarpCand = 256;
-constexpr uint32_t kWarpRefineMin = 48; // more candidates than this: refine the polygon first
+constexpr uint32_t kWarpRefineMin = 64; // more candidates than this: refine the polygon first
 constexpr int kWarpPoly = 64;           // refined polygon capacity of the warp path
 
 // Scratch of the warp path's polygon refinement.
@@ -2051,19 +2097,17 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
     };
     HPt<float>* gs = reinterpret_cast<HPt<float>*>(b.hs_cand) + 2ull * start; // capacity 2n >= next_pow2(n)
     uint32_t m = 0;
+    uint32_t o_next = mem[min(lane, n - 1u)];
+    float2 p_next = xy[min(lane, n - 1u)];
 #pragma unroll 1
     for (uint32_t base = 0; base < n; base += 32)
     {
         const uint32_t i = base + lane;
-        bool keep = false;
-        HPt<float> c{0.0f, 0.0f, 0u};
-        if (i < n)
-        {
-            const uint32_t o = mem[i];
-            const float2 p = xy[i];
-            keep = !inside(p.x, p.y);
-            c = HPt<float>{p.x, p.y, o};
-        }
+        const HPt<float> c{p_next.x, p_next.y, o_next};
+        const uint32_t ahead = min(i + 32u, n - 1u); // (on its way during the tests)
+        o_next = mem[ahead];
+        p_next = xy[ahead];
+        const bool keep = !inside(c.x, c.y) && i < n;
         const uint32_t mask = __ballot_sync(0xffffffffu, keep);
         if (keep)
         {
@@ -2425,7 +2469,7 @@ struct BoxSmem
 constexpr int kBoxWarpVerts = 256; // more: the warps of a CTA share one region, up to kHullSmem
 static_assert(sizeof(BoxSmem<kBoxWarpVerts>) * (kHullThreads / 32) <= kTieDynSmem && sizeof(BoxSmem<kHullSmem>) <= kTieDynSmem);
 
-// The tie repairs (rare), then both boxes of every cluster, a warp for each box. The boxes' FP64 chains
+// The tie repairs (rare), the member counts of the large clusters' hulls, then both boxes of every cluster, a warp for each box. The boxes' FP64 chains
 // (the SM retires an FP64 instruction of a warp every 16 cycles) take longer than finding the hull: one after the other
 // behind the hull, they were more than half of the 62 us that a small scan's longest cluster took; here the two boxes run
 // on different SMs where the scan is small, and the hull kernel's code fits the instruction cache better without them.
@@ -2439,14 +2483,49 @@ __global__ void __launch_bounds__(kHullThreads) k_hull_boxes(BatchDev b, int com
     const uint32_t ntie = b.queue[5]; // the tie count (queue[4] is the small-cluster head)
     for (uint32_t t = blockIdx.x; t < ntie; t += gridDim.x)
         repair_cluster(b, b.tie_list[t], tsm, ss);
+    const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
+    // the large clusters' member counts (37,990 members took the cluster's own CTA 44,000 cycles)
+    const uint32_t nitems = b.queue[6];
+    for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x)
+    {
+        const uint2 item = b.pre_items[it];
+        const uint32_t g = item.x;
+        const uint32_t h = b.pre_nact[g]; // 0: counted with the hull
+        if (h == 0u)
+            continue;
+        const uint32_t start = b.cl_start[g], n = b.cl_cnt[g];
+        const uint32_t* mem = b.members + start;
+        const int* keys = b.hs_stack + 2ull * start + 2ull * b.cl_rank[g];
+        constexpr uint32_t kEach = kPreChunk / kHullThreads;
+        uint32_t o[kEach];
+#pragma unroll
+        for (uint32_t u = 0; u < kEach; ++u)
+        {
+            const uint32_t i = item.y * kPreChunk + u * kHullThreads + threadIdx.x;
+            o[u] = (i < n) ? mem[i] : 0xffffffffu; // (never below a key)
+        }
+#pragma unroll 2
+        for (uint32_t j = 0; j < h; ++j)
+        {
+            const uint32_t key = static_cast<uint32_t>(keys[j]);
+            uint32_t cnt = 0;
+#pragma unroll
+            for (uint32_t u = 0; u < kEach; ++u)
+                cnt += (o[u] < key) ? 1u : 0u;
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
+            if (lane == 0)
+                atomicAdd(&b.hull_tmp[start + j], static_cast<int32_t>(cnt));
+        }
+    }
     if (!compute_obb)
         return;
     const uint32_t nbig = b.queue[2], nsmall = b.queue[3];
-    const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
-    // hulls of more vertices than a warp's region holds (their clusters are large): one per CTA, one box a warp
-    for (uint32_t w = blockIdx.x; w < nbig; w += gridDim.x)
+    const uint32_t K = nbig + nsmall;
+    auto cluster = [&](uint32_t w) { return w < nbig ? work[w] : work[b.ncl - 1u - (w - nbig)]; };
+    // hulls of more vertices than a warp's region holds: one per CTA, one box a warp
+    for (uint32_t w = blockIdx.x; w < K; w += gridDim.x)
     {
-        const uint32_t g = work[w];
+        const uint32_t g = cluster(w);
         const int h = static_cast<int>(b.hull_cnt[g]);
         if (h <= kBoxWarpVerts)
             continue;
@@ -2470,11 +2549,9 @@ __global__ void __launch_bounds__(kHullThreads) k_hull_boxes(BatchDev b, int com
         __syncthreads();
     }
     BoxSmem<kBoxWarpVerts>& bs = reinterpret_cast<BoxSmem<kBoxWarpVerts>*>(tsm)[warp];
-    const uint32_t K = nbig + nsmall;
     for (uint32_t i = blockIdx.x + gridDim.x * warp; i < 2u * K; i += gridDim.x * (kHullThreads / 32))
     {
-        const uint32_t w = i < K ? i : i - K;
-        const uint32_t g = w < nbig ? work[w] : work[b.ncl - 1u - (w - nbig)];
+        const uint32_t g = cluster(i < K ? i : i - K);
         const int h = static_cast<int>(b.hull_cnt[g]);
         if (h > kBoxWarpVerts || b.cl_cnt[g] < 3u) // (fewer than three members: zero, written with the hull)
             continue;
