@@ -191,21 +191,30 @@ __device__ __forceinline__ int32_t flat_voxel(int32_t nr, int32_t na, int32_t r,
 // New voxels are listed (vlist; state[0].n_comp counts the batch's). The grid dimensions
 // (clusterer.cpp:92-99) come from the maxima that k_obs_gather left; the thread of a scan's first
 // obstacle records them.
-__global__ void k_vox_insert(BatchDev b)
+// What bounds it is the L2's atomics: neighbours in a row share their voxel and every new voxel its scan's
+// counters, so the lanes of a warp that fell into one voxel insert it once, and a CTA takes its place in the list
+// and counts its voxels with one atomic each (obstacle by obstacle and warp by warp, 64 scans took 92 us).
+constexpr uint32_t kVoxThreads = 256;
+__global__ void __launch_bounds__(kVoxThreads) k_vox_insert(BatchDev b)
 {
     pdl_enter();
-    const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = o < b.obs_flag[b.npts];
-    bool fresh = false;
-    uint32_t at = 0u;
-    int s = 0;
+    __shared__ uint32_t wnew[kVoxThreads / 32], wbase[kVoxThreads / 32];
+    __shared__ int ends[2]; // the scans of the CTA's first and last obstacle
+    const uint32_t nobs = b.obs_flag[b.npts];
+    const uint32_t o0 = blockIdx.x * kVoxThreads;
+    if (o0 >= nobs)
+        return;
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    const uint32_t o = o0 + threadIdx.x;
+    const bool in = o < nobs;
+    const int s = scan_of_obs(b, min(o, nobs - 1u));
+    const ScanDev& sd = b.scans[s];
+    ScanState& st = b.state[s];
+    const int32_t nr = static_cast<int32_t>(ceilf(__uint_as_float(st.max_r_bits) / sd.res_r) + 1.0f);
+    const int32_t na = static_cast<int32_t>(ceilf(__uint_as_float(st.max_a_bits) / sd.res_a) + 1.0f);
+    uint32_t key = 0u;
     if (in)
     {
-        s = scan_of_obs(b, o);
-        const ScanDev& sd = b.scans[s];
-        ScanState& st = b.state[s];
-        const int32_t nr = static_cast<int32_t>(ceilf(__uint_as_float(st.max_r_bits) / sd.res_r) + 1.0f);
-        const int32_t na = static_cast<int32_t>(ceilf(__uint_as_float(st.max_a_bits) / sd.res_a) + 1.0f);
         if (o == st.obs_off)
         {
             const int32_t ne = static_cast<int32_t>(ceilf(__uint_as_float(st.max_e_bits) / sd.res_e) + 1.0f);
@@ -218,10 +227,17 @@ __global__ void k_vox_insert(BatchDev b)
         const int32_t vr = static_cast<int32_t>(b.obs_r[o] / sd.res_r);
         const int32_t va = static_cast<int32_t>(b.obs_a[o] / sd.res_a);
         const int32_t ve = static_cast<int32_t>(b.obs_e[o] / sd.res_e);
-        const uint32_t key = static_cast<uint32_t>(flat_voxel(nr, na, vr, va, ve));
+        key = static_cast<uint32_t>(flat_voxel(nr, na, vr, va, ve));
+    }
+    const unsigned long long voxel = in ? (static_cast<unsigned long long>(s) << 32) | key : ~0ull;
+    const uint32_t peers = __match_any_sync(0xffffffffu, voxel);
+    const int leader = __ffs(peers) - 1; // the smallest obstacle of the warp's in the voxel
+    bool fresh = false;
+    uint32_t at = kEmpty;
+    if (in && static_cast<int>(lane) == leader)
+    {
         const uint32_t mask = st.hash_mask, off = st.hash_off;
         uint32_t h = hash_mix(key) & mask;
-        at = kEmpty;
         for (uint32_t probe = 0; probe <= mask; ++probe)
         {
             uint32_t* rec = reinterpret_cast<uint32_t*>(&b.hrec[off + h]);
@@ -231,34 +247,44 @@ __global__ void k_vox_insert(BatchDev b)
                 at = off + h;
                 fresh = prev == kEmpty;
                 atomicMin(&rec[1], o - st.obs_off);
-                atomicAdd(&rec[2], 1u);
+                atomicAdd(&rec[2], static_cast<uint32_t>(__popc(peers)));
                 break;
             }
             h = (h + 1u) & mask;
         }
         if (at == kEmpty)
             raise_err(&st, ERR_HASH_FULL);
+    }
+    at = __shfl_sync(0xffffffffu, at, leader);
+    if (in)
         b.obs_hslot[o] = at;
-    }
     const uint32_t m = __ballot_sync(0xffffffffu, fresh);
-    if (m == 0u)
-        return;
-    uint32_t pos = 0u;
-    const int leader = __ffs(m) - 1;
-    if (lane_id() == static_cast<uint32_t>(leader))
-        pos = atomicAdd(&b.state[0].n_comp, static_cast<uint32_t>(__popc(m)));
-    pos = __shfl_sync(0xffffffffu, pos, leader);
-    if (fresh)
-        b.vlist[pos + static_cast<uint32_t>(__popc(m & ((1u << lane_id()) - 1u)))] = at;
-    // voxels per scan (a warp's obstacles mostly belong to one)
-    const int s0 = __shfl_sync(0xffffffffu, s, leader);
-    if (__all_sync(0xffffffffu, !fresh || s == s0))
+    if (lane == 0)
+        wnew[warp] = static_cast<uint32_t>(__popc(m));
+    if (threadIdx.x == 0 || threadIdx.x == kVoxThreads - 1u)
+        ends[threadIdx.x != 0] = s;
+    __syncthreads();
+    if (warp == 0)
     {
-        if (lane_id() == static_cast<uint32_t>(leader))
-            atomicAdd(&b.state[s0].n_vox, static_cast<uint32_t>(__popc(m)));
+        const uint32_t v = (lane < kVoxThreads / 32u) ? wnew[lane] : 0u;
+        const uint32_t incl = warp_incl_scan(v);
+        uint32_t base = 0u;
+        if (lane == 31u && incl)
+        {
+            base = atomicAdd(&b.state[0].n_comp, incl);
+            if (ends[0] == ends[1]) // (the obstacles lie scan by scan)
+                atomicAdd(&st.n_vox, incl);
+        }
+        base = __shfl_sync(0xffffffffu, base, 31);
+        if (lane < kVoxThreads / 32u)
+            wbase[lane] = base + incl - v;
     }
-    else if (fresh)
-        atomicAdd(&b.state[s].n_vox, 1u);
+    __syncthreads();
+    if (!fresh)
+        return;
+    b.vlist[wbase[warp] + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)))] = at;
+    if (ends[0] != ends[1])
+        atomicAdd(&st.n_vox, 1u);
 }
 
 // Every parent pointer is strictly smaller than its index except at roots (links go from the
@@ -558,7 +584,7 @@ void launch_clustering(Launcher& L, const BatchDev& b, const BatchHost& hb)
     };
     scan("k_obs_scan", ObsFlagSrc{b.seg_label, b.npts}, b.obs_flag);
     LP_LAUNCH(L, k_obs_gather, div_up(b.npts, kObsChunk), 256, b);
-    LP_LAUNCH(L, k_vox_insert, div_up(b.npts, T), T, b);
+    LP_LAUNCH(L, k_vox_insert, div_up(b.npts, kVoxThreads), kVoxThreads, b);
     const uint32_t vgrid = std::min(div_up(13u * std::max(b.npts, 1u), T), static_cast<uint32_t>(sm_count()) * 8u);
     LP_LAUNCH(L, k_uf_hook, vgrid, T, b);
     LP_LAUNCH(L, k_uf_flatten, std::min(div_up(b.npts, T), static_cast<uint32_t>(sm_count()) * 8u), T, b);

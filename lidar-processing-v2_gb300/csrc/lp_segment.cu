@@ -884,18 +884,17 @@ __device__ __forceinline__ void ransac_select(const BatchDev& b, int s)
 {
     ScanState& st = b.state[s];
     const unsigned long long valid = b.pvalid[s];
-    uint32_t best = 0;
-    int bi = -1;
-#pragma unroll 10
-    for (int it = 0; it < kMaxRansacIters; ++it)
-    {
-        const uint32_t c = ((valid >> it) & 1ull) ? __ldcg(&b.inliers[s * kMaxRansacIters + it]) : 0u;
-        if (c > best)
-        {
-            best = c;
-            bi = it;
-        }
-    }
+    // a warp: the first hypothesis of the most inliers, two per lane
+    const uint32_t lane = lane_id();
+    auto count = [&](uint32_t it) {
+        return it < static_cast<uint32_t>(kMaxRansacIters) && ((valid >> it) & 1ull) ? __ldcg(&b.inliers[s * kMaxRansacIters + it]) : 0u;
+    };
+    const uint32_t n0 = count(lane), n1 = count(lane + 32u);
+    const uint32_t best = __reduce_max_sync(0xffffffffu, max(n0, n1));
+    const uint32_t m0 = __ballot_sync(0xffffffffu, n0 == best), m1 = __ballot_sync(0xffffffffu, n1 == best);
+    const int bi = m0 ? __ffs(m0) - 1 : 31 + __ffs(m1);
+    if (lane != 0u)
+        return;
     if (best > 0)
     {
         float4 q = b.planes[s * kMaxRansacIters + bi];
@@ -996,7 +995,7 @@ __global__ void __launch_bounds__(256) k_ransac_inliers(BatchDev b)
     if (!last)
         return;
     __threadfence();
-    for (int q = static_cast<int>(threadIdx.x); q < b.nscan; q += static_cast<int>(blockDim.x))
+    for (int q = static_cast<int>(warp); q < b.nscan; q += static_cast<int>(nwarp))
         ransac_select(b, q);
 }
 
@@ -1083,26 +1082,13 @@ __global__ void k_pixel(BatchDev b)
 // segments (zero outside the image: the rectangle is clipped at the border). Dilation changes
 // only ground and empty pixels, never the obstacle channel, so rows are independent. Each warp
 // walks a contiguous run of segments; the queue keeps column order through per-warp counts.
-__device__ __forceinline__ uint32_t obstacle_bits(const uint8_t* st, int32_t H, int32_t W, int32_t h, int32_t seg)
-{
-    uint32_t m = 0u;
-    const int32_t w = seg * 32 + static_cast<int32_t>(lane_id());
-    const bool colok = seg >= 0 && w < W;
-#pragma unroll
-    for (int32_t dh = -2; dh <= 2; ++dh)
-    {
-        const int32_t hh = h + dh;
-        const bool ok = colok && hh >= 0 && hh < H;
-        m |= __ballot_sync(0xffffffffu, ok && st[hh * W + w] == PX_OBSTACLE);
-    }
-    return m;
-}
-
+constexpr int kRowWords = 2048; // 32-column words of the widest image row (65,535 columns)
 __global__ void __launch_bounds__(256) k_dilate_rows(BatchDev b)
 {
     pdl_enter();
     __shared__ uint32_t wcount[8];
     __shared__ uint32_t woff[8];
+    __shared__ uint32_t bits[kRowWords + 2], queued[kRowWords];
     const uint32_t r = blockIdx.x;
     const int s = scan_of_row(b, r);
     const ScanDev& sd = b.scans[s];
@@ -1114,31 +1100,57 @@ __global__ void __launch_bounds__(256) k_dilate_rows(BatchDev b)
     const int32_t nseg = (W + 31) / 32;
     const int32_t per = (nseg + 7) / 8;
     const int32_t s0 = static_cast<int32_t>(warp) * per, s1 = min(nseg, s0 + per);
+    // the obstacles of the rows h - 2 .. h + 2, a bit per column, four words' loads in flight
+    for (int32_t g = s0; g < s1; g += 4)
+    {
+        bool any[4];
+#pragma unroll
+        for (int32_t u = 0; u < 4; ++u)
+        {
+            const int32_t w = (g + u) * 32 + static_cast<int32_t>(lane);
+            any[u] = false;
+#pragma unroll
+            for (int32_t dh = -2; dh <= 2; ++dh)
+                any[u] |= g + u < s1 && w < W && h + dh >= 0 && h + dh < H && st[(h + dh) * W + w] == PX_OBSTACLE;
+        }
+#pragma unroll
+        for (int32_t u = 0; u < 4; ++u)
+        {
+            const uint32_t m = __ballot_sync(0xffffffffu, any[u]);
+            if (lane == 0 && g + u < s1)
+                bits[g + u + 1] = m;
+        }
+    }
+    if (threadIdx.x == 0)
+        bits[0] = bits[nseg + 1] = 0u;
+    __syncthreads();
     // pass 1: dilate, update the states, count the queued (ground -> intersection) pixels
     uint32_t count = 0u;
-    uint32_t left = (s0 < s1) ? obstacle_bits(st, H, W, h, s0 - 1) : 0u;
-    uint32_t cur = (s0 < s1) ? obstacle_bits(st, H, W, h, s0) : 0u;
-    for (int32_t seg = s0; seg < s1; ++seg)
+    for (int32_t g = s0; g < s1; g += 4)
     {
-        const uint32_t right = obstacle_bits(st, H, W, h, seg + 1);
-        const uint32_t d = cur | (cur << 1) | (cur << 2) | (cur >> 1) | (cur >> 2) | (left >> 31) | (left >> 30) |
-                           (right << 31) | (right << 30);
-        const int32_t w = seg * 32 + static_cast<int32_t>(lane);
-        bool inter = false;
-        if (w < W && ((d >> lane) & 1u))
+        uint8_t c[4];
+#pragma unroll
+        for (int32_t u = 0; u < 4; ++u)
         {
-            const uint8_t c = st[h * W + w];
-            if (c == PX_GROUND)
-            {
-                inter = true;
-                st[h * W + w] = PX_INTERSECT;
-            }
-            else if (c == PX_EMPTY)
-                st[h * W + w] = PX_EMPTY_RED;
+            const int32_t seg = min(g + u, nseg - 1), w = seg * 32 + static_cast<int32_t>(lane);
+            const uint32_t left = bits[seg], cur = bits[seg + 1], right = bits[seg + 2];
+            const uint32_t d = cur | (cur << 1) | (cur << 2) | (cur >> 1) | (cur >> 2) | (left >> 31) | (left >> 30) |
+                               (right << 31) | (right << 30);
+            c[u] = (g + u < s1 && w < W && ((d >> lane) & 1u)) ? st[h * W + w] : static_cast<uint8_t>(PX_OBSTACLE);
         }
-        count += static_cast<uint32_t>(__popc(__ballot_sync(0xffffffffu, inter)));
-        left = cur;
-        cur = right;
+#pragma unroll
+        for (int32_t u = 0; u < 4; ++u)
+        {
+            const int32_t w = (g + u) * 32 + static_cast<int32_t>(lane);
+            if (c[u] == PX_GROUND)
+                st[h * W + w] = PX_INTERSECT;
+            else if (c[u] == PX_EMPTY)
+                st[h * W + w] = PX_EMPTY_RED;
+            const uint32_t m = __ballot_sync(0xffffffffu, c[u] == PX_GROUND);
+            if (lane == 0 && g + u < s1)
+                queued[g + u] = m;
+            count += static_cast<uint32_t>(__popc(m));
+        }
     }
     if (lane == 0)
         wcount[warp] = count;
@@ -1165,13 +1177,14 @@ __global__ void __launch_bounds__(256) k_dilate_rows(BatchDev b)
         }
     }
     __syncthreads();
-    // pass 2: queue entries in column order (this row's states now hold the intersections)
+    // pass 2: queue entries in column order
     uint32_t pos = woff[warp];
+#pragma unroll 4
     for (int32_t seg = s0; seg < s1; ++seg)
     {
         const int32_t w = seg * 32 + static_cast<int32_t>(lane);
-        const bool inter = w < W && st[h * W + w] == PX_INTERSECT;
-        const uint32_t m = __ballot_sync(0xffffffffu, inter);
+        const uint32_t m = queued[seg];
+        const bool inter = ((m >> lane) & 1u) != 0u;
         if (inter)
         {
             const uint32_t j = pos + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
@@ -1991,7 +2004,9 @@ void launch_segmentation(Launcher& L, const BatchDev& b, const BatchHost& hb, ui
     LP_LAUNCH(L, k_recm, hb.nslices, kRecmThreads, b);
     LP_LAUNCH(L, k_ransac_draw, static_cast<uint32_t>(b.nscan) * kDrawCtas, kDrawThreads, b);
     // about four CTAs per SM over the batch's tiles
-    LP_LAUNCH(L, k_ransac_inliers, static_cast<uint32_t>(sm_count()) * 4u, 256, b);
+    // (candidates are points: more CTAs than their tiles would only take tickets)
+    LP_LAUNCH(L, k_ransac_inliers, std::min(static_cast<uint32_t>(sm_count()) * 4u,
+                                            b.npts / kInlierTile + static_cast<uint32_t>(b.nscan)), 256, b);
     LP_LAUNCH(L, k_label_depth, div_up(b.npts, T), T, b);
     LP_LAUNCH(L, k_project_key, div_up(b.npts, T), T, b);
     LP_LAUNCH(L, k_pixel, div_up(b.npix, T), T, b);
