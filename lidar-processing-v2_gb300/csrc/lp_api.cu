@@ -91,6 +91,33 @@ bool seg_config_ok(const lp_segmenter_config& c)
            static_cast<int64_t>(c.image_width) * c.image_height < (1 << 28);
 }
 
+// Layout of the scan's projection keys in one 64-bit word (k_label_depth): the squared distance's bits above
+// those of the least one a valid point can have, the cell, the point, its label. False where they need more
+// than 63 bits (all ones: no point).
+bool pack_projection_key(ScanDev& sd, const lp_segmenter_config& c)
+{
+    auto bits = [](float v) {
+        uint32_t u;
+        std::memcpy(&u, &v, 4);
+        return u;
+    };
+    auto width = [](uint64_t v) {
+        uint32_t w = 0;
+        for (; v != 0; v >>= 1)
+            ++w;
+        return w;
+    };
+    // sqrtf(d2) >= min_d and <= max_d: d2 lies within a few roundings of their squares
+    const float lo = c.min_distance_m > 0.0f ? c.min_distance_m * c.min_distance_m * (1.0f - 1e-5f) : 0.0f;
+    const float hi = c.max_distance_m * c.max_distance_m * (1.0f + 1e-5f);
+    if (!(lo <= hi)) // no point is valid
+        return false;
+    sd.key_base = bits(lo);
+    sd.key_cell = 1u + width(sd.n > 0u ? sd.n - 1u : 0u);
+    sd.key_dist = sd.key_cell + width(static_cast<uint64_t>(sd.nslice) * static_cast<uint64_t>(sd.nrad) - 1u);
+    return sd.key_cell < 32u && sd.key_dist + width(bits(hi) - sd.key_base) <= 63u;
+}
+
 // Host-side layout and the configuration constants of every scan (binary32 expressions
 // evaluated exactly as the reference writes them).
 lp_status plan(lp_context* ctx, lp_batch& B)
@@ -147,6 +174,7 @@ lp_status plan(lp_context* ctx, lp_batch& B)
             sd.kthr2 = c.kernel_threshold_distance_m * c.kernel_threshold_distance_m; // :532-533
             sd.amp = c.amplification_factor;
             sd.max_cos = std::cos(std::tan(c.road_maximum_slope_m_per_m)); // :360
+            hb.packed_key = pack_projection_key(sd, c) && hb.packed_key;
             sd.use_ring = ((in.ring != nullptr) || in.compute_ring) && !c.assume_unorganized_cloud;
             if (sd.compute_ring && sd.first_ring < 0)
                 sd.first_ring = c.image_height - 1;
@@ -477,7 +505,8 @@ lp_status execute(lp_context* ctx, lp_batch& B, bool outputs)
         f.add(b.ransac_done, 4, 0u);
         f.add(b.pvalid, S * 8, 0u);
         f.add(b.inliers, S * kMaxRansacIters * 4, 0u);
-        f.add(b.pix_depth, static_cast<size_t>(b.npix) * 4, 0xffffffffu);
+        if (!B.hb.packed_key)
+            f.add(b.pix_depth, static_cast<size_t>(b.npix) * 4, 0xffffffffu);
         f.add(b.pix_key, static_cast<size_t>(b.npix) * 8, 0xffffffffu);
         f.add(b.row_cnt, static_cast<size_t>(b.nrows) * 4, 0u);
     }

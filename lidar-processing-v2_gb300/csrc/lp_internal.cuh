@@ -51,6 +51,8 @@ struct ScanDev
     float zmin_adj, zmax_adj, spacing, min_d, max_d, slice_res;
     float down_rad, rad_per_px;
     float delta, thr, sensor_h, kthr2, amp, max_cos;
+    // projection key (project_key): bits of the least squared distance, shifts of distance and cell
+    uint32_t key_base, key_dist, key_cell;
     int32_t use_ring; // 1: height index from ring; 0: from the elevation angle
     int32_t compute_ring;
     int32_t first_ring;

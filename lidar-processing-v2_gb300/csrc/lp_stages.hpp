@@ -239,6 +239,7 @@ struct BatchHost
     int nscan = 0;
     bool any_compute_ring = false;
     bool any_noise = false;
+    bool packed_key = true; // every scan's projection keys fit one word (k_label_depth)
     uint32_t ntiles = 0;
     uint32_t nslices = 0;
     std::vector<ScanDev> scans;
