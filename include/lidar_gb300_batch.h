@@ -85,7 +85,8 @@ typedef struct lp_tuning
     uint32_t hull_cta_min;     /* clusters of more members take a whole CTA of the hull kernel, smaller
                                   ones one warp (64-512) */
     uint32_t hull_ctas_per_sm; /* persistent hull CTAs per SM (1-4) */
-    uint32_t cell_ctas_per_sm; /* polar-cell sort CTAs per SM (1-16) */
+    uint32_t cell_ctas_per_sm; /* 1-16; kept in tables, no kernel reads it (the polar cells take a CTA per
+                                  azimuth slice) */
     uint32_t jcp_ctas_per_sm;  /* vote-weight CTAs per SM (1-16) */
 } lp_tuning;
 

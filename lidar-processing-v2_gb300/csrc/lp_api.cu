@@ -216,7 +216,6 @@ lp_status plan(lp_context* ctx, lp_batch& B)
     hb.ntiles = static_cast<uint32_t>(tile);
     hb.nslices = static_cast<uint32_t>(slice);
     hb.hull_ctas_per_sm = B.tune.hull_ctas_per_sm;
-    hb.cell_ctas_per_sm = B.tune.cell_ctas_per_sm;
     hb.jcp_ctas_per_sm = B.tune.jcp_ctas_per_sm;
     BatchDev& b = B.b;
     b = BatchDev{};

@@ -10,8 +10,6 @@
 namespace lpg
 {
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems; // 2048 elements per block
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
 {
@@ -25,10 +23,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
     return v;
 }
 
-// ---- TMA bulk copies (global -> shared) completing on an mbarrier ------------------------------
-// cp.async.bulk moves a contiguous range (16-byte aligned, size a multiple of 16) through the
-// tensor memory accelerator; the issuing thread announces the byte count on the mbarrier, and
-// the barrier's phase flips when that many bytes have landed.
+// ---- mbarrier with a bounded wait --------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_addr(const void* p)
 {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -37,18 +32,6 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, uint32_t coun
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, unsigned long long* bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
 }
 // Waits until the barrier has completed the phase with the given parity; gives up after
 // `limit` polls and returns false (the caller reports it and stops using the buffer).
@@ -234,29 +217,6 @@ __device__ void warp_bitonic_smem(T* s, uint32_t n, Less less)
             __syncwarp();
         }
     }
-}
-
-// Bitonic sort of 32 values held one per lane (ascending by lane).
-template <typename T, typename Less>
-__device__ __forceinline__ T warp_bitonic_sort(T v, Less less)
-{
-    const uint32_t lane = lane_id();
-#pragma unroll
-    for (uint32_t k = 2; k <= 32; k <<= 1)
-    {
-#pragma unroll
-        for (uint32_t j = k >> 1; j > 0; j >>= 1)
-        {
-            const T o = __shfl_xor_sync(0xffffffffu, v, j);
-            const bool up = ((lane & k) == 0);
-            const bool lower = ((lane & j) == 0);
-            // lower lane keeps min when ascending
-            const bool take_o = (lower == up) ? less(o, v) : less(v, o);
-            if (take_o)
-                v = o;
-        }
-    }
-    return v;
 }
 
 __host__ __device__ inline uint32_t next_pow2(uint32_t v)

@@ -126,12 +126,6 @@ __device__ __forceinline__ int find_scan(int nscan, uint32_t i, F off_of)
     return lo;
 }
 
-// Order-preserving map of non-negative float bits for atomicMax.
-__device__ __forceinline__ uint32_t fkey(float v)
-{
-    return __float_as_uint(v);
-}
-
 __device__ __forceinline__ uint32_t lane_id()
 {
     return threadIdx.x & 31u;

@@ -245,7 +245,6 @@ struct BatchHost
     std::vector<ScanDev> scans;
     // launch shapes (lp_tuning)
     uint32_t hull_ctas_per_sm = 2;
-    uint32_t cell_ctas_per_sm = 8;
     uint32_t jcp_ctas_per_sm = 8;
 };
 
