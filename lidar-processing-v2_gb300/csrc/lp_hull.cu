@@ -15,9 +15,9 @@
 //      all members,
 //   4. local hull indices = rank of each hull vertex among the cluster's members in input
 //      order (the reference gathers a cluster's points in obstacle order, processor.cpp:640),
-//   5. rotating-calipers box (Shamos antipodal pairs, best area kept as a float exactly like
-//      BoundingBox::area; comparisons screened in FP32) and the PCA box, one warp each (in the CTA
-//      path while the other warps count the ranks).
+//   5. in a kernel of its own (k_hull_boxes), rotating-calipers box (Shamos antipodal pairs, best area
+//      kept as a float exactly like BoundingBox::area; comparisons screened in FP32) and the PCA box,
+//      one warp each.
 #include <atomic>
 #include <cfloat>
 #include <climits>
@@ -944,16 +944,13 @@ __device__ __noinline__ void calipers_box(ScanState* st, const double2* P, const
     }
 }
 
-// Orientation test of the monotone chain for float points: decided in FP32 when the float
-// determinant exceeds 2^-21 (|t1| + |t2|) in magnitude (its rounding error stays below
-// 6 * 2^-24 of that sum, the FP64 form's below 3 * 2^-53), else evaluated in FP64 as written.
 // u * v has an exact binary32 error term (no underflow in the product).
 __device__ __forceinline__ bool prod_err_exact(float u, float v, float t)
 {
     return fabsf(t) >= 1e-30f || u == 0.0f || v == 0.0f;
 }
 
-// The near-ties of ccw_or_colinear_f, out of line: points along a wall are mostly such.
+// The near-ties of chain_pops, out of line: along an exactly straight wall every test is one.
 __device__ __noinline__ bool ccw_or_colinear_near(float ax, float ay, float bx, float by, float cx, float cy)
 {
     const float u = bx - ax, v = cy - ay, w = by - ay, z = cx - ax;
@@ -981,7 +978,9 @@ __device__ __noinline__ bool ccw_or_colinear_near(float ax, float ay, float bx, 
     return ccw_or_colinear(ax, ay, bx, by, cx, cy);
 }
 
-// Does the candidate c pop b (a below it)? The FP32 decision; `near`: it is not one, ask chain_pops_near.
+// Does the candidate c pop b (a below it)? Decided in FP32 when the float determinant exceeds 2^-21 (|t1| +
+// |t2|) in magnitude (its rounding error stays below 6 * 2^-24 of that sum, the FP64 form's below
+// 3 * 2^-53); `near`: it does not, ask chain_pops_near.
 __device__ __forceinline__ bool chain_pops(float ax, float ay, float bx, float by, float cx, float cy, bool& near)
 {
     const float u = bx - ax, v = cy - ay, w = by - ay, z = cx - ax;
