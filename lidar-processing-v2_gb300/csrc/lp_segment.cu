@@ -873,12 +873,15 @@ __global__ void __launch_bounds__(kDrawThreads) k_ransac_draw(BatchDev b)
 // warp holds planes l and l + 32 as a float pair and counts, for the candidates its warp takes,
 // |((n.x p.x + n.y p.y) + n.z p.z) - d| < thr with packed binary32 operations (each half rounds
 // like the scalar operation, in the reference's order). The work is a flat list of tiles of
-// kInlierTile candidates over the batch's scans with usable planes (scan by scan, so a tile
+// kTile candidates over the batch's scans with usable planes (scan by scan, so a tile
 // belongs to one scan), taken grid-strided: a large scan spreads over the whole grid instead of
 // its own share of it. A CTA's tiles come in increasing order, so it follows the scans with a
 // cursor, loads a scan's planes when it reaches it and adds its counts when it leaves it (integer
 // partial counts add up exactly). The last CTA to finish picks every scan's plane (segmenter.cpp:432-443).
+// Batches whose points do not give every CTA a tile of 1,024 take tiles of 256: a warp's 128 candidates in a row
+// were most of the time (32 x 1024 scan 15 -> 9 us, 64 x 2048 16 -> 11, 128 x 4096 19 -> 13).
 constexpr uint32_t kInlierTile = 1024;
+constexpr uint32_t kInlierTileFew = 256;
 
 __device__ __forceinline__ void ransac_select(const BatchDev& b, int s)
 {
@@ -913,17 +916,18 @@ __device__ __forceinline__ void ransac_select(const BatchDev& b, int s)
     }
 }
 
+template <uint32_t kTile>
 __global__ void __launch_bounds__(256) k_ransac_inliers(BatchDev b)
 {
     pdl_enter();
     static_assert(kMaxRansacIters <= 64, "two planes per lane");
-    __shared__ float4 tile[kInlierTile];
+    __shared__ float4 tile[kTile];
     const uint32_t lane = lane_id();
     const uint32_t i0 = lane, i1 = lane + 32u;
     const uint32_t warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     auto tiles_of = [&](int q) -> uint32_t {
-        return (b.pvalid[q] != 0ull) ? div_up(b.state[q].n_cand, kInlierTile) : 0u;
+        return (b.pvalid[q] != 0ull) ? div_up(b.state[q].n_cand, kTile) : 0u;
     };
     int cs = 0; // the cursor: scan cs owns tiles [cbase, cbase + ctiles)
     uint32_t cbase = 0u, ctiles = (b.nscan > 0) ? tiles_of(0) : 0u;
@@ -932,14 +936,44 @@ __global__ void __launch_bounds__(256) k_ransac_inliers(BatchDev b)
     float2 qx = make_float2(0.f, 0.f), qy = qx, qz = qx, nqw = qx;
     float thr = 0.0f;
     uint32_t ca = 0u, cb = 0u;
-    auto flush = [&]() {
+    // The planes' counters take one atomic at a time. With small tiles (few points, many CTAs for them) a CTA's warps
+    // add up in shared memory first; with large ones a CTA meets several scans, and the barriers cost more.
+    constexpr bool together = kTile < kInlierTile;
+    __shared__ uint32_t sum[together ? 64 : 1];
+    if (together)
+    {
+        if (threadIdx.x < 64u)
+            sum[threadIdx.x] = 0u;
+        __syncthreads();
+    }
+    auto flush = [&]() { // (all threads alike)
         if (s < 0)
             return;
-        if (i0 < static_cast<uint32_t>(kMaxRansacIters) && ((valid >> i0) & 1ull) && ca)
-            atomicAdd(&b.inliers[s * kMaxRansacIters + i0], ca);
-        if (i1 < static_cast<uint32_t>(kMaxRansacIters) && ((valid >> i1) & 1ull) && cb)
-            atomicAdd(&b.inliers[s * kMaxRansacIters + i1], cb);
-        ca = cb = 0u;
+        if constexpr (!together)
+        {
+            if (i0 < static_cast<uint32_t>(kMaxRansacIters) && ((valid >> i0) & 1ull) && ca)
+                atomicAdd(&b.inliers[s * kMaxRansacIters + i0], ca);
+            if (i1 < static_cast<uint32_t>(kMaxRansacIters) && ((valid >> i1) & 1ull) && cb)
+                atomicAdd(&b.inliers[s * kMaxRansacIters + i1], cb);
+            ca = cb = 0u;
+        }
+        else
+        {
+            if (ca)
+                atomicAdd(&sum[i0], ca);
+            if (cb)
+                atomicAdd(&sum[i1], cb);
+            ca = cb = 0u;
+            __syncthreads();
+            if (threadIdx.x < 64u)
+            {
+                const uint32_t n = sum[threadIdx.x];
+                sum[threadIdx.x] = 0u;
+                if (n && threadIdx.x < static_cast<uint32_t>(kMaxRansacIters) && ((valid >> threadIdx.x) & 1ull))
+                    atomicAdd(&b.inliers[s * kMaxRansacIters + threadIdx.x], n);
+            }
+            __syncthreads();
+        }
     };
     for (uint32_t it = blockIdx.x;; it += gridDim.x)
     {
@@ -965,8 +999,8 @@ __global__ void __launch_bounds__(256) k_ransac_inliers(BatchDev b)
             thr = b.scans[s].thr;
         }
         const ScanState& st = b.state[s];
-        const uint32_t base = (it - cbase) * kInlierTile;
-        const uint32_t cnt = min(kInlierTile, st.n_cand - base);
+        const uint32_t base = (it - cbase) * kTile;
+        const uint32_t cnt = min(kTile, st.n_cand - base);
         const float4* cand = b.cand + st.cand_off + base;
         // candidates staged in shared memory (coalesced), read by each warp as broadcasts
         __syncthreads();
@@ -2111,8 +2145,10 @@ void launch_segmentation(Launcher& L, const BatchDev& b, const BatchHost& hb, ui
     LP_LAUNCH(L, k_ransac_draw, static_cast<uint32_t>(b.nscan) * kDrawCtas, kDrawThreads, b);
     // about four CTAs per SM over the batch's tiles
     // (candidates are points: more CTAs than their tiles would only take tickets)
-    LP_LAUNCH(L, k_ransac_inliers, std::min(static_cast<uint32_t>(sm_count()) * 4u,
-                                            b.npts / kInlierTile + static_cast<uint32_t>(b.nscan)), 256, b);
+    const uint32_t most = static_cast<uint32_t>(sm_count()) * 4u;
+    const uint32_t each = b.npts < most * kInlierTile ? kInlierTileFew : kInlierTile;
+    L.launch("k_ransac_inliers", each == kInlierTile ? k_ransac_inliers<kInlierTile> : k_ransac_inliers<kInlierTileFew>,
+             std::min(most, b.npts / each + static_cast<uint32_t>(b.nscan)), 256, b);
     const bool many = b.npix > static_cast<uint32_t>(sm_count()) * 10240u; // four pixels per thread fill the SMs
     const uint32_t pix_ctas = div_up(b.npix, many ? 4u * T : T);
     if (hb.packed_key)
