@@ -179,17 +179,24 @@ struct AreaCmpFp64
     }
 };
 
-// The same comparisons decided in FP32 where the float areas differ by more than `tol`, else in
-// FP64. Float areas use coordinates relative to (ox, oy): with every |local vertex| <= R the
+// The same comparisons decided in FP32 where the float areas differ by more than `tol`, else by
+// area_order_near. Float areas use coordinates relative to vertex 0: with every |local vertex| <= R the
 // float area is within 1.02e-6 R^2 of the exact area of the (float-valued) vertices, and the FP64
 // area of the reference within 1e-14 M R (M the largest |coordinate|). tol is at least twice the
-// sum of both bounds, so a decision taken in FP32 is the one FP64 takes.
+// sum of both bounds, so a decision taken in FP32 is the one FP64 takes. The margins are the constructor's:
+// one left at zero would let the approximate areas decide the ties of parallel edges.
 struct AreaCmpFiltered
 {
     const double2* P;
     const float2* Pf; // the same vertices as floats (exact: they are float points)
     float ox, oy, tol;
     float tol2; // of twice the areas, evaluated with two-term differences and products (area_order_near)
+    // m: M; r2: at least R^2
+    __device__ __forceinline__ AreaCmpFiltered(const double2* p, const float2* pf, float m, float r2)
+        : P(p), Pf(pf), ox(pf[0].x), oy(pf[0].y), tol(2.0f * (4e-6f * r2 + 1e-13f * (m * sqrtf(r2))) + 1e-30f),
+          tol2(4e-12f * r2 + 4e-13f * (m * sqrtf(r2)) + 1e-30f)
+    {
+    }
     __device__ __forceinline__ float af(int a, int b, int c) const
     {
         const float ax = Pf[a].x - ox, ay = Pf[a].y - oy;
@@ -914,10 +921,8 @@ __device__ __noinline__ void calipers_box(ScanState* st, const double2* P, const
         }
         r2 = warp_max_f(r2) * 1.001f;
         mabs = warp_max_f(mabs);
-        const float mr = mabs * sqrtf(r2);
-        const AreaCmpFiltered cmp{P, Pf, ox, oy, 2.0f * (4e-6f * r2 + 1e-13f * mr) + 1e-30f, 4e-12f * r2 + 4e-13f * mr + 1e-30f};
         if (lane == 0)
-            npairs = antipodal_pairs(cmp, h, pairs, cap);
+            npairs = antipodal_pairs(AreaCmpFiltered(P, Pf, mabs, r2), h, pairs, cap);
         npairs = __shfl_sync(0xffffffffu, npairs, 0);
         if (npairs > cap)
         {
@@ -2940,8 +2945,7 @@ __global__ void __launch_bounds__(32) k_boxes_single(const double2* P, uint32_t 
     if (lane == 0)
     {
         if (fast)
-            np = antipodal_pairs(AreaCmpFiltered{V, spf, spf[0].x, spf[0].y, 2.0f * (4e-6f * r2 + 1e-13f * mabs * sqrtf(r2)) + 1e-30f},
-                                 static_cast<int>(n), pairs, cap);
+            np = antipodal_pairs(AreaCmpFiltered(V, spf, mabs, r2), static_cast<int>(n), pairs, cap);
         else
             np = antipodal_pairs(AreaCmpFp64{V}, static_cast<int>(n), pairs, cap);
     }

@@ -51,3 +51,41 @@ def test_boxes_sizes(ctx, n, single):
     assert np.array_equal(poly.findAntipodalPairsOfConvexHull(hp), T.o_antipodal(hp))
     assert T.boxes_identical(poly.boundingBoxRotatingCalipers(hp), T.o_calipers(hp))
     assert T.pca_boxes_equal(poly.boundingBoxPrincipalComponentAnalysis(hp), T.o_pca(hp)[0])
+
+
+def parallel_sided(kind, rng):
+    """Polygons whose opposite sides are parallel up to binary32 rounding: the pair walk's area comparisons are ties."""
+    c, s = np.cos(a := rng.uniform(0, 2 * np.pi)), np.sin(a)
+    if kind in ("rectangle", "parallelogram"):
+        w, h, k = rng.uniform(0.2, 12), rng.uniform(0.2, 4), rng.uniform(-1, 1) if kind == "parallelogram" else 0.0
+        p = np.array([[0, 0], [w, 0], [w + k, h], [k, h]])
+    elif kind == "regular":
+        n = 2 * rng.integers(2, 17)
+        p = rng.uniform(0.1, 30) * np.stack([np.cos(t := np.arange(n) * (2 * np.pi / n)), np.sin(t)], 1)
+    else:  # the hull of points along a rectangle's sides
+        t, w, h = rng.random((200, 2)), rng.uniform(1, 6), rng.uniform(1, 3)
+        side = rng.integers(0, 2, 200)
+        p = np.stack([np.where(side == 0, t[:, 0] * w, (t[:, 1] < 0.5) * w), np.where(side == 1, t[:, 0] * h, (t[:, 1] < 0.5) * h)], 1)
+    p = p @ np.array([[c, s], [-s, c]]) + rng.uniform(-1, 1, 2) * rng.choice([0.0, 1.0, 60.0])
+    p = np.ascontiguousarray(p.astype(np.float32).astype(np.float64))
+    return np.ascontiguousarray(p[T.o_hull(p)]) if kind == "footprint" else p
+
+
+@pytest.mark.parametrize("kind", ["rectangle", "parallelogram", "regular", "footprint"])
+def test_boxes_of_parallel_sides(ctx, kind):
+    rng = np.random.default_rng(len(kind))
+    poly = lp.Polygonizer(ctx)
+    for k in range(1000):
+        hp = parallel_sided(kind, rng)
+        if len(hp) < 3:
+            continue
+        assert np.array_equal(poly.findAntipodalPairsOfConvexHull(hp), T.o_antipodal(hp)), (k, hp)
+        assert T.boxes_identical(poly.boundingBoxRotatingCalipers(hp), T.o_calipers(hp)), (k, hp)
+
+
+def test_box_of_a_turned_rectangle(ctx):
+    hp = np.array([[3.01463151, -2.00201011], [3.29160833, -2.88407683], [11.3488865, -0.354019314], [11.071909, 0.528047264]],
+                  np.float32).astype(np.float64)
+    poly = lp.Polygonizer(ctx)
+    assert np.array_equal(poly.findAntipodalPairsOfConvexHull(hp), T.o_antipodal(hp))
+    assert T.boxes_identical(poly.boundingBoxRotatingCalipers(hp), T.o_calipers(hp))
