@@ -949,10 +949,11 @@ __device__ __noinline__ void calipers_box(ScanState* st, const double2* P, const
     }
 }
 
-// u * v has an exact binary32 error term (no underflow in the product).
+// u * v has an exact binary32 error term: the product neither underflows nor overflows (an infinite one
+// would compare as equal to any other).
 __device__ __forceinline__ bool prod_err_exact(float u, float v, float t)
 {
-    return fabsf(t) >= 1e-30f || u == 0.0f || v == 0.0f;
+    return fabsf(t) <= FLT_MAX && (fabsf(t) >= 1e-30f || u == 0.0f || v == 0.0f);
 }
 
 // The near-ties of chain_pops, out of line: along an exactly straight wall every test is one.

@@ -2,6 +2,8 @@
 filter's and the shared-memory sort's sizes, binary32 and genuine binary64 coordinates, clouds that keep
 every point, ties, degenerate and far-off clouds. Index sequences and boxes equal the oracle's (the
 boxes' FP64 expressions are the oracle's, so no tolerance)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -89,3 +91,30 @@ def test_box_of_a_turned_rectangle(ctx):
     poly = lp.Polygonizer(ctx)
     assert np.array_equal(poly.findAntipodalPairsOfConvexHull(hp), T.o_antipodal(hp))
     assert T.boxes_identical(poly.boundingBoxRotatingCalipers(hp), T.o_calipers(hp))
+
+
+def far_points(n, scale, rng):
+    """Binary32 points on an integer grid scaled by a power of two: the products of their differences leave binary32."""
+    if n == 3:
+        return np.array([[0.0, 0.0], [1.0, 1.0], [2.0, 3.0]]) * scale
+    return np.round(rng.normal(size=(n, 2)) * 12).clip(-30, 30) * scale
+
+
+@pytest.mark.parametrize("log2", [59, 62, 65, 100, 122])
+@pytest.mark.parametrize("n", [3, 40, 64, 700, 5000])
+def test_hull_of_far_points(ctx, n, log2):
+    pts = np.ascontiguousarray(far_points(n, 2.0**log2, np.random.default_rng([n, log2])))
+    assert np.array_equal(pts, pts.astype(np.float32))
+    assert np.array_equal(lp.Polygonizer(ctx).convexHull(pts), T.o_hull(pts, T.TIES_LIBSTDCXX))
+
+
+@pytest.mark.parametrize("log2", [65, 100])
+def test_noalloc_hull_of_far_points(ctx, log2):
+    torch = pytest.importorskip("torch")
+    fn = lp.library().lp_convex_hull_noalloc
+    fn.restype, fn.argtypes = ctypes.c_int32, [ctypes.c_void_p, ctypes.c_uint32] + [ctypes.c_void_p] * 3
+    for n in (3, 40, 700):
+        pts = np.ascontiguousarray(far_points(n, 2.0**log2, np.random.default_rng([n, log2])))
+        xy, idx, cnt = torch.from_numpy(pts).cuda(), torch.zeros(n, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        assert fn(xy.data_ptr(), n, idx.data_ptr(), cnt.data_ptr(), None) == lp.LP_OK
+        assert np.array_equal(idx.cpu().numpy()[:int(cnt.item())], T.o_hull(pts, T.TIES_LIBSTDCXX))
