@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kRecmThreads) k_recm(BatchDev b)
     __shared__ float sz[kLargeCellMax]; // the slice's bucket table, then heights to be sorted
     static_assert(4u * kRecmTable <= kLargeCellMax, "counts, minima, maxima and the cells' starts");
     static_assert(kRecmThreads / 32 * kMediumCell <= kLargeCellMax, "the warps' parts fit");
-    __shared__ uint32_t nlarge, ccount[kRecmThreads / 32], cbase[kRecmThreads / 32];
+    __shared__ uint32_t nlarge, nbad, ccount[kRecmThreads / 32], cbase[kRecmThreads / 32];
     __shared__ int32_t sk;
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const int s = scan_of_slice(b, blockIdx.x);
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kRecmThreads) k_recm(BatchDev b)
     const uint32_t slice = blockIdx.x - sd.slice_off;
     const uint32_t off = sd.cell_off + slice * static_cast<uint32_t>(sd.nrad);
     if (threadIdx.x == 0)
-        nlarge = 0u;
+        nlarge = nbad = 0u;
     __syncthreads();
     const int32_t q0 = static_cast<int32_t>(floorf(2.0f * sd.zmin_adj));
     const int32_t nb = static_cast<int32_t>(floorf(2.0f * sd.zmax_adj)) - q0 + 1;
@@ -422,28 +422,22 @@ __global__ void __launch_bounds__(kRecmThreads) k_recm(BatchDev b)
             }
             b.zlow[off + c] = zunord(pick);
             if (below != n)
-                b.large_list[off + atomicAdd(&nlarge, 1u)] = off + c;
+                b.large_list[off + atomicAdd(&nbad, 1u)] = off + c;
         }
         __syncthreads();
-        // cells with a nan: small ones sorted by a warp, the others stay listed
-        const uint32_t nbad = nlarge;
-        if (nbad != 0u)
-        {
-            if (threadIdx.x == 0)
-                nlarge = 0u;
-            __syncthreads();
-            if (warp == 0)
-                for (uint32_t li = 0; li < nbad; ++li)
-                {
-                    const uint32_t c = b.large_list[off + li], n = b.cell_cnt[c];
-                    __syncwarp();
-                    if (n <= static_cast<uint32_t>(kMediumCell))
-                        cell_zlow_sorted(b, c, n, b.cell_start[c], sz);
-                    else if (lane == 0)
-                        b.large_list[off + nlarge++] = c;
-                    __syncwarp();
-                }
-        }
+        // cells with a nan: small ones sorted by a warp, the others stay listed (behind a counter of their own: the
+        // other warps only meet this one at the barrier below)
+        if (warp == 0)
+            for (uint32_t li = 0; li < nbad; ++li)
+            {
+                const uint32_t c = b.large_list[off + li], n = b.cell_cnt[c];
+                __syncwarp();
+                if (n <= static_cast<uint32_t>(kMediumCell))
+                    cell_zlow_sorted(b, c, n, b.cell_start[c], sz);
+                else if (lane == 0)
+                    b.large_list[off + nlarge++] = c; // nlarge <= li
+                __syncwarp();
+            }
     }
     else
     {
