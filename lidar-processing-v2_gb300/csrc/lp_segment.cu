@@ -1606,7 +1606,8 @@ __device__ __forceinline__ bool stale_slot(const BatchDev& b, const ScanDev& sd,
 // first, then (more open pixels than threads only) rounds over the list, then every thread watches
 // its own pixel's open neighbours and repeats the test when one is decided. Each CTA keeps every
 // queued pixel's state in its shared memory and a decision is written into all of them, so
-// watching costs local reads only (scans of more than `cap` queued pixels watch global memory).
+// watching costs local reads only (scans of more than `cap` queued pixels watch global memory). What
+// neither decides within its budget is left to vote_rows.
 // Bound by the chain of hops, about 700 cycles each. Chains of pixels of one row, each hanging on the
 // one to its left, would make 60 hops on a 64 x 2048 scan and 130 on a 32 x 4096 one: where the
 // bounds show that one open neighbour alone decides (it on ground: ground, it on obstacle: obstacle,
@@ -1620,7 +1621,12 @@ __device__ __forceinline__ bool stale_slot(const BatchDev& b, const ScanDev& sd,
 constexpr uint32_t kResolveThreads = 512;
 constexpr uint32_t kResolveStates = 24u * 1024u; // queued pixels whose states fit shared memory (4 bytes each)
 constexpr int kResolveWide = 7;           // scans of a launch up to which a scan takes 8 CTAs
-constexpr uint32_t kResolveSpins = 1u << 20; // polls of a pixel's neighbours before giving up
+// A round takes as long as it has open pixels, and where they hang on one another in chains as long as the image it
+// decides little more than one pixel of each. So rounds (2 us for 4,096 pixels) and watching end where they
+// have cost about half of what vote_rows would (2.5 us for every row and 512 pixels). Stripes over a 64 x 2048 and a
+// 128 x 4096 image: 1.2 and 4.1 ms, against 1,276 and 16,000 without an end. The workloads' scans stay below
+// it; with half of this budget one of 64 did not (107 -> 146 us).
+constexpr uint32_t kSpinsLocal = 32, kSpinsGlobal = 4; // polls of a pixel's neighbours for each step of vote_rows
 
 __device__ __forceinline__ void cluster_barrier()
 {
@@ -1669,6 +1675,117 @@ __device__ __forceinline__ uint32_t wide_state(uint32_t v)
     return (v & 1u) | ((v >> 1) << 12);
 }
 
+// What rounds and watching leave open, by one CTA, row by row as the reference goes: with the rows above decided, a
+// pixel's outcome depends on its two neighbours to the left alone (kernel slots 10 and 11, at most two
+// places back in the queue), so it is a map of the last two outcomes onto the next two, and the maps
+// of 512 pixels are composed by a scan.
+struct RowVote // of one scan
+{
+    volatile uint8_t* st;  // outcomes by queue index
+    const uint32_t* slot;  // record of each open pixel
+    const uint4* rec;      // field f of record r at rec[f * stride + r]
+    size_t stride;
+    const uint32_t* cnt;   // queued pixels of each row
+    const uint16_t* cols;  // their columns
+    const uint32_t* qidx;  // queue index by pixel
+    int32_t H, W;
+};
+
+// A map of the state (outcome before last, last outcome; 1: obstacle): two bits of the next state for each.
+__device__ __forceinline__ uint32_t then_map(uint32_t first, uint32_t second)
+{
+    uint32_t r = 0u;
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u)
+        r |= ((second >> (2u * ((first >> (2u * u)) & 3u))) & 3u) << (2u * u);
+    return r;
+}
+
+__device__ __noinline__ void vote_rows(const RowVote v)
+{
+    constexpr uint32_t kSame = 0xe4u; // the identity
+    __shared__ uint32_t total[kResolveThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    for (int32_t h = 0; h < v.H; ++h)
+    {
+        const uint32_t m = v.cnt[h];
+        const uint32_t q0 = m ? v.qidx[h * v.W + v.cols[h * v.W]] : 0u; // the row's queue entries lie behind one another
+        for (uint32_t j0 = 0; j0 < m; j0 += kResolveThreads)
+        {
+            const uint32_t q = q0 + j0 + tid;
+            const uint32_t is = (j0 + tid < m) ? v.st[q] : V_U;
+            const bool open = is == JST_OPEN;
+            if (!__syncthreads_or(open))
+                continue;
+            uint32_t map = (j0 + tid < m) ? (is == V_O ? 0xddu : 0x88u) : kSame; // decided: (., x) -> (x, outcome)
+            if (open)
+            {
+                const uint4* rec = v.rec + __ldcg(&v.slot[q]);
+                float wn[24];
+#pragma unroll
+                for (uint32_t f = 0; f < 6; ++f)
+                {
+                    const uint4 w = rec[f * v.stride];
+                    wn[4 * f] = __uint_as_float(w.x);
+                    wn[4 * f + 1] = __uint_as_float(w.y);
+                    wn[4 * f + 2] = __uint_as_float(w.z);
+                    wn[4 * f + 3] = __uint_as_float(w.w);
+                }
+                const uint4 masks = rec[9u * v.stride];
+                uint32_t m0 = masks.x & 0xfff000u, m1 = masks.y & 0xfff000u;
+                uint32_t last = 0u, before = 0u; // slots that read the last outcome, the one before
+#pragma unroll
+                for (uint32_t f = 0; f < 3; ++f)
+                {
+                    const uint4 d4 = rec[(6u + f) * v.stride];
+                    const uint32_t d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; ++u)
+                    {
+                        const uint32_t k = 4u * f + u;
+                        const uint32_t x = (d[u] & kDepFixed) ? d[u] & 3u : v.st[d[u]];
+                        if (x != JST_OPEN)
+                        {
+                            m0 |= (x & 1u) << k;
+                            m1 |= (x >> 1) << k;
+                        }
+                        else if (q - d[u] == 1u)
+                            last |= 1u << k;
+                        else
+                            before |= 1u << k;
+                    }
+                }
+                map = 0u;
+#pragma unroll 1
+                for (uint32_t u = 0; u < 4; ++u)
+                {
+                    const uint32_t o = ((u & 1u) ? last : 0u) | ((u & 2u) ? before : 0u); // these on obstacle
+                    const uint32_t x = vote_bounds(wn, m0 | ((last | before) & ~o), m1 | o);
+                    map |= (((u & 1u) << 1) | (x == V_O ? 1u : 0u)) << (2u * u);
+                }
+            }
+            uint32_t incl = map;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const uint32_t below = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= static_cast<uint32_t>(o))
+                    incl = then_map(below, incl);
+            }
+            if (lane == 31u)
+                total[warp] = incl;
+            __syncthreads();
+            uint32_t state = 0u; // (an open pixel never reads outcomes of the step before: those are decided)
+            for (uint32_t w = 0; w < warp; ++w)
+                state = (total[w] >> (2u * state)) & 3u;
+            state = (incl >> (2u * state)) & 3u;
+            if (open)
+                v.st[q] = static_cast<uint8_t>((state & 1u) ? V_O : V_G);
+            __syncthreads();
+        }
+    }
+}
+
 template <uint32_t kCtas>
 __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads) k_jcp_resolve(BatchDev b, uint32_t cap)
 {
@@ -1676,6 +1793,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads)
     constexpr uint32_t kAll = kResolveThreads * kCtas;
     extern __shared__ __align__(16) uint32_t sst[]; // cap + 4 entries
     __shared__ uint32_t s_n[2]; // pixels left open by a round (of the cluster's first CTA), alternating
+    __shared__ uint32_t s_left; // pixels remain for vote_rows (of the cluster's first CTA)
     const int s = static_cast<int>(blockIdx.x / kCtas);
     const uint32_t rank = blockIdx.x % kCtas;
     const ScanDev& sd = b.scans[s];
@@ -1724,6 +1842,8 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads)
     }
     if (tid < 2u)
         s_n[tid] = 0u;
+    if (tid == 2u)
+        s_left = 0u;
     __threadfence();
     cluster_barrier();
     const uint32_t n_addr[2] = {peer_smem(&s_n[0], 0u), peer_smem(&s_n[1], 0u)};
@@ -1780,8 +1900,11 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads)
     uint32_t dep[12], m0, m1;
     uint32_t n = nopen;
     uint32_t *cur = nullptr, *next = b.jlist + sd.jq_off, *other = b.jlist + b.jq_total + sd.jq_off; // null: all positions
-    for (uint32_t round = 0; n > kAll; ++round)
+    const uint32_t steps = static_cast<uint32_t>(sd.H) + nq / kResolveThreads; // of vote_rows
+    uint32_t spent = 0u;
+    for (uint32_t round = 0; n > kAll && 2u * spent <= steps; ++round)
     {
+        spent += 1u + n / (8u * kResolveThreads);
         const uint32_t cnt = n_addr[round & 1u];
         for (uint32_t t0 = warp * 32u; t0 < n; t0 += kAll)
         {
@@ -1816,24 +1939,32 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads)
         if (all == 0u)
             s_n[(round & 1u) ^ 1u] = 0u; // the next round's count (its last readers passed the barrier above)
         cluster_barrier();
-        if (left >= n)
-        {
-            if (all == 0u)
-                raise_err(&b.state[s], ERR_INTERNAL); // (the first open pixel in order is always decided)
-            n = 0u; // (every thread of the cluster alike)
-            break;
-        }
         n = left;
         cur = next;
         next = other;
         other = cur;
     }
-    if (all < n)
+    // what is left to vote_rows: its records by queue index
+    auto leave = [&](uint32_t at, uint32_t q) {
+        next[q] = at;
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer_smem(&s_left, 0u)), "r"(1u) : "memory");
+    };
+    if (n > kAll)
     {
-        const uint32_t q = jrec_load(b, sd.jq_off + (cur ? __ldcg(&cur[all]) : all), wn, dep, m0, m1);
+        for (uint32_t t = all; t < n; t += kAll)
+        {
+            const uint32_t at = cur ? __ldcg(&cur[t]) : t;
+            leave(at, jrec(b, 9u, sd.jq_off + at).z);
+        }
+    }
+    else if (all < n)
+    {
+        const uint32_t at = cur ? __ldcg(&cur[all]) : all;
+        const uint32_t q = jrec_load(b, sd.jq_off + at, wn, dep, m0, m1);
         locate(dep);
         uint32_t x = JST_OPEN, seen = 0xffffffffu, copied = 0u; // copied: the entry this pixel copies
-        for (uint32_t spin = 0; x == JST_OPEN && spin < kResolveSpins; ++spin)
+        const uint32_t spins = (local ? kSpinsLocal : kSpinsGlobal) * steps;
+        for (uint32_t spin = 0; x == JST_OPEN && spin < spins; ++spin)
         {
             if (copied != 0u)
             {
@@ -1857,31 +1988,35 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads)
                 {
                     // the heaviest open neighbour: does it decide alone?
                     float w = -1.0F;
-                    uint32_t at = 0u, bit = 0u;
+                    uint32_t on = 0u, bit = 0u;
 #pragma unroll
                     for (int k = 0; k < 12; ++k)
                         if (((acc >> k) & (acc >> (k + 12)) & 1u) && wn[k] > w)
                         {
                             w = wn[k];
-                            at = dep[k];
+                            on = dep[k];
                             bit = 1u << k;
                         }
                     if (bit != 0u && vote(wn, acc & ~(bit << 12), m0, m1) == V_G && vote(wn, acc & ~bit, m0, m1) == V_O)
                     {
-                        copied = at;
-                        tell(4u * q + 2u, (at - own) / 4u + 1u);
+                        copied = on;
+                        tell(4u * q + 2u, (on - own) / 4u + 1u);
                     }
                 }
             }
             if (x != JST_OPEN)
                 decide(q, x);
         }
-        gst[q] = static_cast<uint8_t>(x);
-        if (x == JST_OPEN)
-            raise_err(&b.state[s], ERR_INTERNAL);
+        if (x != JST_OPEN)
+            gst[q] = static_cast<uint8_t>(x);
+        else
+            leave(at, q);
     }
     __syncwarp();
     cluster_barrier(); // no CTA leaves while another may still write its states
+    if (rank == 0u && s_left != 0u)
+        vote_rows(RowVote{gst, next, b.jrec + sd.jq_off, b.jq_total, b.row_cnt + sd.row_off, b.row_cols + sd.pix_off,
+                          b.pix_depth + sd.pix_off, sd.H, sd.W});
 }
 
 // populateLabels (segmenter.cpp:640-669) and the colour image of Segmenter::image().

@@ -56,3 +56,31 @@ def test_batches_on_both_cluster_sizes(ctx, nscans):
     got = lp.process_batch(ctx, [s[0] for s in scans], pipe, [s[2] for s in scans], [s[1] for s in scans])
     for r, (x, ring, cfg) in zip(got, scans):
         assert np.array_equal(r.seg_labels, T.o_segment(x, ring, cfg))
+
+
+def stripes(H, W, kind, seed=1):
+    """Flat ground on whose returns every n-th pixel of a row, a column or a diagonal stands 0.6 m above it: nearly
+    every ground pixel is queued and hangs on its left and upper neighbours, in chains as long as the image."""
+    h, w = np.meshgrid(np.arange(H), np.arange(W), indexing="ij")
+    el, az = np.radians(2.0 - 26.8 * (h + 0.5) / H), (w + 0.5) * 2 * np.pi / W
+    seen = el < -0.03
+    r = 1.73 / np.tan(np.where(seen, -el, 1.0))
+    high = {"rows": h % 4 == 0, "columns": w % 4 == 0, "diagonals": (w + 2 * h) % 5 == 0,
+            "noise": np.random.default_rng(seed).random((H, W)) < 0.15}[kind]
+    x = np.stack([r * np.cos(az), r * np.sin(az), np.where(high, -1.13, -1.73), 0 * r], -1)[seen].astype(np.float32)
+    cfg = lp.SegmenterConfig.default(image_height=H, image_width=W)
+    return np.ascontiguousarray(x), np.ascontiguousarray(h[seen].astype(np.uint16)), cfg
+
+
+@pytest.mark.parametrize("H,W", [(24, 900), (64, 300), (64, 2048), (128, 4096), (20, 20000), (2000, 64)])
+@pytest.mark.parametrize("kind", ["rows", "columns", "diagonals", "noise"])
+def test_long_chains(ctx, H, W, kind):
+    check(ctx, *stripes(H, W, kind))
+
+
+def test_long_chains_of_many_scans(ctx):
+    scans = [stripes(16 + 5 * k, 700 + 131 * k, kind, k) for k, kind in enumerate(["rows", "columns", "diagonals", "noise"] * 3)]
+    pipe = lp.PipelineConfig.default()
+    got = lp.process_batch(ctx, [s[0] for s in scans], pipe, [s[2] for s in scans], [s[1] for s in scans])
+    for r, (x, ring, cfg) in zip(got, scans):
+        assert np.array_equal(r.seg_labels, T.o_segment(x, ring, cfg))
