@@ -50,6 +50,13 @@ __device__ __forceinline__ bool hpt_less(const HPt<T>& a, const HPt<T>& b)
     return (a.x < b.x) | ((a.x == b.x) & ((a.y < b.y) | ((a.y == b.y) & (a.key < b.key))));
 }
 
+// Members with a NaN coordinate are no candidates: hpt_less would not order them (the sorts by counting
+// need a total order), and the chain, which never pops them, would hold more vertices than the cluster members.
+__device__ __forceinline__ bool has_place(float x, float y)
+{
+    return x == x && y == y;
+}
+
 // polygonizer.cpp:45-50: counter-clockwise or collinear, evaluated in FP64 exactly as written
 __device__ __noinline__ bool ccw_or_colinear(double ax, double ay, double bx, double by, double cx, double cy)
 {
@@ -1656,7 +1663,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int comput
         const uint32_t i = (cur < 0) ? t : act[cur][t];
         const uint32_t o = mem[i];
         const float2 p = xy[i];
-        if (!inside(p.x, p.y))
+        if (!inside(p.x, p.y) && has_place(p.x, p.y))
         {
             const int pos = atomicAdd(&sm.ncand, 1);
             if (pos < kHullSmem)
@@ -1718,7 +1725,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int comput
         const int kl = sm.nhull, ku = sm.grew;
         for (int j = 1; j < ku - 1; ++j)
             H[kl - 1 + j] = H[m + 1 + j];
-        sm.nhull = (m == 0) ? -1 : kl + ku - 2;
+        sm.nhull = (m < 2) ? m : kl + ku - 2;
     }
     __syncthreads();
     const int h = sm.nhull;
@@ -2112,7 +2119,7 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
         const uint32_t ahead = min(i + 32u, n - 1u); // (on its way during the tests)
         o_next = mem[ahead];
         p_next = xy[ahead];
-        const bool keep = !inside(c.x, c.y) && i < n;
+        const bool keep = !inside(c.x, c.y) && i < n && has_place(c.x, c.y);
         const uint32_t mask = __ballot_sync(0xffffffffu, keep);
         if (keep)
         {
@@ -2187,7 +2194,7 @@ __device__ void hull_one_warp(const BatchDev& b, WarpSmem& ws, const float2* dir
             H[kl - 1 + j] = v;
         __syncwarp();
     }
-    const int h = kl + ku - 2; // (m >= 1: the extreme members stay)
+    const int h = (m < 2u) ? static_cast<int>(m) : kl + ku - 2;
     {
         bool tie = false;
         for (int j = static_cast<int>(lane); j < h; j += 32)
