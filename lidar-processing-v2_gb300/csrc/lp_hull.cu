@@ -2806,11 +2806,12 @@ __device__ uint32_t single_filter(SingleSmem& sm, const double2* pts, uint32_t n
     return nact;
 }
 
-// Sort and chain of m candidates (list: their input positions, null for all points): hull indices
-// to out, returns the hull size; *tie: a vertex has an identical candidate.
+// Sort and chain of m candidates (list: their input positions, null for all points; `placed` of them without a NaN
+// coordinate, which alone take part: has_place): hull indices to out, returns the hull size; *tie: a vertex has an
+// identical candidate.
 template <typename T>
-__device__ int single_chain(SingleSmem& sm, const double2* pts, const uint32_t* list, uint32_t m, HPt<T>* gl, int* gstack,
-                            int32_t* out, bool* tie)
+__device__ int single_chain(SingleSmem& sm, const double2* pts, const uint32_t* list, uint32_t m, uint32_t placed, HPt<T>* gl,
+                            int* gstack, int32_t* out, bool* tie)
 {
     auto run = [&](HPt<T>* C, int* H) {
         const uint32_t np2 = next_pow2(m);
@@ -2821,10 +2822,12 @@ __device__ int single_chain(SingleSmem& sm, const double2* pts, const uint32_t* 
             {
                 const uint32_t i = list ? list[t] : t;
                 const double2 p = pts[i];
-                c = HPt<T>{static_cast<T>(p.x), static_cast<T>(p.y), i};
+                if (p.x == p.x && p.y == p.y) // (the others end behind all points)
+                    c = HPt<T>{static_cast<T>(p.x), static_cast<T>(p.y), i};
             }
             C[t] = c;
         }
+        m = placed;
         __syncthreads();
         block_bitonic_sort(C, np2, [](const HPt<T>& x, const HPt<T>& y) { return hpt_less(x, y); });
         if (threadIdx.x < 64u)
@@ -2835,7 +2838,9 @@ __device__ int single_chain(SingleSmem& sm, const double2* pts, const uint32_t* 
                 (upper ? sm.grew : sm.npoly) = k;
         }
         __syncthreads();
-        const int kl = sm.npoly, h = kl + sm.grew - 2;
+        const int kl = sm.npoly;
+        // (a chain without orientations, where they overflow binary64, pops nothing: no more than out holds)
+        const int h = (m < 2u) ? static_cast<int>(m) : min(kl + sm.grew - 2, static_cast<int>(m) + 1);
         bool t = false;
         for (int j = static_cast<int>(threadIdx.x); j < h; j += static_cast<int>(blockDim.x))
         {
@@ -2870,6 +2875,18 @@ __global__ void __launch_bounds__(kSingleThreads) k_hull_single(const double2* p
     }
     exact = __syncthreads_and(exact);
     finite = __syncthreads_and(finite);
+    uint32_t placed = n;
+    if (!finite)
+    {
+        if (threadIdx.x == 0)
+            sm.nact = 0;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+            if (pts[i].x == pts[i].x && pts[i].y == pts[i].y)
+                atomicAdd(&sm.nact, 1);
+        __syncthreads();
+        placed = static_cast<uint32_t>(sm.nact);
+    }
     const size_t bytes = static_cast<size_t>(next_pow2(n)) * sizeof(HPt<double>);
     const size_t lists = bytes - 8ull * n; // the two lists of n entries start here
     uint32_t* act0 = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(scratch) + lists);
@@ -2884,9 +2901,9 @@ __global__ void __launch_bounds__(kSingleThreads) k_hull_single(const double2* p
     bool tie;
     int h;
     if (exact && finite)
-        h = single_chain(sm, pts, all ? nullptr : act0, m, reinterpret_cast<HPt<float>*>(scratch), stack, out, &tie);
+        h = single_chain(sm, pts, all ? nullptr : act0, m, m, reinterpret_cast<HPt<float>*>(scratch), stack, out, &tie);
     else
-        h = single_chain(sm, pts, all ? nullptr : act0, m, scratch, stack, out, &tie);
+        h = single_chain(sm, pts, all ? nullptr : act0, m, finite ? m : placed, scratch, stack, out, &tie);
     if (threadIdx.x == 0)
         *n_out = static_cast<uint32_t>(h);
     if (__syncthreads_or(tie))

@@ -118,3 +118,14 @@ def test_noalloc_hull_of_far_points(ctx, log2):
         xy, idx, cnt = torch.from_numpy(pts).cuda(), torch.zeros(n, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
         assert fn(xy.data_ptr(), n, idx.data_ptr(), cnt.data_ptr(), None) == lp.LP_OK
         assert np.array_equal(idx.cpu().numpy()[:int(cnt.item())], T.o_hull(pts, T.TIES_LIBSTDCXX))
+
+
+@pytest.mark.parametrize("n", [3, 64, 700])
+@pytest.mark.parametrize("value", [np.nan, np.inf, 1e200])
+def test_hull_without_orientations(ctx, n, value):
+    """NaN, infinite and overflowing coordinates: no more indices than the output holds, each of a point."""
+    pts = np.random.default_rng(n).normal(size=(n, 2)) * 5
+    for share in (0.1, 1.0):
+        bad = np.random.default_rng([n, 1]).random((n, 2)) < share
+        hull = lp.Polygonizer(ctx).convexHull(np.where(bad, value * np.sign(pts), pts))
+        assert len(hull) <= n + 1 and (hull >= 0).all() and (hull < n).all()
