@@ -1426,6 +1426,35 @@ __global__ void __launch_bounds__(256) k_hull_pre_ref(BatchDev b)
     }
 }
 
+// Local indices of a hull's h vertices (H: their candidates in C), more than shared memory takes: the members
+// [start, start + n) before each, by a CTA. A vertex per lane, every member once for all of a warp's (from
+// aligned quadruples, the same for all lanes). A warp per vertex read the members for each of them: of the 117 ms that
+// k_hull took for a cluster of 112,000 members and 2,048 vertices all but 10.
+__device__ __noinline__ void count_members(const uint32_t* members, uint32_t start, uint32_t n, const HPt<float>* C, const int* H,
+                                           int h, int32_t* out)
+{
+    const uint32_t a4 = start & 3u;
+    const uint4* mv = reinterpret_cast<const uint4*>(members + (start - a4));
+    const uint32_t nq = (n + a4 + 3u) / 4u;
+    for (int j = static_cast<int>(threadIdx.x); j - static_cast<int>(lane_id()) < h; j += kHullThreads)
+    {
+        const uint32_t key = (j < h) ? C[H[j]].key : 0u;
+        uint32_t cnt = 0;
+#pragma unroll 4
+        for (uint32_t v = 0; v < nq; ++v)
+        {
+            const uint4 o = mv[v];
+            const uint32_t i = 4u * v - a4; // (wraps below the first member: not less than n)
+            cnt += (o.x < key && i < n) ? 1u : 0u;
+            cnt += (o.y < key && i + 1u < n) ? 1u : 0u;
+            cnt += (o.z < key && i + 2u < n) ? 1u : 0u;
+            cnt += (o.w < key && i + 3u < n) ? 1u : 0u;
+        }
+        if (j < h)
+            out[j] = static_cast<int32_t>(cnt);
+    }
+}
+
 // Cluster g of scan s: z range, hull (local indices into hull_tmp at cl_start), boxes.
 __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int compute_obb)
 {
@@ -1863,21 +1892,7 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int comput
             atomicAdd(&sm.diff[cb], cc);
     }
     else
-    {
-        for (int j = static_cast<int>(warp); j < h; j += kHullThreads / 32)
-        {
-            const uint32_t key = C[H[j]].key;
-            uint32_t cnt = 0;
-            for (uint32_t base = 0; base < n; base += 32)
-            {
-                const uint32_t i = base + lane;
-                const bool lt = (i < n) && (mem[i] < key);
-                cnt += __popc(__ballot_sync(0xffffffffu, lt));
-            }
-            if (lane == 0)
-                hull_dst[j] = static_cast<int32_t>(cnt);
-        }
-    }
+        count_members(b.members, start, n, C, H, h, hull_dst);
     __syncthreads();
     if (fast)
     {

@@ -63,3 +63,23 @@ def test_cluster_hull_paths(ctx, kind):
     for k in range(want.n_clusters):
         assert T.boxes_identical(got.obb_calipers[k], want.obb_calipers[k]), k
         assert T.pca_boxes_equal(got.obb_pca[k], want.obb_pca[k]), k
+
+
+@pytest.mark.parametrize("rings,columns", [(3, 1400), (7, 1301), (6, 4096)])
+def test_hull_of_more_vertices_than_shared_memory(ctx, rings, columns):
+    """A wall all around the sensor: one cluster, most of its outermost points hull vertices."""
+    rng = np.random.default_rng(columns)
+    ring, col = np.meshgrid(np.arange(rings), np.arange(columns), indexing="ij")
+    r, az = 20 - 0.02 * ring, (col + 0.5) * 2 * np.pi / columns
+    x = np.stack([r * np.cos(az), r * np.sin(az), 0.5 - 0.3 * ring, 0 * r], -1).reshape(-1, 4).astype(np.float32)
+    order = rng.permutation(len(x))
+    x, ring = np.ascontiguousarray(x[order]), np.ascontiguousarray(ring.ravel()[order].astype(np.uint16))
+    cfg = lp.SegmenterConfig.default(image_height=rings, image_width=columns)
+    pipe = lp.PipelineConfig.default()
+    want = T.o_process(x, ring, cfg, pipe)
+    assert want.n_clusters == 1 and len(want.hull_indices) > 1024
+    got = lp.process_batch(ctx, [x], pipe, [cfg], [ring])[0]
+    assert np.array_equal(got.cluster_labels, want.cluster_labels)
+    assert np.array_equal(got.hull_indices, want.hull_indices)
+    assert T.boxes_identical(got.obb_calipers[0], want.obb_calipers[0])
+    assert T.pca_boxes_equal(got.obb_pca[0], want.obb_pca[0])
