@@ -901,7 +901,13 @@ lp_status direct_finish(lp_context* ctx, lp_batch& B, lp_scan_output* outs)
 
 lp_status run_direct(lp_context* ctx, lp_batch& B, lp_scan_output* outs)
 {
-    LP_TRY(direct_launch(ctx, B, outs));
+    const lp_status st = direct_launch(ctx, B, outs);
+    if (st != LP_OK)
+    {
+        // what was issued before the failure still reads the staging and the caller's buffers
+        cudaStreamSynchronize(B.stream ? B.stream : ctx->stream);
+        return st;
+    }
     return direct_finish(ctx, B, outs);
 }
 
@@ -938,8 +944,10 @@ lp_status run_direct_split(lp_context* ctx, const lp_pipeline_config* cfg, const
             in.push_back(scans[i]);
             sub[k].push_back(outs[i]);
         }
-        LP_CUDA(ctx, cudaStreamWaitEvent(P.stream, ctx->fork, 0));
-        worst = fill_pipeline(ctx, P, cfg, in.data(), static_cast<uint32_t>(in.size()));
+        // (an error here or below leaves through the wait after the loop: earlier parts are running)
+        const cudaError_t e = cudaStreamWaitEvent(P.stream, ctx->fork, 0);
+        worst = e == cudaSuccess ? fill_pipeline(ctx, P, cfg, in.data(), static_cast<uint32_t>(in.size()))
+                                 : cuda_fail(ctx, e, "cudaStreamWaitEvent");
         if (worst == LP_OK)
             worst = direct_launch(ctx, P, sub[k].data());
         if (worst == LP_OK)
