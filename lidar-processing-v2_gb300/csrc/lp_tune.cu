@@ -302,8 +302,8 @@ lp_status lp_autotune(lp_context* ctx, const lp_pipeline_config* cfg, const lp_s
     if (st0 != LP_OK)
         return st0;
     const float start_ms = cur_ms;
-    // coordinate descent: each field in turn over its candidates, keeping a change only when it
-    // is at least 1 % faster than the current choice
+    // coordinate descent: each field that a launch reads (not cell_ctas_per_sm) in turn over its
+    // candidates, keeping a change only when it is at least 1 % faster than the current choice
     struct Field
     {
         uint32_t lp_tuning::*member;
@@ -314,7 +314,6 @@ lp_status lp_autotune(lp_context* ctx, const lp_pipeline_config* cfg, const lp_s
         {&lp_tuning::balance_parts, {0u, 1u}},
         {&lp_tuning::hull_cta_min, {128u, 256u, 512u}},
         {&lp_tuning::hull_ctas_per_sm, {1u, 2u, 3u, 4u}},
-        {&lp_tuning::cell_ctas_per_sm, {4u, 8u, 12u}},
         {&lp_tuning::jcp_ctas_per_sm, {4u, 8u, 12u}},
     };
     for (const Field& f : fields)

@@ -104,3 +104,16 @@ def test_autotune(ctx):
     assert t_used.as_dict() == best.as_dict()
     for i, (g, w) in enumerate(zip(got, want)):
         compare_scan(g, w, f"tuned scan {i}")
+
+
+def test_autotune_leaves_unread_fields(ctx):
+    """cell_ctas_per_sm stays in tables and files, but no launch reads it: no candidate differs in it, so timing noise
+    cannot store a choice of it."""
+    data = [T.synth_scan(5, i) for i in range(4)]
+    start = lp.Tuning.default(cell_ctas_per_sm=3)
+    tab = lp.TuningTable()
+    xs, rings, cfgs = [d[0] for d in data], [d[1] for d in data], [d[2] for d in data]
+    tab.set(lp.tuning_key(xs, cfgs), start, 1.0)
+    best, rep = lp.autotune(ctx, xs, lp.PipelineConfig.default(), cfgs, rings, iters=2, table=tab)
+    assert best.cell_ctas_per_sm == 3
+    assert {c["cell_ctas_per_sm"] for c, _ in rep["candidates"]} == {3}
