@@ -1623,9 +1623,9 @@ constexpr uint32_t kResolveStates = 24u * 1024u; // queued pixels whose states f
 constexpr int kResolveWide = 7;           // scans of a launch up to which a scan takes 8 CTAs
 // A round takes as long as it has open pixels, and where they hang on one another in chains as long as the image it
 // decides little more than one pixel of each. So rounds (2 us for 4,096 pixels) and watching end where they
-// have cost about half of what vote_rows would (2.5 us for every row and 512 pixels). Stripes over a 64 x 2048 and a
-// 128 x 4096 image: 1.2 and 4.1 ms, against 1,276 and 16,000 without an end. The workloads' scans stay below
-// it; with half of this budget one of 64 did not (107 -> 146 us).
+// have cost about what vote_rows would (2 us for every row and 512 pixels). Stripes over a 64 x 2048 and a 128 x 4096
+// image: 1.1 and 4.3 ms, against 1,276 and 16,000 without an end. The workloads' scans stay below it; with half of
+// this budget one scan each of two 64-scan batches did not (107 -> 146 us; 1.79 -> 1.80 ms a batch).
 constexpr uint32_t kSpinsLocal = 32, kSpinsGlobal = 4; // polls of a pixel's neighbours for each step of vote_rows
 
 __device__ __forceinline__ void cluster_barrier()
@@ -1755,13 +1755,24 @@ __device__ __noinline__ void vote_rows(const RowVote v)
                             before |= 1u << k;
                     }
                 }
+                // the sums of slots 0-9 once, the others for every state (vote_bounds for a known state, its terms in the same order)
+                auto term = [&](uint32_t k, uint32_t g, uint32_t o) {
+                    return make_float2(((g >> k) & 1u) ? wn[k] : 0.0F, ((o >> k) & 1u) ? wn[k] : 0.0F);
+                };
+                float2 head = make_float2(0.0F, 0.0F); // (ground, obstacle)
+#pragma unroll
+                for (uint32_t k = 0; k < 10; ++k)
+                    head = __fadd2_rn(head, term(k, m0, m1));
                 map = 0u;
-#pragma unroll 1
+#pragma unroll
                 for (uint32_t u = 0; u < 4; ++u)
                 {
                     const uint32_t o = ((u & 1u) ? last : 0u) | ((u & 2u) ? before : 0u); // these on obstacle
-                    const uint32_t x = vote_bounds(wn, m0 | ((last | before) & ~o), m1 | o);
-                    map |= (((u & 1u) << 1) | (x == V_O ? 1u : 0u)) << (2u * u);
+                    float2 sum = head;
+#pragma unroll
+                    for (uint32_t k = 10; k < 24; ++k)
+                        sum = __fadd2_rn(sum, term(k, m0 | ((last | before) & ~o), m1 | o));
+                    map |= (((u & 1u) << 1) | (sum.y > sum.x ? 1u : 0u)) << (2u * u);
                 }
             }
             uint32_t incl = map;
@@ -1902,7 +1913,7 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kResolveThreads)
     uint32_t *cur = nullptr, *next = b.jlist + sd.jq_off, *other = b.jlist + b.jq_total + sd.jq_off; // null: all positions
     const uint32_t steps = static_cast<uint32_t>(sd.H) + nq / kResolveThreads; // of vote_rows
     uint32_t spent = 0u;
-    for (uint32_t round = 0; n > kAll && 2u * spent <= steps; ++round)
+    for (uint32_t round = 0; n > kAll && spent <= steps; ++round)
     {
         spent += 1u + n / (8u * kResolveThreads);
         const uint32_t cnt = n_addr[round & 1u];
