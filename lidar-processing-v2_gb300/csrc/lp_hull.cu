@@ -1891,8 +1891,9 @@ __device__ void hull_one(const BatchDev& b, HullSmem& sm, uint32_t g, int comput
         if (cc > 0 && cb < h)
             atomicAdd(&sm.diff[cb], cc);
     }
-    else
-        count_members(b.members, start, n, C, H, h, hull_dst);
+    else // (candidates and stack lie in global memory)
+        count_members(b.members, start, n, reinterpret_cast<const HPt<float>*>(b.hs_cand) + 2ull * start,
+                      b.hs_stack + 2ull * start + 2ull * b.cl_rank[g], h, hull_dst);
     __syncthreads();
     if (fast)
     {
