@@ -126,7 +126,6 @@ lp_status plan(lp_context* ctx, lp_batch& B)
     BatchHost& hb = B.hb;
     hb = BatchHost{};
     hb.nscan = static_cast<int>(R.scans.size());
-    hb.any_noise = (R.stages & ST_NOISE) != 0;
     uint64_t pt = 0, pix = 0, row = 0, tile = 0, slice = 0, cell = 0, nearc = 0, hash = 0, cl = 0, queue = 0;
     const bool seg = (R.stages & ST_SEG) != 0;
     for (const ScanIn& in : R.scans)

@@ -75,7 +75,6 @@ struct ScanState
 {
     uint32_t err;
     uint32_t n_pts;     // points entering segmentation (after noise removal)
-    uint32_t reserved_dror[2];
     // RANSAC (segmenter.cpp:321-479)
     uint32_t n_cand, cand_off;
     int32_t ransac_ok;
@@ -88,13 +87,12 @@ struct ScanState
     uint32_t n_vox;
     uint32_t n_comp; // of the batch's first scan: voxels listed (all scans)
     uint32_t n_clusters;
-    uint32_t cl_base; // clusters of earlier scans (work-queue numbering)
-    uint32_t n_hull;
     // jump convolution: queued pixels, those the weights pass left open, and of these the ones whose
     // window leaves the image
     uint32_t n_queue, n_open, n_border;
-    uint32_t pad[1];
+    uint32_t pad[7]; // to a line of 128 bytes: scans' counters do not share one
 };
+static_assert(sizeof(ScanState) == 128);
 
 // First statement of every kernel. Launches of a run carry the programmatic-serialisation attribute
 // (Launcher), so a kernel's CTAs may be set up while the one before it drains: it waits here until that
@@ -149,11 +147,5 @@ __host__ __device__ constexpr uint32_t scan_words_max(uint32_t n)
 {
     return scan_words(n) > scan_words(1u << 20) ? scan_words(n) : scan_words(n < (1u << 20) ? n : 1u << 20);
 }
-
-// Kernel launch bookkeeping (counted by the host wrapper for instrumentation).
-struct LaunchCounter
-{
-    uint64_t n = 0;
-};
 
 } // namespace lpg

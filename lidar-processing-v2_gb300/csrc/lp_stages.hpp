@@ -117,16 +117,6 @@ struct Launcher
         note();
     }
     template <typename K, typename... Args>
-    void launch2d(const char* name, K kernel, dim3 grid, uint32_t block, Args... args)
-    {
-        if (grid.x == 0 || grid.y == 0 || err != cudaSuccess)
-            return;
-        begin(name);
-        issue(kernel, grid, block, 0, args...);
-        end();
-        note();
-    }
-    template <typename K, typename... Args>
     void launch_smem(const char* name, K kernel, uint32_t grid, uint32_t block, size_t smem, Args... args)
     {
         if (grid == 0 || err != cudaSuccess)
@@ -177,7 +167,6 @@ struct Launcher
 };
 
 #define LP_LAUNCH(L, k, grid, block, ...) (L).launch(#k, k, grid, block, __VA_ARGS__)
-#define LP_LAUNCH2D(L, k, grid, block, ...) (L).launch2d(#k, k, grid, block, __VA_ARGS__)
 #define LP_LAUNCH_SMEM(L, k, grid, block, smem, ...) (L).launch_smem(#k, k, grid, block, smem, __VA_ARGS__)
 
 // One-time kernel attributes (dynamic shared memory opt-in); called when a context is created.
@@ -238,7 +227,6 @@ struct BatchHost
 {
     int nscan = 0;
     bool any_compute_ring = false;
-    bool any_noise = false;
     bool packed_key = true; // every scan's projection keys fit one word (k_label_depth)
     uint32_t ntiles = 0;
     uint32_t nslices = 0;
