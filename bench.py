@@ -382,7 +382,12 @@ def run_dror(args):
 # jump convolution, label write-back); prefix scans count with the stage of the kernel before them.
 SEG_KERNELS = {"k_quadrant", "k_ring_count", "k_ring_apply", "k_bin", "k_scatter", "k_recm", "k_ransac_draw",
                "k_ransac_inliers", "k_label_depth", "k_project_key", "k_pixel", "k_dilate_rows", "k_jcp_weights",
-               "k_jcp_resolve", "k_jcp_rows", "k_populate"}
+               "k_jcp_resolve", "k_jcp_rows", "k_populate"}  # (k_jcp_rows: in earlier libraries' profiles)
+
+# Kernels whose algorithmic bytes do not follow from what a batch returns (queued pixels, occupied voxels,
+# hypotheses): the roofline takes the longest of the others.
+UNCOUNTED = {"k_prepare", "k_ransac_draw", "k_ransac_inliers", "k_jcp_weights", "k_jcp_resolve", "k_vox_insert",
+             "k_uf_hook", "k_uf_flatten", "k_hull_worklist", "k_hull_pre_ext", "k_hull_pre_ref", "k_hull_finish"}
 
 
 def stage_ms(prof, kernels):
@@ -476,12 +481,17 @@ def main():
     batch = lp.PreparedBatch(ctx, xs, pipe, cfgs, rings)
     batch_tuning = batch.tuning.as_dict()
 
-    # per-kernel profile of one un-captured execution (dominant kernel for the roofline)
+    # launches of one un-captured execution (a graph replay makes the same), counted by the library; without its
+    # count, from the profile
+    launched = getattr(ctx, "launches", None)
     batch.execute()
     batch.synchronize()
+    kernels_per_step = ctx.launches - launched if launched is not None else 0
+    # per-kernel profile (dominant kernel for the roofline)
     prof, agg = kernel_profile(batch)
-    kernels_per_step = sum(1 for n, _ in prof if n != "k_scan") + 3 * sum(1 for n, _ in prof if n == "k_scan")
-    top_name = max(agg.items(), key=lambda kv: kv[1][1])[0]
+    if not kernels_per_step:
+        kernels_per_step = sum(1 for n, _ in prof if n != "k_scan") + 3 * sum(1 for n, _ in prof if n == "k_scan")
+    top_name = max(((n, a) for n, a in agg.items() if n not in UNCOUNTED), key=lambda kv: kv[1][1])[0]
     res = batch.download()
     n_obs = sum(r.n_obstacles for r in res)
     n_clusters = sum(r.n_clusters for r in res)
@@ -511,8 +521,11 @@ def main():
     top_launches = agg2[top_name][0]
     top_ms = agg2[top_name][1] / top_launches
     alg = {
-        "k_hull": 8 * n_clustered + 4 * n_hull + 64 * n_clusters,
-        "k_jcp_rows": 20 * npts,
+        "k_bin": 28 * npts,  # point and ring in; cell, slot and pixel out
+        "k_recm": 4 * npts,  # the heights
+        "k_label_depth": 28 * npts,  # point, cell, pixel, key
+        "k_hull": 8 * n_clustered + 20 * n_hull,  # members; local indices and vertices out
+        "k_hull_boxes": 32 * n_hull + 160 * n_clusters,  # vertices for either box
         "k_obs_gather": 20 * n_obs,
     }
     alg_bytes = alg.get(top_name, 20 * npts) / top_launches
