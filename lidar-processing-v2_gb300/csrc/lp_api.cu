@@ -351,7 +351,6 @@ size_t carve(lp_batch& B, char* base)
         put(b.jq, b.jq_total + 1);
         put(b.jw, static_cast<size_t>(b.nrows) * 3u * kJwStride); // the last three queued pixels of each row
         put(b.jst, static_cast<size_t>(b.jq_total) + 16);
-        put(b.jrec, static_cast<size_t>(b.jq_total) * kJrecFields + 1);
         put(b.jlist, 2ull * b.jq_total + 1);
         put(b.jborder, b.jq_total + 1);
         if (R.stages & ST_IMAGE)
@@ -388,12 +387,6 @@ size_t carve(lp_batch& B, char* base)
         put(b.cl_zmax, b.ncl);
         put(b.obb_c, b.ncl);
         put(b.obb_p, b.ncl);
-        uint8_t* cand;
-        put(cand, static_cast<size_t>(2) * N * 12 + 64);
-        b.hs_cand = cand;
-        put(b.hs_stack, static_cast<size_t>(2) * N + 2ull * b.ncl + 8);
-        put(b.hs_pts, static_cast<size_t>(N) + 8);
-        put(b.hs_pairs, static_cast<size_t>(4) * N + 16ull * b.ncl + 16);
         put(b.queue, 10);
         put(b.tie_list, b.ncl + 1);
         put(b.pre_items, N / 4096u + b.ncl + 1);
@@ -401,7 +394,25 @@ size_t carve(lp_batch& B, char* base)
         put(b.pre_pk, 16ull * b.ncl + 16);
         put(b.pre_nact, b.ncl + 1);
     }
-    return c.off + 4096;
+    // the vote's records and the hulls' scratch share their place: the vote has ended when the hulls begin
+    const size_t shared = c.off;
+    size_t end = shared;
+    if (seg)
+    {
+        put(b.jrec, static_cast<size_t>(b.jq_total) * kJrecFields + 1);
+        end = c.off;
+        c.off = shared;
+    }
+    if (hull)
+    {
+        uint8_t* cand;
+        put(cand, static_cast<size_t>(2) * N * 12 + 64);
+        b.hs_cand = cand;
+        put(b.hs_stack, static_cast<size_t>(2) * N + 2ull * b.ncl + 8);
+        put(b.hs_pts, static_cast<size_t>(N) + 8);
+        put(b.hs_pairs, static_cast<size_t>(4) * N + 16ull * b.ncl + 16);
+    }
+    return std::max(end, c.off) + 4096;
 }
 
 lp_status build(lp_context* ctx, lp_batch& B)
