@@ -2650,7 +2650,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_hull_finish(BatchDev b)
 // What bounds them: nearly every point of a cluster lies inside its hull, and sorting all of them
 // (24-byte records, about log2(n)^2 / 2 passes) and walking them with one thread's FP64 orientation
 // tests took most of the 62 ms that twelve polygons of 3 to 20,000 points needed for hull and both
-// boxes (now 1.9 ms, 54 us a call). The points proven inside a polygon of input points
+// boxes (now 1.9 ms, 52 us a call). The points proven inside a polygon of input points
 // are dropped first (Quickhull rounds as in hull_one, coordinates as floats), so the sort and the
 // chain see a few dozen to a few hundred; 1,024 threads because the rounds stream over all points.
 // Points whose coordinates are binary32 values (the processor's are) also take the FP32-screened
