@@ -380,7 +380,7 @@ def run_dror(args):
 
 # Kernels of the segmentation stage (ring partition, polar grid, RECM, RANSAC, projection, dilation,
 # jump convolution, label write-back); prefix scans count with the stage of the kernel before them.
-SEG_KERNELS = {"k_quadrant", "k_ring_count", "k_ring_apply", "k_bin", "k_scatter", "k_recm", "k_ransac_draw",
+SEG_KERNELS = {"k_quadrant", "k_ring_count", "k_ring_apply", "k_bin", "k_scatter", "k_recm", "k_recm_sparse", "k_ransac_draw",
                "k_ransac_inliers", "k_label_depth", "k_project_key", "k_pixel", "k_dilate_rows", "k_jcp_weights",
                "k_jcp_resolve", "k_jcp_rows", "k_populate"}  # (k_jcp_rows: in earlier libraries' profiles)
 
