@@ -229,7 +229,8 @@ lp_status lp_cluster(lp_context* ctx, const float* xyz, uint32_t stride, uint32_
                      const lp_clusterer_config* cfg, int32_t* labels_out);
 
 /* Convex hull (Andrew's monotone chain). xy: n x 2 doubles. indices_out: capacity >= n + 1;
- * *n_out receives the hull size. Counter-clockwise, starting at the lexicographic minimum. */
+ * *n_out receives the hull size. Counter-clockwise, starting at the lexicographic minimum. Points with
+ * a NaN coordinate take no part. */
 lp_status lp_convex_hull(lp_context* ctx, const double* xy, uint32_t n, int32_t* indices_out,
                          uint32_t* n_out);
 
